@@ -225,7 +225,8 @@ def nblist_build_batch(cells, binum, coords, rcut, umax, is_cart=True, pbc=(True
     B, npad = int(coords.shape[0]), int(coords.shape[1])
     dev = coords.device
     npdt = np.float64 if suf == "f64" else np.float32
-    dcells = torch.from_numpy(np.ascontiguousarray(np.asarray(cells, dtype=npdt).reshape(B, 9))).to(dev)
+    # (asynchronous: the driver takes pageable host memory into its own buffer before the call returns)
+    dcells = torch.from_numpy(np.ascontiguousarray(np.asarray(cells, dtype=npdt).reshape(B, 9))).to(dev, non_blocking=True)
     hpbc = np.ascontiguousarray([1 if p else 0 for p in pbc], np.int32)
     binum = binum.to(torch.int32).contiguous()
     out = dict(binum=binum, bilist=torch.empty(B, npad, dtype=torch.int32, device=dev),

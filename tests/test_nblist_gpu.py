@@ -247,3 +247,46 @@ def test_lanes_as_centres_kernel_on_small_cases(checkers, dt, monkeypatch):
     nn, fn, rc, st = capi.NeighborBuilder().build(c1, dpos, 6.0, 8)
     st = st.cpu().numpy()
     assert st[1] == 1 and st[0] == ref[0].max() and nn.max().item() == 8
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.float32])
+@pytest.mark.parametrize("n,density,umax,pbc", [
+    (1, 0.03, 64, (1, 1, 1)),
+    (37, 0.03, 100, (1, 1, 1)),          # cell narrower than the cutoff: candidates come in pieces
+    (2048, 0.03, 64, (1, 1, 1)),         # last size that one block bins
+    (2049, 0.03, 63, (1, 1, 1)),         # first size that is binned by several launches; rows without 16-byte alignment
+    (2048, 0.03, 64, (0, 1, 0)),
+    (2500, 0.03, 64, (0, 0, 0)),         # extents looked up by a cluster of blocks
+    (8100, 0.005, 32, (1, 1, 1)),        # sparse bins: two warps per bin
+    (8100, 0.0015, 32, (1, 1, 1)),       # ... one warp per bin
+    (8100, 0.14, 256, (1, 1, 1)),        # crowded bins: more candidates than the table holds
+])
+def test_build_at_the_edges_of_its_forms(checkers, dt, n, density, umax, pbc):
+    chk = _chk(checkers)
+    rng = np.random.default_rng(n)
+    L = (n / density) ** (1.0 / 3.0)
+    cell = (np.eye(3) * L + np.array([[0, 0, 0], [0.1, 0, 0], [0.05, -0.1, 0]]) * L).astype(dt)
+    pos = (rng.random((n, 3)) @ cell.astype(np.float64) + rng.normal(0, 0.3, (n, 3))).astype(dt)
+    types = np.zeros(n, np.int32)
+    rcut = 5.0 if density < 0.1 else 4.0
+    a = _gpu(cell, types, pos, rcut, umax, pbc=pbc)
+    b = chk.nblist(cell, types, pos, rcut, umax, pbc=pbc)
+    util.assert_nblist_equal(a, b[:3])
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.float32])
+@pytest.mark.parametrize("sizes,umax", [((600, 512, 1), 64), ((17, 16, 15), 66)])
+def test_batched_build_tiles_and_chunks(checkers, dt, sizes, umax):
+    """Structures longer than one tile of the batched build, exactly one tile, and sizes around its chunk of centres."""
+    chk = _chk(checkers)
+    rng = np.random.default_rng(4)
+    B, npad = len(sizes), max(sizes)
+    cells = np.stack([np.eye(3) * 3.0 * max(2.0, n ** (1.0 / 3.0)) for n in sizes]).astype(dt)
+    coords = np.zeros((B, npad, 3), dt)
+    for b, n in enumerate(sizes):
+        coords[b, :n] = rng.random((n, 3)) * cells[b, 0, 0]
+    out = capi.nblist_build_batch(cells, torch.tensor(sizes, dtype=torch.int32).cuda(), torch.from_numpy(coords).cuda(), 4.0, umax)
+    for b, n in enumerate(sizes):
+        nn, fn, rc, ty, mx = chk.nblist(cells[b], np.zeros(n, np.int32), coords[b, :n], 4.0, umax)
+        util.assert_nblist_equal((out["bnumneigh"][b, :n].cpu().numpy(), out["bfirstneigh"][b, :n].cpu().numpy(),
+                                  out["brcs"][b, :n].cpu().numpy()), (nn, fn, rc))
