@@ -1,26 +1,25 @@
 // NEP energy / force / virial kernel specialised for models with at most NMAX radial and NMAX
 // angular functions (NMAX = 4 covers the reference's defaults, ai2pot/models/nep/nep.py:36-40).
-// Included by nep_kernels.cu after the shared helpers (NepArgs, nep_radial, NEP_FOR_EACH_LM).
+// Included by nep_kernels.cu after the shared helpers (NepArgs, NEP_FOR_EACH_LM).
 //
-// Same mapping as the general kernel (eight lanes per centre atom, lanes = neighbours) and the
-// same math (nep.h:320-529), with the per-atom instruction count cut about in half:
-//   * the coefficient table [ti][tj][2 NMAX][CSP] is zero-padded into shared memory by the block
-//     itself (no separate padding launch) and read with 16-byte loads;
-//   * radial pass: q_n accumulate in registers over the neighbour chunks, one group reduction at
-//     the end; the contracted derivatives g'_n(r_j) are kept per neighbour in shared memory, so
-//     the radial force pass does not rebuild the basis;
-//   * angular sums S[mu][lm] = sum_j g_mu(j) B_lm(j): the lanes stage g and B_lm of their
-//     neighbour in shared memory and lane s accumulates the 3 NMAX sums lm = 3s..3s+2 for every
-//     mu (a small matrix product) instead of 3 NMAX eight-lane transpose-reductions;
-//   * angular force pass: the harmonic polynomials and their gradients are consumed one lm at a
-//     time against the adjoints of all mu (4 NMAX accumulators), never held as 96 registers;
-//   * the network weights of all types sit in shared memory as zero-padded rows (16-byte loads,
-//     compile-time trip counts);
-//   * energy and virial accumulate per lane over all atoms a group visits and are reduced once
-//     per block at the end of the kernel (or when the structure index changes), so the loop over
-//     atoms has no block-wide barrier;
-//   * structures' atom offsets are read from the workspace only for batches of more than one
-//     structure.
+// Same math as the general kernel (nep.h:320-529). A warp evaluates 32 / G atoms, G lanes each, and all of its lanes run the
+// same trip counts: with loops per group (8 lanes, own neighbour count) the four groups of a warp drift apart and every phase
+// is issued up to four times. What bounds it is instruction issue, so every phase is written for few instructions:
+//   * set-up: nep_prep_kernel lays the model out once per call (padded rows, signs and constants folded in) and zeroes the
+//     outputs; a block takes the table with a handful of 16-byte copies;
+//   * radial pass, lanes = neighbours of the group's atom: Chebyshev sums of all functions and their derivatives in packed
+//     pairs, cutoff from two short polynomials; g'_n(r_j) / r_j are kept per neighbour in shared memory;
+//   * angular pass, lanes = angular neighbours of all atoms of the warp, back to back: only a fifth of the neighbours are
+//     inside the angular cutoff (6.5 of 29, or 2.2 of 17), so lanes that belong to one atom would mostly idle. The harmonics
+//     of a neighbour go through shared memory to the lanes that own its atom's sums S[mu][lm];
+//   * network: lanes = neurons, then lanes = descriptors;
+//   * angular forces, lanes as in the angular pass (the neighbour's functions are still in registers): the adjoints are
+//     first contracted over the radial functions, sum_mu g_mu e_{mu,lm} and sum_mu g'_mu e_{mu,lm}, which leaves one
+//     polynomial and one gradient per neighbour instead of NMAX. The radial force of the neighbour joins here, so every
+//     neighbour receives one set of atomics;
+//   * radial forces of the other neighbours from the cached derivatives.
+// G: 32 lanes per atom when there are few atoms (the chip is filled by atoms x G threads), 8 for many.
+// Measured (fp32, whole call, 29 / 6.5 neighbours): see launch_nep_fast.
 #pragma once
 
 namespace ai2b {
@@ -57,186 +56,307 @@ __device__ __forceinline__ void store_vec(T *__restrict__ p, const T (&v)[N])
     }
 }
 
+// Two values that are worked on together: one packed register pair and one instruction in single precision.
+template <typename T> struct Pk { T a, b; };
+template <> struct Pk<float> { unsigned long long v; };
+__device__ __forceinline__ Pk<float> pk(float a, float b) { Pk<float> r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ Pk<double> pk(double a, double b) { return {a, b}; }
+__device__ __forceinline__ float pk_lo(Pk<float> p) { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v)); return a; }
+__device__ __forceinline__ float pk_hi(Pk<float> p) { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v)); return b; }
+__device__ __forceinline__ double pk_lo(Pk<double> p) { return p.a; }
+__device__ __forceinline__ double pk_hi(Pk<double> p) { return p.b; }
+__device__ __forceinline__ Pk<float> pk_fma(Pk<float> a, Pk<float> b, Pk<float> c)
+{
+    Pk<float> r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ Pk<double> pk_fma(Pk<double> a, Pk<double> b, Pk<double> c) { return {fma(a.a, b.a, c.a), fma(a.b, b.b, c.b)}; }
+__device__ __forceinline__ Pk<float> pk_mul(Pk<float> a, Pk<float> b)
+{
+    Pk<float> r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ Pk<double> pk_mul(Pk<double> a, Pk<double> b) { return {a.a * b.a, a.b * b.b}; }
+template <int N>
+__device__ __forceinline__ void load_pk(const float *p, Pk<float> (&v)[N])
+{
+    static_assert(N % 2 == 0, "16-byte loads");
+#pragma unroll
+    for (int i = 0; i < N / 2; i++) {
+        const ulonglong2 t = reinterpret_cast<const ulonglong2 *>(p)[i];
+        v[2 * i].v = t.x; v[2 * i + 1].v = t.y;
+    }
+}
+template <int N>
+__device__ __forceinline__ void load_pk(const double *p, Pk<double> (&v)[N])
+{
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const double2 t = reinterpret_cast<const double2 *>(p)[i];
+        v[i].a = t.x; v[i].b = t.y;
+    }
+}
+
 // padded descriptor count: rows of the network's first layer are 16-byte aligned and an odd
 // number of 16-byte chunks long (conflict-free when eight lanes read eight rows)
 template <int NMAX>
 struct NepFastDims {
     static constexpr int ND = 5 * NMAX;                                   // >= n_r + n_a * l_max
     static constexpr int NDP = ((ND / 4) & 1) ? ND : ND + 4;
+    static constexpr int CS = 8;                                          // Chebyshev rows
+    static constexpr int TROW = 2 * NMAX * CS + 4;                        // one type pair; rows of different pairs start in different banks
+    static constexpr int RS = NMAX + NEP_NLM + (NMAX == 8 ? 4 : 0);       // staging row: g[NMAX] | B_lm[24], conflict-free 16-byte stores
+    static constexpr int ESR = NMAX * NEP_NLM + 4;                        // adjoints of an atom's sums, [mu][24]
 };
 __host__ __device__ inline int nep_r4(int n) { return (n + 3) & ~3; }
 __host__ __device__ inline int nep_r32(int n) { return (n + 31) & ~31; }   // neurons per type, padded
-// shared-memory elements (of T) per atom slot of the specialised kernel
+
+// The model as the kernel reads it (elements of T): Chebyshev rows [ti][tj][k][radial | angular], then (unless descriptors
+// only) first-layer rows [type][neuron][NDP], biases, second-layer weights, 1 / q_scaler
 template <int NMAX>
-__host__ __device__ inline int nep_fast_atom_elems(int nneu, int umax, bool cache)
+struct NepTab {
+    int w0, b0, w1, iqs, total;
+    __host__ __device__ NepTab(int ntypes, int nneu, bool net)
+    {
+        using D = NepFastDims<NMAX>;
+        const int nrow = ntypes * nep_r32(nneu);
+        w0 = nep_r4(ntypes * ntypes * D::TROW);
+        b0 = w0 + (net ? nrow * D::NDP : 0);
+        w1 = b0 + (net ? nrow : 0);
+        iqs = w1 + (net ? nrow : 0);
+        total = iqs + (net ? nep_r4(D::NDP) : 0);
+    }
+};
+
+// One launch in front of the kernel: the table, the structures' atom offsets, zeroed outputs.
+// Row 0 of a function holds 2 c_0 + sum_k c_k (the constant part of sum c_k (T_k + 1)); row k holds s_k c_k with the signs
+// s = + + - - + + - -, which turn the recurrences T_k+1 = 2 x T_k - T_k-1 and T'_k+1 = 2 T_k + 2 x T'_k - T'_k-1 into sums.
+template <typename T, int NMAX>
+__global__ void nep_prep_kernel(const NepArgs<T> A, const T *__restrict__ coeffs, T *__restrict__ tab, int *__restrict__ prefix, int net, int tab_blocks,
+                                T *__restrict__ z0, size_t n0, T *__restrict__ z1, size_t n1, T *__restrict__ z2, size_t n2)
 {
-    const int sea = 2 * NEP_NLM * NMAX + nep_r32(nneu);       // S, ES, act ...
-    const int stage = NEP_GROUP * (NMAX + NEP_NLM);           // ... share their space with the staging rows
-    return 2 * NepFastDims<NMAX>::NDP + (sea > stage ? sea : stage) + (cache ? umax * NMAX : 0);
-}
-// elements (of T) of the block-wide tables: coefficients, then (unless descriptors only) W0, b0, w1
-template <int NMAX, int CSP>
-__host__ __device__ inline int nep_fast_table_elems(int ntypes, int nneu, bool net)
-{
-    int n = nep_r4(ntypes * ntypes * 2 * NMAX * CSP);
-    if (net) n += ntypes * nep_r32(nneu) * (NepFastDims<NMAX>::NDP + 2);
-    return n;
+    using D = NepFastDims<NMAX>;
+    chain_release();
+    chain_wait();
+    if ((int)blockIdx.x < tab_blocks) {
+        const NepTab<NMAX> L(A.ntypes, A.nneu, net != 0);
+        const int NP = nep_r32(A.nneu), nfun = A.n_r + A.n_a;
+        if (blockIdx.x == 0 && A.B > 1 && threadIdx.x < 32) {      // exclusive sum of the structures' sizes
+            int carry = 0;
+            for (int b0 = 0; b0 < A.B; b0 += 32) {
+                const int b = b0 + threadIdx.x;
+                int inc = b < A.B ? A.binum[b] : 0;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(FULL_MASK, inc, o); if ((int)threadIdx.x >= o) inc += v; }
+                if (b < A.B) prefix[b + 1] = carry + inc;
+                carry += __shfl_sync(FULL_MASK, inc, 31);
+            }
+            if (threadIdx.x == 0) prefix[0] = 0;
+        }
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < L.total; i += tab_blocks * blockDim.x) {
+            T v = T(0);
+            if (i < L.w0) {
+                const int pair = i / D::TROW, o = i % D::TROW, k = o / (2 * NMAX), f = o % (2 * NMAX);
+                const int row = f < NMAX ? (f < A.n_r ? f : -1) : (f - NMAX < A.n_a ? A.n_r + f - NMAX : -1);
+                if (pair < A.ntypes * A.ntypes && k < A.cs && row >= 0) {
+                    const T *c = coeffs + ((size_t)pair * nfun + row) * A.cs;
+                    if (k == 0) {
+                        v = T(2) * c[0];
+                        for (int q = 1; q < A.cs; q++) v += c[q];
+                    } else {
+                        v = (k & 2) ? -c[k] : c[k];
+                    }
+                }
+            } else if (i < L.b0) {
+                const int row = (i - L.w0) / D::NDP, k = (i - L.w0) % D::NDP, t = row / NP, p = row % NP;
+                if (k < A.nd && p < A.nneu) v = A.w0[((size_t)t * A.nneu + p) * A.nd + k];
+            } else if (i < L.iqs) {
+                const int row = (i - L.b0) % (A.ntypes * NP), t = row / NP, p = row % NP;
+                if (p < A.nneu) v = (i < L.w1 ? A.b0 : A.w1)[t * A.nneu + p];
+            } else if (i - L.iqs < A.nd) {
+                v = T(1) / A.qs[i - L.iqs];
+            }
+            tab[i] = v;
+        }
+        return;
+    }
+    const size_t i0 = (size_t)(blockIdx.x - tab_blocks) * blockDim.x + threadIdx.x, step = (size_t)(gridDim.x - tab_blocks) * blockDim.x;
+    for (size_t i = i0; i < n0; i += step) z0[i] = T(0);
+    for (size_t i = i0; i < n1; i += step) z1[i] = T(0);
+    for (size_t i = i0; i < n2; i += step) z2[i] = T(0);
 }
 
-template <typename T, int CSP, int MODE, int NMAX, int MINB>
-__global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_fast_kernel(const NepArgs<T> A, const T *__restrict__ coeffs)
+// sin and cos of pi t / 2, 0 <= t <= 1, s = t - 1: polynomials in t^2 fitted to the functions (sin(pi t / 2) / t, and
+// cos(pi t / 2) / (1 - t^2), so that the cosine keeps its relative precision towards t = 1); relative error 1.2e-7 and 6e-8
+__device__ __forceinline__ void quarter_wave(float t, float s, float &sn, float &cs)
 {
-    constexpr int RS = NMAX + NEP_NLM;     // staging row: g[NMAX] | B_lm[24]
-    constexpr int TROW = 2 * NMAX * CSP;   // coefficient rows of one (ti,tj) pair
-    constexpr bool CACHE = MODE != NEP_DESC;
-    extern __shared__ __align__(16) unsigned char nep_smem[];
-    constexpr int NDP = NepFastDims<NMAX>::NDP;
+    const float x = t * t;
+    sn = t * fmaf(fmaf(fmaf(fmaf(1.5167852689e-04f, x, -4.6741575934e-03f), x, 7.9689927399e-02f), x, -6.4596378803e-01f), x, 1.5707963705f);
+    cs = -s * (t + 1.f) * fmaf(fmaf(fmaf(fmaf(2.3601285648e-05f, x, -8.9353672229e-04f), x, 1.9968606532e-02f), x, -2.3370051384e-01f), x, 1.f);
+}
+__device__ __forceinline__ void quarter_wave(double t, double, double &sn, double &cs) { sincospi(0.5 * t, &sn, &cs); }
+
+// 1 / sqrt(v) with a Newton step behind the hardware's estimate in single precision
+__device__ __forceinline__ float inv_sqrt(float v) { const float y = rsqrtf(v); return y * fmaf(-0.5f * v * y, y, 1.5f); }
+__device__ __forceinline__ double inv_sqrt(double v) { return rsqrt(v); }
+
+// Radial functions g_n (basis.h:300-333,519-530) of one pair, and their derivatives, in pairs of functions. tc: the pair's
+// first Chebyshev row (of the radial or the angular functions); t = r / rc.
+template <typename T, int NMAX, bool DERIV>
+__device__ __forceinline__ void nep_functions(const T *tc, T t, T inv_rc, Pk<T> (&g)[NMAX / 2], Pk<T> (&dg)[NMAX / 2])
+{
+    constexpr int NP = NMAX / 2, ROW = 2 * NMAX;
+    const T s = t - T(1), x = T(2) * s * s - T(1), x2 = T(2) * x;
+    const Pk<T> plus = pk(x2, x2), minus = pk(-x2, -x2), p2 = pk(T(2), T(2)), m2 = pk(T(-2), T(-2));
+    Pk<T> u0 = pk(T(1), T(1)), u1 = pk(x, x), v0 = pk(T(0), T(0)), v1 = pk(T(1), T(1));
+    Pk<T> S[NP], dS[NP], c[NP];
+    load_pk<NP>(tc, S);
+    load_pk<NP>(tc + ROW, c);
+#pragma unroll
+    for (int n = 0; n < NP; n++) { S[n] = pk_fma(c[n], u1, S[n]); if (DERIV) dS[n] = c[n]; }
+#pragma unroll
+    for (int k = 2; k < NepFastDims<NMAX>::CS; k++) {
+        const Pk<T> f = (k & 1) ? plus : minus;
+        const Pk<T> u2 = pk_fma(f, u1, u0);
+        load_pk<NP>(tc + k * ROW, c);
+        if (DERIV) {
+            const Pk<T> v2 = pk_fma(f, v1, pk_fma((k & 1) ? p2 : m2, u1, v0));
+#pragma unroll
+            for (int n = 0; n < NP; n++) dS[n] = pk_fma(c[n], v2, dS[n]);
+            v0 = v1; v1 = v2;
+        }
+#pragma unroll
+        for (int n = 0; n < NP; n++) S[n] = pk_fma(c[n], u2, S[n]);
+        u0 = u1; u1 = u2;
+    }
+    T sn, cs;
+    quarter_wave(t, s, sn, cs);
+    const T fh = T(0.5) * cs * cs;      // half the cutoff function cos^2(pi t / 2)
+    const Pk<T> f2 = pk(fh, fh);
+#pragma unroll
+    for (int n = 0; n < NP; n++) g[n] = pk_mul(f2, S[n]);
+    if (DERIV) {
+        const T df = T(-0.5 * 3.14159265358979323846) * inv_rc * cs * sn, fx = fh * (T(4) * inv_rc) * s;
+        const Pk<T> d2 = pk(df, df), x3 = pk(fx, fx);
+#pragma unroll
+        for (int n = 0; n < NP; n++) dg[n] = pk_fma(x3, dS[n], pk_mul(d2, S[n]));
+    }
+}
+
+// N per-lane values (a power of two) summed over the G lanes of every group: lane `sub` of a group returns the total of value
+// sub / (G / N) (N <= G). All lanes of the warp take part.
+template <typename T, int N, int G>
+__device__ __forceinline__ T group_xreduce(T (&v)[N], int lane)
+{
+    static_assert(N <= G, "one value per lane at most");
+    int o = G / 2;
+#pragma unroll
+    for (int h = N / 2; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < h; i++) {
+            const T send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+            v[i] = keep + __shfl_xor_sync(FULL_MASK, send, o);
+        }
+    }
+    T r = v[0];
+    for (; o >= 1; o >>= 1) r += __shfl_xor_sync(FULL_MASK, r, o);
+    return r;
+}
+
+// f[0..2] += (x, y, z): in single precision one 8-byte and one 4-byte atomic (which of the two comes first follows from the
+// address: rows of three floats start on 8-byte boundaries or 4 bytes past one)
+__device__ __forceinline__ void add3(float *f, float x, float y, float z)
+{
+    const bool even = (reinterpret_cast<size_t>(f) & 4) == 0;
+    float *p2 = even ? f : f + 1, *p1 = even ? f + 2 : f;
+    const float a = even ? x : y, b = even ? y : z, c = even ? z : x;
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p2), "f"(a), "f"(b) : "memory");
+    atomicAdd(p1, c);
+}
+__device__ __forceinline__ void add3(double *f, double x, double y, double z) { atomicAdd(f, x); atomicAdd(f + 1, y); atomicAdd(f + 2, z); }
+
+// shared-memory elements (of T) per warp behind the model table; the neighbour lists follow (two bytes per neighbour)
+template <int NMAX, int G>
+__host__ __device__ inline int nep_fast_warp_elems(int nneu, int umax, bool net)
+{
+    using D = NepFastDims<NMAX>;
+    constexpr int AW = 32 / G;
+    const int stage = 32 * D::RS, es = AW * D::ESR;                 // staging rows, later the adjoints of the sums
+    return (stage > es ? stage : es) + AW * 2 * D::NDP +            // descriptors, their adjoints
+           (net ? AW * (nep_r32(nneu) + 4) + 96 + AW * umax * NMAX : 0);   // neurons, angular forces, cached derivatives
+}
+
+template <typename T, int G, int MODE, int NMAX, int MINB>
+__global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_fast_kernel(const NepArgs<T> A, const T *__restrict__ tab, int early_release)
+{
+    using D = NepFastDims<NMAX>;
+    constexpr int AW = 32 / G, NP2 = NMAX / 2, NDP = D::NDP, RS = D::RS, ESR = D::ESR, ROW = 2 * NMAX;
+    constexpr int LM = (NEP_NLM + G - 1) / G;            // sums per lane and function
+    constexpr int NPL = 32 / G;                          // neurons per lane and round
     constexpr bool NET = MODE != NEP_DESC;
+    extern __shared__ __align__(16) unsigned char nep_smem[];
     __shared__ T blk_acc[10];
     __shared__ int blk_b;
-    __shared__ T iqs[NDP];           // 1 / q_scaler, zero beyond the descriptor count
     __shared__ T fac_s[NEP_NLM];     // (2 - delta_m0) * 2 * C_lm
     __shared__ T c3w_s[NEP_NLM];     // (2 - delta_m0) * C_lm
-    __shared__ unsigned char pm_mu[NDP], pm_l[NDP];   // angular descriptor p -> (mu, l)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    chain_release();
-    const int sub = lane & (NEP_GROUP - 1), grp = lane / NEP_GROUP;
-    const int slot_in_block = warp * NEP_APW + grp;
-    const unsigned gmask_shift = grp * NEP_GROUP;
-    const unsigned gmask = 0xffu << gmask_shift;
-    const int per_atom = nep_fast_atom_elems<NMAX>(A.nneu, A.umax, CACHE);
-    const int ntab = A.ntypes * A.ntypes * TROW;
-    const int NP = nep_r32(A.nneu), nrow = A.ntypes * NP;   // zero rows pad every type to NP neurons
-    T *ctab_s = reinterpret_cast<T *>(nep_smem);
-    T *W0s = ctab_s + nep_r4(ntab);              // [ntypes * nneu][NDP], zero-padded rows
-    T *B0s = W0s + (NET ? nrow * NDP : 0);
-    T *W1s = B0s + (NET ? nrow : 0);
-    T *atoms_s = ctab_s + nep_fast_table_elems<NMAX, CSP>(A.ntypes, A.nneu, NET);
-    T *q = atoms_s + (size_t)slot_in_block * per_atom;   // [NDP]
-    T *Eq = q + NDP;                       // [NDP]
-    T *S = Eq + NDP;                       // [NMAX][24]
-    T *ES = S + NEP_NLM * NMAX;            // [24][NMAX]
-    T *act = ES + NEP_NLM * NMAX;
-    T *stage = S;                          // staging rows of the angular sums (before S, ES, act are written)
-    const int sea = 2 * NEP_NLM * NMAX + NP, stg = NEP_GROUP * RS;
-    T *dcache = S + (sea > stg ? sea : stg);   // [umax][NMAX]: g'_n of every neighbour
-    unsigned short *alist = reinterpret_cast<unsigned short *>(atoms_s + (size_t)NEP_APB * per_atom) + (size_t)slot_in_block * A.umax;
-    const int ntot_n = A.n_r + A.n_a;
+    const int sub = lane % G, grp = lane / G;
+    if (early_release) chain_release();
+    const NepTab<NMAX> L(A.ntypes, A.nneu, NET);
+    T *tab_s = reinterpret_cast<T *>(nep_smem);
+    const int per_warp = nep_fast_warp_elems<NMAX, G>(A.nneu, A.umax, NET), NP = nep_r32(A.nneu), NPP = NP + 4;
+    T *stage = tab_s + L.total + (size_t)warp * per_warp;
+    T *es = stage;                                       // [AW][ESR]
+    T *q = stage + (32 * RS > AW * ESR ? 32 * RS : AW * ESR) + grp * NDP;
+    T *Eq0 = q - grp * NDP + AW * NDP, *Eq = Eq0 + grp * NDP;
+    T *act0 = Eq0 + AW * NDP, *act = act0 + (NET ? grp * NPP : 0);
+    T *fbuf = act0 + (NET ? AW * NPP : 0);               // [32][3]
+    T *dcache0 = fbuf + 96, *dcache = dcache0 + (size_t)grp * A.umax * NMAX;      // [umax][NMAX]: g'_n / r of every neighbour
+    unsigned short *alist0 = reinterpret_cast<unsigned short *>(tab_s + L.total + (size_t)NEP_WARPS * per_warp) + (size_t)warp * AW * A.umax;
+    unsigned short *alist = alist0 + grp * A.umax;
     const int nlm = A.l_max * A.l_max + 2 * A.l_max;
     const int nq_a = A.l_max > 0 ? A.n_a * A.l_max : 0;
+    const T inv_rcr = T(1) / A.rc_r, inv_rca = T(1) / A.rc_a;
 
-    // block prologue: zero-padded tables, 1/q_scaler, 3-body factors, descriptor index map.
-    // The tables [coefficients | W0 rows | b0 | w1] are one contiguous run of shared memory; every
-    // thread first issues all of its (independent) global loads of the coefficients, then stores.
-    {
-        T qsv = T(1);
-        if (NET && (int)threadIdx.x < A.nd) qsv = A.qs[threadIdx.x];
-        const int n0 = nep_r4(ntab), n1 = n0 + (NET ? nrow * NDP : 0), n2 = n1 + (NET ? nrow : 0);
-        const int nall = n2 + (NET ? nrow : 0);
-        // neurons per type are padded to a multiple of 32: a power of two for the usual sizes, so the row -> (type,
-        // neuron) split is a shift instead of an integer division per staged element
-        const int np_shift = (NP & (NP - 1)) == 0 ? __ffs(NP) - 1 : -1;
-        auto split = [&](int row, int &t, int &pn) {
-            if (np_shift >= 0) { t = row >> np_shift; pn = row & (NP - 1); }
-            else { t = row / NP; pn = row % NP; }
-        };
-        auto load = [&](int i) -> T {
-            if (i < n0) {
-                if (i >= ntab) return T(0);
-                const int k = i % CSP, n = (i / CSP) % (2 * NMAX), pair = i / TROW;
-                const int row = n < NMAX ? (n < A.n_r ? n : -1) : (n - NMAX < A.n_a ? A.n_r + n - NMAX : -1);
-                return (k < A.cs && row >= 0) ? coeffs[((size_t)pair * ntot_n + row) * A.cs + k] : T(0);
-            }
-            if (i < n1) {
-                const int row = (i - n0) / NDP, k = (i - n0) % NDP;
-                int t, pn;
-                split(row, t, pn);
-                return (k < A.nd && pn < A.nneu) ? A.w0[((size_t)t * A.nneu + pn) * A.nd + k] : T(0);
-            }
-            const int row = i < n2 ? i - n1 : i - n2;
-            int t, pn;
-            split(row, t, pn);
-            if (pn >= A.nneu) return T(0);
-            return i < n2 ? A.b0[t * A.nneu + pn] : A.w1[t * A.nneu + pn];
-        };
-        // coefficients: through registers (the radial pass of the first atom needs them at once)
-        constexpr int U = 8;
-        for (int i0 = threadIdx.x; i0 < n0; i0 += U * blockDim.x) {
-            T v[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int i = i0 + u * blockDim.x;
-                v[u] = i < n0 ? load(i) : T(0);
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int i = i0 + u * blockDim.x;
-                if (i < n0) ctab_s[i] = v[u];
-            }
-        }
-        // network tables: asynchronous copies straight into shared memory, awaited before the first atom's network
-        // (they travel during its radial and angular passes); padding entries are plain zero stores
-        for (int i = n0 + threadIdx.x; i < nall; i += blockDim.x) {
-            const T *src = nullptr;
-            if (i < n1) {
-                const int row = (i - n0) / NDP, k = (i - n0) % NDP;
-                int t, pn;
-                split(row, t, pn);
-                if (k < A.nd && pn < A.nneu) src = A.w0 + ((size_t)t * A.nneu + pn) * A.nd + k;
-            } else {
-                const int row = i < n2 ? i - n1 : i - n2;
-                int t, pn;
-                split(row, t, pn);
-                if (pn < A.nneu) src = (i < n2 ? A.b0 : A.w1) + t * A.nneu + pn;
-            }
-            if (src) __pipeline_memcpy_async(ctab_s + i, src, sizeof(T));
-            else ctab_s[i] = T(0);
-        }
-        __pipeline_commit();
-        if (NET && threadIdx.x < NDP) iqs[threadIdx.x] = (int)threadIdx.x < A.nd ? T(1) / qsv : T(0);
-    }
     if (threadIdx.x < NEP_NLM) {
         const int lm = threadIdx.x;
         const bool m0 = lm == 0 || lm == 3 || lm == 8 || lm == 15;
         c3w_s[lm] = (m0 ? T(1) : T(2)) * (T)c_C3B[lm];
         fac_s[lm] = (m0 ? T(1) : T(2)) * T(2) * (T)c_C3B[lm];
     }
-    for (int p = threadIdx.x; p < NDP; p += blockDim.x) {
-        const bool in = p < nq_a;
-        pm_mu[p] = (unsigned char)(in ? p / A.l_max : 0);
-        pm_l[p] = (unsigned char)(in ? p % A.l_max + 1 : 0);
-    }
     // descriptors and their adjoints are read as NDP-long vectors: the padding stays zero
-    for (int i = threadIdx.x; i < NEP_APB * 2 * NDP; i += blockDim.x) atoms_s[(size_t)(i / (2 * NDP)) * per_atom + i % (2 * NDP)] = T(0);
-    __syncthreads();
-    chain_wait();        // the prologue read the model only: it ran while the kernels before this one drained
-
+    for (int i = lane; i < AW * 2 * NDP; i += 32) (q - grp * NDP)[i] = T(0);
+    chain_wait();        // the table and the offsets are the previous launch's
+    for (int i = threadIdx.x; i < L.total * (int)sizeof(T) / 16; i += NEP_WARPS * 32)
+        __pipeline_memcpy_async(reinterpret_cast<float4 *>(tab_s) + i, reinterpret_cast<const float4 *>(tab) + i, 16);
+    __pipeline_commit();
     const int ntot = A.B == 1 ? A.binum[0] : A.prefix[A.B];
-    const int ngroups = gridDim.x * NEP_APB;
-    const int gidx = blockIdx.x * NEP_APB + slot_in_block;
-    const int rounds = (ntot + ngroups - 1) / ngroups;
+    const int nwarps = gridDim.x * NEP_WARPS;
+    __pipeline_wait_prior(0);
+    __syncthreads();
 
-    // energy / virial of the atoms this lane has worked on, all of structure `bcur`
+    // energy / virial of the atoms this warp has worked on, all of structure `bcur`
     T e_acc = T(0), vir[9];
 #pragma unroll
     for (int k = 0; k < 9; k++) vir[k] = T(0);
     int bcur = -1;
-    auto flush_group = [&]() {   // called by all lanes of a group together
-        e_acc = group_sum(e_acc, gmask);
-        if (sub == 0) atomicAdd(A.etot + bcur, e_acc);
-        e_acc = T(0);
-        if (MODE == NEP_EFV) {
+    auto flush_to = [&](int b, T *e_dst, T *v_dst) {     // whole warp, one structure
+        T r[16];
 #pragma unroll
-            for (int k = 0; k < 9; k++) {
-                const T v = group_sum(vir[k], gmask);
-                if (sub == 0) atomicAdd(A.virial + 9 * bcur + k, v);
-                vir[k] = T(0);
-            }
-        }
+        for (int k = 0; k < 16; k++) r[k] = k == 0 ? e_acc : (MODE == NEP_EFV && k < 10) ? vir[k < 10 ? k - 1 : 0] : T(0);
+        const T s = group_xreduce<T, 16, 32>(r, lane);
+        const int k = lane >> 1;
+        if ((lane & 1) == 0 && (k == 0 || (MODE == NEP_EFV && k < 10))) atomicAdd(k == 0 ? e_dst : v_dst + k - 1, s);
+        e_acc = T(0);
+#pragma unroll
+        for (int k2 = 0; k2 < 9; k2++) vir[k2] = T(0);
     };
 
-    for (int it = 0; it < rounds; it++) {
-        const int t = it * ngroups + gidx;
+    for (int t0 = (blockIdx.x * NEP_WARPS + warp) * AW; t0 < ntot; t0 += nwarps * AW) {
+        const int t = t0 + grp;
         const bool valid = t < ntot;
         int b = 0;
         if (valid && A.B > 1) {
@@ -244,348 +364,417 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_fast_kernel(const Ne
             while (hi - lo > 1) { int mid = (lo + hi) >> 1; if (A.prefix[mid] <= t) lo = mid; else hi = mid; }
             b = lo;
         }
-        const int ii = valid ? (A.B > 1 ? t - A.prefix[b] : t) : 0;
-        const size_t slot = (size_t)b * A.npad + ii;
+        const int slot = b * A.npad + (valid ? (A.B > 1 ? t - A.prefix[b] : t) : 0);
         const int ci = valid ? A.bilist[slot] : 0;
         const int nn = valid ? min(A.numneigh[slot], A.umax) : 0;
-        const int *types = A.types + (size_t)b * (A.npad + (MODE == NEP_DESC ? 0 : A.nghost));
+        const size_t tstride = A.npad + (MODE == NEP_DESC ? 0 : A.nghost);
+        const int *types = A.types + (size_t)b * tstride;
         const int ti = valid ? types[ci] : 0;
-        const int *fn = A.firstneigh + slot * A.umax;
-        const T *rc = A.rcs + slot * A.umax * 3;
-        const T *ctab = ctab_s + (size_t)ti * A.ntypes * TROW;
-
-        if (NET && valid && b != bcur) {
-            if (bcur >= 0) flush_group();
-            bcur = b;
+        const int *fn = A.firstneigh + (size_t)slot * A.umax;
+        const T *rc = A.rcs + (size_t)slot * A.umax * 3;
+        const int nnmax = __reduce_max_sync(FULL_MASK, nn);
+        // atoms of one structure accumulate energy and virial in registers; a warp across a boundary adds its own at once
+        bool mixed = false;
+        if (NET) {
+            const int b0 = __shfl_sync(FULL_MASK, b, 0);
+            mixed = A.B > 1 && !__all_sync(FULL_MASK, !valid || b == b0);
+            if (mixed || b0 != bcur) {
+                if (bcur >= 0) flush_to(bcur, A.etot + bcur, A.virial + 9 * bcur);
+                bcur = mixed ? -1 : b0;
+            }
         }
 
-        // ---- 1. radial pass: q_n, cached g'_n, compaction of the angular neighbours ----------------
-        T qacc[NMAX];
+        // ---- 1. radial pass: q_n, cached g'_n / r, lists of the angular neighbours --------------------
+        Pk<T> qa[NP2];
 #pragma unroll
-        for (int n = 0; n < NMAX; n++) qacc[n] = T(0);
+        for (int n = 0; n < NP2; n++) qa[n] = pk(T(0), T(0));
         int nang = 0;
-        // the next chunk's positions and indices are requested before this chunk is worked on
-        T xn = 0, yn = 0, zn = 0;
-        int njn = 0;
-        if (sub < nn) { xn = rc[3 * sub]; yn = rc[3 * sub + 1]; zn = rc[3 * sub + 2]; njn = fn[sub]; }
-        for (int j0 = 0; j0 < nn; j0 += NEP_GROUP) {
-            const int j = j0 + sub;
-            bool on = j < nn;
-            const T x = xn, y = yn, z = zn;
-            const int tj = on ? types[njn] : 0;
-            {
-                const int jn = j + NEP_GROUP;
-                xn = yn = zn = T(0);
-                if (jn < nn) { xn = rc[3 * jn]; yn = rc[3 * jn + 1]; zn = rc[3 * jn + 2]; njn = fn[jn]; }
-            }
-            const T r = gsqrt(x * x + y * y + z * z);
-            on = on && r <= A.rc_r && r > T(0);
-            T f[CSP], df[CSP];
-            nep_radial<T, CSP>(on ? r : A.rc_r, A.rc_r, f, df);
-            const T *crow = ctab + (size_t)tj * TROW;
-            T dgv[NMAX];
-#pragma unroll
-            for (int n = 0; n < NMAX; n++) {
-                T c[CSP];
-                load_vec<T, CSP>(crow + n * CSP, c);
-                T g = T(0), dg = T(0);
-#pragma unroll
-                for (int k = 0; k < CSP; k++) {
-                    g = fma(c[k], f[k], g);
-                    if (CACHE) dg = fma(c[k], df[k], dg);
+        {
+            T xn = 0, yn = 0, zn = 0;
+            int njn = 0;
+            if (sub < nn) { xn = rc[3 * sub]; yn = rc[3 * sub + 1]; zn = rc[3 * sub + 2]; njn = fn[sub]; }
+            for (int j0 = 0; j0 < nnmax; j0 += G) {
+                const int j = j0 + sub;
+                bool on = j < nn;
+                const T x = xn, y = yn, z = zn;
+                const int tj = on ? types[njn] : 0;
+                {   // the next chunk's positions and indices are requested before this chunk is worked on
+                    const int jn = j + G;
+                    xn = yn = zn = T(0);
+                    if (jn < nn) { xn = rc[3 * jn]; yn = rc[3 * jn + 1]; zn = rc[3 * jn + 2]; njn = fn[jn]; }
                 }
-                qacc[n] += on ? g : T(0);
-                dgv[n] = on ? dg : T(0);
-            }
-            if (CACHE && j < A.umax) store_vec<T, NMAX>(dcache + (size_t)j * NMAX, dgv);
-            const bool ang = on && r <= A.rc_a && A.l_max > 0;
-            const unsigned bal = (__ballot_sync(gmask, ang) >> gmask_shift) & 0xffu;
-            // list entry: neighbour slot (10 bits) | neighbour type (4 bits)
-            if (ang) alist[nang + __popc(bal & ((1u << sub) - 1u))] = (unsigned short)(j | (tj << 10));
-            nang += __popc(bal);
-        }
+                const T r2 = x * x + y * y + z * z;
+                on = on && r2 > T(0);
+                const T rinv = inv_sqrt(on ? r2 : T(1)), r = r2 * rinv;
+                const bool ang = on && r <= A.rc_a && A.l_max > 0;
+                on = on && r <= A.rc_r;
+                Pk<T> g[NP2], dg[NP2];
+                nep_functions<T, NMAX, NET>(tab_s + (ti * A.ntypes + tj) * D::TROW, on ? r * inv_rcr : T(1), inv_rcr, g, dg);
+                const T w = on ? T(1) : T(0);
+                const Pk<T> w2 = pk(w, w);
 #pragma unroll
-        for (int n = 0; n < NMAX; n++) {
-            const T s = group_sum(qacc[n], gmask);
-            if (sub == (n & (NEP_GROUP - 1)) && n < A.n_r) q[n] = s;
+                for (int n = 0; n < NP2; n++) qa[n] = pk_fma(w2, g[n], qa[n]);
+                if (NET && j < A.umax) {
+                    const T wr = on ? rinv : T(0);
+                    T d[NMAX];
+#pragma unroll
+                    for (int n = 0; n < NP2; n++) { d[2 * n] = wr * pk_lo(dg[n]); d[2 * n + 1] = wr * pk_hi(dg[n]); }
+                    store_vec<T, NMAX>(dcache + (size_t)j * NMAX, d);
+                }
+                const unsigned bal = __ballot_sync(FULL_MASK, ang) >> (G == 32 ? 0 : grp * G) & (G == 32 ? FULL_MASK : (1u << (G & 31)) - 1u);
+                // list entry: neighbour slot (10 bits) | neighbour type (4 bits)
+                if (ang) alist[nang + __popc(bal & ((1u << sub) - 1u))] = (unsigned short)(j | (tj << 10));
+                nang += __popc(bal);
+            }
         }
-        __syncwarp(gmask);
+        {
+            T v[NMAX];
+#pragma unroll
+            for (int n = 0; n < NP2; n++) { v[2 * n] = pk_lo(qa[n]); v[2 * n + 1] = pk_hi(qa[n]); }
+            if constexpr (NMAX <= G) {
+                const T s = group_xreduce<T, NMAX, G>(v, lane);
+                if (sub % (G / NMAX) == 0 && sub / (G / NMAX) < A.n_r) q[sub / (G / NMAX)] = s;
+            } else {
+#pragma unroll
+                for (int n = 0; n < NMAX; n++) {
+                    T s = v[n];
+#pragma unroll
+                    for (int o = G / 2; o >= 1; o >>= 1) s += __shfl_xor_sync(FULL_MASK, s, o);
+                    if (sub == n % G && n < A.n_r) q[n] = s;
+                }
+            }
+        }
+        __syncwarp();
 
-        // ---- 2. angular sums: lane `sub` ends with S[mu][3 sub .. 3 sub + 2] ------------------------
-        T Sacc[NMAX][3];
+        // ---- 2. angular sums: lane `sub` of a group ends with S[mu][LM sub .. LM sub + LM - 1] of its atom ------
+        // the angular neighbours of the warp's atoms in one sequence: group g's are first[g] .. first[g] + nang - 1
+        int first = 0, total = 0;
 #pragma unroll
-        for (int mu = 0; mu < NMAX; mu++) Sacc[mu][0] = Sacc[mu][1] = Sacc[mu][2] = T(0);
-        for (int k0 = 0; k0 < nang; k0 += NEP_GROUP) {
-            const bool on = k0 + sub < nang;
-            T x = 0, y = 0, z = 0, rinv = 0, r = A.rc_a;
-            int tj = 0;
-            if (on) {
-                const int ent = alist[k0 + sub], j = ent & 1023;
-                tj = ent >> 10;
-                x = rc[3 * j]; y = rc[3 * j + 1]; z = rc[3 * j + 2];
-                r = gsqrt(x * x + y * y + z * z);
-                rinv = T(1) / r;
+        for (int g = 0; g < AW; g++) {
+            const int c = __shfl_sync(FULL_MASK, nang, g * G);
+            if (g == grp) first = total;
+            total += c;
+        }
+        const bool keep = total <= 32;          // one step: what it computes stays in registers for the force pass
+        Pk<T> S[LM][NP2];
+#pragma unroll
+        for (int i = 0; i < LM; i++)
+#pragma unroll
+            for (int n = 0; n < NP2; n++) S[i][n] = pk(T(0), T(0));
+        // the angular neighbour that this lane works on
+        Pk<T> g[NP2], dg[NP2];
+        T ux = 0, uy = 0, uz = 0, rinv = 0, rr = 0;
+        int pg = 0, pj = 0;
+        bool pon = false;
+        auto take_pair = [&](int p) {
+            pon = p < total;
+            int k = p;
+            pg = 0;
+#pragma unroll
+            for (int a = 0; a < AW - 1; a++) {
+                const int c = __shfl_sync(FULL_MASK, nang, a * G);
+                if (pg == a && k >= c) { k -= c; pg = a + 1; }
             }
+            const int pslot = __shfl_sync(FULL_MASK, slot, pg * G), pti = __shfl_sync(FULL_MASK, ti, pg * G);
+            T x = T(0), y = T(0), z = A.rc_a;
+            int tj = 0;
+            pj = 0;
+            if (pon) {
+                const int ent = alist0[pg * A.umax + k];
+                pj = ent & 1023;
+                tj = ent >> 10;
+                const T *pr = A.rcs + ((size_t)pslot * A.umax + pj) * 3;
+                x = pr[0]; y = pr[1]; z = pr[2];
+            }
+            const T r2 = x * x + y * y + z * z;
+            rinv = inv_sqrt(r2);
+            rr = r2 * rinv;
+            ux = x * rinv; uy = y * rinv; uz = z * rinv;
+            nep_functions<T, NMAX, NET>(tab_s + (pti * A.ntypes + tj) * D::TROW + NMAX, rr * inv_rca, inv_rca, g, dg);
+        };
+        for (int p0 = 0; p0 < total; p0 += 32) {
+            take_pair(p0 + lane);
             {
-                T f[CSP], df[CSP], row[RS];
-                nep_radial<T, CSP>(r, A.rc_a, f, df);
-                const T *crow = ctab + (size_t)tj * TROW + NMAX * CSP;
+                T row[RS];
 #pragma unroll
-                for (int mu = 0; mu < NMAX; mu++) {
-                    T c[CSP];
-                    load_vec<T, CSP>(crow + mu * CSP, c);
-                    T g = T(0);
-#pragma unroll
-                    for (int k = 0; k < CSP; k++) g = fma(c[k], f[k], g);
-                    row[mu] = on ? g : T(0);
-                }
-                const T ux = x * rinv, uy = y * rinv, uz = z * rinv;
+                for (int n = 0; n < NP2; n++) { row[2 * n] = pk_lo(g[n]); row[2 * n + 1] = pk_hi(g[n]); }
                 {
-                    const T x_ = ux, y_ = uy, z_ = uz;
-                    NEP_POLY_COMMON(x_, y_, z_)
+                    NEP_POLY_COMMON(ux, uy, uz)
 #define NEP_X(k, val, gx, gy, gz) row[NMAX + k] = (val);
-                    NEP_FOR_EACH_LM(NEP_X, x_, y_, z_)
+                    NEP_FOR_EACH_LM(NEP_X, ux, uy, uz)
 #undef NEP_X
                 }
-                store_vec<T, RS>(stage + sub * RS, row);
-            }
-            __syncwarp(gmask);
-            const int cnt = min(NEP_GROUP, nang - k0);
-            for (int jj = 0; jj < cnt; jj++) {
-                const T *rj = stage + jj * RS;
-                T gj[NMAX];
-                load_vec<T, NMAX>(rj, gj);
-                const T b0 = rj[NMAX + 3 * sub], b1 = rj[NMAX + 3 * sub + 1], b2 = rj[NMAX + 3 * sub + 2];
 #pragma unroll
-                for (int mu = 0; mu < NMAX; mu++) {
-                    Sacc[mu][0] = fma(gj[mu], b0, Sacc[mu][0]);
-                    Sacc[mu][1] = fma(gj[mu], b1, Sacc[mu][1]);
-                    Sacc[mu][2] = fma(gj[mu], b2, Sacc[mu][2]);
+                for (int k = NMAX + NEP_NLM; k < RS; k++) row[k] = T(0);
+                if (pon) store_vec<T, RS>(stage + lane * RS, row);
+            }
+            __syncwarp();
+            const int k0 = max(first - p0, 0), k1 = min(first + nang - p0, 32);       // this group's rows of the step
+            const int steps = __reduce_max_sync(FULL_MASK, k1 - k0);
+            for (int k = k0; k < k0 + steps; k++) {
+                if (k < k1) {
+                    const T *row = stage + k * RS;
+                    Pk<T> gj[NP2];
+                    load_pk<NP2>(row, gj);
+#pragma unroll
+                    for (int i = 0; i < LM; i++) {
+                        const int lm = LM * sub + i;
+                        const T bv = lm < NEP_NLM ? row[NMAX + lm] : T(0);
+                        const Pk<T> b2 = pk(bv, bv);
+#pragma unroll
+                        for (int n = 0; n < NP2; n++) S[i][n] = pk_fma(gj[n], b2, S[i][n]);
+                    }
                 }
             }
-            __syncwarp(gmask);
+            __syncwarp();
         }
-#pragma unroll
-        for (int mu = 0; mu < NMAX; mu++) {
-            S[mu * NEP_NLM + 3 * sub] = Sacc[mu][0];
-            S[mu * NEP_NLM + 3 * sub + 1] = Sacc[mu][1];
-            S[mu * NEP_NLM + 3 * sub + 2] = Sacc[mu][2];
-        }
-        __syncwarp(gmask);
 
-        // ---- 3. angular descriptors, network ------------------------------------------------------------
-        for (int p = sub; p < nq_a; p += NEP_GROUP) {
-            const int mu = pm_mu[p], l = pm_l[p];
-            const T *Srow = S + mu * NEP_NLM + l * l - 1;
-            const T *cw = c3w_s + l * l - 1;
-            T acc = T(0);
-            for (int mp = 0; mp < 2 * l + 1; mp++) acc += cw[mp] * Srow[mp] * Srow[mp];
-            q[A.n_r + p] = acc;
+        // ---- 3. angular descriptors q_{mu,l} = sum_m w_m C_lm S^2, network --------------------------------------
+        T *tq = es + grp * ESR;
+#pragma unroll
+        for (int i = 0; i < LM; i++) {
+            const int lm = LM * sub + i;
+            if (lm < NEP_NLM) {
+#pragma unroll
+                for (int n = 0; n < NP2; n++) {
+                    tq[2 * n * NEP_NLM + lm] = c3w_s[lm] * pk_lo(S[i][n]) * pk_lo(S[i][n]);
+                    tq[(2 * n + 1) * NEP_NLM + lm] = c3w_s[lm] * pk_hi(S[i][n]) * pk_hi(S[i][n]);
+                }
+            }
         }
-        __syncwarp(gmask);
+        __syncwarp();
+        for (int p = sub; p < nq_a; p += G) {
+            const int mu = p / A.l_max, l = p - mu * A.l_max + 1;
+            const T *row = tq + mu * NEP_NLM + l * l - 1;
+            T s = row[0] + row[1] + row[2];
+            for (int m = 3; m < 2 * l + 1; m += 2) s += row[m] + row[m + 1];
+            q[A.n_r + p] = s;
+        }
+        __syncwarp();
         if constexpr (MODE == NEP_DESC) {
             if (valid)
-                for (int k = sub; k < A.nd; k += NEP_GROUP) A.desc[slot * A.nd + k] = q[k];
-            __syncwarp(gmask);
+                for (int k = sub; k < A.nd; k += G) A.desc[(size_t)slot * A.nd + k] = q[k];
+            __syncwarp();
         } else {
-        // network on the scaled descriptors; rows and vectors are zero-padded to NDP
-        if (it == 0) {      // the network tables requested in the prologue have to be there now
-            __pipeline_wait_prior(0);
-            __syncthreads();
-        }
-        for (int k = sub; k < A.nd; k += NEP_GROUP) Eq[k] = q[k] * iqs[k];
-        __syncwarp(gmask);
-        T es = T(0);
-        const T *W0t = W0s + (size_t)ti * NP * NDP;
-        for (int p0 = 0; p0 < NP; p0 += 4 * NEP_GROUP) {   // four neurons per lane at a time
-            T h[4][4];
+        for (int k = sub; k < A.nd; k += G) Eq[k] = q[k] * tab_s[L.iqs + k];
+        __syncwarp();
+        T e_at = T(0);
+        const T *W0t = tab_s + L.w0 + ti * NP * NDP, *B0t = tab_s + L.b0 + ti * NP, *W1t = tab_s + L.w1 + ti * NP;
+        for (int p0 = 0; p0 < NP; p0 += NPL * G) {      // lanes = neurons, NPL at a time
+            Pk<T> h[NPL];
 #pragma unroll
-            for (int i = 0; i < 4; i++) h[i][0] = h[i][1] = h[i][2] = h[i][3] = T(0);
+            for (int i = 0; i < NPL; i++) h[i] = pk(T(0), T(0));
 #pragma unroll
             for (int c = 0; c < NDP / 4; c++) {
-                T e[4];
-                load_vec<T, 4>(Eq + 4 * c, e);
+                Pk<T> e[2];
+                load_pk<2>(Eq + 4 * c, e);
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    T w[4];
-                    load_vec<T, 4>(W0t + (size_t)(p0 + sub + NEP_GROUP * i) * NDP + 4 * c, w);
-#pragma unroll
-                    for (int k = 0; k < 4; k++) h[i][k] = fma(w[k], e[k], h[i][k]);
+                for (int i = 0; i < NPL; i++) {
+                    Pk<T> w[2];
+                    load_pk<2>(W0t + (p0 + sub + G * i) * NDP + 4 * c, w);
+                    h[i] = pk_fma(w[0], e[0], h[i]);
+                    h[i] = pk_fma(w[1], e[1], h[i]);
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int p = p0 + sub + NEP_GROUP * i;
-                const T th = gtanh((h[i][0] + h[i][1]) + (h[i][2] + h[i][3]) + B0s[ti * NP + p]);
-                const T w1 = W1s[ti * NP + p];   // zero for padding neurons
-                es += w1 * th;
+            for (int i = 0; i < NPL; i++) {
+                const int p = p0 + sub + G * i;
+                const T th = gtanh(pk_lo(h[i]) + pk_hi(h[i]) + B0t[p]);
+                const T w1 = W1t[p];                    // zero for padding neurons
+                e_at += w1 * th;
                 act[p] = w1 * (T(1) - th * th);
             }
         }
-        if (valid) e_acc += es + (sub == 0 ? A.bias[ti] : T(0));
-        __syncwarp(gmask);
-        for (int c = sub; c < NDP / 4; c += NEP_GROUP) {   // lane c: descriptors 4c .. 4c+3
-            const T *wcol = W0t + 4 * c;
-            T a[4][4];
+        if (valid) e_at += sub == 0 ? A.bias[ti] : T(0);
+        else e_at = T(0);
+        __syncwarp();
+        {   // adjoints of the descriptors: lanes = four descriptors each, the neurons in G / 8 parts
+            constexpr int PARTS = G >= 8 ? G / 8 : 1, CL = G >= 8 ? 8 : G;
+            const int part = sub / CL, pb = part * (NP / PARTS), pe = pb + NP / PARTS;
+            for (int c0 = 0; c0 < NDP / 4; c0 += CL) {
+                const int c = c0 + sub % CL;
+                const bool in = c < NDP / 4;
+                const T *wcol = W0t + 4 * (in ? c : 0);
+                Pk<T> a[2][2];
+                a[0][0] = a[0][1] = a[1][0] = a[1][1] = pk(T(0), T(0));
+#pragma unroll 2
+                for (int p = pb; p < pe; p += 4) {
+                    T x[4];
+                    load_vec<T, 4>(act + p, x);
 #pragma unroll
-            for (int i = 0; i < 4; i++) a[i][0] = a[i][1] = a[i][2] = a[i][3] = T(0);
-            for (int p = 0; p < NP; p += 4) {
-                T x[4];
-                load_vec<T, 4>(act + p, x);
+                    for (int i = 0; i < 4; i++) {
+                        Pk<T> w[2];
+                        load_pk<2>(wcol + (p + i) * NDP, w);
+                        const Pk<T> x2 = pk(x[i], x[i]);
+                        a[i & 1][0] = pk_fma(x2, w[0], a[i & 1][0]);
+                        a[i & 1][1] = pk_fma(x2, w[1], a[i & 1][1]);
+                    }
+                }
+                T r[4] = {pk_lo(a[0][0]) + pk_lo(a[1][0]), pk_hi(a[0][0]) + pk_hi(a[1][0]), pk_lo(a[0][1]) + pk_lo(a[1][1]), pk_hi(a[0][1]) + pk_hi(a[1][1])};
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    T w[4];
-                    load_vec<T, 4>(wcol + (size_t)(p + i) * NDP, w);
+                for (int o = CL; o < G; o <<= 1)
 #pragma unroll
-                    for (int k = 0; k < 4; k++) a[i][k] = fma(x[i], w[k], a[i][k]);
+                    for (int k = 0; k < 4; k++) r[k] += __shfl_xor_sync(FULL_MASK, r[k], o);
+                if (in && part == 0) {
+#pragma unroll
+                    for (int k = 0; k < 4; k++) r[k] *= tab_s[L.iqs + 4 * c + k];
+                    store_vec<T, 4>(Eq + 4 * c, r);
                 }
             }
-            T r[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) r[k] = ((a[0][k] + a[1][k]) + (a[2][k] + a[3][k])) * iqs[4 * c + k];
-            store_vec<T, 4>(Eq + 4 * c, r);
         }
-        __syncwarp(gmask);
-        // adjoints of the sums, layout [lm][NMAX] for 16-byte broadcast loads in the force pass
+        __syncwarp();
+        // adjoints of the sums, [mu][24] (the descriptors' terms that lay there have been read)
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
-            const int lm = 3 * sub + i;
-            const int l = lm >= 15 ? 4 : lm >= 8 ? 3 : lm >= 3 ? 2 : 1;
-            T e[NMAX];
+        for (int i = 0; i < LM; i++) {
+            const int lm = LM * sub + i;
+            if (lm < NEP_NLM) {
+                const int l = lm >= 15 ? 4 : lm >= 8 ? 3 : lm >= 3 ? 2 : 1;
 #pragma unroll
-            for (int mu = 0; mu < NMAX; mu++)
-                e[mu] = (lm < nlm && mu < A.n_a) ? fac_s[lm] * Eq[A.n_r + mu * A.l_max + l - 1] * Sacc[mu][i] : T(0);
-            store_vec<T, NMAX>(ES + lm * NMAX, e);
+                for (int mu = 0; mu < NMAX; mu++) {
+                    const T s = (mu & 1) ? pk_hi(S[i][mu / 2]) : pk_lo(S[i][mu / 2]);
+                    tq[mu * NEP_NLM + lm] = (lm < nlm && mu < A.n_a) ? fac_s[lm] * Eq[A.n_r + mu * A.l_max + l - 1] * s : T(0);
+                }
+            }
         }
-        T eqr[NMAX];
-#pragma unroll
-        for (int n = 0; n < NMAX; n++) eqr[n] = n < A.n_r ? Eq[n] : T(0);
-        __syncwarp(gmask);
+        __syncwarp();
 
-        // ---- 4. force / virial -------------------------------------------------------------------------
-        T *frc = A.force + (size_t)b * (A.npad + A.nghost) * 3;
-        T fcx = 0, fcy = 0, fcz = 0;
-        auto scatter = [&](bool on, int nj, T gx, T gy, T gz, T x, T y, T z) {
-            if (!on) return;
-            fcx += gx; fcy += gy; fcz += gz;
-            atomicAdd(frc + 3 * nj + 0, -gx);
-            atomicAdd(frc + 3 * nj + 1, -gy);
-            atomicAdd(frc + 3 * nj + 2, -gz);
+        // ---- 4. forces and virial --------------------------------------------------------------------------------
+        T fx = T(0), fy = T(0), fz = T(0);            // on this group's atom
+        auto add_virial = [&](T gx, T gy, T gz, T x, T y, T z) {
             if (MODE == NEP_EFV) {
                 vir[0] -= gx * x; vir[1] -= gx * y; vir[2] -= gx * z;
                 vir[3] -= gy * x; vir[4] -= gy * y; vir[5] -= gy * z;
                 vir[6] -= gz * x; vir[7] -= gz * y; vir[8] -= gz * z;
             }
         };
-        xn = yn = zn = T(0);
-        if (sub < nn) { xn = rc[3 * sub]; yn = rc[3 * sub + 1]; zn = rc[3 * sub + 2]; njn = fn[sub]; }
-        for (int j0 = 0; j0 < nn; j0 += NEP_GROUP) {     // radial part from the cached g'_n
-            const int j = j0 + sub;
-            bool on = j < nn;
-            const T x = xn, y = yn, z = zn;
-            const int nj = njn;
-            {
-                const int jn = j + NEP_GROUP;
-                xn = yn = zn = T(0);
-                if (jn < nn) { xn = rc[3 * jn]; yn = rc[3 * jn + 1]; zn = rc[3 * jn + 2]; njn = fn[jn]; }
-            }
-            T dgv[NMAX];
+        for (int p0 = 0; p0 < total; p0 += 32) {       // angular neighbours, with their radial part
+            if (!keep) take_pair(p0 + lane);
+            const T *ep = es + pg * ESR;
+            T V = T(0), U = T(0), Gx = T(0), Gy = T(0), Gz = T(0);     // sum D B, sum l A B, sum A grad B
+            Pk<T> gg[NMAX], dd[NMAX];
 #pragma unroll
-            for (int n = 0; n < NMAX; n++) dgv[n] = T(0);
-            if (on) load_vec<T, NMAX>(dcache + (size_t)j * NMAX, dgv);
-            const T r = gsqrt(x * x + y * y + z * z);
-            on = on && r <= A.rc_r && r > T(0);
-            T gr = T(0);
-#pragma unroll
-            for (int n = 0; n < NMAX; n++) gr = fma(eqr[n], dgv[n], gr);
-            const T s = on ? gr / r : T(0);
-            scatter(on, nj, s * x, s * y, s * z, x, y, z);
-        }
-        for (int k0 = 0; k0 < nang; k0 += NEP_GROUP) {   // angular part
-            const bool on = k0 + sub < nang;
-            T x = 0, y = 0, z = 0, rinv = 0, r = A.rc_a;
-            int nj = 0, tj = 0;
-            if (on) {
-                const int ent = alist[k0 + sub], j = ent & 1023;
-                tj = ent >> 10;
-                x = rc[3 * j]; y = rc[3 * j + 1]; z = rc[3 * j + 2];
-                nj = fn[j];
-                r = gsqrt(x * x + y * y + z * z);
-                rinv = T(1) / r;
+            for (int n = 0; n < NP2; n++) {
+                gg[2 * n] = pk(pk_lo(g[n]), pk_lo(g[n])); gg[2 * n + 1] = pk(pk_hi(g[n]), pk_hi(g[n]));
+                dd[2 * n] = pk(pk_lo(dg[n]), pk_lo(dg[n])); dd[2 * n + 1] = pk(pk_hi(dg[n]), pk_hi(dg[n]));
             }
-            const T ux = x * rinv, uy = y * rinv, uz = z * rinv;
-            T g[NMAX], dg[NMAX];
-            {
-                T f[CSP], df[CSP];
-                nep_radial<T, CSP>(r, A.rc_a, f, df);
-                const T *crow = ctab + (size_t)tj * TROW + NMAX * CSP;
+            T Av[NEP_NLM], Dv[NEP_NLM];
+#pragma unroll
+            for (int c = 0; c < NEP_NLM / 4; c++) {
+                Pk<T> a[2], d[2];
 #pragma unroll
                 for (int mu = 0; mu < NMAX; mu++) {
-                    T c[CSP];
-                    load_vec<T, CSP>(crow + mu * CSP, c);
-                    T a = T(0), d = T(0);
+                    Pk<T> e[2];
+                    load_pk<2>(ep + mu * NEP_NLM + 4 * c, e);
 #pragma unroll
-                    for (int k = 0; k < CSP; k++) {
-                        a = fma(c[k], f[k], a);
-                        d = fma(c[k], df[k], d);
+                    for (int h = 0; h < 2; h++) {
+                        a[h] = mu ? pk_fma(gg[mu], e[h], a[h]) : pk_mul(gg[mu], e[h]);
+                        d[h] = mu ? pk_fma(dd[mu], e[h], d[h]) : pk_mul(dd[mu], e[h]);
                     }
-                    g[mu] = a; dg[mu] = d;
+                }
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    Av[4 * c + 2 * h] = pk_lo(a[h]); Av[4 * c + 2 * h + 1] = pk_hi(a[h]);
+                    Dv[4 * c + 2 * h] = pk_lo(d[h]); Dv[4 * c + 2 * h + 1] = pk_hi(d[h]);
                 }
             }
-            T Pv[NMAX], Gx[NMAX], Gy[NMAX], Gz[NMAX];
-#pragma unroll
-            for (int mu = 0; mu < NMAX; mu++) Pv[mu] = Gx[mu] = Gy[mu] = Gz[mu] = T(0);
             {
                 NEP_POLY_COMMON(ux, uy, uz)
-#define NEP_X(k, val, gx_, gy_, gz_)                                      \
-    {                                                                     \
-        T e[NMAX];                                                        \
-        load_vec<T, NMAX>(ES + (k) * NMAX, e);                            \
-        nep_acc<T, NMAX>(e, (val), Pv);                                   \
-        nep_acc<T, NMAX>(e, (gx_), Gx);                                   \
-        nep_acc<T, NMAX>(e, (gy_), Gy);                                   \
-        nep_acc<T, NMAX>(e, (gz_), Gz);                                   \
+#define NEP_X(k, val, gx_, gy_, gz_)                                                      \
+    {                                                                                     \
+        const T b_ = (val), ab_ = Av[k] * b_;                                             \
+        V = fma(Dv[k], b_, V);                                                            \
+        U = fma(T((k) >= 15 ? 4 : (k) >= 8 ? 3 : (k) >= 3 ? 2 : 1), ab_, U);              \
+        nep_acc1<T>(Av[k], (gx_), Gx);                                                    \
+        nep_acc1<T>(Av[k], (gy_), Gy);                                                    \
+        nep_acc1<T>(Av[k], (gz_), Gz);                                                    \
     }
                 NEP_FOR_EACH_LM(NEP_X, ux, uy, uz)
 #undef NEP_X
             }
-            T gx = 0, gy = 0, gz = 0;
+            // u . grad B_lm = l B_lm: the part of the gradient along u needs no dot product
+            const T *Eqp = Eq0 + pg * NDP;
+            T *dc = dcache0 + ((size_t)pg * A.umax + pj) * NMAX;
+            T d[NMAX], gr = T(0);
+            load_vec<T, NMAX>(dc, d);
 #pragma unroll
-            for (int mu = 0; mu < NMAX; mu++) {
-                const T ug = ux * Gx[mu] + uy * Gy[mu] + uz * Gz[mu];
-                const T c = g[mu] * rinv, a = dg[mu] * Pv[mu] - c * ug;
-                gx += a * ux + c * Gx[mu];
-                gy += a * uy + c * Gy[mu];
-                gz += a * uz + c * Gz[mu];
+            for (int n = 0; n < NMAX; n++) gr = fma(n < A.n_r ? Eqp[n] : T(0), d[n], gr);
+            const T au = V - rinv * U + gr * rr;
+            const T gx = pon ? fma(au, ux, rinv * Gx) : T(0), gy = pon ? fma(au, uy, rinv * Gy) : T(0), gz = pon ? fma(au, uz, rinv * Gz) : T(0);
+            fbuf[3 * lane] = gx; fbuf[3 * lane + 1] = gy; fbuf[3 * lane + 2] = gz;
+            const int pslot = __shfl_sync(FULL_MASK, slot, pg * G), pb = __shfl_sync(FULL_MASK, b, pg * G);
+            if (pon) {
+                const int nj = A.firstneigh[(size_t)pslot * A.umax + pj];
+                add3(A.force + ((size_t)pb * (A.npad + A.nghost) + nj) * 3, -gx, -gy, -gz);
+                const T x = ux * rr, y = uy * rr, z = uz * rr;
+                if (!mixed) add_virial(gx, gy, gz, x, y, z);
+                else if (MODE == NEP_EFV) {
+                    T *v = A.virial + 9 * pb;
+                    atomicAdd(v, -gx * x); atomicAdd(v + 1, -gx * y); atomicAdd(v + 2, -gx * z);
+                    atomicAdd(v + 3, -gy * x); atomicAdd(v + 4, -gy * y); atomicAdd(v + 5, -gy * z);
+                    atomicAdd(v + 6, -gz * x); atomicAdd(v + 7, -gz * y); atomicAdd(v + 8, -gz * z);
+                }
+#pragma unroll
+                for (int n = 0; n < NMAX; n++) d[n] = T(0);
+                store_vec<T, NMAX>(dc, d);            // done: the radial pass leaves this neighbour out
             }
-            scatter(on, nj, gx, gy, gz, x, y, z);
+            __syncwarp();
+            const int k1 = min(first + nang - p0, 32);
+            for (int k = max(first - p0, 0) + sub; k < k1; k += G) { fx += fbuf[3 * k]; fy += fbuf[3 * k + 1]; fz += fbuf[3 * k + 2]; }
+            __syncwarp();
         }
-        fcx = group_sum(fcx, gmask); fcy = group_sum(fcy, gmask); fcz = group_sum(fcz, gmask);
-        if (sub == 0 && valid) {
-            atomicAdd(frc + 3 * ci + 0, fcx);
-            atomicAdd(frc + 3 * ci + 1, fcy);
-            atomicAdd(frc + 3 * ci + 2, fcz);
+        {
+            T eqr[NMAX];
+#pragma unroll
+            for (int n = 0; n < NMAX; n++) eqr[n] = n < A.n_r ? Eq[n] : T(0);
+            T *frc = A.force + (size_t)b * (A.npad + A.nghost) * 3;
+            for (int j = sub; j < nn; j += G) {        // radial neighbours
+                T d[NMAX], s = T(0);
+                load_vec<T, NMAX>(dcache + (size_t)j * NMAX, d);
+#pragma unroll
+                for (int n = 0; n < NMAX; n++) s = fma(eqr[n], d[n], s);
+                if (s != T(0)) {
+                    const T x = rc[3 * j], y = rc[3 * j + 1], z = rc[3 * j + 2];
+                    const T gx = s * x, gy = s * y, gz = s * z;
+                    fx += gx; fy += gy; fz += gz;
+                    add3(frc + 3 * (size_t)fn[j], -gx, -gy, -gz);
+                    add_virial(gx, gy, gz, x, y, z);
+                }
+            }
+            __syncwarp();
+            T f4[4] = {fx, fy, fz, T(0)};
+            const T s = group_xreduce<T, 4, G>(f4, lane);
+            const int k = sub / (G / 4);
+            if (valid && sub % (G / 4) == 0 && k < 3) atomicAdd(frc + 3 * ci + k, s);
         }
+        e_acc += e_at;
+        if (mixed) {      // per group, straight to the outputs
+            T r[10];
+            r[0] = e_acc;
+#pragma unroll
+            for (int k = 0; k < 9; k++) r[1 + k] = vir[k];
+#pragma unroll
+            for (int k = 0; k < (MODE == NEP_EFV ? 10 : 1); k++) {
+#pragma unroll
+                for (int o = G / 2; o >= 1; o >>= 1) r[k] += __shfl_xor_sync(FULL_MASK, r[k], o);
+                if (valid && sub == 0) atomicAdd(k == 0 ? A.etot + b : A.virial + 9 * b + k - 1, r[k]);
+            }
+            e_acc = T(0);
+#pragma unroll
+            for (int k = 0; k < 9; k++) vir[k] = T(0);
+        }
+        __syncwarp();     // the cached derivatives and lists are rewritten by the next atoms
         }   // MODE != NEP_DESC
     }
 
-    // energy / virial: groups whose atoms belong to the structure of the block's first group
-    // combine in shared memory, the others add to the outputs directly
+    // energy / virial: warps whose atoms belong to the structure of the block's first warp combine in shared memory, the
+    // others add to the outputs directly
     if (NET) {
         if (threadIdx.x == 0) blk_b = bcur;
         if (threadIdx.x < 10) blk_acc[threadIdx.x] = T(0);
         __syncthreads();
         if (bcur >= 0) {
-            const bool local = bcur == blk_b;
-            e_acc = group_sum(e_acc, gmask);
-            if (sub == 0) atomicAdd(local ? &blk_acc[0] : A.etot + bcur, e_acc);
-            if (MODE == NEP_EFV) {
-#pragma unroll
-                for (int k = 0; k < 9; k++) {
-                    const T v = group_sum(vir[k], gmask);
-                    if (sub == 0) atomicAdd(local ? &blk_acc[1 + k] : A.virial + 9 * bcur + k, v);
-                }
-            }
+            if (bcur == blk_b) flush_to(bcur, &blk_acc[0], &blk_acc[1]);
+            else flush_to(bcur, A.etot + bcur, A.virial + 9 * bcur);
         }
         __syncthreads();
         if (threadIdx.x < 10 && blk_b >= 0) {

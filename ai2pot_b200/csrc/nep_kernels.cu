@@ -40,6 +40,7 @@ struct NepArgs {
     const int *prefix;
     int B, npad, ntypes, umax, nghost, cs, n_r, n_a, l_max, nneu, nd, nS;
     T rc_r, rc_a;
+    int zero = 0;          // the outputs are zeroed before anything is added to them
 };
 
 // 3-body coefficients as the reference stores them: double literals, some written with an `f`
@@ -97,6 +98,8 @@ __device__ __forceinline__ void nep_acc(const T (&e)[N], T v, T (&acc)[N])
 }
 template <typename T, int N>
 __device__ __forceinline__ void nep_acc(const T (&)[N], NepZero, T (&)[N]) {}
+template <typename T> __device__ __forceinline__ void nep_acc1(T e, T v, T &acc) { acc = fma(e, v, acc); }
+template <typename T> __device__ __forceinline__ void nep_acc1(T, NepZero, T &) {}
 
 // Harmonic polynomials b[l*l-1+m] (l = 1..4) at (x,y,z) and their Cartesian gradients (closed
 // forms tabulated in nep_utilities.h:100-383), as a list X(index, value, d/dx, d/dy, d/dz) over
@@ -523,88 +526,116 @@ __global__ void __launch_bounds__(NEP_WARPS * 32) nep_atom_kernel(const NepArgs<
 namespace ai2b {
 
 // ---------------------------------------------------------------------------------------------
+// scratch of the general kernel: atom offsets, padded radial coefficients
+static size_t nep_prefix_bytes(int B) { return (((size_t)(B > 0 ? B : 0) + 1) * sizeof(int) + 255) & ~size_t(255); }
+static size_t nep_ws_min(int B, int ntypes, int n_r, int n_a, int csp, size_t elem)
+{
+    return nep_prefix_bytes(B) + (((size_t)ntypes * ntypes * (n_r + n_a) * csp * elem + 255) & ~size_t(255));
+}
+// what a caller is asked for: also room for the specialised kernel's model table
+constexpr size_t NEP_TAB_BYTES = 96 * 1024;
+constexpr size_t NEP_FAST_SMEM = 110 * 1024;      // two blocks per SM at least
 static size_t nep_ws_bytes(int B, int ntypes, int n_r, int n_a, int csp, size_t elem)
 {
-    size_t pre = (((size_t)(B > 0 ? B : 0) + 1) * sizeof(int) + 255) & ~size_t(255);
-    size_t co = ((size_t)ntypes * ntypes * (n_r + n_a) * csp * elem + 255) & ~size_t(255);
-    return pre + co;
+    return std::max(nep_ws_min(B, ntypes, n_r, n_a, csp, elem), nep_prefix_bytes(B) + NEP_TAB_BYTES);
 }
 
-static int nep_grid(const void *kern, size_t smem, int B, int npad, long *blocks)
+template <typename T, int MODE, int NMAX, int G>
+static int launch_nep_fast_g(const NepArgs<T> &A, const T *tab, size_t tab_elems, cudaStream_t st, bool *done)
 {
-    int sms = 148, dev = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    AI2B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NEP_WARPS * 32, smem));
-    if (per_sm < 1) per_sm = 1;
-    *blocks = (long)sms * per_sm;
-    const long need_blocks = ((long)B * npad + NEP_APB - 1) / NEP_APB;
-    if (*blocks > need_blocks) *blocks = need_blocks;
-    return AI2B_OK;
-}
-
-// Specialised kernel for n_radial, n_angular <= NMAX. *done = false if the model's tables or the
-// neighbour width do not fit its shared-memory plan (the general kernel then runs).
-template <typename T, int CSP, int MODE, int NMAX>
-static int launch_nep_fast(const NepArgs<T> &A, const T *coeffs, cudaStream_t st, bool *done)
-{
-    constexpr int MINB = sizeof(T) == 4 ? 4 : 2;
     constexpr bool NET = MODE != NEP_DESC;
+    constexpr int MINB = sizeof(T) == 4 ? 4 : 2;
     *done = false;
-    if (A.ntypes > 16 || A.nneu > 256 || A.umax > 1024) return AI2B_OK;
-    const size_t smem = ((size_t)nep_fast_table_elems<NMAX, CSP>(A.ntypes, A.nneu, NET) +
-                         (size_t)NEP_APB * nep_fast_atom_elems<NMAX>(A.nneu, A.umax, NET)) * sizeof(T) +
-                        (size_t)NEP_APB * A.umax * sizeof(unsigned short) + 16;
-    if (smem > 96 * 1024) return AI2B_OK;
-    auto kern = nep_fast_kernel<T, CSP, MODE, NMAX, MINB>;
+    const size_t smem = (tab_elems + (size_t)NEP_WARPS * nep_fast_warp_elems<NMAX, G>(A.nneu, A.umax, NET)) * sizeof(T) +
+                        (size_t)NEP_WARPS * (32 / G) * A.umax * sizeof(unsigned short) + 16;
+    if (smem > NEP_FAST_SMEM) return AI2B_OK;
+    auto kern = nep_fast_kernel<T, G, MODE, NMAX, MINB>;
     static KernelSetup setup;
-    if (int rc = kernel_setup(setup, kern, smem)) return rc;
-    long blocks = 0;
-    int rc = nep_grid((const void *)kern, smem, A.B, A.npad, &blocks);
-    if (rc != AI2B_OK) return rc;
-    AI2B_CUDA(launch_chained(kern, (unsigned)blocks, NEP_WARPS * 32, smem, st, A, coeffs));
+    int per_sm = 1;
+    if (int rc = kernel_setup(setup, kern, smem, NEP_WARPS * 32, &per_sm)) return rc;
+    long blocks = ((long)A.B * A.npad * G + NEP_WARPS * 32 - 1) / (NEP_WARPS * 32);
+    const long room = (long)sm_count() * per_sm;
+    // the next kernel of the chain may move in early only where this one leaves room for it
+    const int early = blocks * 2 <= room;
+    if (blocks > room) blocks = room;
+    AI2B_CUDA(launch_chained(kern, (unsigned)blocks, NEP_WARPS * 32, smem, st, A, tab, early));
     *done = true;
     return AI2B_OK;
+}
+
+// Specialised kernel for n_radial, n_angular <= NMAX. *done = false if the model's tables, the neighbour width or the
+// workspace do not fit its plan (the general kernel then runs).
+template <typename T, int MODE, int NMAX>
+static int launch_nep_fast(NepArgs<T> A, const T *coeffs, void *ws, size_t ws_bytes, cudaStream_t st, bool *done)
+{
+    constexpr bool NET = MODE != NEP_DESC;
+    *done = false;
+    if (A.ntypes > 16 || A.umax > 1024 || (long)A.B * A.npad >= (1L << 31)) return AI2B_OK;
+    const NepTab<NMAX> L(A.ntypes, A.nneu, NET);
+    const size_t tab_bytes = (size_t)L.total * sizeof(T);
+    if (tab_bytes > NEP_TAB_BYTES || nep_prefix_bytes(A.B) + tab_bytes > ws_bytes) return AI2B_OK;
+    T *tab = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(ws) + nep_prefix_bytes(A.B));
+    auto fits = [&](int lanes) {
+        const int warp = lanes == 32 ? nep_fast_warp_elems<NMAX, 32>(A.nneu, A.umax, NET) : nep_fast_warp_elems<NMAX, 8>(A.nneu, A.umax, NET);
+        return tab_bytes + (size_t)NEP_WARPS * warp * sizeof(T) + (size_t)NEP_WARPS * (32 / lanes) * A.umax * 2 + 16 <= NEP_FAST_SMEM;
+    };
+    if (!fits(32)) return AI2B_OK;
+    {   // table, offsets, zeroed outputs
+        T *z[3] = {NET ? A.etot : A.desc, A.force, A.virial};
+        const size_t nz[3] = {NET ? (size_t)A.B : (size_t)A.B * A.npad * A.nd, NET ? 3 * (size_t)A.B * (A.npad + A.nghost) : 0, A.virial ? 9 * (size_t)A.B : 0};
+        const size_t nzero = A.zero ? nz[0] + nz[1] + nz[2] : 0;
+        size_t zb = (nzero + 4 * 256 - 1) / (4 * 256);
+        if (zb > 4096) zb = 4096;
+        const int tb = (L.total + 4 * 256 - 1) / (4 * 256);
+        AI2B_CUDA(launch_chained(nep_prep_kernel<T, NMAX>, (unsigned)(tb + zb), 256, 0, st, A, coeffs, tab, const_cast<int *>(A.prefix), NET ? 1 : 0, tb,
+                                 z[0], A.zero ? nz[0] : 0, z[1], A.zero ? nz[1] : 0, z[2], A.zero ? nz[2] : 0));
+    }
+    const long atoms = (long)A.B * A.npad;
+    // Lanes per atom. Few atoms: more lanes, the chip is filled by atoms x lanes. Whole call in us, fp32, 29 / 6.5 neighbours
+    // (in brackets eight lanes per atom and a trip count per group):
+    //   216 atoms: 32 lanes 9.8, 16 lanes 10.6 [20.2];   1,157: 12.6, 12.2 [20.3];   4,000: 16 lanes 14.7, 8 lanes 18.1 [24.5];
+    //   13,824: 16 lanes 30.5, 8 lanes 30.0 [48.7];   60,000: 8 lanes 80, 4 lanes 110 [176]
+    // Four lanes pay when the rows are short enough for four blocks per SM and angular neighbours are few (17 / 2.2
+    // neighbours, 1,048,576 atoms: 945, eight lanes 1083 [1435]); narrow rows stand for that.
+    if constexpr (NET && NMAX == 4 && sizeof(T) == 4)
+        if (atoms >= 50000 && A.umax <= 32) return launch_nep_fast_g<T, MODE, NMAX, 4>(A, tab, L.total, st, done);
+    if (atoms <= (NET ? 1000 : 4000) || !fits(8)) return launch_nep_fast_g<T, MODE, NMAX, 32>(A, tab, L.total, st, done);
+    if constexpr (NET)
+        if (atoms <= 6000) return launch_nep_fast_g<T, MODE, NMAX, 16>(A, tab, L.total, st, done);
+    return launch_nep_fast_g<T, MODE, NMAX, 8>(A, tab, L.total, st, done);
 }
 
 template <typename T, int CSP, int MODE>
 static int launch_nep_csp(NepArgs<T> A, const T *coeffs, void *ws, size_t ws_bytes, cudaStream_t st)
 {
-    const size_t need = nep_ws_bytes(A.B, A.ntypes, A.n_r, A.n_a, CSP, sizeof(T));
+    const size_t need = nep_ws_min(A.B, A.ntypes, A.n_r, A.n_a, CSP, sizeof(T));
     AI2B_REQUIRE(ws && ws_bytes >= need, AI2B_ERR_WORKSPACE, "NEP workspace too small: %zu < %zu bytes", ws_bytes, need);
     int *prefix = reinterpret_cast<int *>(ws);
-    T *cpad = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(ws) + ((((size_t)A.B + 1) * sizeof(int) + 255) & ~size_t(255)));
+    T *cpad = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(ws) + nep_prefix_bytes(A.B));
     A.prefix = prefix;
     A.coeffs_pad = cpad;
-    bool have_prefix = false;
     if constexpr (CSP == 8) {
         if (A.n_r <= 8 && A.n_a <= 8) {
-            // the specialised kernel reads the atom offsets only for batches of several structures
-            if (A.B > 1) {
-                nep_prefix_kernel<<<1, 32, 0, st>>>(A.binum, A.B, prefix);
-                have_prefix = true;
-            }
             bool done = false;
-            int rc = (A.n_r <= 4 && A.n_a <= 4) ? launch_nep_fast<T, CSP, MODE, 4>(A, coeffs, st, &done)
-                                                : launch_nep_fast<T, CSP, MODE, 8>(A, coeffs, st, &done);
+            int rc = (A.n_r <= 4 && A.n_a <= 4) ? launch_nep_fast<T, MODE, 4>(A, coeffs, ws, ws_bytes, st, &done)
+                                                : launch_nep_fast<T, MODE, 8>(A, coeffs, ws, ws_bytes, st, &done);
             if (rc != AI2B_OK || done) return rc;
         }
     }
-    if (!have_prefix) nep_prefix_kernel<<<1, 32, 0, st>>>(A.binum, A.B, prefix);
+    if (A.zero)
+        if (int rc = nep_zero_outputs<T>(MODE == NEP_DESC ? A.desc : A.etot, MODE == NEP_DESC ? (size_t)A.B * A.npad * A.nd : (size_t)A.B, A.force,
+                                         MODE == NEP_DESC ? 0 : 3 * (size_t)A.B * (A.npad + A.nghost), A.virial, A.virial ? 9 * (size_t)A.B : 0, st))
+            return rc;
+    nep_prefix_kernel<<<1, 32, 0, st>>>(A.binum, A.B, prefix);
     const int rows = A.ntypes * A.ntypes * (A.n_r + A.n_a);
     nep_pad_coeffs_kernel<T><<<(rows * CSP + 255) / 256, 256, 0, st>>>(coeffs, cpad, rows, A.cs, CSP);
     const size_t smem = (size_t)NEP_APB * (nep_atom_elems(A.nd, A.nS, A.nneu) * sizeof(T) + (size_t)A.umax * sizeof(unsigned short)) + 16;
     AI2B_REQUIRE(smem <= 200 * 1024, AI2B_ERR_UNSUPPORTED, "NEP model/umax need %zu bytes of shared memory per block", smem);
     auto kern = nep_atom_kernel<T, CSP, MODE>;
     static KernelSetup setup;
-    if (int rc = kernel_setup(setup, kern, smem)) return rc;
-    int sms = 148, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int per_sm = 0;
-    AI2B_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NEP_WARPS * 32, smem));
-    if (per_sm < 1) per_sm = 1;
-    long blocks = (long)sms * per_sm;
+    int per_sm = 1;
+    if (int rc = kernel_setup(setup, kern, smem, NEP_WARPS * 32, &per_sm)) return rc;
+    long blocks = (long)sm_count() * per_sm;
     const long need_blocks = ((long)A.B * A.npad + NEP_APB - 1) / NEP_APB;
     if (blocks > need_blocks) blocks = need_blocks;
     kern<<<(unsigned)blocks, NEP_WARPS * 32, smem, st>>>(A);
@@ -619,9 +650,12 @@ static int launch_nep(NepArgs<T> A, const T *coeffs, void *ws, size_t ws_bytes, 
     AI2B_REQUIRE(A.l_max >= 0 && A.l_max <= 4, AI2B_ERR_INVALID, "l_max %d outside 0..4", A.l_max);
     AI2B_REQUIRE(A.n_r >= 0 && A.n_a >= 0 && A.n_r + A.n_a > 0 && A.nneu >= 1 && A.ntypes >= 1, AI2B_ERR_INVALID, "bad NEP sizes");
     AI2B_REQUIRE(A.B >= 0 && A.npad >= 0 && A.umax >= 0 && A.umax < 65536 && A.nghost >= 0, AI2B_ERR_INVALID, "bad batch sizes");
-    if (A.B == 0 || A.npad == 0) return AI2B_OK;
+    if (A.B == 0) return AI2B_OK;
     A.nd = A.l_max == 0 ? A.n_r : A.n_r + A.n_a * A.l_max;
     A.nS = A.l_max == 0 ? 0 : A.n_a * (A.l_max * A.l_max + 2 * A.l_max);
+    if (A.npad == 0)      // no atoms: nothing but the outputs
+        return A.zero && MODE != NEP_DESC ? nep_zero_outputs<T>(A.etot, (size_t)A.B, A.force, 3 * (size_t)A.B * A.nghost, A.virial, A.virial ? 9 * (size_t)A.B : 0, st)
+                                          : AI2B_OK;
     if (A.cs <= 8) return launch_nep_csp<T, 8, MODE>(A, coeffs, ws, ws_bytes, st);
     return launch_nep_csp<T, 16, MODE>(A, coeffs, ws, ws_bytes, st);
 }
@@ -646,13 +680,9 @@ extern "C" size_t ai2b_nep_workspace_bytes(int batch_size, int ntypes, int n_rad
         AI2B_REQUIRE(etot && force && coeffs && w0 && b0 && w1 && bias && qs && binum && bilist && numneigh &&  \
                          firstneigh && rcs && types, AI2B_ERR_INVALID, "ai2b_nep_efv: NULL argument");          \
         cudaStream_t st = (cudaStream_t)stream;                                                                 \
-        if (zero && B > 0 && npad >= 0) {                                                                       \
-            if (int rc = nep_zero_outputs<T>(etot, (size_t)B, force, 3 * (size_t)B * (npad + nghost), virial,   \
-                                             virial ? 9 * (size_t)B : 0, st)) return rc;                        \
-        }                                                                                                       \
         NepArgs<T> A{etot, force, virial, nullptr, nullptr, w0, b0, w1, bias, qs, binum, bilist, numneigh,      \
                      firstneigh, types, rcs, nullptr, B, npad, ntypes, umax, nghost, cs, n_r, n_a, l_max, nneu, \
-                     0, 0, rc_r, rc_a};                                                                         \
+                     0, 0, rc_r, rc_a, zero ? 1 : 0};                                                           \
         return virial ? launch_nep<T, NEP_EFV>(A, coeffs, ws, ws_bytes, st)                                     \
                       : launch_nep<T, NEP_EF>(A, coeffs, ws, ws_bytes, st);                                     \
     }                                                                                                           \
@@ -687,11 +717,9 @@ extern "C" size_t ai2b_nep_workspace_bytes(int batch_size, int ntypes, int n_rad
         AI2B_REQUIRE(desc && coeffs && binum && bilist && numneigh && firstneigh && rcs && types,               \
                      AI2B_ERR_INVALID, "ai2b_nep_descriptors: NULL argument");                                  \
         cudaStream_t st = (cudaStream_t)stream;                                                                 \
-        const int nd = l_max == 0 ? n_r : n_r + n_a * l_max;                                                    \
-        if (B > 0 && npad > 0) AI2B_CUDA(cudaMemsetAsync(desc, 0, sizeof(T) * (size_t)B * npad * nd, st));      \
         NepArgs<T> A{nullptr, nullptr, nullptr, desc, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,     \
                      binum, bilist, numneigh, firstneigh, types, rcs, nullptr, B, npad, ntypes, umax, nghost,   \
-                     cs, n_r, n_a, l_max, 1, 0, 0, rc_r, rc_a};                                                 \
+                     cs, n_r, n_a, l_max, 1, 0, 0, rc_r, rc_a, 1};                                              \
         return launch_nep<T, NEP_DESC>(A, coeffs, ws, ws_bytes, st);                                            \
     }
 
@@ -758,7 +786,7 @@ extern "C" int ai2b_nep_efv_static_scratch_f32(float *etot, float *force, float 
                  AI2B_ERR_INVALID, "ai2b_nep_efv_static_scratch_f32: NULL argument");
     AI2B_REQUIRE(B >= 0 && ntypes >= 1 && n_r >= 0 && n_a >= 0 && cs >= 1 && cs <= 16, AI2B_ERR_INVALID,
                  "ai2b_nep_efv_static_scratch_f32: bad sizes");
-    const size_t need = nep_ws_bytes(B, ntypes, n_r, n_a, cs <= 8 ? 8 : 16, sizeof(float));
+    const size_t need = nep_ws_min(B, ntypes, n_r, n_a, cs <= 8 ? 8 : 16, sizeof(float));
     AI2B_REQUIRE(need <= NEP_STATIC_SCRATCH_BYTES, AI2B_ERR_WORKSPACE,
                  "ai2b_nep_efv_static_scratch_f32: this batch/model needs %zu bytes of scratch, the built-in array holds %zu; "
                  "use ai2b_nep_efv_f32 with a caller-owned workspace",
@@ -773,13 +801,9 @@ extern "C" int ai2b_nep_efv_static_scratch_f32(float *etot, float *force, float 
         scratch_of_device[dev] = p;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    if (B > 0 && npad >= 0) {
-        if (int rc = nep_zero_outputs<float>(etot, (size_t)B, force, 3 * (size_t)B * (npad + nghost), virial,
-                                             virial ? 9 * (size_t)B : 0, st)) return rc;
-    }
     NepArgs<float> A{etot, force, virial, nullptr, nullptr, w0, b0, w1, bias, qs, binum, bilist, numneigh,
                      firstneigh, types, rcs, nullptr, B, npad, ntypes, umax, nghost, cs, n_r, n_a, l_max, nneu,
-                     0, 0, rc_r, rc_a};
+                     0, 0, rc_r, rc_a, 1};
     return virial ? launch_nep<float, NEP_EFV>(A, coeffs, scratch_of_device[dev], NEP_STATIC_SCRATCH_BYTES, st)
                   : launch_nep<float, NEP_EF>(A, coeffs, scratch_of_device[dev], NEP_STATIC_SCRATCH_BYTES, st);
 }

@@ -191,3 +191,59 @@ def test_g4_full_size_properties():
     e2, f2, v2 = ev.compute(coords + shift)
     assert abs(float(e2) - float(e)) < 2e-5 * abs(float(e))
     assert float((f2 - f).abs().max()) < 1e-3 * fs                                     # fp32 positions at |x| ~ 400 A move rcs by ~3e-5 A
+
+
+def _f64(model):
+    return util.to64(model)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n,model_kw,umax", [
+    (5, dict(rmax_angular=5.5), 96),                                         # 125 atoms, 32 lanes each; many angular neighbours
+    (11, dict(), 64),                                                        # 1,331 atoms, 16 lanes each
+    (11, dict(n_radial=8, n_angular=7, num_neurons=33, rmax_angular=5.5), 64),
+    (11, dict(n_radial=3, n_angular=1, l_max=2, chebyshev_size=5, num_neurons=7), 64),
+    (19, dict(rmax_angular=5.5), 64),                                        # 6,859 atoms, 8 lanes each: more angular neighbours than one step holds
+    (19, dict(l_max=0, num_neurons=64), 64),                                 # no angular part
+    (37, dict(rmax_radial=5.0), 32),                                         # 50,653 atoms in narrow rows: 4 lanes each (fp32)
+])
+def test_lanes_per_atom_forms(checkers, dt, n, model_kw, umax):
+    chk = _chk(checkers)
+    rng = np.random.default_rng(n)
+    cell, pos = synth.cubic_lattice(n, 3.0, 0.1, rng, dt)
+    types = rng.integers(0, 3, len(pos)).astype(np.int32)
+    model = synth.nep_model(3, rng, dt, **model_kw)
+    model["type_bias"] = rng.normal(0, 0.1, 3).astype(dt)
+    model["q_scaler"] = rng.uniform(0.5, 1.5, len(model["q_scaler"])).astype(dt)
+    nb0 = capi.NeighborBuilder()
+    nn, fn, rc, st = (t.cpu().numpy() for t in nb0.build(cell, torch.from_numpy(pos).cuda(), model["rmax_radial"], umax))
+    assert st[1] == 0
+    nb = synth.batch_from_nblist(nn, fn, rc, types, 3)
+    got, *_ = _run(model, nb)
+    nb64 = dict(nb, brcs=nb["brcs"].astype(np.float64))
+    want = chk.nep_efv(_f64(model), nb64)
+    for a, b, name in zip(got, want, ("energy", "force", "virial")):
+        assert util.relerr(a, b) < (1e-10 if dt == np.float64 else 1e-5), name
+    ef, *_ = _run(model, nb, virial=False)
+    assert util.relerr(ef[1], want[1]) < (1e-10 if dt == np.float64 else 1e-5)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("B,nmin,nmax", [(40, 1, 9), (50, 100, 130)])
+def test_ragged_batch_warps_across_structures(checkers, dt, B, nmin, nmax):
+    """Structures much smaller than, and no multiple of, the atoms a warp takes: energies and virials stay apart."""
+    chk = _chk(checkers)
+    rng = np.random.default_rng(B)
+    model = synth.nep_model(3, rng, dt)
+    lists = []
+    for _ in range(B):
+        n = int(rng.integers(nmin, nmax + 1))
+        edge = int(np.ceil(n ** (1 / 3) - 1e-9))
+        cell, pos = synth.cubic_lattice(edge, 3.2, 0.15, rng, dt, nocc=n)
+        types = rng.integers(0, 3, n).astype(np.int32)
+        lists.append(chk.nblist(cell, types, pos, 6.0, 64)[:4])
+    nb = synth.pad_batch(lists, 3, 64)
+    got, *_ = _run(model, nb)
+    want = chk.nep_efv(_f64(model), dict(nb, brcs=nb["brcs"].astype(np.float64)))
+    for a, b, name in zip(got, want, ("energy", "force", "virial")):
+        assert util.relerr(a, b) < (1e-10 if dt == np.float64 else 1e-5), name
