@@ -32,6 +32,7 @@ def lib():
         _lib.ai2b_nblist_workspace_bytes.restype = C.c_size_t
         _lib.ai2b_nep_workspace_bytes.restype = C.c_size_t
         _lib.ai2b_mtp_loss_workspace_bytes.restype = C.c_size_t
+        _lib.ai2b_evaluate.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
     return _lib
 
 
@@ -50,8 +51,38 @@ def _ptr(t):
     return C.c_void_p(t.data_ptr())
 
 
+def raw_stream(device_index):
+    """Address of the current stream of a device (what torch.cuda.current_stream() wraps)."""
+    return torch._C._cuda_getCurrentRawStream(device_index)
+
+
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(raw_stream(torch.cuda.current_device()))
+
+
+class Evaluation(C.Structure):
+    """ai2b_evaluation: one structure, one model, as ai2b_evaluate() takes them."""
+    _fields_ = ([(k, C.c_int) for k in ("is_f64", "natoms", "umax", "ntypes")] + [("cell", C.c_double * 9), ("rcut", C.c_double), ("mtp", C.c_void_p)] +
+                [(k, C.c_int) for k in ("chebyshev_size", "n_radial", "n_angular", "l_max", "num_neurons")] +
+                [(k, C.c_double) for k in ("scaling", "rmax", "rmin", "rmax_angular")] +
+                [(k, C.c_void_p) for k in ("d_coeffs", "d_linear_coeffs", "d_w0", "d_b0", "d_w1", "d_type_bias", "d_q_scaler", "d_binum", "d_ilist",
+                                           "d_types", "d_numneigh", "d_firstneigh", "d_status", "d_rcs", "d_etot", "d_force", "d_virial",
+                                           "d_nblist_workspace")] +
+                [("nblist_workspace_bytes", C.c_size_t), ("d_workspace", C.c_void_p), ("workspace_bytes", C.c_size_t)])
+
+
+CHAINED_COPY_BYTES = 1 << 20    # up to here a kernel of the chain beats the copy engine's hand-over
+
+
+def copy_around_call(dst, src):
+    """dst.copy_(src) on the current stream; between device and pinned host memory, small contiguous copies go through
+    ai2b_chained_copy."""
+    n = dst.numel() * dst.element_size()
+    if (n <= CHAINED_COPY_BYTES and dst.dtype == src.dtype and dst.shape == src.shape and dst.is_contiguous() and src.is_contiguous()
+            and all(t.is_cuda or t.is_pinned() for t in (dst, src))):
+        _check(lib().ai2b_chained_copy(C.c_void_p(dst.data_ptr()), C.c_void_p(src.data_ptr()), C.c_size_t(n), _stream()))
+    else:
+        dst.copy_(src, non_blocking=True)
 
 
 def _suf(dtype):

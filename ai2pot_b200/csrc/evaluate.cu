@@ -1,0 +1,78 @@
+// One structure, one model: positions -> neighbour list -> energy, forces, virial in one host call.
+//
+// The reference's calculators assemble the list and the model's arguments on the host for every call
+// (ai2pot/models/potential_utils.py:217-268). Here everything but the positions is described once; a call then is
+// the neighbour build and the evaluation back to back, with no argument handling in between: at a few hundred atoms
+// the host's share of a call through two separate entry points (50 us) exceeded the device's (31 us).
+#include "common.cuh"
+
+using namespace ai2b;
+
+template <typename T>
+static int evaluate_t(const ai2b_evaluation *e, const T *coords, void *stream)
+{
+    const int pbc[3] = {1, 1, 1};
+    T cell[9];
+    for (int k = 0; k < 9; k++) cell[k] = (T)e->cell[k];
+    int rc;
+    if constexpr (sizeof(T) == 8)
+        rc = ai2b_nblist_build_f64(e->natoms, cell, coords, 1, e->rcut, pbc, e->umax, e->d_numneigh, e->d_firstneigh, (T *)e->d_rcs, e->d_status,
+                                   e->d_nblist_workspace, e->nblist_workspace_bytes, stream);
+    else
+        rc = ai2b_nblist_build_f32(e->natoms, cell, coords, 1, e->rcut, pbc, e->umax, e->d_numneigh, e->d_firstneigh, (T *)e->d_rcs, e->d_status,
+                                   e->d_nblist_workspace, e->nblist_workspace_bytes, stream);
+    if (rc != AI2B_OK) return rc;
+    T *etot = (T *)e->d_etot, *force = (T *)e->d_force, *virial = (T *)e->d_virial;
+    const T *co = (const T *)e->d_coeffs, *bias = (const T *)e->d_type_bias, *qs = (const T *)e->d_q_scaler, *rcs = (const T *)e->d_rcs;
+    if (e->mtp) {
+        const T *lin = (const T *)e->d_linear_coeffs;
+        if constexpr (sizeof(T) == 8)
+            return ai2b_mtp_efv_f64(e->mtp, etot, force, virial, e->chebyshev_size, e->scaling, co, lin, bias, 1, e->natoms, e->d_binum, e->d_ilist,
+                                    e->d_numneigh, e->d_firstneigh, rcs, e->d_types, e->ntypes, e->umax, 0, e->rmax, e->rmin, qs, e->d_workspace,
+                                    e->workspace_bytes, stream);
+        else
+            return ai2b_mtp_efv_f32(e->mtp, etot, force, virial, e->chebyshev_size, (T)e->scaling, co, lin, bias, 1, e->natoms, e->d_binum, e->d_ilist,
+                                    e->d_numneigh, e->d_firstneigh, rcs, e->d_types, e->ntypes, e->umax, 0, (T)e->rmax, (T)e->rmin, qs,
+                                    e->d_workspace, e->workspace_bytes, stream);
+    }
+    const T *w0 = (const T *)e->d_w0, *b0 = (const T *)e->d_b0, *w1 = (const T *)e->d_w1;
+    if constexpr (sizeof(T) == 8)
+        return ai2b_nep_efv_f64(etot, force, virial, e->chebyshev_size, e->n_radial, e->n_angular, e->l_max, e->num_neurons, co, w0, b0, w1, bias, 1,
+                                e->natoms, e->d_binum, e->d_ilist, e->d_numneigh, e->d_firstneigh, rcs, e->d_types, e->ntypes, e->umax, 0, e->rmax,
+                                e->rmax_angular, qs, e->d_workspace, e->workspace_bytes, stream);
+    else
+        return ai2b_nep_efv_f32(etot, force, virial, e->chebyshev_size, e->n_radial, e->n_angular, e->l_max, e->num_neurons, co, w0, b0, w1, bias, 1,
+                                e->natoms, e->d_binum, e->d_ilist, e->d_numneigh, e->d_firstneigh, rcs, e->d_types, e->ntypes, e->umax, 0, (T)e->rmax,
+                                (T)e->rmax_angular, qs, e->d_workspace, e->workspace_bytes, stream);
+}
+
+extern "C" int ai2b_evaluate(const ai2b_evaluation *e, const void *d_coords, void *stream)
+{
+    AI2B_REQUIRE(e && (d_coords || e->natoms == 0), AI2B_ERR_INVALID, "ai2b_evaluate: NULL argument");
+    return e->is_f64 ? evaluate_t<double>(e, (const double *)d_coords, stream) : evaluate_t<float>(e, (const float *)d_coords, stream);
+}
+
+// Copy by a kernel that is part of the chain. Between two kernels a copy engine costs the hand-over there and back, several
+// microseconds for a few kilobytes; either side may be pinned host memory.
+__global__ void chained_copy_kernel(unsigned char *__restrict__ dst, const unsigned char *__restrict__ src, size_t bytes)
+{
+    chain_release();
+    chain_wait();
+    const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    size_t done = 0;
+    if (((reinterpret_cast<size_t>(dst) | reinterpret_cast<size_t>(src)) & 15) == 0) {
+        for (size_t i = i0; i < bytes / 16; i += step) reinterpret_cast<int4 *>(dst)[i] = reinterpret_cast<const int4 *>(src)[i];
+        done = bytes & ~size_t(15);
+    }
+    for (size_t i = done + i0; i < bytes; i += step) dst[i] = src[i];
+}
+
+extern "C" int ai2b_chained_copy(void *dst, const void *src, size_t bytes, void *stream)
+{
+    if (bytes == 0) return AI2B_OK;
+    AI2B_REQUIRE(dst && src, AI2B_ERR_INVALID, "ai2b_chained_copy: NULL argument");
+    size_t blocks = (bytes + 16 * 256 - 1) / (16 * 256);
+    if (blocks > 148) blocks = 148;
+    AI2B_CUDA(launch_chained(chained_copy_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, (unsigned char *)dst, (const unsigned char *)src, bytes));
+    return AI2B_OK;
+}

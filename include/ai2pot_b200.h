@@ -535,6 +535,34 @@ AI2B_DECL_PEER_EXCHANGE(f32, float)
 AI2B_DECL_PEER_RETURN(f64, double)
 AI2B_DECL_PEER_RETURN(f32, float)
 
+/* ------------------------------------------------------------------------------------------
+ * One structure, one model: neighbour list and energy / forces / virial in one call (what the
+ * reference's calculators do per call, ai2pot/models/potential_utils.py:217-268).
+ * Everything but the positions is described once; the pointed-to arrays stay the caller's.
+ * The cell is fully periodic. rmax is the radial cutoff of either kind of model.
+ * ---------------------------------------------------------------------------------------- */
+typedef struct ai2b_evaluation {
+    int is_f64, natoms, umax, ntypes;
+    double cell[9], rcut;
+    const ai2b_mtp_program *mtp;                       /* NULL: NEP */
+    int chebyshev_size, n_radial, n_angular, l_max, num_neurons;
+    double scaling, rmax, rmin, rmax_angular;
+    const void *d_coeffs, *d_linear_coeffs, *d_w0, *d_b0, *d_w1, *d_type_bias, *d_q_scaler;
+    const int *d_binum, *d_ilist, *d_types;            /* [1] = natoms, [natoms] = 0, 1, ..., [natoms] */
+    int *d_numneigh, *d_firstneigh, *d_status;         /* neighbour list of the call */
+    void *d_rcs;
+    void *d_etot, *d_force, *d_virial;                 /* results */
+    void *d_nblist_workspace;
+    size_t nblist_workspace_bytes;
+    void *d_workspace;
+    size_t workspace_bytes;
+} ai2b_evaluation;
+int ai2b_evaluate(const ai2b_evaluation *e, const void *d_coords, void *stream);
+
+/* dst[0..bytes) = src[0..bytes) by a kernel on `stream`; either pointer may be pinned host memory.
+ * Meant for the few kilobytes around a call, where handing over to a copy engine costs more than the copy. */
+int ai2b_chained_copy(void *dst, const void *src, size_t bytes, void *stream);
+
 #ifdef __cplusplus
 }
 #endif
