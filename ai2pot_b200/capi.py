@@ -6,6 +6,7 @@ no CPU implementation behind these calls: a missing library or a non-CUDA tensor
 """
 import ctypes as C
 import os
+import sys
 
 import numpy as np
 import torch
@@ -504,6 +505,9 @@ class MdSession:
 
     def __init__(self, model, umax, prog=None):
         self.h = C.c_void_p()
+        self._spare = []
+        self._out = np.zeros(7, np.float64)      # energy, six virial components of a step
+        self._out_p = (C.c_void_p(self._out.ctypes.data), C.c_void_p(self._out.ctypes.data + 8))
         f32 = lambda a: np.ascontiguousarray(np.asarray(a).ravel(), np.float32)
         hp = lambda a: a.ctypes.data_as(C.c_void_p)
         self.kind = model["kind"]
@@ -521,17 +525,28 @@ class MdSession:
                 C.c_int(int(model["ntypes"])), C.c_int(int(prog.nmus)), C.c_int(int(prog.ns)), *[hp(x) for x in a],
                 C.c_float(model["rmax"]), C.c_float(model["rmin"]), C.c_int(int(umax))))
 
+    def _force_array(self, n):
+        """An array for the forces of n atoms. Memory whose last array the caller has dropped is used again (two blocks at most,
+        returned with the session): fresh pages cost more than the forces themselves."""
+        for base in self._spare:
+            if base.shape[0] == n and sys.getrefcount(base) == 3:      # the list, the loop variable, the argument
+                return base.view()
+        base = np.empty((n, 3), np.float64)
+        self._spare = [base] + self._spare[:1]
+        return base.view()
+
     def compute(self, nlocal, nghost, x, model_type, want_virial=True):
         x = np.ascontiguousarray(x, np.float64)
         t = np.ascontiguousarray(model_type, np.int32)
-        f = np.zeros((nlocal + nghost, 3), np.float64)
-        e = C.c_double(0.0)
-        v = np.zeros(6, np.float64)
+        f = self._force_array(nlocal + nghost)
+        out = self._out
+        out[:] = 0.0
         mx = C.c_int(0)
-        _check(lib().ai2b_md_session_compute(self.h, C.c_int(nlocal), C.c_int(nghost), x.ctypes.data_as(C.c_void_p),
-                                             t.ctypes.data_as(C.c_void_p), C.c_int(int(want_virial)), f.ctypes.data_as(C.c_void_p),
-                                             C.byref(e), v.ctypes.data_as(C.c_void_p), C.byref(mx)))
-        return e.value, f, v, mx.value
+        rc = lib().ai2b_md_session_forces(self.h, C.c_int(nlocal), C.c_int(nghost), C.c_void_p(x.ctypes.data), C.c_void_p(t.ctypes.data),
+                                          C.c_int(int(want_virial)), C.c_void_p(f.ctypes.data), self._out_p[0], self._out_p[1], C.byref(mx))
+        if rc:
+            _check(rc)
+        return float(out[0]), f, out[1:7].copy(), mx.value
 
     def close(self):
         if self.h:

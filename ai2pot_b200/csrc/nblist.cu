@@ -1409,6 +1409,14 @@ static int nblist_build_batch(int B, int npad, const int *d_binum, const T *d_ce
     return AI2B_OK;
 }
 
+// rows in single precision from double positions; open_ext (optional): lowest and highest fractional coordinates
+int nblist_build_rows32(int n, int ncentres, const double *h_cell, const double *d_coords, double rcut, const int *h_pbc, const double *open_ext, int umax,
+                        int *d_numneigh, int *d_firstneigh, float *d_rcs, int *d_status, void *ws, size_t ws_bytes, cudaStream_t st)
+{
+    return nblist_build<double, float>(n, ncentres, h_cell, d_coords, 1, rcut, h_pbc, umax, d_numneigh, d_firstneigh, d_rcs, d_status, ws, ws_bytes, st, 0,
+                                       false, open_ext);
+}
+
 }  // namespace ai2b
 
 using namespace ai2b;

@@ -416,6 +416,10 @@ void ai2b_md_session_destroy(ai2b_md_session *session);
 int ai2b_md_session_compute(ai2b_md_session *session, int nlocal, int nghost, const double *h_x,
                             const int *h_model_type, int want_virial, double *h_f,
                             double *h_eng, double *h_virial6, int *h_max_neighbours);
+/* The same step, storing the forces instead of adding them (h_f need not be initialised). */
+int ai2b_md_session_forces(ai2b_md_session *session, int nlocal, int nghost, const double *h_x,
+                           const int *h_model_type, int want_virial, double *h_f,
+                           double *h_eng, double *h_virial6, int *h_max_neighbours);
 
 /* Neighbour rows in single precision from double-precision positions (r_j - r_i formed in
  * double, rounded once: pair_ai2pot.cpp:232-235); otherwise as ai2b_nblist_build_ghost_f64. */
