@@ -2,8 +2,8 @@
 //
 // Tables of the reference's template levels 6 to 16 (monomial degree <= 6, four radial functions at most):
 //   mtp_fwd_atoms_kernel    (mtp_atoms.cu) lanes = atoms, basic moments in registers -> Mb[tile][basic row][32 atoms]
-//   mtp_contract_seg_kernel lanes = atoms, one tile of 32 atoms per block at a time: the product rows and the adjoint
-//                           sweep run out of shared memory, every moment owned by one warp; site energies; adjoints
+//   mtp_contract_pair_kernel lanes = atoms, one tile of 32 atoms per block at a time: the product rows and the adjoint
+//                           sweep run out of shared memory, every moment owned by a group of lanes; site energies; adjoints
 //                           of the basic moments -> Eb[tile][dense monomial][32 atoms] (or the descriptors)
 //   mtp_force_atoms_kernel  (mtp_atoms.cu) lanes = atoms: polynomial of every radial function and its gradient per
 //                           neighbour; pair force g = f' P u + f/r (G - (u.G) u); F_i += g, F_j -= g, V -= g (x) r
@@ -14,7 +14,7 @@
 // tables while the kernel before it drains, then waits for it.
 //
 // Reference semantics: source/descriptor/mtpr/include/mtpBasis.h:400-534, linearMtp.h:190-352.
-#include "mtp_device.cuh"
+#include "mtp_pairs.cuh"
 #include <cuda_pipeline.h>
 
 namespace ai2b {
@@ -437,131 +437,52 @@ __global__ void __launch_bounds__(MTP_CWARPS * 32, 1) mtp_contract_kernel(const 
 }
 
 
-// ---- kernel B, segment form: lanes = atoms, one worker (warp) owns a moment ------------------------
-// The flat-stream kernel above spends ~30 instructions around the two FP64 instructions of a product row
-// (offset unpacking, multiplier conversion, flag test, shared-memory atomic flush). Here the tables are
-// compiled into segments (mtp_program.cuh): a header {moment, row count, multiplier} followed by rows of
-// two element offsets, every moment owned by one warp, so a row is one 8-byte broadcast load, two address
-// adds, two operand loads and one FMA, and a moment is finished with a plain store. Tiles of 32 atoms;
-// the workspace holds them tile by tile ([tile][row][32 atoms]; per-atom rows from the warp-per-atom forward
-// kernels are transposed on the way in and out, row stride 33 keeps those accesses spread over the banks),
-// the next tile's rows travelling in registers while the current tile is processed.
-// Shared memory: M[nm][33], E[nm][33] (not for descriptors), headers, rows, seeds, worker tables.
-constexpr int MTP_SEG_EWARPS = 8;   // warps that sum the site energies of a tile
+// ---- kernel B: products and adjoints out of shared memory (row loop: mtp_pairs.cuh) -----------------------
+// Tiles of 32 atoms, one block per SM walking over them; the next tile's rows travel in registers while the current tile is
+// processed. A moment is finished with a plain store by the group of lanes that owns it, so the result is the same bit for
+// bit from run to run. Shared memory: M[nm][32], E[nm][32] (not for descriptors), row records, adjoint seeds, small tables.
+constexpr int MTP_PAIR_EWARPS = 8;   // warps that sum the site energies of a tile
+template <typename T> constexpr int pair_gl() { return MTP_TILE * (int)sizeof(T) / 16; }      // lanes per row
 template <typename T>
-struct SegSmem {
+struct PairSmem {
     T *M, *E, *seed, *wsc;     // wsc[s] = lin[s] / q[s]; seed[m] = sum of wsc over the scalars mapped to moment m
-    int *mapo;                 // element offset of the moment of scalar s
-    T *ep;                     // [MTP_SEG_EWARPS][33] partial site energies
-    int *db;                   // [ndense] element offset of the basic moment of dense index d (-1: none)
-    int4 *hdr;
-    int2 *row;
-    int *wseg, *wrow;
+    T *ep;                     // [MTP_PAIR_EWARPS][32] partial site energies
+    int2 *row, *warp;
+    int *map, *db;             // moment of scalar s; basic moment of dense index d (-1: none)
 };
 template <typename T, int MODE>
-__host__ __device__ inline size_t seg_smem_layout(const MtpProgramDev &P, unsigned char *base, SegSmem<T> *out)
+__host__ __device__ inline size_t pair_smem_layout(const MtpProgramDev &P, unsigned char *base, PairSmem<T> *out)
 {
+    constexpr int K = pair_gl<T>() == 16 ? 0 : 1, G = 32 / pair_gl<T>();
     size_t o = 0;
     auto take = [&](size_t bytes) { size_t r = o; o += (bytes + 15) & ~size_t(15); return r; };
-    const size_t oM = take(sizeof(T) * (size_t)P.nm * MTP_SEG_LD);
-    const size_t oE = MODE == MODE_DESC ? oM : take(sizeof(T) * (size_t)P.nm * MTP_SEG_LD);
-    const size_t oh = take(sizeof(int4) * (size_t)P.nseg);
-    const size_t orow = take(sizeof(int2) * (size_t)P.nseg_rows);
+    const size_t oM = take(sizeof(T) * (size_t)P.nm * MTP_TILE);
+    const size_t oE = MODE == MODE_DESC ? oM : take(sizeof(T) * (size_t)P.nm * MTP_TILE);
+    const size_t orow = take(sizeof(int2) * (size_t)P.stream[K].nrows * G);
+    const size_t ow = take(sizeof(int2) * (size_t)(2 * P.nlev) * MTP_PAIR_WARPS);
     const size_t os = take(sizeof(T) * (size_t)P.nm);
     const size_t osc = take(sizeof(T) * (size_t)P.ns);
-    const size_t omo = take(sizeof(int) * (size_t)P.ns);
-    const size_t oep = take(MODE == MODE_DESC ? 0 : sizeof(T) * MTP_SEG_EWARPS * MTP_SEG_LD);
+    const size_t oep = take(MODE == MODE_DESC ? 0 : sizeof(T) * MTP_PAIR_EWARPS * MTP_TILE);
+    const size_t om = take(sizeof(int) * (size_t)P.ns);
     const size_t odb = take(MODE == MODE_DESC ? 0 : sizeof(int) * (size_t)P.ndense);
-    const size_t ow = take(sizeof(int) * (size_t)(2 * P.nlev) * (MTP_SEG_WORKERS + 1));
-    const size_t owr = take(sizeof(int) * (size_t)(2 * P.nlev) * MTP_SEG_WORKERS);
     if (out) {
         out->M = reinterpret_cast<T *>(base + oM); out->E = reinterpret_cast<T *>(base + oE);
-        out->hdr = reinterpret_cast<int4 *>(base + oh); out->row = reinterpret_cast<int2 *>(base + orow);
+        out->row = reinterpret_cast<int2 *>(base + orow); out->warp = reinterpret_cast<int2 *>(base + ow);
         out->seed = reinterpret_cast<T *>(base + os); out->wsc = reinterpret_cast<T *>(base + osc);
-        out->wseg = reinterpret_cast<int *>(base + ow); out->wrow = reinterpret_cast<int *>(base + owr);
-        out->mapo = reinterpret_cast<int *>(base + omo);
         out->ep = reinterpret_cast<T *>(base + oep);
-        out->db = reinterpret_cast<int *>(base + odb);
+        out->map = reinterpret_cast<int *>(base + om); out->db = reinterpret_cast<int *>(base + odb);
     }
     return o;
 }
-
-// Shared-memory accesses of the row loop, by 32-bit shared-window address (explicit ld.shared / st.shared: the
-// loop is bound by instruction issue and shared-memory bandwidth, so it must not fall back to generic addressing).
-__device__ __forceinline__ int2 lds_int2(unsigned a)
-{
-    int2 v;
-    asm volatile("ld.shared.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ int4 lds_int4(unsigned a)
-{
-    int4 v;
-    asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ double lds_val(unsigned a, double)
-{
-    double v;
-    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ float lds_val(unsigned a, float)
-{
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ void sts_val(unsigned a, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
-__device__ __forceinline__ void sts_val(unsigned a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
-
-// one phase for one worker. xl, yl = shared addresses of this lane's column of the arrays a row's first / second
-// offset refers to, dl = of the destination array; hdr, row, seed = shared addresses of the tables
-template <typename T, bool SEEDED>
-__device__ __forceinline__ void seg_phase(int h, int hend, unsigned hdr, unsigned rp, unsigned seed, unsigned xl, unsigned yl, unsigned dl)
-{
-    constexpr unsigned ES = (unsigned)sizeof(T);
-    T dsum = T(0);
-    for (; h < hend; h++) {
-        // a worker's rows follow one another across its segments, so the first two row records are requested together
-        // with the header (they are simply not used if the segment is shorter), and inside a segment the next pair is
-        // requested before the current pair's products are formed
-        const int4 hd = lds_int4(hdr + 16u * (unsigned)h);
-        int2 r0 = lds_int2(rp), r1 = lds_int2(rp + 8u);
-        const int n = hd.y & 0x3fffffff;
-        T acc0 = T(0), acc1 = T(0);
-        const unsigned rend = rp + 8u * (unsigned)n;
-#pragma unroll 1
-        while (rp + 8u < rend) {
-            const T x0 = lds_val(xl + (unsigned)r0.x * ES, T()), y0 = lds_val(yl + (unsigned)r0.y * ES, T());
-            const T x1 = lds_val(xl + (unsigned)r1.x * ES, T()), y1 = lds_val(yl + (unsigned)r1.y * ES, T());
-            rp += 16u;
-            r0 = lds_int2(rp); r1 = lds_int2(rp + 8u);
-            acc0 = fma(x0, y0, acc0);
-            acc1 = fma(x1, y1, acc1);
-        }
-        if (rp < rend) {
-            acc0 = fma(lds_val(xl + (unsigned)r0.x * ES, T()), lds_val(yl + (unsigned)r0.y * ES, T()), acc0);
-            rp += 8u;
-        }
-        const T mult = (T)__hiloint2double(hd.w, hd.z);
-        const T acc = acc0 + acc1;
-        dsum = (hd.y & (1 << 30)) ? mult * acc : fma(mult, acc, dsum);
-        if (hd.y < 0) {                                  // bit 31: last segment of the moment
-            T out = dsum;
-            if (SEEDED) out += lds_val(seed + (unsigned)(hd.x / MTP_SEG_LD) * ES, T());
-            sts_val(dl + (unsigned)hd.x * ES, out);
-        }
-    }
-}
+template <typename T> static bool pair_fits(const MtpProgramDev &P, size_t smem) { return P.stream[pair_gl<T>() == 16 ? 0 : 1].nrows > 0 && smem <= 226 * 1024; }
 
 template <typename T, int MODE>
-__global__ void __launch_bounds__(MTP_SEG_WORKERS * 32, 1) mtp_contract_seg_kernel(const MtpProgramDev P, const MtpArgs<T> A)
+__global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_contract_pair_kernel(const MtpProgramDev P, const MtpArgs<T> A)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int NT = MTP_SEG_WORKERS * 32;
-    SegSmem<T> S;
-    seg_smem_layout<T, MODE>(P, smem_raw, &S);
+    constexpr int NT = MTP_PAIR_WARPS * 32, GL = pair_gl<T>(), G = 32 / GL, K = GL == 16 ? 0 : 1;
+    PairSmem<T> S;
+    pair_smem_layout<T, MODE>(P, smem_raw, &S);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     chain_release();
     const int ntot = total_atoms(A);
@@ -572,62 +493,52 @@ __global__ void __launch_bounds__(MTP_SEG_WORKERS * 32, 1) mtp_contract_seg_kern
     }
 
     // tables, staged once per block
-    for (int i = threadIdx.x; i < P.nseg; i += NT) S.hdr[i] = P.seg_hdr[i];
-    for (int i = threadIdx.x; i < P.nseg_rows; i += NT) S.row[i] = P.seg_row[i];
-    for (int i = threadIdx.x; i < 2 * P.nlev * (MTP_SEG_WORKERS + 1); i += NT) S.wseg[i] = P.seg_wseg[i];
-    for (int i = threadIdx.x; i < 2 * P.nlev * MTP_SEG_WORKERS; i += NT) S.wrow[i] = P.seg_wrow[i];
+    for (int i = threadIdx.x; i < P.stream[K].nrows * G; i += NT) S.row[i] = stream_rows<T>(P.stream[K])[i];
+    for (int i = threadIdx.x; i < 2 * P.nlev * MTP_PAIR_WARPS; i += NT) S.warp[i] = P.stream[K].warp[i];
+    for (int s = threadIdx.x; s < P.ns; s += NT) S.map[s] = P.map[s];
     if (MODE != MODE_DESC) {
         for (int i = threadIdx.x; i < P.nm; i += NT) S.seed[i] = T(0);
         __syncthreads();
         // adjoint seeds lin[s] / q[s] (linearMtp.h:292-295); a moment may serve several scalars
         for (int s = threadIdx.x; s < P.ns; s += NT) {
             const T w = A.lin[s] / A.qs[s];
-            const int m = P.map[s];
             S.wsc[s] = w;
-            S.mapo[s] = m * MTP_SEG_LD;
-            atomicAdd(S.seed + m, w);
+            atomicAdd(S.seed + P.map[s], w);
         }
-        for (int d = threadIdx.x; d < P.ndense; d += NT) {
-            const int r = P.dense_basic[d];
-            S.db[d] = r >= 0 ? r * MTP_SEG_LD : -1;
-        }
-    } else {
-        for (int s = threadIdx.x; s < P.ns; s += NT) S.mapo[s] = P.map[s] * MTP_SEG_LD;
+        for (int d = threadIdx.x; d < P.ndense; d += NT) S.db[d] = P.dense_basic[d];
     }
 
-    // basic-moment rows of a tile: warp w fetches atom w, lanes run over the row; fetched one tile ahead
+    // basic-moment rows of a tile: warp w fetches the rows w, w + 32, ..., lanes run over the atoms; fetched one tile ahead
     const bool can_prefetch = P.nb <= 32 * MTP_PREF;
+    auto basic = [&](int tile, int i) -> T {
+        if (A.tiled) return A.Mb[((size_t)tile * A.nbp + i) * MTP_TILE + lane];
+        const int t = tile * MTP_TILE + lane;
+        return t < ntot ? A.Mb[(size_t)t * A.nbp + i] : T(0);
+    };
     T pre[MTP_PREF];
-    // (tiled workspace: warp w fetches the rows w, w + 32, ... of the tile, lanes run over its atoms)
     auto fetch = [&](int tile) {
 #pragma unroll
         for (int k = 0; k < MTP_PREF; k++) {
-            if (A.tiled) {
-                const int i = warp + 32 * k;
-                pre[k] = i < P.nb ? A.Mb[((size_t)tile * A.nbp + i) * MTP_TILE + lane] : T(0);
-            } else {
-                const int i = lane + 32 * k, t = tile * MTP_TILE + warp;
-                pre[k] = (t < ntot && i < P.nb) ? A.Mb[(size_t)t * A.nbp + i] : T(0);
-            }
+            const int i = warp + 32 * k;
+            pre[k] = i < P.nb ? basic(tile, i) : T(0);
         }
     };
     chain_wait();        // everything above reads the program's tables and the model only
     if (can_prefetch) fetch(blockIdx.x);
-    // shared-window addresses of this lane's columns and of the tables
-    const unsigned ml = (unsigned)__cvta_generic_to_shared(S.M + lane), el = (unsigned)__cvta_generic_to_shared(S.E + lane);
-    const unsigned a_hdr = (unsigned)__cvta_generic_to_shared(S.hdr), a_row = (unsigned)__cvta_generic_to_shared(S.row),
-                   a_seed = (unsigned)__cvta_generic_to_shared(S.seed);
+    // shared-window addresses of this lane's 16 bytes of every row, of its group's records, of the seeds
+    const unsigned ml = (unsigned)__cvta_generic_to_shared(S.M) + 16u * (lane % GL), el = (unsigned)__cvta_generic_to_shared(S.E) + 16u * (lane % GL);
+    const unsigned a_row = (unsigned)__cvta_generic_to_shared(S.row) + 8u * (lane / GL), a_seed = (unsigned)__cvta_generic_to_shared(S.seed);
     auto run_phase = [&](int p, auto seeded, unsigned xl, unsigned yl, unsigned dl) {
-        const int h = S.wseg[p * (MTP_SEG_WORKERS + 1) + warp], hend = S.wseg[p * (MTP_SEG_WORKERS + 1) + warp + 1];
-        seg_phase<T, decltype(seeded)::value>(h, hend, a_hdr, a_row + 8u * (unsigned)S.wrow[p * MTP_SEG_WORKERS + warp], a_seed, xl, yl, dl);
+        const int2 w = S.warp[p * MTP_PAIR_WARPS + warp];
+        pair_phase<T, GL, decltype(seeded)::value>(a_row + 8u * G * (unsigned)w.x, w.y, xl, yl, dl, a_seed);
     };
 
     __syncthreads();         // tables staged
     if (MODE != MODE_DESC) {
         // moments no product reads: their adjoint is their seed for every atom of every tile, written once
-        for (int i = warp; i < P.nseg_init; i += MTP_SEG_WORKERS) {
-            const int m = P.seg_init[i];
-            S.E[m * MTP_SEG_LD + lane] = S.seed[m];
+        for (int i = warp; i < P.n_adj_const; i += MTP_PAIR_WARPS) {
+            const int m = P.adj_const[i];
+            S.E[m * MTP_TILE + lane] = S.seed[m];
         }
     }
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -636,17 +547,12 @@ __global__ void __launch_bounds__(MTP_SEG_WORKERS * 32, 1) mtp_contract_seg_kern
         if (can_prefetch) {
 #pragma unroll
             for (int k = 0; k < MTP_PREF; k++) {
-                const int i = (A.tiled ? warp : lane) + 32 * k;
-                if (i < P.nb) S.M[i * MTP_SEG_LD + (A.tiled ? lane : warp)] = pre[k];
+                const int i = warp + 32 * k;
+                if (i < P.nb) S.M[i * MTP_TILE + lane] = pre[k];
             }
             if (tile + (int)gridDim.x < ntiles) fetch(tile + gridDim.x);   // in flight during this tile
-        } else if (A.tiled) {
-            const T *src = A.Mb + (size_t)tile * A.nbp * MTP_TILE + lane;
-            for (int i = warp; i < P.nb; i += MTP_SEG_WORKERS) S.M[i * MTP_SEG_LD + lane] = src[(size_t)i * MTP_TILE];
         } else {
-            const int t = tile * MTP_TILE + warp;
-            const T *src = A.Mb + (size_t)t * A.nbp;
-            for (int i = lane; i < P.nb; i += 32) S.M[i * MTP_SEG_LD + warp] = t < ntot ? src[i] : T(0);
+            for (int i = warp; i < P.nb; i += MTP_PAIR_WARPS) S.M[i * MTP_TILE + lane] = basic(tile, i);
         }
         __syncthreads();
 
@@ -679,22 +585,22 @@ __global__ void __launch_bounds__(MTP_SEG_WORKERS * 32, 1) mtp_contract_seg_kern
 
         if (MODE == MODE_DESC) {
             if (valid)
-                for (int s = warp; s < P.ns; s += MTP_SEG_WORKERS) A.desc[slot * P.ns + s] = S.M[S.mapo[s] + lane];
+                for (int s = warp; s < P.ns; s += MTP_PAIR_WARPS) A.desc[slot * P.ns + s] = S.M[S.map[s] * MTP_TILE + lane];
             __syncthreads();     // the moments are overwritten by the next tile
             continue;
         }
 
-        // site energies (linearMtp.h:281-289) by the first MTP_SEG_EWARPS warps, which meet at a barrier of their own;
+        // site energies (linearMtp.h:281-289) by the first MTP_PAIR_EWARPS warps, which meet at a barrier of their own;
         // the other warps go on to the adjoints (they read the moments and write the adjoint array only)
-        if (warp < MTP_SEG_EWARPS) {
+        if (warp < MTP_PAIR_EWARPS) {
             T es = T(0);
-            for (int s = warp; s < P.ns; s += MTP_SEG_EWARPS) es = fma(S.wsc[s], S.M[S.mapo[s] + lane], es);
-            S.ep[warp * MTP_SEG_LD + lane] = es;
-            asm volatile("bar.sync 1, %0;" ::"n"(MTP_SEG_EWARPS * 32) : "memory");
+            for (int s = warp; s < P.ns; s += MTP_PAIR_EWARPS) es = fma(S.wsc[s], S.M[S.map[s] * MTP_TILE + lane], es);
+            S.ep[warp * MTP_TILE + lane] = es;
+            asm volatile("bar.sync 1, %0;" ::"n"(MTP_PAIR_EWARPS * 32) : "memory");
             if (warp == 0) {
                 T e = ebias;
 #pragma unroll
-                for (int k = 0; k < MTP_SEG_EWARPS; k++) e += S.ep[k * MTP_SEG_LD + lane];
+                for (int k = 0; k < MTP_PAIR_EWARPS; k++) e += S.ep[k * MTP_TILE + lane];
                 if (!valid) e = T(0);
                 // one atomic per structure present in these 32 atoms
                 const int key = valid ? b : -1;
@@ -720,19 +626,15 @@ __global__ void __launch_bounds__(MTP_SEG_WORKERS * 32, 1) mtp_contract_seg_kern
             __syncthreads();
         }
         if (P.nlev < 2) __syncthreads();     // the energy warps still read the moments the next tile overwrites
-        // adjoints of the basic moments: whole rows of the tile, or back to per-atom rows (warp w writes atom w)
+        // adjoints of the basic moments: whole rows of the tile, or back to per-atom rows
         if (A.tiled) {      // in dense monomial order, the order the force kernel evaluates its polynomials in
             T *dstp = A.Eb + (size_t)tile * A.ndp * MTP_TILE + lane;
-            for (int d = warp; d < P.ndense; d += MTP_SEG_WORKERS) {
-                const int o = S.db[d];
-                dstp[(size_t)d * MTP_TILE] = o >= 0 ? S.E[o + lane] : T(0);
+            for (int d = warp; d < P.ndense; d += MTP_PAIR_WARPS) {
+                const int i = S.db[d];
+                dstp[(size_t)d * MTP_TILE] = i >= 0 ? S.E[i * MTP_TILE + lane] : T(0);
             }
-        } else {
-            const int t = tile * MTP_TILE + warp;
-            if (t < ntot) {
-                T *dstp = A.Eb + (size_t)t * A.nbp;
-                for (int i = lane; i < A.nbp; i += 32) dstp[i] = i < P.nb ? S.E[i * MTP_SEG_LD + warp] : T(0);
-            }
+        } else if (valid) {
+            for (int i = warp; i < A.nbp; i += MTP_PAIR_WARPS) A.Eb[(size_t)t * A.nbp + i] = i < P.nb ? S.E[i * MTP_TILE + lane] : T(0);
         }
     }
 }
@@ -932,15 +834,15 @@ template <typename T, int MODE>
 static int dispatch_contract(const MtpProgramDev &P, const MtpArgs<T> &A, long atoms_upper, cudaStream_t st)
 {
     const size_t cap = 222 * 1024;
-    {   // segment form: whole tables and a tile of 32 atoms in shared memory
-        const size_t smem = seg_smem_layout<T, MODE>(P, nullptr, nullptr);
-        if (smem <= 226 * 1024 && P.nseg > 0) {
-            auto kern = mtp_contract_seg_kernel<T, MODE>;
+    {   // whole tables and a tile of 32 atoms in shared memory
+        const size_t smem = pair_smem_layout<T, MODE>(P, nullptr, nullptr);
+        if (pair_fits<T>(P, smem)) {
+            auto kern = mtp_contract_pair_kernel<T, MODE>;
             static KernelSetup setup;
             if (int rc = kernel_setup(setup, kern, smem)) return rc;
             long tiles = (atoms_upper + MTP_TILE - 1) / MTP_TILE;
             if (tiles > sm_count()) tiles = sm_count();      // persistent: one block per SM walks over the tiles
-            AI2B_CUDA(launch_chained(kern, (unsigned)tiles, MTP_SEG_WORKERS * 32, smem, st, P, A));
+            AI2B_CUDA(launch_chained(kern, (unsigned)tiles, MTP_PAIR_WARPS * 32, smem, st, P, A));
             return AI2B_OK;
         }
     }
@@ -978,8 +880,8 @@ static int launch_mtp_v(const ai2b_mtp_program *prog, MtpArgs<T> A, void *ws, cu
     // lanes-as-atoms forward and force kernels around the segment contraction, where all three apply
     bool atoms_path = false;
     if constexpr (KD <= 6 && CSP == 8)
-        atoms_path = mtp_atoms_supported(P, A.ntypes, A.cs, sizeof(T), (long)A.npad + A.nghost) && P.nseg > 0 &&
-                     seg_smem_layout<T, MODE>(P, nullptr, nullptr) <= 226 * 1024;
+        atoms_path = mtp_atoms_supported(P, A.ntypes, A.cs, sizeof(T), (long)A.npad + A.nghost) &&
+                     pair_fits<T>(P, pair_smem_layout<T, MODE>(P, nullptr, nullptr));
     const bool need_pad = A.cs != CSP || (reinterpret_cast<size_t>(A.coeffs) % (2 * sizeof(T))) != 0;
     if (atoms_path && A.B == 1 && !need_pad) {
         // one structure, coefficient rows usable as they are: no set-up launch; the forward kernel zeroes the outputs

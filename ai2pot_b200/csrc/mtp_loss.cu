@@ -17,7 +17,7 @@
 // moments and their directional derivatives, a tile kernel with lanes = atoms for all product-row
 // sweeps, and a per-atom kernel that evaluates the two polynomials per neighbour and reduces the
 // coefficient gradient over the lanes of each neighbour type.
-#include "mtp_device.cuh"
+#include "mtp_pairs.cuh"
 
 namespace ai2b {
 
@@ -371,6 +371,122 @@ __global__ void __launch_bounds__(MTP_CWARPS * 32, 1) mtp_loss_contract_kernel(c
     if (wid == 0) group_add(ce, valid ? b * A.ntypes + ti : -1, L.dbias + (size_t)b * A.ntypes + ti);
 }
 
+// ---- kernel B', tables that fit: row loop of mtp_pairs.cuh with eight lanes per row -----------------------------------
+// Four arrays of a tile in shared memory (moments, directional derivatives, adjoints, second-order adjoints): 16 atoms in
+// double, 32 in single precision. Two sweeps: products with their derivatives, then adjoints and second-order adjoints
+// together (a source's second-order adjoint needs the two of its products, which belong to deeper levels). A row of the second
+// sweep reads four operands where three sweeps of their own read six. Walks over the tiles with the tables staged once.
+// Level 16, fp64, 9,323 atoms: 86 us; 171 us with one row per warp, a block per tile and the table staged for each.
+template <typename T>
+struct LossPairSmem {
+    T *M, *E, *seed;
+    int2 *row, *warp;
+    int *map;
+};
+template <typename T> constexpr int loss_ta() { return 8 * 16 / (int)sizeof(T); }
+template <typename T>
+__host__ __device__ inline size_t loss_pair_smem(const MtpProgramDev &P, unsigned char *base, LossPairSmem<T> *out)
+{
+    size_t o = 0;
+    auto take = [&](size_t bytes) { size_t r = o; o += (bytes + 15) & ~size_t(15); return r; };
+    const size_t oM = take(sizeof(T) * 2 * (size_t)P.nm * loss_ta<T>()), oE = take(sizeof(T) * 2 * (size_t)P.nm * loss_ta<T>());
+    const size_t orow = take(sizeof(int2) * (size_t)P.stream[1].nrows * 4), ow = take(sizeof(int2) * (size_t)(2 * P.nlev) * MTP_PAIR_WARPS);
+    const size_t os = take(sizeof(T) * (size_t)P.nm), om = take(sizeof(int) * (size_t)P.ns);
+    if (out) {
+        out->M = reinterpret_cast<T *>(base + oM); out->E = reinterpret_cast<T *>(base + oE); out->seed = reinterpret_cast<T *>(base + os);
+        out->row = reinterpret_cast<int2 *>(base + orow); out->warp = reinterpret_cast<int2 *>(base + ow); out->map = reinterpret_cast<int *>(base + om);
+    }
+    return o;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_loss_pair_kernel(const MtpProgramDev P, const MtpArgs<T> A, const LossArgs<T> L)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int NT = MTP_PAIR_WARPS * 32, TA = loss_ta<T>(), RW = 32 / TA, G = 4;    // RW: moment rows per warp when lanes are atoms
+    LossPairSmem<T> S;
+    loss_pair_smem<T>(P, smem_raw, &S);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int at = lane % TA, rw = warp * RW + lane / TA;
+    T *D = S.M + (size_t)P.nm * TA, *Gm = S.E + (size_t)P.nm * TA;
+    const unsigned off = (unsigned)(sizeof(T) * (size_t)P.nm * TA);
+    chain_release();
+    for (int i = threadIdx.x; i < P.stream[1].nrows * G; i += NT) S.row[i] = stream_rows<T>(P.stream[1])[i];
+    for (int i = threadIdx.x; i < 2 * P.nlev * MTP_PAIR_WARPS; i += NT) S.warp[i] = P.stream[1].warp[i];
+    for (int s = threadIdx.x; s < P.ns; s += NT) S.map[s] = P.map[s];
+    for (int i = threadIdx.x; i < P.nm; i += NT) S.seed[i] = T(0);
+    __syncthreads();
+    for (int s = threadIdx.x; s < P.ns; s += NT) atomicAdd(S.seed + P.map[s], A.lin[s] / A.qs[s]);
+    __syncthreads();
+    // moments no product reads: adjoint = seed, no second-order adjoint
+    for (int i = rw; i < P.n_adj_const; i += MTP_PAIR_WARPS * RW) {
+        const int m = P.adj_const[i];
+        S.E[m * TA + at] = S.seed[m];
+        Gm[m * TA + at] = T(0);
+    }
+    chain_wait();        // everything above reads the program's tables and the model only
+    const int ntot = A.prefix[A.B], ntiles = (ntot + TA - 1) / TA;
+    const unsigned ml = (unsigned)__cvta_generic_to_shared(S.M) + 16u * (lane % 8), el = (unsigned)__cvta_generic_to_shared(S.E) + 16u * (lane % 8);
+    const unsigned a_row = (unsigned)__cvta_generic_to_shared(S.row) + 8u * (lane / 8), a_seed = (unsigned)__cvta_generic_to_shared(S.seed);
+
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int t = tile * TA + at;
+        const bool valid = t < ntot;
+        for (int i = rw; i < P.nb; i += MTP_PAIR_WARPS * RW) {
+            // rows per atom, or [tile of 32 atoms][row][32]
+            const size_t src = A.tiled ? ((size_t)(t >> 5) * A.nbp + i) * 32 + (t & 31) : (size_t)t * A.nbp + i;
+            S.M[i * TA + at] = valid ? A.Mb[src] : T(0);
+            D[i * TA + at] = valid ? L.Db[src] : T(0);
+        }
+        int b = 0, ti = 0;
+        T ce = T(0);
+        if (valid) {
+            b = find_structure(A.prefix, A.B, t);
+            const size_t slot = (size_t)b * A.npad + (t - A.prefix[b]);
+            ti = (A.types + (size_t)b * (A.npad + A.nghost))[A.bilist[slot]];
+            ce = T(2) * L.ew / T(A.binum[b]) * (L.e_ml[b] - L.e_dft[b]);
+        }
+        __syncthreads();
+        for (int p = 0; p < P.nlev; p++) {
+            const int2 w = S.warp[p * MTP_PAIR_WARPS + warp];
+            pair_phase_deriv<T, 8>(a_row + 8u * G * (unsigned)w.x, w.y, ml, off);
+            __syncthreads();
+        }
+        for (int p = P.nlev; p < 2 * P.nlev; p++) {
+            const int2 w = S.warp[p * MTP_PAIR_WARPS + warp];
+            pair_phase_second<T, 8>(a_row + 8u * G * (unsigned)w.x, w.y, el, ml, off, a_seed);
+            __syncthreads();
+        }
+        // for the coefficient kernel: E and X = ce E + G of the basic moments
+        if (valid)
+            for (int i = rw; i < P.nb; i += MTP_PAIR_WARPS * RW) {
+                const T e = S.E[i * TA + at];
+                A.Eb[(size_t)t * A.nbp + i] = e;
+                L.Xb[(size_t)t * A.nbp + i] = fma(ce, e, Gm[i * TA + at]);
+            }
+        // gradients w.r.t. the linear coefficients and the type bias: one atomic per entry when the tile lies in one structure
+        const int b0 = __shfl_sync(FULL_MASK, b, 0);
+        const bool uniform = __all_sync(FULL_MASK, !valid || b == b0);      // (the same in every warp: they share the tile's atoms)
+        for (int s0 = 0; s0 < P.ns; s0 += MTP_PAIR_WARPS * RW) {
+            const int s = s0 + rw;
+            T val = T(0);
+            if (s < P.ns && valid) {
+                const int m = S.map[s];
+                val = (ce * S.M[m * TA + at] + D[m * TA + at]) / A.qs[s];
+            }
+            if (uniform) {
+#pragma unroll
+                for (int o = TA / 2; o >= 1; o >>= 1) val += __shfl_xor_sync(FULL_MASK, val, o);
+                if (s < P.ns && at == 0) atomicAdd(L.dlinear + (size_t)b0 * P.ns + s, val);
+            } else if (s < P.ns && valid) {
+                atomicAdd(L.dlinear + (size_t)b * P.ns + s, val);
+            }
+        }
+        if (warp == 0 && lane < TA && valid) atomicAdd(L.dbias + (size_t)b * A.ntypes + ti, ce);
+        __syncthreads();     // the moments are overwritten by the next tile
+    }
+}
+
 // ---- kernel C': gradient w.r.t. the radial coefficients -------------------------------------------
 template <typename T, int KD, int CSP>
 __global__ void __launch_bounds__(MTP_WARPS * 32, 3) mtp_loss_coeff_kernel(const MtpProgramDev P, const MtpArgs<T> A, const LossArgs<T> L)
@@ -545,6 +661,16 @@ static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArg
         const size_t cap = 222 * 1024;
         int rc = AI2B_ERR_UNSUPPORTED;
         bool done = false;
+        const size_t pair_bytes = loss_pair_smem<T>(P, nullptr, nullptr);
+        if (P.stream[1].nrows > 0 && pair_bytes <= 226 * 1024) {
+            auto kern = mtp_loss_pair_kernel<T>;
+            static KernelSetup setup;
+            if ((rc = kernel_setup(setup, kern, pair_bytes))) return rc;
+            long tiles = (atoms_upper + loss_ta<T>() - 1) / loss_ta<T>();
+            if (tiles > sm_count()) tiles = sm_count();
+            AI2B_CUDA(launch_chained(kern, (unsigned)tiles, MTP_PAIR_WARPS * 32, pair_bytes, st, P, A, L));
+            done = true;
+        }
 #define AI2B_TRY(TA_)                                                                                                   \
     if (!done && (long)P.nm * (TA_ + 1) <= 65535) {                                                                     \
         if (loss_contract_smem(P, sizeof(T), TA_, true) <= cap) { rc = launch_loss_contract<T, TA_, true>(P, A, L, atoms_upper, st); done = true; } \

@@ -296,10 +296,9 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
     for (int s = 0; s < ns; s++)
         AI2B_REQUIRE(map[s] >= 0 && map[s] < nm, AI2B_ERR_INVALID, "alpha_moment_mapping[%d] out of range", s);
 
-    // segment streams (see mtp_program.cuh)
-    std::vector<int4> seg_hdr;
-    std::vector<int2> seg_row;
-    std::vector<int> seg_wseg, seg_wrow, seg_init;
+    // row streams (see mtp_program.cuh)
+    std::vector<int2> stream_d[2], stream_f[2], stream_warp[2];
+    std::vector<int> adj_const;
     {
         std::vector<char> is_source(nm, 0), is_mapped(nm, 0);
         for (int t = 0; t < nt; t++) { is_source[times[4 * t]] = 1; is_source[times[4 * t + 1]] = 1; }
@@ -307,87 +306,128 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
         // moments whose adjoint is just their seed: scalars that are no operand of any product, and basic
         // moments nothing uses (seed 0); every other adjoint that is read is written by a gather phase
         for (int m = 0; m < nm; m++)
-            if (!is_source[m] && (is_mapped[m] || m < nb)) seg_init.push_back(m);
+            if (!is_source[m] && (is_mapped[m] || m < nb)) adj_const.push_back(m);
         struct Row { int x, y, mult; };
-        auto emit_phase = [&](const std::vector<std::pair<int, std::vector<Row>>> &moments) {
-            // longest processing time first over the workers; a segment (rows of one multiplier) costs about as much as
-            // two and a half of its rows (header, multiplier, final store)
-            std::vector<long> cost(moments.size());
-            for (size_t i = 0; i < moments.size(); i++) {
-                std::vector<int> mults;
-                for (const Row &r : moments[i].second) mults.push_back(r.mult);
-                std::sort(mults.begin(), mults.end());
-                const long nseg = (long)(std::unique(mults.begin(), mults.end()) - mults.begin());
-                cost[i] = 2 * (long)moments[i].second.size() + 5 * nseg;
-            }
-            std::vector<size_t> order(moments.size());
-            for (size_t i = 0; i < order.size(); i++) order[i] = i;
-            std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return cost[a] > cost[b]; });
-            std::vector<std::vector<size_t>> mine(MTP_SEG_WORKERS);
-            std::vector<long> load(MTP_SEG_WORKERS, 0);
-            for (size_t i : order) {
-                int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-                mine[w].push_back(i);
-                load[w] += cost[i];
-            }
-            for (int w = 0; w < MTP_SEG_WORKERS; w++) {
-                seg_wseg.push_back((int)seg_hdr.size());
-                seg_wrow.push_back((int)seg_row.size());
-                for (size_t i : mine[w]) {
-                    std::vector<Row> rows = moments[i].second;
-                    std::stable_sort(rows.begin(), rows.end(), [](const Row &a, const Row &b) { return a.mult < b.mult; });
-                    size_t r = 0;
-                    bool first = true;
-                    while (r < rows.size()) {
-                        size_t e = r;
-                        while (e < rows.size() && rows[e].mult == rows[r].mult) e++;
-                        const double mult = (double)rows[r].mult;
-                        long long bits;
-                        memcpy(&bits, &mult, 8);
-                        unsigned flags = (unsigned)(e - r) | (first ? 1u << 30 : 0u) | (e == rows.size() ? 1u << 31 : 0u);
-                        seg_hdr.push_back(make_int4(moments[i].first * MTP_SEG_LD, (int)flags, (int)(bits & 0xffffffffll), (int)(bits >> 32)));
-                        for (size_t k = r; k < e; k++) seg_row.push_back(make_int2(rows[k].x * MTP_SEG_LD, rows[k].y * MTP_SEG_LD));
-                        first = false;
-                        r = e;
-                    }
-                }
-            }
-            seg_wseg.push_back((int)seg_hdr.size());
-        };
+        struct Moment { int m; std::vector<Row> rows; };
+        std::vector<std::vector<Moment>> phases;
         for (int lev = 1; lev <= P.nlev; lev++) {
-            std::vector<std::pair<int, std::vector<Row>>> moments;
+            phases.emplace_back();
             for (int m = 0; m < nm; m++)
                 if (depth[m] == lev && !rows_of[m].empty()) {
-                    std::vector<Row> rows;
-                    for (int t : rows_of[m]) rows.push_back(Row{times[4 * t], times[4 * t + 1], times[4 * t + 2]});
-                    moments.emplace_back(m, rows);
+                    Moment q{m, {}};
+                    for (int t : rows_of[m]) q.rows.push_back(Row{times[4 * t], times[4 * t + 1], times[4 * t + 2]});
+                    phases.back().push_back(q);
                 }
-            emit_phase(moments);
         }
-        for (int k = 0; k < P.nlev; k++) {
-            const int lev = P.nlev - 1 - k;
-            std::vector<std::pair<int, std::vector<Row>>> moments;
+        for (int lev = P.nlev - 1; lev >= 0; lev--) {
+            phases.emplace_back();
             for (int m = 0; m < nm; m++)
                 if (depth[m] == lev && !occ_of[m].empty()) {
-                    std::vector<Row> rows;
+                    Moment q{m, {}};
                     for (int o : occ_of[m]) {
                         const int t = o >> 1;
-                        const int other = (o & 1) ? times[4 * t] : times[4 * t + 1];
-                        rows.push_back(Row{times[4 * t + 3], other, times[4 * t + 2]});
+                        q.rows.push_back(Row{times[4 * t + 3], (o & 1) ? times[4 * t] : times[4 * t + 1], times[4 * t + 2]});
                     }
-                    moments.emplace_back(m, rows);
+                    phases.back().push_back(q);
                 }
-            emit_phase(moments);
         }
-        for (const int4 &h : seg_hdr)
-            AI2B_REQUIRE((h.y & 0x3fffffff) < (1 << 24), AI2B_ERR_UNSUPPORTED, "a product segment has too many rows");
+        for (int k = 0; k < 2; k++) {
+            const size_t groups = k == 0 ? 2 : 4;
+            P.stream[k].nrows = 0;
+            if (nm > 2046 || nt == 0) continue;      // the completed moment has 11 bits
+            for (const auto &ph : phases) {
+                // A phase lasts as long as its longest warp, and a few moments have many times the rows of the others (69
+                // against 13 on average in the last phase of level 16). Moments with more rows than `wide` are therefore split
+                // over all groups of a warp; the others go to single groups. Both by decreasing row count to the least loaded
+                // place, completing a moment taken as a row. `wide` is chosen per phase by a cost: a row of the longest warp
+                // waits for about 60 cycles, a row of any warp takes about 5 of its scheduler's issue slots.
+                std::vector<size_t> order(ph.size());
+                for (size_t i = 0; i < order.size(); i++) order[i] = i;
+                std::stable_sort(order.begin(), order.end(), [&](size_t i, size_t j) { return ph[i].rows.size() > ph[j].rows.size(); });
+                using Deal = std::vector<std::vector<size_t>>;
+                auto deal = [&](size_t wide, Deal &of_warp, Deal &of_group) -> size_t {
+                    of_warp.assign(MTP_PAIR_WARPS, {});
+                    of_group.assign(MTP_PAIR_WARPS * groups, {});
+                    std::vector<size_t> wload(MTP_PAIR_WARPS, 0), wrows(MTP_PAIR_WARPS, 0), grows(MTP_PAIR_WARPS * groups, 0);
+                    size_t i = 0;
+                    for (; i < order.size() && ph[order[i]].rows.size() > wide; i++) {
+                        const size_t w = std::min_element(wload.begin(), wload.end()) - wload.begin(), n = (ph[order[i]].rows.size() + groups - 1) / groups;
+                        of_warp[w].push_back(order[i]);
+                        wload[w] += n + 1;
+                        wrows[w] += n;
+                    }
+                    std::vector<size_t> gload(MTP_PAIR_WARPS * groups);
+                    for (size_t g = 0; g < gload.size(); g++) gload[g] = wload[g / groups];
+                    for (; i < order.size(); i++) {
+                        const size_t g = std::min_element(gload.begin(), gload.end()) - gload.begin(), n = ph[order[i]].rows.size();
+                        of_group[g].push_back(order[i]);
+                        gload[g] += n + 1;
+                        grows[g] += n;
+                    }
+                    size_t longest = 0, sum = 0;
+                    for (size_t w = 0; w < MTP_PAIR_WARPS; w++) {
+                        const size_t len = wrows[w] + *std::max_element(grows.begin() + w * groups, grows.begin() + (w + 1) * groups);
+                        longest = std::max(longest, len);
+                        sum += len;
+                    }
+                    return 60 * longest + 5 * sum;
+                };
+                Deal of_warp, of_group;
+                size_t best = ~size_t(0), best_wide = 0;
+                for (size_t i : order) {
+                    const size_t wide = ph[i].rows.size(), cost = deal(wide, of_warp, of_group);
+                    if (cost < best) { best = cost; best_wide = wide; }
+                }
+                deal(best_wide, of_warp, of_group);
+                for (size_t w = 0; w < MTP_PAIR_WARPS; w++) {
+                    std::vector<std::vector<int2>> rd(groups), rf(groups);
+                    auto put = [&](size_t g, int xy, int mult, int done) {
+                        const double md = mult;
+                        const float mf = (float)mult;
+                        long long bd;
+                        int bf;
+                        memcpy(&bd, &md, 8);
+                        memcpy(&bf, &mf, 4);
+                        rd[g].push_back(make_int2(xy, (int)(bd >> 32) | done));
+                        rf[g].push_back(make_int2(xy, bf | done));
+                    };
+                    for (size_t i : of_warp[w]) {
+                        const Moment &q = ph[i];
+                        const size_t n = (q.rows.size() + groups - 1) / groups;
+                        for (size_t r = 0; r < n; r++)
+                            for (size_t g = 0; g < groups; g++) {
+                                const size_t at = r * groups + g;
+                                const int done = r + 1 == n ? (q.m + 1) | MTP_PAIR_WIDE : 0;
+                                if (at < q.rows.size()) put(g, q.rows[at].x | (q.rows[at].y << 16), q.rows[at].mult, done);
+                                else put(g, q.rows[0].x | (q.rows[0].y << 16), 0, done);      // (operands that are written by then)
+                            }
+                    }
+                    size_t len = 0;
+                    for (size_t g = 0; g < groups; g++) {
+                        for (size_t i : of_group[w * groups + g]) {
+                            const Moment &q = ph[i];
+                            for (size_t r = 0; r < q.rows.size(); r++)
+                                put(g, q.rows[r].x | (q.rows[r].y << 16), q.rows[r].mult, r + 1 == q.rows.size() ? q.m + 1 : 0);
+                        }
+                        len = std::max(len, rd[g].size());
+                    }
+                    stream_warp[k].push_back(make_int2((int)(stream_d[k].size() / groups), (int)len));
+                    for (size_t r = 0; r < len; r++)
+                        for (size_t g = 0; g < groups; g++) {
+                            stream_d[k].push_back(r < rd[g].size() ? rd[g][r] : make_int2(0, 0));
+                            stream_f[k].push_back(r < rf[g].size() ? rf[g][r] : make_int2(0, 0));
+                        }
+                }
+            }
+            for (size_t g = 0; g < 2 * groups; g++) { stream_d[k].push_back(make_int2(0, 0)); stream_f[k].push_back(make_int2(0, 0)); }   // read ahead
+            P.stream[k].nrows = (int)(stream_d[k].size() / groups);
+        }
     }
-    P.nseg = (int)seg_hdr.size();
-    P.nseg_rows = (int)seg_row.size();
-    P.nseg_init = (int)seg_init.size();
+    P.n_adj_const = (int)adj_const.size();
 
     Blob blob;
-    size_t o_sh = blob.add(seg_hdr), o_sr = blob.add(seg_row), o_sws = blob.add(seg_wseg), o_swr = blob.add(seg_wrow), o_si = blob.add(seg_init);
+    size_t o_ac = blob.add(adj_const), o_sd[2], o_sf[2], o_sw[2];
+    for (int k = 0; k < 2; k++) { o_sd[k] = blob.add(stream_d[k]); o_sf[k] = blob.add(stream_f[k]); o_sw[k] = blob.add(stream_warp[k]); }
     size_t o_bd = blob.add(basic_dense), o_db = blob.add(dense_basic), o_e4d = blob.add(e4d), o_g = blob.add(e4g), o_m = blob.add(e4m), o_fd = blob.add(fwd_dst),
            o_fr = blob.add(fwd_ab), o_fmf = blob.add(fwd_mf), o_fmd = blob.add(fwd_md), o_rm = blob.add(rev_mom),
            o_re = blob.add(rev_od), o_rmf = blob.add(rev_mf), o_rmd = blob.add(rev_md), o_map = blob.add(map);
@@ -423,11 +463,12 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
     P.rev_ents = (const int2 *)(b + o_rent);
     P.fwd_flat = (const int2 *)(b + o_ff);
     P.rev_flat = (const int2 *)(b + o_rf);
-    P.seg_hdr = (const int4 *)(b + o_sh);
-    P.seg_row = (const int2 *)(b + o_sr);
-    P.seg_wseg = (const int *)(b + o_sws);
-    P.seg_wrow = (const int *)(b + o_swr);
-    P.seg_init = (const int *)(b + o_si);
+    P.adj_const = (const int *)(b + o_ac);
+    for (int k = 0; k < 2; k++) {
+        P.stream[k].row_d = (const int2 *)(b + o_sd[k]);
+        P.stream[k].row_f = (const int2 *)(b + o_sf[k]);
+        P.stream[k].warp = (const int2 *)(b + o_sw[k]);
+    }
     prog->dev = P;
     *out = prog;
     return AI2B_OK;

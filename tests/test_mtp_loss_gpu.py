@@ -143,3 +143,29 @@ def test_loss_op_autograd(checkers):
     assert util.relerr(bias.grad.cpu().numpy(), G["train_dbias"].mean(0)) < 1e-10
     out = fromcc.linearMtpToEFLossOp(1.0, 1.0, c(t["E"], dt), c(t["F"][:, :npad], dt), *tail)
     assert len(out) == 3
+
+
+@pytest.mark.parametrize("dt", [torch.float64, torch.float32])
+@pytest.mark.parametrize("level,B,nmin,nmax", [(6, 1, 1, 2), (6, 3, 8, 40), (10, 5, 1, 17), (16, 1, 16, 17), (16, 9, 1, 34)])
+def test_contraction_tile_edges(checkers, level, B, nmin, nmax, dt):
+    """Structures of 1 to 33 atoms: tiles of 16 and 32 atoms that are nearly empty, full, ragged and shared by several
+    structures, at every template level, forward and gradients."""
+    chk = _chk(checkers)
+    g, nb = util.training_batch(chk, level=level, B=B, seed=5, nmin=nmin, nmax=nmax)
+    if dt == torch.float32:      # the checker in double precision on the values that single precision holds
+        g["model"] = {k: (v.astype(np.float32).astype(v.dtype) if isinstance(v, np.ndarray) and v.dtype == np.float64 else v) for k, v in g["model"].items()}
+        nb["brcs"] = nb["brcs"].astype(np.float32).astype(np.float64)
+    er, fr, vr = chk.mtp_efv(g["model"], nb)
+    t = g["targets"]; npad = nb["bilist"].shape[1]
+    ref = chk.mtp_loss_backward(g["model"], nb, g["weights"], er, t["E"], fr, t["F"][:, :npad], vr, t["V"])
+    nbt = dict(nb, brcs=nb["brcs"].astype(np.float64 if dt == torch.float64 else np.float32))
+    prog, md, nbd, (E, F, V) = _dev(g, nbt, dt)
+    tol = 1e-10 if dt == torch.float64 else 1e-5
+    for a, r, name in zip(capi.mtp_efv(prog, md, nbd), (er, fr, vr), ("energy", "force", "virial")):
+        assert util.relerr(a.cpu().numpy(), r) < tol, name
+    e, f, v = (torch.from_numpy(x).to(dt).cuda() for x in (er, fr, vr))
+    got = capi.mtp_loss_backward(prog, md, nbd, g["weights"], e, E, f, F, v, V)
+    for a, r, name in zip(got, ref, ("coeffs", "linear", "bias")):
+        assert util.relerr(a.cpu().numpy(), r) < 2 * tol, name
+    if dt == torch.float64:
+        assert util.relerr(capi.mtp_descriptors(prog, md, nbd).cpu().numpy(), chk.mtp_descriptors(g["model"], nb)) < tol
