@@ -56,6 +56,8 @@ __device__ __forceinline__ void pair_weight(const MtpArgs<T> &A, const LossArgs<
 
 // Lanes-as-atoms forward / force kernels (mtp_atoms.cu): available for the tables they are compiled for.
 bool mtp_atoms_supported(const MtpProgramDev &P, int ntypes, int cs, size_t elem, long atom_ids);
+// whether ai2b_mtp_efv_* / ai2b_mtp_ef_* leave the basic moments of these sizes in tiles in their workspace (mtp_kernels.cu)
+template <typename T> bool mtp_moments_tiled(const MtpProgramDev &P, const MtpArgs<T> &A);
 template <typename T> int mtp_fwd_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, cudaStream_t st);
 template <typename T, int MODE> int mtp_force_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, cudaStream_t st);
 // directional derivatives of the basic moments along the loss gradient's pair weights -> L.Db (tiled)

@@ -857,6 +857,15 @@ static int dispatch_contract(const MtpProgramDev &P, const MtpArgs<T> &A, long a
     return AI2B_ERR_UNSUPPORTED;
 }
 
+template <typename T>
+bool mtp_moments_tiled(const MtpProgramDev &P, const MtpArgs<T> &A)
+{
+    return P.kmax <= 6 && A.cs <= 8 && mtp_atoms_supported(P, A.ntypes, A.cs, sizeof(T), (long)A.npad + A.nghost) &&
+           pair_fits<T>(P, pair_smem_layout<T, MODE_EFV>(P, nullptr, nullptr));
+}
+template bool mtp_moments_tiled<float>(const MtpProgramDev &, const MtpArgs<float> &);
+template bool mtp_moments_tiled<double>(const MtpProgramDev &, const MtpArgs<double> &);
+
 template <typename T, int MODE, int KD, int CSP>
 static int launch_mtp_v(const ai2b_mtp_program *prog, MtpArgs<T> A, void *ws, cudaStream_t st)
 {
@@ -877,11 +886,13 @@ static int launch_mtp_v(const ai2b_mtp_program *prog, MtpArgs<T> A, void *ws, cu
         Z.p[1] = A.force; Z.n[1] = 3 * (size_t)A.B * (A.npad + A.nghost);
         if (A.virial) { Z.p[2] = A.virial; Z.n[2] = 9 * (size_t)A.B; }
     }
-    // lanes-as-atoms forward and force kernels around the segment contraction, where all three apply
+    // lanes-as-atoms forward and force kernels around the contraction in shared memory, where all three apply
     bool atoms_path = false;
-    if constexpr (KD <= 6 && CSP == 8)
-        atoms_path = mtp_atoms_supported(P, A.ntypes, A.cs, sizeof(T), (long)A.npad + A.nghost) &&
-                     pair_fits<T>(P, pair_smem_layout<T, MODE>(P, nullptr, nullptr));
+    if constexpr (KD <= 6 && CSP == 8) {
+        if (MODE != MODE_DESC) atoms_path = mtp_moments_tiled<T>(P, A);
+        else atoms_path = mtp_atoms_supported(P, A.ntypes, A.cs, sizeof(T), (long)A.npad + A.nghost) &&
+                          pair_fits<T>(P, pair_smem_layout<T, MODE>(P, nullptr, nullptr));
+    }
     const bool need_pad = A.cs != CSP || (reinterpret_cast<size_t>(A.coeffs) % (2 * sizeof(T))) != 0;
     if (atoms_path && A.B == 1 && !need_pad) {
         // one structure, coefficient rows usable as they are: no set-up launch; the forward kernel zeroes the outputs

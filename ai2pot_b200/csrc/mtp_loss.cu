@@ -23,14 +23,16 @@ namespace ai2b {
 
 // ---- loss and squared-error sums ---------------------------------------------------------------
 // one block per structure; se[0..2] accumulate sum dE^2 (of the energy per atom if e_per_atom: the NEP ops'
-// definition, nepLoss_cpu_launcher.h:300-345), sum dF^2, sum dV^2, se[3] the atom count
+// definition, nepLoss_cpu_launcher.h:300-345), sum dF^2, sum dV^2, se[3] the atom count. With a row of se per structure
+// (rows) the sums are stored and added up by mtp_rmse_kernel: no memset ahead of the launch, no atomics.
 template <typename T>
-__global__ void mtp_loss_kernel(T *__restrict__ loss, T *__restrict__ se, int e_per_atom, int npad, int nghost, const int *__restrict__ binum,
+__global__ void mtp_loss_kernel(T *__restrict__ loss, T *__restrict__ se, int rows, int e_per_atom, int npad, int nghost, const int *__restrict__ binum,
                                 const int *__restrict__ bilist, T ew, T fw, T vw, const T *__restrict__ e_ml,
                                 const T *__restrict__ e_dft, const T *__restrict__ f_ml, const T *__restrict__ f_dft,
                                 const T *__restrict__ v_ml, const T *__restrict__ v_dft)
 {
     __shared__ T sh[32];
+    chain_wait();
     const int b = blockIdx.x, n = binum[b];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     T fs = T(0);
@@ -53,19 +55,28 @@ __global__ void mtp_loss_kernel(T *__restrict__ loss, T *__restrict__ se, int e_
         T l = fw / T(3 * n) * f2 + ew / T(n) * de * de;
         if (v_ml) l += vw / T(9 * n) * v2;
         loss[b] = n > 0 ? l : T(0);
-        atomicAdd(se + 0, e_per_atom ? (n > 0 ? (de / T(n)) * (de / T(n)) : T(0)) : de * de);
-        atomicAdd(se + 1, f2);
-        atomicAdd(se + 2, v2);
-        atomicAdd(se + 3, T(n));
+        const T e2 = e_per_atom ? (n > 0 ? (de / T(n)) * (de / T(n)) : T(0)) : de * de, sum[4] = {e2, f2, v2, T(n)};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (rows) se[4 * b + k] = sum[k];
+            else atomicAdd(se + k, sum[k]);
+        }
     }
 }
 template <typename T>
-__global__ void mtp_rmse_kernel(T *__restrict__ rmse, const T *__restrict__ se, int B)
+__global__ void mtp_rmse_kernel(T *__restrict__ rmse, const T *__restrict__ se, int nrows, int B)
 {
+    chain_wait();
+    T sum[4] = {T(0), T(0), T(0), T(0)};
+    for (int b = threadIdx.x; b < nrows; b += 32)
+#pragma unroll
+        for (int k = 0; k < 4; k++) sum[k] += se[4 * b + k];
+#pragma unroll
+    for (int k = 0; k < 4; k++) sum[k] = warp_sum(sum[k]);
     if (threadIdx.x == 0) {
-        rmse[0] = sqrt(se[0] / T(B));
-        rmse[1] = sqrt(se[1] / (T(3) * se[3]));
-        rmse[2] = sqrt(se[2] / T(9 * B));
+        rmse[0] = sqrt(sum[0] / T(B));
+        rmse[1] = sqrt(sum[1] / (T(3) * sum[3]));
+        rmse[2] = sqrt(sum[2] / T(9 * B));
     }
 }
 
@@ -402,7 +413,7 @@ __host__ __device__ inline size_t loss_pair_smem(const MtpProgramDev &P, unsigne
 template <typename T>
 __global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_loss_pair_kernel(const MtpProgramDev P, const MtpArgs<T> A, const LossArgs<T> L)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(32) unsigned char smem_raw[];
     constexpr int NT = MTP_PAIR_WARPS * 32, TA = loss_ta<T>(), RW = 32 / TA, G = 4;    // RW: moment rows per warp when lanes are atoms
     LossPairSmem<T> S;
     loss_pair_smem<T>(P, smem_raw, &S);
@@ -501,6 +512,7 @@ __global__ void __launch_bounds__(MTP_WARPS * 32, 3) mtp_loss_coeff_kernel(const
     T *Xd = Ed + A.nbp;
     T *am = Xd + A.nbp;
     T *bm = am + MTP_MAX_MU * 32;
+    chain_wait();
     const int ntot = A.prefix[A.B];
     const int nw = gridDim.x * MTP_WARPS;
     const int nval = P.nmus * CSP;   // values per neighbour type: (mu, xi)
@@ -621,7 +633,7 @@ static int launch_loss_contract(const MtpProgramDev &P, const MtpArgs<T> &A, con
 }
 
 template <typename T, int KD, int CSP>
-static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArgs<T> L, void *ws, cudaStream_t st)
+static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArgs<T> L, void *ws, const void *kept, cudaStream_t st)
 {
     const MtpProgramDev &P = prog->dev;
     const LossWs W = loss_ws_layout(P, A.B, A.npad, A.ntypes, sizeof(T));
@@ -635,7 +647,11 @@ static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArg
     L.Xb = reinterpret_cast<T *>(w + W.xb);
     A.ndp = ndense_pad(P);
     A.nbp = nbasic_pad(P);
-    A.coeffs_pad = mtp_prepare<T>(A.binum, A.B, const_cast<int *>(A.prefix), A.coeffs, cpad, A.ntypes * A.ntypes * P.nmus, A.cs, CSP, st);
+    MtpZero<T> Z;
+    Z.p[0] = L.dcoeffs; Z.n[0] = (size_t)A.B * L.ncoef;
+    Z.p[1] = L.dlinear; Z.n[1] = (size_t)A.B * P.ns;
+    Z.p[2] = L.dbias; Z.n[2] = (size_t)A.B * A.ntypes;
+    A.coeffs_pad = mtp_prepare<T>(A.binum, A.B, const_cast<int *>(A.prefix), A.coeffs, cpad, A.ntypes * A.ntypes * P.nmus, A.cs, CSP, st, Z);
     AI2B_CUDA(cudaGetLastError());
     const long atoms_upper = (long)A.B * A.npad;
     const long need = (atoms_upper + MTP_WARPS - 1) / MTP_WARPS;
@@ -644,7 +660,9 @@ static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArg
     if constexpr (KD <= 6 && CSP == 8) atoms_path = mtp_atoms_supported(P, A.ntypes, A.cs, sizeof(T), (long)A.npad + A.nghost);
     if (atoms_path) {
         A.tiled = 1;
-        if (int rc = mtp_fwd_atoms<T>(P, A, st)) return rc;
+        // the energy and force call left the basic moments in its workspace if it took the same kernels
+        if (kept && mtp_moments_tiled<T>(P, A)) A.Mb = reinterpret_cast<T *>(const_cast<unsigned char *>(reinterpret_cast<const unsigned char *>(kept)) + W.base.mb);
+        else if (int rc = mtp_fwd_atoms<T>(P, A, st)) return rc;
         if (int rc = mtp_dfwd_atoms<T>(P, A, L, st)) return rc;
     } else {
         const size_t smem = sizeof(T) * (size_t)(2 * A.ndp + 2 * MTP_MAX_MU * 32) * MTP_WARPS;
@@ -689,8 +707,7 @@ static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArg
         if (int rc = kernel_setup(setup, kern, smem, MTP_WARPS * 32, &per_sm)) return rc;
         long blocks = (long)sm_count() * per_sm;
         if (blocks > need) blocks = need;
-        kern<<<(unsigned)blocks, MTP_WARPS * 32, smem, st>>>(P, A, L);
-        AI2B_CUDA(cudaGetLastError());
+        AI2B_CUDA(launch_chained(kern, (unsigned)blocks, MTP_WARPS * 32, smem, st, P, A, L));
     }
     return AI2B_OK;
 }
@@ -717,12 +734,53 @@ static int loss_forward(int e_per_atom, T *loss, T *rmse, int B, int npad, int n
     AI2B_REQUIRE(ws && ws_bytes >= 4 * sizeof(T), AI2B_ERR_WORKSPACE, "loss: workspace too small");
     cudaStream_t st = (cudaStream_t)stream;
     T *se = reinterpret_cast<T *>(ws);
-    AI2B_CUDA(cudaMemsetAsync(se, 0, 4 * sizeof(T), st));
-    mtp_loss_kernel<T><<<B, 256, 0, st>>>(loss, se, e_per_atom, npad, nghost, binum, bilist, ew, fw, vw, e_ml, e_dft, f_ml, f_dft, v_ml,
-                                          v_dft);
-    mtp_rmse_kernel<T><<<1, 32, 0, st>>>(rmse, se, B);
-    AI2B_CUDA(cudaGetLastError());
+    const int rows = ws_bytes >= 4 * sizeof(T) * (size_t)B;
+    if (!rows) AI2B_CUDA(cudaMemsetAsync(se, 0, 4 * sizeof(T), st));
+    AI2B_CUDA(launch_chained(mtp_loss_kernel<T>, (unsigned)B, 256, 0, st, loss, se, rows, e_per_atom, npad, nghost, binum, bilist, ew, fw, vw,
+                             e_ml, e_dft, f_ml, f_dft, v_ml, v_dft));
+    AI2B_CUDA(launch_chained(mtp_rmse_kernel<T>, 1u, 32, 0, st, rmse, se, rows ? B : 1, B));
     return AI2B_OK;
+}
+
+#define AI2B_LOSS_BWD_ARGS(T)                                                                                      \
+    const ai2b_mtp_program *prog, T *dcoeffs, T *dlinear, T *dbias, T ew, T fw, T vw, const T *e_ml,               \
+        const T *e_dft, const T *f_ml, const T *f_dft, const T *v_ml, const T *v_dft, int cs, T scaling,           \
+        const T *coeffs, const T *lin, const T *bias, int B, int npad, const int *binum, const int *bilist,        \
+        const int *numneigh, const int *firstneigh, const T *rcs, const int *types, int ntypes, int umax,          \
+        int nghost, T rmax, T rmin, const T *qs
+#define AI2B_LOSS_BWD_PASS                                                                                         \
+    prog, dcoeffs, dlinear, dbias, ew, fw, vw, e_ml, e_dft, f_ml, f_dft, v_ml, v_dft, cs, scaling, coeffs, lin,    \
+        bias, B, npad, binum, bilist, numneigh, firstneigh, rcs, types, ntypes, umax, nghost, rmax, rmin, qs
+
+// kept: workspace of the energy and force call on the same inputs (NULL: everything is computed here)
+template <typename T>
+static int loss_backward(AI2B_LOSS_BWD_ARGS(T), void *ws, size_t ws_bytes, const void *kept, void *stream)
+{
+    AI2B_REQUIRE(prog && dcoeffs && dlinear && dbias && e_ml && e_dft && f_ml && f_dft && (!v_ml == !v_dft) && coeffs && lin && qs &&
+                     binum && bilist && numneigh && firstneigh && rcs && types,
+                 AI2B_ERR_INVALID, "ai2b_mtp_loss_backward: NULL argument");
+    (void)bias;
+    AI2B_REQUIRE(cs >= 1 && cs <= 16, AI2B_ERR_UNSUPPORTED, "chebyshev_size %d outside 1..16", cs);
+    AI2B_REQUIRE(B >= 0 && npad >= 0 && umax >= 0 && ntypes >= 1, AI2B_ERR_INVALID, "negative size");
+    AI2B_REQUIRE(nghost == 0, AI2B_ERR_UNSUPPORTED, "the loss gradient is defined for nghost = 0 only");
+    const MtpProgramDev &P = prog->dev;
+    const int ncoef = ntypes * ntypes * P.nmus * cs;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (B == 0) return AI2B_OK;
+    if (npad == 0) {
+        AI2B_CUDA(cudaMemsetAsync(dcoeffs, 0, sizeof(T) * (size_t)B * ncoef, st));
+        AI2B_CUDA(cudaMemsetAsync(dlinear, 0, sizeof(T) * (size_t)B * P.ns, st));
+        AI2B_CUDA(cudaMemsetAsync(dbias, 0, sizeof(T) * (size_t)B * ntypes, st));
+        return AI2B_OK;
+    }
+    const size_t need = loss_ws_layout(P, B, npad, ntypes, sizeof(T)).total;
+    AI2B_REQUIRE(ws && ws_bytes >= need, AI2B_ERR_WORKSPACE, "MTP loss workspace too small: %zu < %zu bytes", ws_bytes, need);
+    MtpArgs<T> A{nullptr, nullptr, nullptr, nullptr, coeffs, lin, bias, qs, nullptr, binum, bilist, numneigh,
+                 firstneigh, types, rcs, nullptr, nullptr, nullptr, B, npad, ntypes, umax, nghost, cs, 0, 0,
+                 scaling, rmax, rmin};
+    LossArgs<T> L{e_ml, e_dft, f_ml, f_dft, v_ml, v_dft, dcoeffs, dlinear, dbias, nullptr, nullptr, ew, fw, vw, ncoef};
+    if (P.kmax <= 6 && cs <= 8) return launch_loss_bwd_v<T, 6, 8>(prog, A, L, ws, kept, st);
+    return launch_loss_bwd_v<T, 8, 16>(prog, A, L, ws, kept, st);
 }
 
 #define AI2B_DEF_LOSS(SUF, T)                                                                                      \
@@ -742,38 +800,15 @@ static int loss_forward(int e_per_atom, T *loss, T *rmse, int B, int npad, int n
         return loss_forward<T>(1, loss, rmse, B, npad, nghost, binum, bilist, ew, fw, vw, e_ml, e_dft, f_ml, f_dft, \
                                v_ml, v_dft, ws, ws_bytes, stream);                                                 \
     }                                                                                                              \
-    extern "C" int ai2b_mtp_loss_backward_##SUF(                                                                   \
-        const ai2b_mtp_program *prog, T *dcoeffs, T *dlinear, T *dbias, T ew, T fw, T vw, const T *e_ml,           \
-        const T *e_dft, const T *f_ml, const T *f_dft, const T *v_ml, const T *v_dft, int cs, T scaling,           \
-        const T *coeffs, const T *lin, const T *bias, int B, int npad, const int *binum, const int *bilist,        \
-        const int *numneigh, const int *firstneigh, const T *rcs, const int *types, int ntypes, int umax,          \
-        int nghost, T rmax, T rmin, const T *qs, void *ws, size_t ws_bytes, void *stream)                          \
+    extern "C" int ai2b_mtp_loss_backward_##SUF(AI2B_LOSS_BWD_ARGS(T), void *ws, size_t ws_bytes, void *stream)     \
     {                                                                                                              \
-        AI2B_REQUIRE(prog && dcoeffs && dlinear && dbias && e_ml && e_dft && f_ml && f_dft && (!v_ml == !v_dft) && \
-                         coeffs && lin && qs && binum && bilist && numneigh && firstneigh && rcs && types,         \
-                     AI2B_ERR_INVALID, "ai2b_mtp_loss_backward: NULL argument");                                   \
-        (void)bias;                                                                                                \
-        AI2B_REQUIRE(cs >= 1 && cs <= 16, AI2B_ERR_UNSUPPORTED, "chebyshev_size %d outside 1..16", cs);            \
-        AI2B_REQUIRE(B >= 0 && npad >= 0 && umax >= 0 && ntypes >= 1, AI2B_ERR_INVALID, "negative size");          \
-        AI2B_REQUIRE(nghost == 0, AI2B_ERR_UNSUPPORTED, "the loss gradient is defined for nghost = 0 only");       \
-        const MtpProgramDev &P = prog->dev;                                                                        \
-        const int ncoef = ntypes * ntypes * P.nmus * cs;                                                           \
-        cudaStream_t st = (cudaStream_t)stream;                                                                    \
-        if (B == 0) return AI2B_OK;                                                                                \
-        AI2B_CUDA(cudaMemsetAsync(dcoeffs, 0, sizeof(T) * (size_t)B * ncoef, st));                                 \
-        AI2B_CUDA(cudaMemsetAsync(dlinear, 0, sizeof(T) * (size_t)B * P.ns, st));                                  \
-        AI2B_CUDA(cudaMemsetAsync(dbias, 0, sizeof(T) * (size_t)B * ntypes, st));                                  \
-        if (npad == 0) return AI2B_OK;                                                                             \
-        const size_t need = loss_ws_layout(P, B, npad, ntypes, sizeof(T)).total;                                   \
-        AI2B_REQUIRE(ws && ws_bytes >= need, AI2B_ERR_WORKSPACE, "MTP loss workspace too small: %zu < %zu bytes",  \
-                     ws_bytes, need);                                                                              \
-        MtpArgs<T> A{nullptr, nullptr, nullptr, nullptr, coeffs, lin, bias, qs, nullptr, binum, bilist, numneigh,  \
-                     firstneigh, types, rcs, nullptr, nullptr, nullptr, B, npad, ntypes, umax, nghost, cs, 0, 0,   \
-                     scaling, rmax, rmin};                                                                         \
-        LossArgs<T> L{e_ml, e_dft, f_ml, f_dft, v_ml, v_dft, dcoeffs, dlinear, dbias, nullptr, nullptr, ew, fw,    \
-                      vw, ncoef};                                                                                  \
-        if (P.kmax <= 6 && cs <= 8) return launch_loss_bwd_v<T, 6, 8>(prog, A, L, ws, st);                         \
-        return launch_loss_bwd_v<T, 8, 16>(prog, A, L, ws, st);                                                    \
+        return loss_backward<T>(AI2B_LOSS_BWD_PASS, ws, ws_bytes, nullptr, stream);                                \
+    }                                                                                                              \
+    extern "C" int ai2b_mtp_loss_backward_kept_##SUF(AI2B_LOSS_BWD_ARGS(T), const void *efv_ws, void *ws,          \
+                                                     size_t ws_bytes, void *stream)                                \
+    {                                                                                                              \
+        AI2B_REQUIRE(efv_ws || B == 0, AI2B_ERR_INVALID, "ai2b_mtp_loss_backward_kept: NULL workspace");           \
+        return loss_backward<T>(AI2B_LOSS_BWD_PASS, ws, ws_bytes, efv_ws, stream);                                 \
     }
 
 AI2B_DEF_LOSS(f64, double)

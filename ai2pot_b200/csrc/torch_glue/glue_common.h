@@ -7,6 +7,11 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/custom_class.h>
+#include <c10/util/accumulate.h>
+
+#include <type_traits>
+#include <vector>
 
 #include "../../../include/ai2pot_b200.h"
 
@@ -46,28 +51,66 @@ inline at::Tensor workspace(size_t bytes, const at::Tensor &like)
     return at::empty({(int64_t)(bytes < 256 ? 256 : bytes)}, like.options().dtype(at::kByte));
 }
 
+// Several device buffers in one allocation: take() every size, then allocate() once. A training step of small cells spends its
+// time on the host, and an allocation costs as much there as half a launch.
+struct Slab {
+    at::Tensor bytes;
+    size_t used = 0;
+    size_t take(size_t n)
+    {
+        const size_t o = used;
+        used += (n + 255) & ~size_t(255);
+        return o;
+    }
+    void allocate(const at::Tensor &like) { bytes = workspace(used, like); }
+    template <typename T> T *at(size_t o) const { return reinterpret_cast<T *>(static_cast<unsigned char *>(bytes.data_ptr()) + o); }
+    at::Tensor view(size_t o, at::IntArrayRef sizes, const at::Tensor &like) const
+    {
+        const int64_t n = c10::multiply_integers(sizes) * (int64_t)like.element_size();
+        return bytes.narrow(0, (int64_t)o, n).view(like.scalar_type()).view(sizes);
+    }
+};
+
 // g[B] @ parts[k][B, n_k] for every k in one launch (what a training op's backward returns per parameter
-// tensor); results are views into one flat tensor, in the order of `parts`
-inline std::vector<at::Tensor> weighted_sums(const at::Tensor &g, const std::vector<at::Tensor> &parts)
+// tensor, in the shape of that parameter); results are views into one flat tensor, in the order of `parts`
+template <typename T>
+inline std::vector<at::Tensor> weighted_sums(const at::Tensor &g, const std::vector<const T *> &parts, const std::vector<at::Tensor> &params,
+                                             const std::vector<int> &n)
 {
     const int B = (int)g.numel(), np = (int)parts.size();
-    std::vector<int> n(np);
-    std::vector<const void *> ptr(np);
     int64_t total = 0;
-    for (int k = 0; k < np; k++) { n[k] = B ? (int)(parts[k].numel() / B) : 0; ptr[k] = parts[k].data_ptr(); total += n[k]; }
-    at::Tensor flat = at::zeros({total}, g.options());
+    for (int k = 0; k < np; k++) {
+        TORCH_CHECK(params[k].numel() == n[k], "a parameter has ", params[k].numel(), " entries, its gradient ", n[k]);
+        total += n[k];
+    }
+    at::Tensor flat = B > 0 ? at::empty({total}, g.options()) : at::zeros({total}, g.options());
     if (B > 0 && total > 0) {
         int rc;
-        if (g.scalar_type() == at::kDouble)
-            rc = ai2b_weighted_sum_rows_f64(np, (const double *const *)ptr.data(), n.data(), B, g.data_ptr<double>(), flat.data_ptr<double>(), stream());
-        else
-            rc = ai2b_weighted_sum_rows_f32(np, (const float *const *)ptr.data(), n.data(), B, g.data_ptr<float>(), flat.data_ptr<float>(), stream());
+        if constexpr (std::is_same<T, double>::value) rc = ai2b_weighted_sum_rows_f64(np, parts.data(), n.data(), B, g.data_ptr<T>(), flat.data_ptr<T>(), stream());
+        else rc = ai2b_weighted_sum_rows_f32(np, parts.data(), n.data(), B, g.data_ptr<T>(), flat.data_ptr<T>(), stream());
         TORCH_CHECK(rc == AI2B_OK, "ai2b_weighted_sum_rows: ", ai2b_last_error_string());
     }
     std::vector<at::Tensor> out(np);
     int64_t off = 0;
-    for (int k = 0; k < np; k++) { out[k] = flat.narrow(0, off, n[k]); off += n[k]; }
+    for (int k = 0; k < np; k++) {
+        out[k] = flat.as_strided(params[k].sizes(), c10::contiguous_strides(params[k].sizes()), off);
+        off += n[k];
+    }
     return out;
+}
+
+// Scalars of a training op that its backward needs (one object instead of an entry per value in the context's dictionary)
+struct LossScalars : torch::CustomClassHolder {
+    bool with_virial;
+    double w[6];
+    int64_t i[4];
+    size_t off[4];      // of e, f, v and the workspace in the saved slab
+};
+
+// [B,9] contiguous view or copy of the virial targets
+inline at::Tensor virial_rows(const at::Tensor &v, int B)
+{
+    return v.dim() == 2 && v.size(0) == B && v.size(1) == 9 && v.is_contiguous() ? v : v.reshape({B, 9}).contiguous();
 }
 
 // ZBL parameters of an op call (zbl_rmax <= 0: no correction)

@@ -88,6 +88,23 @@ struct Nb {
     int B, npad, umax, ntypes;
 };
 
+// ai2b_mtp_efv_* on raw outputs (v NULL: energy and forces)
+template <typename T>
+void efv_call(const ai2b_mtp_program *prog, T *e, T *f, T *v, int64_t cs, double scaling, const at::Tensor &coeffs, const at::Tensor &lin,
+              const at::Tensor &bias, const at::Tensor &binum, const at::Tensor &bilist, const at::Tensor &bnumneigh,
+              const at::Tensor &bfirstneigh, const at::Tensor &brcs, const at::Tensor &btypes, int ntypes, int64_t nghost, double rmax,
+              double rmin, const at::Tensor &qs, void *ws, size_t ws_bytes)
+{
+    auto call = [&](auto fn) {
+        return fn(prog, e, f, v, (int)cs, (T)scaling, fptr<T>(coeffs, brcs, "coeffs"), fptr<T>(lin, brcs, "linear_coeffs"),
+                  fptr<T>(bias, brcs, "type_bias"), (int)binum.size(0), (int)bnumneigh.size(1), iptr(binum, "binum"), iptr(bilist, "bilist"),
+                  iptr(bnumneigh, "bnumneigh"), iptr(bfirstneigh, "bfirstneigh"), fptr<T>(brcs, brcs, "brcs"), iptr(btypes, "btypes"), ntypes,
+                  (int)bfirstneigh.size(2), (int)nghost, (T)rmax, (T)rmin, fptr<T>(qs, brcs, "q_scaler"), ws, ws_bytes, stream());
+    };
+    if constexpr (std::is_same<T, double>::value) check(call(ai2b_mtp_efv_f64), "ai2b_mtp_efv");
+    else check(call(ai2b_mtp_efv_f32), "ai2b_mtp_efv");
+}
+
 template <typename T>
 variable_list efv_impl(bool with_virial, int64_t cs, double scaling, const at::Tensor &coeffs, const at::Tensor &lin,
                        const at::Tensor &bias, int64_t nm, const at::Tensor &basic, const at::Tensor &times, const at::Tensor &map,
@@ -97,30 +114,14 @@ variable_list efv_impl(bool with_virial, int64_t cs, double scaling, const at::T
 {
     require_cuda(brcs, "brcs");
     c10::cuda::CUDAGuard guard(brcs.device());
-    const int B = (int)binum.size(0), npad = (int)bnumneigh.size(1), umax = (int)bfirstneigh.size(2), ntypes = (int)type_map.size(0);
+    const int B = (int)binum.size(0), npad = (int)bnumneigh.size(1), ntypes = (int)type_map.size(0);
     const ai2b_mtp_program *prog = program_for((int)nm, basic, times, map, (int)nmus, brcs.get_device());
     // outputs shaped as the reference allocates them (src/linearMtpOp.cc:2890-2892)
     at::Tensor e = at::empty({B}, brcs.options()), f = at::empty({B, npad + nghost, 3}, brcs.options());
     at::Tensor v = with_virial ? at::empty({B, 9}, brcs.options()) : at::Tensor();
     at::Tensor ws = workspace(ai2b_mtp_workspace_bytes(prog, B, npad, ntypes), brcs);
-    auto fn = [&](auto tag) {
-        using U = decltype(tag);
-        if constexpr (std::is_same<U, double>::value)
-            return ai2b_mtp_efv_f64(prog, e.data_ptr<double>(), f.data_ptr<double>(), with_virial ? v.data_ptr<double>() : nullptr,
-                                    (int)cs, scaling, fptr<double>(coeffs, brcs, "coeffs"), fptr<double>(lin, brcs, "linear_coeffs"),
-                                    fptr<double>(bias, brcs, "type_bias"), B, npad, iptr(binum, "binum"), iptr(bilist, "bilist"),
-                                    iptr(bnumneigh, "bnumneigh"), iptr(bfirstneigh, "bfirstneigh"), fptr<double>(brcs, brcs, "brcs"),
-                                    iptr(btypes, "btypes"), ntypes, umax, (int)nghost, rmax, rmin, fptr<double>(qs, brcs, "q_scaler"),
-                                    ws.data_ptr(), (size_t)ws.numel(), stream());
-        else
-            return ai2b_mtp_efv_f32(prog, e.data_ptr<float>(), f.data_ptr<float>(), with_virial ? v.data_ptr<float>() : nullptr,
-                                    (int)cs, (float)scaling, fptr<float>(coeffs, brcs, "coeffs"), fptr<float>(lin, brcs, "linear_coeffs"),
-                                    fptr<float>(bias, brcs, "type_bias"), B, npad, iptr(binum, "binum"), iptr(bilist, "bilist"),
-                                    iptr(bnumneigh, "bnumneigh"), iptr(bfirstneigh, "bfirstneigh"), fptr<float>(brcs, brcs, "brcs"),
-                                    iptr(btypes, "btypes"), ntypes, umax, (int)nghost, (float)rmax, (float)rmin,
-                                    fptr<float>(qs, brcs, "q_scaler"), ws.data_ptr(), (size_t)ws.numel(), stream());
-    };
-    check(fn(T{}), "ai2b_mtp_efv");
+    efv_call<T>(prog, e.data_ptr<T>(), f.data_ptr<T>(), with_virial ? v.data_ptr<T>() : nullptr, cs, scaling, coeffs, lin, bias, binum, bilist,
+                bnumneigh, bfirstneigh, brcs, btypes, ntypes, nghost, rmax, rmin, qs, ws.data_ptr(), (size_t)ws.numel());
     if (with_virial) return {e, f, v};
     return {e, f};
 }

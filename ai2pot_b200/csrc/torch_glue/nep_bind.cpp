@@ -9,6 +9,24 @@ using torch::autograd::variable_list;
 
 namespace {
 
+// ai2b_nep_efv_* on raw outputs (v NULL: energy and forces)
+template <typename T>
+void nep_efv_call(T *e, T *f, T *v, int64_t cs, int64_t n_r, int64_t n_a, int64_t l_max, const at::Tensor &coeffs, const at::Tensor &w0,
+                  const at::Tensor &b0, const at::Tensor &w1, const at::Tensor &bias, const at::Tensor &binum, const at::Tensor &bilist,
+                  const at::Tensor &bnumneigh, const at::Tensor &bfirstneigh, const at::Tensor &brcs, const at::Tensor &btypes, int ntypes,
+                  int64_t nghost, double rc_r, double rc_a, const at::Tensor &qs, void *ws, size_t ws_bytes)
+{
+    auto call = [&](auto fn) {
+        return fn(e, f, v, (int)cs, (int)n_r, (int)n_a, (int)l_max, (int)(w1.numel() / ntypes), fptr<T>(coeffs, brcs, "coeffs"),
+                  fptr<T>(w0, brcs, "w0"), fptr<T>(b0, brcs, "b0"), fptr<T>(w1, brcs, "w1"), fptr<T>(bias, brcs, "type_bias"),
+                  (int)binum.size(0), (int)bnumneigh.size(1), iptr(binum, "binum"), iptr(bilist, "bilist"), iptr(bnumneigh, "bnumneigh"),
+                  iptr(bfirstneigh, "bfirstneigh"), fptr<T>(brcs, brcs, "brcs"), iptr(btypes, "btypes"), ntypes, (int)bfirstneigh.size(2),
+                  (int)nghost, (T)rc_r, (T)rc_a, fptr<T>(qs, brcs, "q_scaler"), ws, ws_bytes, stream());
+    };
+    if constexpr (std::is_same<T, double>::value) check(call(ai2b_nep_efv_f64), "ai2b_nep_efv");
+    else check(call(ai2b_nep_efv_f32), "ai2b_nep_efv");
+}
+
 variable_list nep_efv(bool with_virial, int64_t cs, int64_t n_r, int64_t n_a, int64_t l_max, const at::Tensor &coeffs,
                       const at::Tensor &w0, const at::Tensor &b0, const at::Tensor &w1, const at::Tensor &bias,
                       const at::Tensor &binum, const at::Tensor &bilist, const at::Tensor &bnumneigh, const at::Tensor &bfirstneigh,
@@ -17,29 +35,20 @@ variable_list nep_efv(bool with_virial, int64_t cs, int64_t n_r, int64_t n_a, in
 {
     require_cuda(brcs, "brcs");
     c10::cuda::CUDAGuard guard(brcs.device());
-    const int B = (int)binum.size(0), npad = (int)bnumneigh.size(1), umax = (int)bfirstneigh.size(2), ntypes = (int)type_map.size(0);
-    const int nneu = (int)(w1.numel() / ntypes);
+    const int B = (int)binum.size(0), npad = (int)bnumneigh.size(1), ntypes = (int)type_map.size(0);
     at::Tensor e = at::empty({B}, brcs.options()), f = at::empty({B, npad + nghost, 3}, brcs.options());
     at::Tensor v = with_virial ? at::empty({B, 9}, brcs.options()) : at::Tensor();
     const bool f64 = brcs.scalar_type() == at::kDouble;
     TORCH_CHECK(f64 || brcs.scalar_type() == at::kFloat, "brcs must be float32 or float64");
     at::Tensor ws = workspace(ai2b_nep_workspace_bytes(B, ntypes, (int)n_r, (int)n_a, (int)cs, f64 ? 1 : 0), brcs);
-    int rc;
-    if (f64)
-        rc = ai2b_nep_efv_f64(e.data_ptr<double>(), f.data_ptr<double>(), with_virial ? v.data_ptr<double>() : nullptr, (int)cs, (int)n_r,
-                              (int)n_a, (int)l_max, nneu, fptr<double>(coeffs, brcs, "coeffs"), fptr<double>(w0, brcs, "w0"),
-                              fptr<double>(b0, brcs, "b0"), fptr<double>(w1, brcs, "w1"), fptr<double>(bias, brcs, "type_bias"), B, npad,
-                              iptr(binum, "binum"), iptr(bilist, "bilist"), iptr(bnumneigh, "bnumneigh"), iptr(bfirstneigh, "bfirstneigh"),
-                              fptr<double>(brcs, brcs, "brcs"), iptr(btypes, "btypes"), ntypes, umax, (int)nghost, rc_r, rc_a,
-                              fptr<double>(qs, brcs, "q_scaler"), ws.data_ptr(), (size_t)ws.numel(), stream());
-    else
-        rc = ai2b_nep_efv_f32(e.data_ptr<float>(), f.data_ptr<float>(), with_virial ? v.data_ptr<float>() : nullptr, (int)cs, (int)n_r,
-                              (int)n_a, (int)l_max, nneu, fptr<float>(coeffs, brcs, "coeffs"), fptr<float>(w0, brcs, "w0"),
-                              fptr<float>(b0, brcs, "b0"), fptr<float>(w1, brcs, "w1"), fptr<float>(bias, brcs, "type_bias"), B, npad,
-                              iptr(binum, "binum"), iptr(bilist, "bilist"), iptr(bnumneigh, "bnumneigh"), iptr(bfirstneigh, "bfirstneigh"),
-                              fptr<float>(brcs, brcs, "brcs"), iptr(btypes, "btypes"), ntypes, umax, (int)nghost, (float)rc_r, (float)rc_a,
-                              fptr<float>(qs, brcs, "q_scaler"), ws.data_ptr(), (size_t)ws.numel(), stream());
-    check(rc, "ai2b_nep_efv");
+    auto run = [&](auto tag) {
+        using T = decltype(tag);
+        nep_efv_call<T>(e.data_ptr<T>(), f.data_ptr<T>(), with_virial ? v.data_ptr<T>() : nullptr, cs, n_r, n_a, l_max, coeffs, w0, b0, w1,
+                        bias, binum, bilist, bnumneigh, bfirstneigh, brcs, btypes, ntypes, nghost, rc_r, rc_a, qs, ws.data_ptr(),
+                        (size_t)ws.numel());
+    };
+    if (f64) run(double{});
+    else run(float{});
     apply_zbl(zbl, e, f, v, binum, bilist, bnumneigh, bfirstneigh, brcs, btypes, type_map, nghost);
     if (with_virial) return {e, f, v};
     return {e, f};

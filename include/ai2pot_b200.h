@@ -105,14 +105,18 @@ AI2B_DECL_MTP_DESC(f32, float)
  * rmse[3] = {energy, force, virial} (LinearMtpLoss<T>::find_loss / find_ef_loss,
  * source/descriptor/mtpr/include/linearMtpLoss.h:138-210; RMSE definitions
  * source/descriptor/mtpr/src/linearMtpOp.cc:885-911). d_bvirial_ml / d_bvirial_dft NULL gives
- * the energy + force variant. Needs 32 bytes of workspace.
+ * the energy + force variant. Needs 32 bytes of workspace; with 4 * batch_size values of T or more
+ * it takes one launch fewer.
  * ai2b_mtp_loss_backward_*: analytic gradient of every structure's loss w.r.t. coeffs
  * [B,ntypes*ntypes*nmus*chebyshev_size], linear_coeffs [B,alpha_scalar_moments] and type_bias
  * [B,ntypes] (find_loss_backward / find_ef_loss_backward, linearMtpLoss.h:212-569; CUDA
  * launcher gpu/include/linearMtpLoss.cuh:1015). The model E/F/V of the same inputs are passed
  * in (the reference recomputes them inside its backward). Outputs are overwritten.
  * d_bforce_ml has row stride natoms_pad + nghost, d_bforce_dft natoms_pad; nghost must be 0
- * for the gradient. Workspace: ai2b_mtp_loss_workspace_bytes. */
+ * for the gradient. Workspace: ai2b_mtp_loss_workspace_bytes.
+ * ai2b_mtp_loss_backward_kept_*: the same with the workspace that an ai2b_mtp_efv_* / ai2b_mtp_ef_*
+ * call was given for the same program, coefficients, lists and sizes, unchanged since that call:
+ * basic moments that it left there are not computed again. */
 size_t ai2b_mtp_loss_workspace_bytes(const ai2b_mtp_program *prog, int batch_size, int natoms_pad,
                                      int ntypes);
 #define AI2B_DECL_MTP_LOSS(SUF, T)                                                               \
@@ -131,6 +135,17 @@ size_t ai2b_mtp_loss_workspace_bytes(const ai2b_mtp_program *prog, int batch_siz
         int natoms_pad, const int *d_binum, const int *d_bilist, const int *d_bnumneigh,         \
         const int *d_bfirstneigh, const T *d_brcs, const int *d_btypes, int ntypes, int umax,    \
         int nghost, T rmax, T rmin, const T *d_q_scaler, void *d_workspace,                      \
+        size_t workspace_bytes, void *stream);                                                   \
+    int ai2b_mtp_loss_backward_kept_##SUF(                                                       \
+        const ai2b_mtp_program *prog, T *d_bloss_der2coeffs, T *d_bloss_der2linear_coeffs,       \
+        T *d_bloss_der2type_bias, T e_weight, T f_weight, T v_weight, const T *d_betot_ml,       \
+        const T *d_betot_dft, const T *d_bforce_ml, const T *d_bforce_dft,                       \
+        const T *d_bvirial_ml, const T *d_bvirial_dft, int chebyshev_size, T scaling,            \
+        const T *d_coeffs, const T *d_linear_coeffs, const T *d_type_bias, int batch_size,       \
+        int natoms_pad, const int *d_binum, const int *d_bilist, const int *d_bnumneigh,         \
+        const int *d_bfirstneigh, const T *d_brcs, const int *d_btypes, int ntypes, int umax,    \
+        int nghost, T rmax, T rmin, const T *d_q_scaler,                                         \
+        const void *d_efv_workspace, void *d_workspace,                                          \
         size_t workspace_bytes, void *stream);
 AI2B_DECL_MTP_LOSS(f64, double)
 AI2B_DECL_MTP_LOSS(f32, float)

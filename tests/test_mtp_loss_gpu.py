@@ -169,3 +169,32 @@ def test_contraction_tile_edges(checkers, level, B, nmin, nmax, dt):
         assert util.relerr(a.cpu().numpy(), r) < 2 * tol, name
     if dt == torch.float64:
         assert util.relerr(capi.mtp_descriptors(prog, md, nbd).cpu().numpy(), chk.mtp_descriptors(g["model"], nb)) < tol
+
+
+@pytest.mark.parametrize("B,cs,dt", [(1, 8, torch.float64), (9, 8, torch.float64), (9, 8, torch.float32), (3, 9, torch.float64)])
+def test_loss_op_keeps_the_moments(checkers, B, cs, dt):
+    """Backward of the op on the moments of its forward (and, with nine Chebyshev functions, without) against the backward
+    that computes everything itself; twice through the same graph, unequal weights, RMSEs in the graph."""
+    from ai2pot_b200 import fromcc
+    g, nb = util.training_batch(_chk(checkers), level=16, B=B, seed=8, nmin=5, nmax=40)
+    m, tb = dict(g["model"]), g["model"]["tables"]
+    if cs != m["chebyshev_size"]:
+        m["chebyshev_size"], m["coeffs"] = cs, np.random.default_rng(1).normal(0, 0.1, 9 * tb["nmus"] * cs)
+        g["model"] = m
+    nb = dict(nb, brcs=nb["brcs"].astype(np.float64 if dt == torch.float64 else np.float32))
+    prog, md, nbd, (E, F, V) = _dev(g, nb, dt)
+    e, f, v = capi.mtp_efv(prog, md, nbd)
+    ref = capi.mtp_loss_backward(prog, md, nbd, (1.0, 2.0, 0.5), e, E, f, F, v, V)
+    c = lambda a, d=None: torch.from_numpy(np.ascontiguousarray(a)).to("cuda", d)
+    params = [c(m[k], dt).requires_grad_(True) for k in ("coeffs", "linear_coeffs", "type_bias")]
+    z = torch.zeros(36, dtype=dt, device="cuda")
+    out = fromcc.linearMtpToLossOp(1.0, 2.0, 0.5, E, F, V, cs, m["scaling"], *params, tb["alpha_moments_count"], c(tb["alpha_index_basic"]),
+                                   c(tb["alpha_index_times"]), c(tb["alpha_moment_mapping"]), tb["nmus"],
+                                   *(nbd[k] for k in ("binum", "bilist", "bnumneigh", "bfirstneigh", "brcs", "btypes")),
+                                   torch.arange(3, dtype=torch.int32, device="cuda"), 0, m["rmax"], m["rmin"], c(m["q_scaler"], dt), 0.0, 0.0, z, z)
+    w = torch.linspace(0.5, 1.5, B, dtype=dt, device="cuda")
+    total = (w * out[0]).sum()
+    tol = 1e-10 if dt == torch.float64 else 1e-5
+    for _ in range(2):
+        for p, a, r in zip(params, torch.autograd.grad(total, params, retain_graph=True), ref):
+            assert a.shape == p.shape and util.relerr(a.cpu().numpy(), (w.double() @ r.reshape(B, -1).double()).cpu().numpy()) < tol
