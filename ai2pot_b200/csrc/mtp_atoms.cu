@@ -279,29 +279,40 @@ __global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_ke
                 }
                 __syncthreads();
                 if constexpr (NACC > 0) {
-#pragma unroll 2
+                    // (the four warps run code of their own; the derivatives twice over would not stay in the instruction cache)
+#pragma unroll (DERIV ? 1 : 2)
                     for (int jj = 0; jj < cnt; jj++) {
                         const T *s = st + (size_t)jj * NV * 32 + lane;
                         Powers<T, KD> pw;
                         pw.set(s[0], s[32], s[64]);
-                        T f[SIG::NMUS], a[SIG::NMUS], qx = T(0), qy = T(0), qz = T(0);
+                        T f[SIG::NMUS], a[SIG::NMUS], dx[KD + 1], dy[KD + 1], dz[KD + 1];
                         static_for<0, SIG::NMUS>([&](auto mm) { f[decltype(mm)::value] = s[(3 + decltype(mm)::value) * 32]; });
                         if constexpr (DERIV) {
                             static_for<0, SIG::NMUS>([&](auto mm) { a[decltype(mm)::value] = s[(3 + SIG::NMUS + decltype(mm)::value) * 32]; });
-                            qx = s[(3 + 2 * SIG::NMUS) * 32]; qy = s[(4 + 2 * SIG::NMUS) * 32]; qz = s[(5 + 2 * SIG::NMUS) * 32];
+                            const T qx = s[(3 + 2 * SIG::NMUS) * 32], qy = s[(4 + 2 * SIG::NMUS) * 32], qz = s[(5 + 2 * SIG::NMUS) * 32];
+#pragma unroll
+                            for (int k = 1; k <= KD; k++) {      // q_x d/dx of the powers, and so on
+                                dx[k] = T(k) * qx * pw.x[k - 1]; dy[k] = T(k) * qy * pw.y[k - 1]; dz[k] = T(k) * qz * pw.z[k - 1];
+                            }
                         }
                         static_for<0, KD + 1>([&](auto dd) {
                             constexpr int D = decltype(dd)::value;
                             if constexpr (SIG::group(D) == G) {
                                 static_for<0, ndeg(D)>([&](auto qq) {
                                     constexpr int Q = decltype(qq)::value;
-                                    const T m = mono<T, KD, D, Q>(pw);
-                                    T dm = T(0);
-                                    if constexpr (DERIV) {   // q . grad of the monomial
+                                    T m, dm = T(0);
+                                    if constexpr (DERIV) {   // the monomial x^a (y^b z^c) and q . grad of it by the product rule
                                         constexpr Exp3 e = deg_exp(D, Q);
-                                        if constexpr (e.x > 0) dm = fma(qx * T(e.x), pw.x[e.x - 1] * pw.y[e.y] * pw.z[e.z], dm);
-                                        if constexpr (e.y > 0) dm = fma(qy * T(e.y), pw.x[e.x] * pw.y[e.y - 1] * pw.z[e.z], dm);
-                                        if constexpr (e.z > 0) dm = fma(qz * T(e.z), pw.x[e.x] * pw.y[e.y] * pw.z[e.z - 1], dm);
+                                        const T yz = e.y == 0 ? pw.z[e.z] : e.z == 0 ? pw.y[e.y] : pw.y[e.y] * pw.z[e.z];
+                                        T dyz = T(0);
+                                        if constexpr (e.y > 0 && e.z > 0) dyz = fma(dy[e.y], pw.z[e.z], pw.y[e.y] * dz[e.z]);
+                                        else if constexpr (e.y > 0) dyz = dy[e.y];
+                                        else if constexpr (e.z > 0) dyz = dz[e.z];
+                                        if constexpr (e.x == 0) { m = yz; dm = dyz; }
+                                        else if constexpr (e.x == D) { m = pw.x[e.x]; dm = dx[e.x]; }
+                                        else { m = pw.x[e.x] * yz; dm = fma(dx[e.x], yz, pw.x[e.x] * dyz); }
+                                    } else {
+                                        m = mono<T, KD, D, Q>(pw);
                                     }
                                     static_for<0, SIG::cnt(D)>([&](auto mm) {
                                         constexpr int mu = decltype(mm)::value;
@@ -488,6 +499,184 @@ __global__ void __launch_bounds__(AT_WARPS * 32, 3) mtp_force_atoms_kernel(const
     }
 }
 
+// ---- gradient w.r.t. the radial coefficients (linearMtpLoss.h:436-569) ---------------------------------
+// d loss / d c[ti][tj][mu][xi] = sum over pairs of W_mu f_xi + D_mu f'_xi with W_mu = X_mu + q . grad E_mu, D_mu = (p . u) E_mu:
+// E_mu, X_mu the polynomials of the two adjoint rows, p the pair weight, q its part across u over r.
+// A block works on a tile of 32 atoms, lanes = atoms, CO_WARPS neighbour slots at a time:
+//  1. every warp takes a slot: value of X, value and directional derivative of E come out of one nested sum (three multiply-adds
+//     per coefficient); W, D, f, f' and the neighbour type go to shared memory as [slot][value][32 atoms];
+//  2. every thread owns entries (mu, xi) of its atom and adds the slots to its place in a table [tj][mu, xi][32 atoms]: no
+//     atomics, no reduction across lanes. The table is summed over the atoms of a type once per tile.
+// Level 16, fp64, 9,323 atoms: 87 us and 17 million warp instructions; a warp per atom with lanes = neighbours and a transposing
+// reduction per type took 99 us and 40 million. Bound by latency: one block of 16 warps per SM is what registers and shared
+// memory hold. (The derivatives of the forward kernel by the product rule instead of three products each: 76 -> 68 us.)
+constexpr int CO_WARPS = 16;
+constexpr int CO_NV = 24;       // values of a pair: W[4], D[4], f[8], f'[8]
+constexpr int CO_RS = 33;       // row stride of the table: atoms along a row, read down the columns at the end
+template <typename T, typename SIG>
+constexpr size_t coeff_atoms_smem(int ntypes)
+{
+    return sizeof(T) * (2 * (size_t)SIG::NDENSE * 32 + (size_t)CO_WARPS * CO_NV * 32 + (((size_t)ntypes * 32 * CO_RS + 3) & ~size_t(3))) +
+           sizeof(int) * (CO_WARPS + 2) * 32 + tile_rows_bytes<T>();
+}
+
+template <typename T, typename SIG, int CSP>
+__global__ void __launch_bounds__(CO_WARPS * 32, 1) mtp_coeff_atoms_kernel(const MtpProgramDev P, const MtpArgs<T> A, const LossArgs<T> L)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int KD = SIG::KD, NT = CO_WARPS * 32;
+    static_assert(SIG::NMUS <= 4 && CSP == 8, "32 entries (mu, xi)");
+    using V2 = typename Vec2<T>::type;
+    V2 *EXs = reinterpret_cast<V2 *>(smem_raw);      // {E, X} [NDENSE][32]
+    T *recs = reinterpret_cast<T *>(EXs + (size_t)SIG::NDENSE * 32);
+    T *table = recs + (size_t)CO_WARPS * CO_NV * 32;
+    int *tjs = reinterpret_cast<int *>(table + (((size_t)A.ntypes * 32 * CO_RS + 3) & ~size_t(3)));      // [slot][32]; -1: no pair
+    int *at_ti = tjs + CO_WARPS * 32, *at_b = at_ti + 32;
+    TileRows<T> tr;
+    tr.bind(reinterpret_cast<unsigned char *>(at_b + 32));
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const T inv_range = T(1) / (A.rmax - A.rmin);
+    chain_wait();
+    const int ntot = total_atoms(A);
+    const int ntiles = (ntot + MTP_TILE - 1) / MTP_TILE;
+
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        if (tile != (int)blockIdx.x) __syncthreads();     // the previous tile's rows and table are no longer read
+        {
+            const T *src = L.Xb + 2 * (size_t)tile * A.ndp * MTP_TILE;
+            T *dst = reinterpret_cast<T *>(EXs);
+            constexpr int CH = 16 / (int)sizeof(T);
+            for (int c = threadIdx.x; c < 2 * SIG::NDENSE * 32 / CH; c += NT) __pipeline_memcpy_async(dst + c * CH, src + c * CH, 16);
+            __pipeline_commit();
+        }
+        TileAtom<T> at;
+        at.set(A, tile * MTP_TILE + lane, ntot);
+        const int nmax = warp_max_int(at.nn);
+        const size_t row = at.slot * A.umax;
+        const int nstruct = at.valid ? A.binum[at.b] : 1;
+        if (warp == 0) {
+            tr.describe(lane, row, (size_t)(at.types_b - A.types), at.nn);
+            at_ti[lane] = at.ti;
+            at_b[lane] = at.b;
+        }
+        for (int i = threadIdx.x; i < A.ntypes * 32 * CO_RS; i += NT) table[i] = T(0);
+        __syncthreads();
+        tr.template stage<NT>(A.rcs, A.firstneigh, A.types, A.umax);
+        __pipeline_wait_prior(0);
+
+        const V2 *exl = EXs + lane;
+        for (int j0 = 0; j0 < nmax; j0 += CO_WARPS) {
+            __syncthreads();     // rows staged / the previous slots added up
+            const int j = j0 + warp;
+            if (j < nmax) {
+                T x = T(0), y = T(0), z = T(0);
+                int nj = 0, tj = 0;
+                bool act = j < at.nn;
+                if (j < TR_SLOTS) {
+                    const T *p = tr.pos + lane * TR_RS + 3 * j;
+                    const int w = tr.idx[lane * TR_IS + j];
+                    if (act) { x = p[0]; y = p[1]; z = p[2]; }
+                    nj = w & TR_INDEX_MASK;
+                    tj = w >> TR_TYPE_SHIFT;
+                } else if (act) {
+                    const T *rc = A.rcs + (row + j) * 3;
+                    x = rc[0]; y = rc[1]; z = rc[2];
+                    nj = A.firstneigh[row + j];
+                    tj = at.types_b[nj];
+                }
+                const T r2 = x * x + y * y + z * z;
+                const T ri = r2 > T(0) ? grsqrt(r2) : T(0), r = r2 * ri;
+                act = act && (r <= A.rmax) && (r > T(0));
+                T px = T(0), py = T(0), pz = T(0);
+                if (act) pair_weight(A, L, at.b, nstruct, at.ci, nj, x, y, z, px, py, pz);
+                T *my = recs + (size_t)warp * CO_NV * 32 + lane;
+                {
+                    T q[CSP], dq[CSP];
+                    mtp_radial_basis<T, CSP>(act ? r : A.rmax, A.rmax, A.rmin, A.scaling, q, dq, inv_range);
+#pragma unroll
+                    for (int k = 0; k < CSP; k++) { my[(8 + k) * 32] = q[k]; my[(16 + k) * 32] = dq[k]; }
+                }
+                tjs[warp * 32 + lane] = act ? tj : -1;
+                const T rinv = act ? ri : T(0), ux = x * rinv, uy = y * rinv, uz = z * rinv;
+                const T ppar = px * ux + py * uy + pz * uz;
+                const T qx = (px - ppar * ux) * rinv, qy = (py - ppar * uy) * rinv, qz = (pz - ppar * uz) * rinv;
+                T X[KD + 1], Y[KD + 1], Z[KD + 1], dX[KD + 1], dY[KD + 1], dZ[KD + 1];
+                X[0] = Y[0] = Z[0] = T(1);
+                if constexpr (KD >= 1) { X[1] = ux; Y[1] = uy; Z[1] = uz; }
+#pragma unroll
+                for (int k = 2; k <= KD; k++) {
+                    X[k] = X[k / 2] * X[k - k / 2]; Y[k] = Y[k / 2] * Y[k - k / 2]; Z[k] = Z[k / 2] * Z[k - k / 2];
+                }
+#pragma unroll
+                for (int k = 1; k <= KD; k++) { dX[k] = T(k) * qx * X[k - 1]; dY[k] = T(k) * qy * Y[k - 1]; dZ[k] = T(k) * qz * Z[k - 1]; }
+                static_for<0, SIG::NMUS>([&](auto mm) {
+                    constexpr int mu = decltype(mm)::value, K = SIG::k(mu), base = SIG::doff(mu);
+                    // E, q . grad E and X of this radial function by nested sums over the z, y and x exponents
+                    T Pv = T(0), Pd = T(0), Xv = T(0);
+                    static_for<0, K + 1>([&](auto aa) {
+                        constexpr int a = decltype(aa)::value;
+                        T S = T(0), Sd = T(0), SX = T(0);
+                        static_for<0, K - a + 1>([&](auto bb) {
+                            constexpr int b = decltype(bb)::value;
+                            T R = T(0), Rd = T(0), RX = T(0);
+                            static_for<0, K - a - b + 1>([&](auto cc) {
+                                constexpr int c = decltype(cc)::value, I = (base + canon_index(a, b, c)) * 32;
+                                const V2 ex = exl[I];
+                                const T e = ex.x, xe = ex.y;
+                                if constexpr (c == 0) { R = e; RX = xe; }
+                                else { R = fma(e, Z[c], R); RX = fma(xe, Z[c], RX); Rd = fma(e, dZ[c], Rd); }
+                            });
+                            if constexpr (b == 0) { S = R; SX = RX; Sd = Rd; }
+                            else { S = fma(Y[b], R, S); SX = fma(Y[b], RX, SX); Sd = fma(Y[b], Rd, fma(dY[b], R, Sd)); }
+                        });
+                        if constexpr (a == 0) { Pv = S; Xv = SX; Pd = Sd; }
+                        else { Pv = fma(X[a], S, Pv); Xv = fma(X[a], SX, Xv); Pd = fma(X[a], Sd, fma(dX[a], S, Pd)); }
+                    });
+                    my[mu * 32] = Xv + Pd;
+                    my[(4 + mu) * 32] = ppar * Pv;
+                });
+            }
+            __syncthreads();
+            const int cnt = min(CO_WARPS, nmax - j0);
+            constexpr int NE = SIG::NMUS * CSP, EPT = (NE + CO_WARPS - 1) / CO_WARPS;
+            for (int s = 0; s < cnt; s++) {
+                const T *v = recs + (size_t)s * CO_NV * 32 + lane;
+                const int tj = tjs[s * 32 + lane];
+                if (tj >= 0) {
+#pragma unroll
+                    for (int k = 0; k < EPT; k++) {
+                        const int e = warp + k * CO_WARPS, mu = e >> 3, xi = e & 7;
+                        if (e < NE) {
+                            T *o = table + ((size_t)tj * 32 + e) * CO_RS + lane;
+                            *o = fma(v[mu * 32], v[(8 + xi) * 32], fma(v[(4 + mu) * 32], v[(16 + xi) * 32], *o));
+                        }
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        // entry (tj, mu, xi) summed over the atoms of type ti; a tile may hold the atoms of several structures
+        for (int i = threadIdx.x; i < A.ntypes * A.ntypes * 32; i += NT) {
+            const int e = i & 31, tj = (i >> 5) % A.ntypes, ti = (i >> 5) / A.ntypes, mu = e >> 3, xi = e & 7;
+            if (mu >= SIG::NMUS || xi >= A.cs) continue;
+            const T *v = table + ((size_t)tj * 32 + e) * CO_RS;
+            T *out = L.dcoeffs + ((size_t)(ti * A.ntypes + tj) * SIG::NMUS + mu) * A.cs + xi;
+            T acc = T(0);
+            int b = at_b[0];
+#pragma unroll 4
+            for (int l = 0; l < 32; l++) {
+                if (at_b[l] != b) {
+                    if (acc != T(0)) atomicAdd(out + (size_t)b * L.ncoef, acc);
+                    acc = T(0);
+                    b = at_b[l];
+                }
+                if (at_ti[l] == ti) acc += v[l];
+            }
+            if (acc != T(0)) atomicAdd(out + (size_t)b * L.ncoef, acc);
+        }
+    }
+}
+
 // ---- host side ------------------------------------------------------------------------------------
 template <typename SIG>
 static bool sig_matches(const MtpProgramDev &P)
@@ -527,6 +716,14 @@ bool mtp_atoms_supported(const MtpProgramDev &P, int ntypes, int cs, size_t elem
     return false;
 }
 
+bool mtp_coeff_atoms_supported(const MtpProgramDev &P, int ntypes, size_t elem)
+{
+#define AI2B_SIG_FITS(S) return (elem == 8 ? coeff_atoms_smem<double, S>(ntypes) : coeff_atoms_smem<float, S>(ntypes)) <= 226 * 1024;
+    AI2B_FOR_SIG(P, AI2B_SIG_FITS)
+#undef AI2B_SIG_FITS
+    return false;
+}
+
 template <typename T, typename SIG, bool DERIV>
 static int launch_fwd_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, const LossArgs<T> &L, cudaStream_t st)
 {
@@ -557,6 +754,31 @@ static int launch_force_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, cudaS
     if (blocks > tiles) blocks = tiles;
     AI2B_CUDA(launch_chained(kern, (unsigned)blocks, AT_WARPS * 32, smem, st, P, A));
     return AI2B_OK;
+}
+
+template <typename T, typename SIG>
+static int launch_coeff_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, const LossArgs<T> &L, cudaStream_t st)
+{
+    const size_t smem = coeff_atoms_smem<T, SIG>(A.ntypes);
+    auto kern = mtp_coeff_atoms_kernel<T, SIG, AT_CSP>;
+    static KernelSetup setup;
+    int per_sm = 1;
+    if (int rc = kernel_setup(setup, kern, smem, CO_WARPS * 32, &per_sm)) return rc;
+    long tiles = ((long)A.B * A.npad + MTP_TILE - 1) / MTP_TILE;
+    long blocks = (long)sm_count() * per_sm;
+    if (blocks > tiles) blocks = tiles;
+    AI2B_CUDA(launch_chained(kern, (unsigned)blocks, CO_WARPS * 32, smem, st, P, A, L));
+    return AI2B_OK;
+}
+
+template <typename T>
+int mtp_coeff_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, const LossArgs<T> &L, cudaStream_t st)
+{
+#define AI2B_SIG_COEFF(S) return launch_coeff_atoms<T, S>(P, A, L, st);
+    AI2B_FOR_SIG(P, AI2B_SIG_COEFF)
+#undef AI2B_SIG_COEFF
+    set_error("no lanes-as-atoms MTP kernel for these tables");
+    return AI2B_ERR_UNSUPPORTED;
 }
 
 template <typename T>
@@ -593,6 +815,8 @@ template int mtp_fwd_atoms<float>(const MtpProgramDev &, const MtpArgs<float> &,
 template int mtp_fwd_atoms<double>(const MtpProgramDev &, const MtpArgs<double> &, cudaStream_t);
 template int mtp_dfwd_atoms<float>(const MtpProgramDev &, const MtpArgs<float> &, const LossArgs<float> &, cudaStream_t);
 template int mtp_dfwd_atoms<double>(const MtpProgramDev &, const MtpArgs<double> &, const LossArgs<double> &, cudaStream_t);
+template int mtp_coeff_atoms<float>(const MtpProgramDev &, const MtpArgs<float> &, const LossArgs<float> &, cudaStream_t);
+template int mtp_coeff_atoms<double>(const MtpProgramDev &, const MtpArgs<double> &, const LossArgs<double> &, cudaStream_t);
 template int mtp_force_atoms<float, MODE_EFV>(const MtpProgramDev &, const MtpArgs<float> &, cudaStream_t);
 template int mtp_force_atoms<float, MODE_EF>(const MtpProgramDev &, const MtpArgs<float> &, cudaStream_t);
 template int mtp_force_atoms<double, MODE_EFV>(const MtpProgramDev &, const MtpArgs<double> &, cudaStream_t);

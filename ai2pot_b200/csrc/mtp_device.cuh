@@ -33,6 +33,7 @@ struct LossArgs {
     T *Db, *Xb;                                             // [atoms][nbp] workspace rows
     T ew, fw, vw;
     int ncoef;
+    int dense = 0;      // E and X are written as pairs to Xb, [tile][dense monomial][32 atoms]
 };
 
 // pair weight vector p of the loss gradient
@@ -62,6 +63,10 @@ template <typename T> int mtp_fwd_atoms(const MtpProgramDev &P, const MtpArgs<T>
 template <typename T, int MODE> int mtp_force_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, cudaStream_t st);
 // directional derivatives of the basic moments along the loss gradient's pair weights -> L.Db (tiled)
 template <typename T> int mtp_dfwd_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, const LossArgs<T> &L, cudaStream_t st);
+
+// gradient w.r.t. the radial coefficients from {E, X} rows of whole tiles (dense monomial order, in L.Xb) -> L.dcoeffs
+bool mtp_coeff_atoms_supported(const MtpProgramDev &P, int ntypes, size_t elem);
+template <typename T> int mtp_coeff_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, const LossArgs<T> &L, cudaStream_t st);
 
 // exclusive prefix sum of binum -> prefix[0..B]; one block
 static __device__ __forceinline__ void prefix_binum_block(const int *__restrict__ binum, int B, int *__restrict__ prefix)

@@ -19,6 +19,8 @@
 // coefficient gradient over the lanes of each neighbour type.
 #include "mtp_pairs.cuh"
 
+#include <algorithm>
+
 namespace ai2b {
 
 // ---- loss and squared-error sums ---------------------------------------------------------------
@@ -392,7 +394,7 @@ template <typename T>
 struct LossPairSmem {
     T *M, *E, *seed;
     int2 *row, *warp;
-    int *map;
+    int *map, *db;
 };
 template <typename T> constexpr int loss_ta() { return 8 * 16 / (int)sizeof(T); }
 template <typename T>
@@ -402,8 +404,9 @@ __host__ __device__ inline size_t loss_pair_smem(const MtpProgramDev &P, unsigne
     auto take = [&](size_t bytes) { size_t r = o; o += (bytes + 15) & ~size_t(15); return r; };
     const size_t oM = take(sizeof(T) * 2 * (size_t)P.nm * loss_ta<T>()), oE = take(sizeof(T) * 2 * (size_t)P.nm * loss_ta<T>());
     const size_t orow = take(sizeof(int2) * (size_t)P.stream[1].nrows * 4), ow = take(sizeof(int2) * (size_t)(2 * P.nlev) * MTP_PAIR_WARPS);
-    const size_t os = take(sizeof(T) * (size_t)P.nm), om = take(sizeof(int) * (size_t)P.ns);
+    const size_t os = take(sizeof(T) * (size_t)P.nm), om = take(sizeof(int) * (size_t)P.ns), od = take(sizeof(int) * (size_t)P.ndense);
     if (out) {
+        out->db = reinterpret_cast<int *>(base + od);
         out->M = reinterpret_cast<T *>(base + oM); out->E = reinterpret_cast<T *>(base + oE); out->seed = reinterpret_cast<T *>(base + os);
         out->row = reinterpret_cast<int2 *>(base + orow); out->warp = reinterpret_cast<int2 *>(base + ow); out->map = reinterpret_cast<int *>(base + om);
     }
@@ -425,6 +428,7 @@ __global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_loss_pair_kernel(c
     for (int i = threadIdx.x; i < P.stream[1].nrows * G; i += NT) S.row[i] = stream_rows<T>(P.stream[1])[i];
     for (int i = threadIdx.x; i < 2 * P.nlev * MTP_PAIR_WARPS; i += NT) S.warp[i] = P.stream[1].warp[i];
     for (int s = threadIdx.x; s < P.ns; s += NT) S.map[s] = P.map[s];
+    for (int d = threadIdx.x; d < P.ndense; d += NT) S.db[d] = P.dense_basic[d];
     for (int i = threadIdx.x; i < P.nm; i += NT) S.seed[i] = T(0);
     __syncthreads();
     for (int s = threadIdx.x; s < P.ns; s += NT) atomicAdd(S.seed + P.map[s], A.lin[s] / A.qs[s]);
@@ -469,7 +473,16 @@ __global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_loss_pair_kernel(c
             __syncthreads();
         }
         // for the coefficient kernel: E and X = ce E + G of the basic moments
-        if (valid)
+        if (L.dense) {
+            for (int d = rw; d < P.ndense; d += MTP_PAIR_WARPS * RW) {
+                const int i = S.db[d];
+                const T e = i >= 0 ? S.E[i * TA + at] : T(0), g = i >= 0 ? Gm[i * TA + at] : T(0);
+                const size_t o = ((size_t)(t >> 5) * A.ndp + d) * 32 + (t & 31);
+                typename Vec2<T>::type ex;
+                ex.x = e; ex.y = fma(ce, e, g);
+                reinterpret_cast<typename Vec2<T>::type *>(L.Xb)[o] = ex;
+            }
+        } else if (valid)
             for (int i = rw; i < P.nb; i += MTP_PAIR_WARPS * RW) {
                 const T e = S.E[i * TA + at];
                 A.Eb[(size_t)t * A.nbp + i] = e;
@@ -609,7 +622,7 @@ static LossWs loss_ws_layout(const MtpProgramDev &P, int B, int npad, int ntypes
     const size_t atoms = ((size_t)(B > 0 ? B : 0) * (npad > 0 ? npad : 0) + 31) & ~size_t(31);   // whole tiles of 32 atoms
     L.db = L.base.total;
     L.xb = L.db + up256(atoms * nbasic_pad(P) * elem);
-    L.total = L.xb + up256(atoms * nbasic_pad(P) * elem);
+    L.total = L.xb + up256(atoms * std::max(2 * ndense_pad(P), nbasic_pad(P)) * elem);
     return L;
 }
 
@@ -675,12 +688,16 @@ static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArg
         kern<<<(unsigned)blocks, MTP_WARPS * 32, smem, st>>>(P, A, L);
         AI2B_CUDA(cudaGetLastError());
     }
+    const size_t pair_bytes = loss_pair_smem<T>(P, nullptr, nullptr);
+    const bool pair = P.stream[1].nrows > 0 && pair_bytes <= 226 * 1024;
+    // the coefficient gradient by tiles pays once they occupy half of the SMs; below that a warp per atom is over sooner
+    // (level 10, fp32, 240 atoms: 11 against 14 us; level 16, fp64, 9,323 atoms: 99 against 87)
+    L.dense = pair && atoms_path && atoms_upper >= MTP_TILE * (long)sm_count() / 2 && mtp_coeff_atoms_supported(P, A.ntypes, sizeof(T));
     {
         const size_t cap = 222 * 1024;
         int rc = AI2B_ERR_UNSUPPORTED;
         bool done = false;
-        const size_t pair_bytes = loss_pair_smem<T>(P, nullptr, nullptr);
-        if (P.stream[1].nrows > 0 && pair_bytes <= 226 * 1024) {
+        if (pair) {
             auto kern = mtp_loss_pair_kernel<T>;
             static KernelSetup setup;
             if ((rc = kernel_setup(setup, kern, pair_bytes))) return rc;
@@ -699,6 +716,7 @@ static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArg
         if (!done) set_error("MTP tables with %d moments do not fit the loss-gradient kernel's shared memory", P.nm);
         if (rc) return rc;
     }
+    if (L.dense) return mtp_coeff_atoms<T>(P, A, L, st);
     {
         const size_t smem = sizeof(T) * (size_t)(5 * A.ndp + 2 * A.nbp + 2 * MTP_MAX_MU * 32) * MTP_WARPS;
         auto kern = mtp_loss_coeff_kernel<T, KD, CSP>;
