@@ -64,7 +64,6 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_loss_fast_kernel(con
     const int sub = lane & (NEP_GROUP - 1), grp = lane / NEP_GROUP;
     const int slot_in_block = warp * NEP_APW + grp;
     const unsigned gmask_shift = grp * NEP_GROUP;
-    const unsigned gmask = 0xffu << gmask_shift;
     const int b = blockIdx.y;
     const int nfun = A.n_r + A.n_a, nd = A.nd, nneu = A.nneu;
     const int NP = nep_r32(nneu), nrow = A.ntypes * NP;
@@ -154,11 +153,14 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_loss_fast_kernel(con
     for (int it = 0; it < rounds; it++) {
         const int ii = it * ngroups + blockIdx.x * NEP_APB + slot_in_block;
         const bool valid = ii < n;
-        if (valid) {
-            const size_t slot = (size_t)b * A.npad + ii;
+        // All groups of a warp run the same trip counts, one without an atom with an empty row: with counts of their own the four
+        // groups drift apart and every phase is issued up to four times.
+        if (__any_sync(FULL_MASK, valid)) {
+            const size_t slot = (size_t)b * A.npad + (valid ? ii : 0);
             const int ci = A.bilist[slot];
-            const int nn = min(A.numneigh[slot], A.umax);
+            const int nn = valid ? min(A.numneigh[slot], A.umax) : 0;
             const int ti = types[ci];
+            const int nnw = __reduce_max_sync(FULL_MASK, nn);
             const int *fn = A.firstneigh + slot * A.umax;
             const T *rc = A.rcs + slot * A.umax * 3;
             const T *ctab = ctab_s + (size_t)ti * A.ntypes * TROW;
@@ -174,15 +176,15 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_loss_fast_kernel(con
             };
             for (int i = sub; i < 2 * A.ntypes * 8; i += NEP_GROUP) Fs[i] = T(0);
             for (int i = sub; i < A.ntypes * NMAX * 8; i += NEP_GROUP) Ga[i] = T(0);
-            if (sub == 0) atomicOr(&tmask[it & 1][ti], 1u << slot_in_block);
-            __syncwarp(gmask);
+            if (sub == 0 && valid) atomicOr(&tmask[it & 1][ti], 1u << slot_in_block);
+            __syncwarp();
 
             // ---- 1. radial pass --------------------------------------------------------------------------
             T qacc[NMAX], uacc[NMAX];
 #pragma unroll
             for (int k = 0; k < NMAX; k++) qacc[k] = uacc[k] = T(0);
             int nang = 0;
-            for (int j0 = 0; j0 < nn; j0 += NEP_GROUP) {
+            for (int j0 = 0; j0 < nnw; j0 += NEP_GROUP) {
                 const int j = j0 + sub;
                 bool on = j < nn;
                 T x = 0, y = 0, z = 0;
@@ -209,33 +211,34 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_loss_fast_kernel(con
                 // per-type sums of f_xi and f'_xi (r^.p): lane xi of the group ends up with entry xi
                 for (int t = 0; t < A.ntypes; t++) {
                     const bool mine = on && tj == t;
-                    if (__ballot_sync(gmask, mine) & gmask) {
+                    if (__any_sync(FULL_MASK, mine)) {
                         T v[CSP], w[CSP];
 #pragma unroll
                         for (int xi = 0; xi < CSP; xi++) { v[xi] = mine ? f[xi] : T(0); w[xi] = mine ? df[xi] * vp : T(0); }
-                        Fs[t * 8 + sub] += group_xreduce8(v, sub, gmask);
-                        Fs[(A.ntypes + t) * 8 + sub] += group_xreduce8(w, sub, gmask);
+                        Fs[t * 8 + sub] += group_xreduce8(v, sub, FULL_MASK);
+                        Fs[(A.ntypes + t) * 8 + sub] += group_xreduce8(w, sub, FULL_MASK);
                     }
                 }
                 const bool ang = on && r <= A.rc_a && A.l_max > 0;
-                const unsigned bal = (__ballot_sync(gmask, ang) >> gmask_shift) & 0xffu;
+                const unsigned bal = (__ballot_sync(FULL_MASK, ang) >> gmask_shift) & 0xffu;
                 if (ang) alist[nang + __popc(bal & ((1u << sub) - 1u))] = (unsigned short)(j | (tj << 10));
                 nang += __popc(bal);
             }
 #pragma unroll
             for (int k = 0; k < NMAX; k++) {
-                const T sq = group_sum(qacc[k], gmask), su = group_sum(uacc[k], gmask);
+                const T sq = group_sum(qacc[k], FULL_MASK), su = group_sum(uacc[k], FULL_MASK);
                 if (sub == (k & (NEP_GROUP - 1)) && k < A.n_r) { q[k] = sq; u[k] = su; }
             }
-            __syncwarp(gmask);
+            __syncwarp();
 
+            const int nangw = __reduce_max_sync(FULL_MASK, nang);
             // ---- 2. angular sums and their directional derivatives: lane owns lm = 3 sub .. 3 sub + 2 ----------
             T Sacc[NMAX][3], Dacc[NMAX][3];
 #pragma unroll
             for (int mu = 0; mu < NMAX; mu++)
 #pragma unroll
                 for (int i = 0; i < 3; i++) Sacc[mu][i] = Dacc[mu][i] = T(0);
-            for (int k0 = 0; k0 < nang; k0 += NEPL_STAGE) {
+            for (int k0 = 0; k0 < nangw; k0 += NEPL_STAGE) {
                 const bool on = sub < NEPL_STAGE && k0 + sub < nang;
                 if (sub < NEPL_STAGE) {   // the first lanes of the group stage one neighbour each
                     T x = 0, y = 0, z = 0, rinv = 0, r = A.rc_a;
@@ -273,8 +276,8 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_loss_fast_kernel(con
                     }
                     store_vec<T, RS>(stage + sub * RS, row);
                 }
-                __syncwarp(gmask);
-                const int cnt = min(NEPL_STAGE, nang - k0);
+                __syncwarp();
+                const int cnt = min(NEPL_STAGE, nangw - k0);      // (rows past a group's own count are zero)
                 for (int jj = 0; jj < cnt; jj++) {
                     const T *rj = stage + jj * RS;
                     T gj[NMAX], gv[NMAX];
@@ -290,7 +293,7 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_loss_fast_kernel(con
                         }
                     }
                 }
-                __syncwarp(gmask);
+                __syncwarp();
             }
             // descriptors q_{mu,l} and u_{mu,l}: partial sums over this lane's lm, combined per (mu, l) through shared memory
             // (the staging rows are free now): tq[mu][lm], tu[mu][lm]
@@ -304,20 +307,20 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_loss_fast_kernel(con
                         tq[mu * NEP_NLM + lm] = c3w_s[lm] * Sacc[mu][i] * Sacc[mu][i];
                         tu[mu * NEP_NLM + lm] = T(2) * c3w_s[lm] * Sacc[mu][i] * Dacc[mu][i];
                     }
-                __syncwarp(gmask);
+                __syncwarp();
                 for (int p = sub; p < nq_a; p += NEP_GROUP) {
                     const int mu = pm_mu[p], l = pm_l[p];
                     T aq = T(0), au = T(0);
                     for (int mp = 0; mp < 2 * l + 1; mp++) { aq += tq[mu * NEP_NLM + l * l - 1 + mp]; au += tu[mu * NEP_NLM + l * l - 1 + mp]; }
                     q[A.n_r + p] = aq; u[A.n_r + p] = au;
                 }
-                __syncwarp(gmask);
+                __syncwarp();
             }
 
             // ---- 3. network with second-order terms --------------------------------------------------------------
             // q, u become q / qs, u / qs (what the first layer sees and what its weight gradient needs)
             for (int k = sub; k < nd; k += NEP_GROUP) { q[k] *= iqs[k]; u[k] *= iqs[k]; }
-            __syncwarp(gmask);
+            __syncwarp();
             const T *W0t = W0s + (size_t)ti * NP * NDP;
             for (int p0 = 0; p0 < NP; p0 += 4 * NEP_GROUP) {
                 T h[4], sv[4];
@@ -346,7 +349,7 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_loss_fast_kernel(con
                     gw1s[pn] = lam * t + d1 * sv[i];
                 }
             }
-            __syncwarp(gmask);
+            __syncwarp();
             // adjoints: av = dE/dq, be = coefficient of dq/dc  (overwrite the scaled copies)
             for (int c = sub; c < NDP / 4; c += NEP_GROUP) {
                 const T *wcol = W0t + 4 * c;
@@ -369,7 +372,7 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_loss_fast_kernel(con
                 store_vec<T, 4>(av + 4 * c, ra);
                 store_vec<T, 4>(be + 4 * c, rb);
             }
-            __syncwarp(gmask);
+            __syncwarp();
             // polynomial coefficients per (lm, mu): x = w2c (be S + av DS), y = w2c av S
 #pragma unroll
             for (int i = 0; i < 3; i++) {
@@ -388,10 +391,10 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_loss_fast_kernel(con
                 store_vec<T, NMAX>(xc + lm * NMAX, xr);
                 store_vec<T, NMAX>(yc + lm * NMAX, yr);
             }
-            __syncwarp(gmask);
+            __syncwarp();
 
             // ---- 4. coefficient gradient, angular functions (the radial part is an outer product: see the round's end) ----
-            for (int k0 = 0; k0 < nang; k0 += NEP_GROUP) {
+            for (int k0 = 0; k0 < nangw; k0 += NEP_GROUP) {
                 const bool on = k0 + sub < nang;
                 int tj = 0;
                 T vp = T(0), f[CSP], df[CSP];
@@ -429,20 +432,20 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_loss_fast_kernel(con
                 // sum over the group's neighbours of each type; lane xi adds entry xi to the atom's record
                 for (int t = 0; t < A.ntypes; t++) {
                     const bool mine = on && tj == t;
-                    if (__ballot_sync(gmask, mine) & gmask) {
+                    if (__any_sync(FULL_MASK, mine)) {
 #pragma unroll
                         for (int mu = 0; mu < NMAX; mu++) {
                             const T wv = X[mu] + GY[mu], wd = Y[mu] * vp;
                             T v[CSP];
 #pragma unroll
                             for (int xi = 0; xi < CSP; xi++) v[xi] = mine ? wv * f[xi] + wd * df[xi] : T(0);
-                            const T tot = group_xreduce8(v, sub, gmask);
+                            const T tot = group_xreduce8(v, sub, FULL_MASK);
                             Ga[(t * NMAX + mu) * 8 + sub] += tot;
                         }
                     }
                 }
             }
-            __syncwarp(gmask);
+            __syncwarp();
         }
         // ---- end of the round: the block adds its atoms' records to the accumulators; one owner per element ----
         __syncthreads();
