@@ -12,7 +12,9 @@
 //   * angular pass, lanes = angular neighbours of all atoms of the warp, back to back: only a fifth of the neighbours are
 //     inside the angular cutoff (6.5 of 29, or 2.2 of 17), so lanes that belong to one atom would mostly idle. The harmonics
 //     of a neighbour go through shared memory to the lanes that own its atom's sums S[mu][lm];
-//   * network: lanes = neurons, then lanes = descriptors;
+//   * network: lanes = neurons; up to NMAX = 4 a neuron's row is read once, for its input and for the descriptors' adjoints, with
+//     the angular sums parked in shared memory (1,048,576 atoms of a crystal: 950 -> 827 us; with a second walk over the rows,
+//     lanes = descriptors, the shared-memory pipe was 82 % busy; without parking the spills made it 1,058 us);
 //   * angular forces, lanes as in the angular pass (the neighbour's functions are still in registers): the adjoints are
 //     first contracted over the radial functions, sum_mu g_mu e_{mu,lm} and sum_mu g'_mu e_{mu,lm}, which leaves one
 //     polynomial and one gradient per neighbour instead of NMAX. The radial force of the neighbour joins here, so every
@@ -296,6 +298,8 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_fast_kernel(const Ne
     constexpr int AW = 32 / G, NP2 = NMAX / 2, NDP = D::NDP, RS = D::RS, ESR = D::ESR, ROW = 2 * NMAX;
     constexpr int LM = (NEP_NLM + G - 1) / G;            // sums per lane and function
     constexpr int NPL = 32 / G;                          // neurons per lane and round
+    constexpr bool PARK = NMAX == 4 && sizeof(T) == 4 && G <= 16;      // the sums wait in shared memory while the network has the registers
+    constexpr bool ONEPASS = NMAX == 4;                  // a row of the first layer, the inputs and the adjoints fit in registers
     constexpr bool NET = MODE != NEP_DESC;
     extern __shared__ __align__(16) unsigned char nep_smem[];
     __shared__ T blk_acc[10];
@@ -558,71 +562,128 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_fast_kernel(const Ne
         } else {
         for (int k = sub; k < A.nd; k += G) Eq[k] = q[k] * tab_s[L.iqs + k];
         __syncwarp();
+        if constexpr (PARK) {      // (the descriptors' terms that lay here have been read)
+            static_assert(LM * NP2 * 64 <= 32 * RS, "a lane's sums fit in the staging rows");
+#pragma unroll
+            for (int i = 0; i < LM; i++)
+#pragma unroll
+                for (int n = 0; n < NP2; n++) reinterpret_cast<Pk<T> *>(stage)[(i * NP2 + n) * 32 + lane] = S[i][n];
+        }
         T e_at = T(0);
         const T *W0t = tab_s + L.w0 + ti * NP * NDP, *B0t = tab_s + L.b0 + ti * NP, *W1t = tab_s + L.w1 + ti * NP;
-        for (int p0 = 0; p0 < NP; p0 += NPL * G) {      // lanes = neurons, NPL at a time
-            Pk<T> h[NPL];
+        if constexpr (ONEPASS) {
+            // A neuron's row is read once and used twice, for its input and for its share of the descriptors' adjoints: the
+            // shared-memory pipe is what bounds this phase (four wavefronts per 16-byte load, whatever the lanes share).
+            Pk<T> e[NDP / 2], a[NDP / 2];
+            load_pk<NDP / 2>(Eq, e);
 #pragma unroll
-            for (int i = 0; i < NPL; i++) h[i] = pk(T(0), T(0));
+            for (int k = 0; k < NDP / 2; k++) a[k] = pk(T(0), T(0));
+            for (int p = sub; p < NP; p += G) {
+                Pk<T> w[NDP / 2], h0 = pk(B0t[p], T(0)), h1 = pk(T(0), T(0));
+                load_pk<NDP / 2>(W0t + p * NDP, w);
 #pragma unroll
-            for (int c = 0; c < NDP / 4; c++) {
-                Pk<T> e[2];
-                load_pk<2>(Eq + 4 * c, e);
-#pragma unroll
-                for (int i = 0; i < NPL; i++) {
-                    Pk<T> w[2];
-                    load_pk<2>(W0t + (p0 + sub + G * i) * NDP + 4 * c, w);
-                    h[i] = pk_fma(w[0], e[0], h[i]);
-                    h[i] = pk_fma(w[1], e[1], h[i]);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < NPL; i++) {
-                const int p = p0 + sub + G * i;
-                const T th = gtanh(pk_lo(h[i]) + pk_hi(h[i]) + B0t[p]);
+                for (int k = 0; k < NDP / 2; k += 2) { h0 = pk_fma(w[k], e[k], h0); h1 = pk_fma(w[k + 1], e[k + 1], h1); }
+                const T th = gtanh((pk_lo(h0) + pk_hi(h0)) + (pk_lo(h1) + pk_hi(h1)));
                 const T w1 = W1t[p];                    // zero for padding neurons
                 e_at += w1 * th;
-                act[p] = w1 * (T(1) - th * th);
+                const T x = w1 * (T(1) - th * th);
+                const Pk<T> x2 = pk(x, x);
+#pragma unroll
+                for (int k = 0; k < NDP / 2; k++) a[k] = pk_fma(x2, w[k], a[k]);
             }
+            // over the lanes of the group: two exchanging steps leave a quarter of the descriptors per lane, the rest adds up
+            constexpr int H = NDP / 2, Q = NDP / 4;
+            T r[H];
+            const bool up1 = sub & 1, up2 = sub & 2;
+#pragma unroll
+            for (int k = 0; k < H; k++) {
+                const T lo = (k & 1) ? pk_hi(a[k / 2]) : pk_lo(a[k / 2]), hi = ((k + H) & 1) ? pk_hi(a[(k + H) / 2]) : pk_lo(a[(k + H) / 2]);
+                r[k] = (up1 ? hi : lo) + __shfl_xor_sync(FULL_MASK, up1 ? lo : hi, 1);
+            }
+#pragma unroll
+            for (int k = 0; k < Q; k++) {
+                r[k] = (up2 ? r[k + Q] : r[k]) + __shfl_xor_sync(FULL_MASK, up2 ? r[k] : r[k + Q], 2);
+#pragma unroll
+                for (int o = 4; o < G; o <<= 1) r[k] += __shfl_xor_sync(FULL_MASK, r[k], o);
+            }
+            const int k0 = (up1 ? H : 0) + (up2 ? Q : 0);
+            __syncwarp();
+            if (sub < 4)
+#pragma unroll
+                for (int k = 0; k < Q; k++) Eq[k0 + k] = r[k] * tab_s[L.iqs + k0 + k];
+        } else {
+            for (int p0 = 0; p0 < NP; p0 += NPL * G) {      // lanes = neurons, NPL at a time
+                Pk<T> h[NPL];
+#pragma unroll
+                for (int i = 0; i < NPL; i++) h[i] = pk(T(0), T(0));
+#pragma unroll
+                for (int c = 0; c < NDP / 4; c++) {
+                    Pk<T> e[2];
+                    load_pk<2>(Eq + 4 * c, e);
+#pragma unroll
+                    for (int i = 0; i < NPL; i++) {
+                        Pk<T> w[2];
+                        load_pk<2>(W0t + (p0 + sub + G * i) * NDP + 4 * c, w);
+                        h[i] = pk_fma(w[0], e[0], h[i]);
+                        h[i] = pk_fma(w[1], e[1], h[i]);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < NPL; i++) {
+                    const int p = p0 + sub + G * i;
+                    const T th = gtanh(pk_lo(h[i]) + pk_hi(h[i]) + B0t[p]);
+                    const T w1 = W1t[p];                    // zero for padding neurons
+                    e_at += w1 * th;
+                    act[p] = w1 * (T(1) - th * th);
+                }
+            }
+            __syncwarp();
+            {   // adjoints of the descriptors: lanes = four descriptors each, the neurons in G / 8 parts
+                constexpr int PARTS = G >= 8 ? G / 8 : 1, CL = G >= 8 ? 8 : G;
+                const int part = sub / CL, pb = part * (NP / PARTS), pe = pb + NP / PARTS;
+                for (int c0 = 0; c0 < NDP / 4; c0 += CL) {
+                    const int c = c0 + sub % CL;
+                    const bool in = c < NDP / 4;
+                    const T *wcol = W0t + 4 * (in ? c : 0);
+                    Pk<T> a[2][2];
+                    a[0][0] = a[0][1] = a[1][0] = a[1][1] = pk(T(0), T(0));
+#pragma unroll 2
+                    for (int p = pb; p < pe; p += 4) {
+                        T x[4];
+                        load_vec<T, 4>(act + p, x);
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            Pk<T> w[2];
+                            load_pk<2>(wcol + (p + i) * NDP, w);
+                            const Pk<T> x2 = pk(x[i], x[i]);
+                            a[i & 1][0] = pk_fma(x2, w[0], a[i & 1][0]);
+                            a[i & 1][1] = pk_fma(x2, w[1], a[i & 1][1]);
+                        }
+                    }
+                    T r[4] = {pk_lo(a[0][0]) + pk_lo(a[1][0]), pk_hi(a[0][0]) + pk_hi(a[1][0]), pk_lo(a[0][1]) + pk_lo(a[1][1]), pk_hi(a[0][1]) + pk_hi(a[1][1])};
+#pragma unroll
+                    for (int o = CL; o < G; o <<= 1)
+#pragma unroll
+                        for (int k = 0; k < 4; k++) r[k] += __shfl_xor_sync(FULL_MASK, r[k], o);
+                    if (in && part == 0) {
+#pragma unroll
+                        for (int k = 0; k < 4; k++) r[k] *= tab_s[L.iqs + 4 * c + k];
+                        store_vec<T, 4>(Eq + 4 * c, r);
+                    }
+                }
+            }
+            __syncwarp();
         }
         if (valid) e_at += sub == 0 ? A.bias[ti] : T(0);
         else e_at = T(0);
         __syncwarp();
-        {   // adjoints of the descriptors: lanes = four descriptors each, the neurons in G / 8 parts
-            constexpr int PARTS = G >= 8 ? G / 8 : 1, CL = G >= 8 ? 8 : G;
-            const int part = sub / CL, pb = part * (NP / PARTS), pe = pb + NP / PARTS;
-            for (int c0 = 0; c0 < NDP / 4; c0 += CL) {
-                const int c = c0 + sub % CL;
-                const bool in = c < NDP / 4;
-                const T *wcol = W0t + 4 * (in ? c : 0);
-                Pk<T> a[2][2];
-                a[0][0] = a[0][1] = a[1][0] = a[1][1] = pk(T(0), T(0));
-#pragma unroll 2
-                for (int p = pb; p < pe; p += 4) {
-                    T x[4];
-                    load_vec<T, 4>(act + p, x);
+        if constexpr (PARK) {
 #pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        Pk<T> w[2];
-                        load_pk<2>(wcol + (p + i) * NDP, w);
-                        const Pk<T> x2 = pk(x[i], x[i]);
-                        a[i & 1][0] = pk_fma(x2, w[0], a[i & 1][0]);
-                        a[i & 1][1] = pk_fma(x2, w[1], a[i & 1][1]);
-                    }
-                }
-                T r[4] = {pk_lo(a[0][0]) + pk_lo(a[1][0]), pk_hi(a[0][0]) + pk_hi(a[1][0]), pk_lo(a[0][1]) + pk_lo(a[1][1]), pk_hi(a[0][1]) + pk_hi(a[1][1])};
+            for (int i = 0; i < LM; i++)
 #pragma unroll
-                for (int o = CL; o < G; o <<= 1)
-#pragma unroll
-                    for (int k = 0; k < 4; k++) r[k] += __shfl_xor_sync(FULL_MASK, r[k], o);
-                if (in && part == 0) {
-#pragma unroll
-                    for (int k = 0; k < 4; k++) r[k] *= tab_s[L.iqs + 4 * c + k];
-                    store_vec<T, 4>(Eq + 4 * c, r);
-                }
-            }
+                for (int n = 0; n < NP2; n++) S[i][n] = reinterpret_cast<const Pk<T> *>(stage)[(i * NP2 + n) * 32 + lane];
+            __syncwarp();
         }
-        __syncwarp();
         // adjoints of the sums, [mu][24] (the descriptors' terms that lay there have been read)
 #pragma unroll
         for (int i = 0; i < LM; i++) {
