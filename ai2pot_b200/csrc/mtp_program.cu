@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cstring>
 #include <fstream>
+#include <queue>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -345,24 +346,35 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
                 for (size_t i = 0; i < order.size(); i++) order[i] = i;
                 std::stable_sort(order.begin(), order.end(), [&](size_t i, size_t j) { return ph[i].rows.size() > ph[j].rows.size(); });
                 using Deal = std::vector<std::vector<size_t>>;
-                auto deal = [&](size_t wide, Deal &of_warp, Deal &of_group) -> size_t {
-                    of_warp.assign(MTP_PAIR_WARPS, {});
-                    of_group.assign(MTP_PAIR_WARPS * groups, {});
-                    std::vector<size_t> wload(MTP_PAIR_WARPS, 0), wrows(MTP_PAIR_WARPS, 0), grows(MTP_PAIR_WARPS * groups, 0);
+                Deal of_warp, of_group;
+                auto deal = [&](size_t wide, bool keep) -> size_t {
+                    using Place = std::pair<size_t, size_t>;      // load, index: the least loaded place on top, the first of equals
+                    using Heap = std::priority_queue<Place, std::vector<Place>, std::greater<Place>>;
+                    std::vector<Place> start(MTP_PAIR_WARPS, Place(0, 0));
+                    for (size_t w = 0; w < MTP_PAIR_WARPS; w++) start[w].second = w;
+                    std::vector<size_t> wrows(MTP_PAIR_WARPS, 0), wload(MTP_PAIR_WARPS, 0), grows(MTP_PAIR_WARPS * groups, 0);
+                    if (keep) { of_warp.assign(MTP_PAIR_WARPS, {}); of_group.assign(MTP_PAIR_WARPS * groups, {}); }
                     size_t i = 0;
+                    Heap warps(std::greater<Place>(), start);
                     for (; i < order.size() && ph[order[i]].rows.size() > wide; i++) {
-                        const size_t w = std::min_element(wload.begin(), wload.end()) - wload.begin(), n = (ph[order[i]].rows.size() + groups - 1) / groups;
-                        of_warp[w].push_back(order[i]);
-                        wload[w] += n + 1;
-                        wrows[w] += n;
+                        const Place p = warps.top();
+                        const size_t n = (ph[order[i]].rows.size() + groups - 1) / groups;
+                        warps.pop();
+                        warps.push(Place(p.first + n + 1, p.second));
+                        wload[p.second] += n + 1;
+                        wrows[p.second] += n;
+                        if (keep) of_warp[p.second].push_back(order[i]);
                     }
-                    std::vector<size_t> gload(MTP_PAIR_WARPS * groups);
-                    for (size_t g = 0; g < gload.size(); g++) gload[g] = wload[g / groups];
+                    start.resize(MTP_PAIR_WARPS * groups);
+                    for (size_t g = 0; g < start.size(); g++) start[g] = Place(wload[g / groups], g);
+                    Heap places(std::greater<Place>(), start);
                     for (; i < order.size(); i++) {
-                        const size_t g = std::min_element(gload.begin(), gload.end()) - gload.begin(), n = ph[order[i]].rows.size();
-                        of_group[g].push_back(order[i]);
-                        gload[g] += n + 1;
-                        grows[g] += n;
+                        const Place p = places.top();
+                        const size_t n = ph[order[i]].rows.size();
+                        places.pop();
+                        places.push(Place(p.first + n + 1, p.second));
+                        grows[p.second] += n;
+                        if (keep) of_group[p.second].push_back(order[i]);
                     }
                     size_t longest = 0, sum = 0;
                     for (size_t w = 0; w < MTP_PAIR_WARPS; w++) {
@@ -372,13 +384,15 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
                     }
                     return 60 * longest + 5 * sum;
                 };
-                Deal of_warp, of_group;
-                size_t best = ~size_t(0), best_wide = 0;
+                size_t best = ~size_t(0), best_wide = 0, last = ~size_t(0);
                 for (size_t i : order) {
-                    const size_t wide = ph[i].rows.size(), cost = deal(wide, of_warp, of_group);
+                    const size_t wide = ph[i].rows.size();
+                    if (wide == last) continue;      // (sorted: every row count is tried once)
+                    last = wide;
+                    const size_t cost = deal(wide, false);
                     if (cost < best) { best = cost; best_wide = wide; }
                 }
-                deal(best_wide, of_warp, of_group);
+                deal(best_wide, true);
                 for (size_t w = 0; w < MTP_PAIR_WARPS; w++) {
                     std::vector<std::vector<int2>> rd(groups), rf(groups);
                     auto put = [&](size_t g, int xy, int mult, int done) {
