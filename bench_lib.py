@@ -209,7 +209,7 @@ def run_md_benchmark(w, steps, warmup, dist, sampler):
                 "note": "host-timed synchronous call; the kernels are those of the nep workload", "max_neighbours": int(mx),
                 "local_atoms": nlocal, "ghost_atoms": nghost}
     nall = nlocal + nghost
-    return dict(t_dev=t, t_e2e=t, clocks=clocks, launches=(9 + 1) * steps, h2d=nall * 28, d2h=nall * 12 + 48, units=nlocal,
+    return dict(t_dev=t, t_e2e=t, clocks=clocks, launches=(4 + 2) * steps, h2d=nall * 28, d2h=nall * 12 + 48, units=nlocal,
                 e2e_path="host double positions + types of local and ghost atoms -> ai2b_md_session_compute -> host forces (+=), energy, virial[6]",
                 roofline=roofline, parts_ms=None, host_ms_per_call=1e3 * t / steps)
 
@@ -344,7 +344,7 @@ def run_training_benchmark(w, steps, warmup, dist, sampler):
                 "unit": "TFLOP/s", "frac": achieved / peak, "peak_source": "FMA-chain microbenchmark in this run (of measured)",
                 "flops_per_atom": fl, "mean_neighbours": mean_nn, "traffic": None}
     name = "nep" if is_nep else "mtp"
-    return dict(t_dev=t_dev, t_e2e=t_e2e, clocks=clocks, launches=((2 + 2 + 1 + 1) if is_nep else (4 + 2 + 4 + 1)) * steps, h2d=0,
+    return dict(t_dev=t_dev, t_e2e=t_e2e, clocks=clocks, launches=((2 + 2 + 1 + 1) if is_nep else (4 + 2 + 5 + 1)) * steps, h2d=0,
                 d2h=hgrad.numel() * hgrad.element_size(), units=natoms,
                 e2e_path=f"resident neighbour tensors -> ai2b_{name}_efv -> ai2b_{name}_loss -> ai2b_{name}_loss_backward -> D2H summed gradient",
                 roofline=roofline, parts_ms=None, cuda_graph=graph is not None, host_ms_per_call=1e3 * t_host)
@@ -524,7 +524,7 @@ def run_single_benchmark(w, steps, warmup, dist, sampler):
     hbm, hbm_src = hbm_peak()
     key = ("mtp16" if m["kind"] == "mtp" else "nep") + f"_{n}_efv"
     traffic, traffic_src = profiled_traffic(key)
-    roofline = {"kernel": "mtp_fwd_atoms + mtp_contract_seg + mtp_force_atoms (the three E/F/V kernels of a call)" if m["kind"] == "mtp" else "nep_fast_kernel",
+    roofline = {"kernel": "mtp_fwd_atoms + mtp_contract_pair + mtp_force_atoms (the three E/F/V kernels of a call)" if m["kind"] == "mtp" else "nep_fast_kernel",
                 "bound": bound,
                 "achieved": achieved, "peak": peak_meas, "unit": "TFLOP/s", "frac": achieved / peak_meas,
                 "peak_source": "FMA-chain microbenchmark in this run (of measured)", "peak_nominal": peak_nom,
