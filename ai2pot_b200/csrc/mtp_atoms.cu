@@ -279,8 +279,8 @@ __global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_ke
                 }
                 __syncthreads();
                 if constexpr (NACC > 0) {
-                    // (the four warps run code of their own; the derivatives twice over would not stay in the instruction cache)
-#pragma unroll (DERIV ? 1 : 2)
+                    // (the four warps run code of their own; twice over it does not stay in the instruction cache: training step 334 -> 329 us)
+#pragma unroll 1
                     for (int jj = 0; jj < cnt; jj++) {
                         const T *s = st + (size_t)jj * NV * 32 + lane;
                         Powers<T, KD> pw;
