@@ -134,7 +134,7 @@ struct WsParts {
     int nparts;
 };
 // A block takes 32 columns and deals the rows to eight warps: with one thread per column the launch was a few blocks of
-// serial chains (f64, 64 rows, 383 columns: 19 us; now 5).
+// serial chains (f64, 64 rows, 383 columns: 19 us; now 7).
 constexpr int WS_WARPS = 8;
 template <typename T>
 __global__ void __launch_bounds__(WS_WARPS * 32) weighted_sum_rows_kernel(WsParts<T> P, int B, const T *__restrict__ w, T *__restrict__ out)
