@@ -25,7 +25,7 @@ class Evaluator:
         self.prog = capi.MtpProgram(model["tables"]) if self.kind == "mtp" else None
         self.device = dev
         self.builder = capi.NeighborBuilder()
-        self.lists = capi.NeighborBuilder.new_outputs(n, self.umax, dtype, dev)     # numneigh, firstneigh, rcs, status
+        self._new_lists()
         self.nb_static = dict(binum=torch.tensor([n], dtype=torch.int32, device=dev),
                               bilist=torch.arange(n, dtype=torch.int32, device=dev)[None].contiguous(),
                               btypes=torch.from_numpy(np.ascontiguousarray(types, np.int32)).to(dev)[None].contiguous(),
@@ -33,58 +33,109 @@ class Evaluator:
         # E, virial and forces in one piece, [E | virial (9) | pad | forces (3 n)], so that a host reads them with one copy
         self.outbuf = torch.empty(16 + 3 * n, dtype=dtype, device=dev)
         self.out = (self.outbuf[0:1], self.outbuf[16:].view(1, n, 3), self.outbuf[1:10].view(1, 9))
-        self.status = self.lists[3]
+        self.ws = None
+        self.nb_ws = torch.empty(max(256, capi.lib().ai2b_nblist_workspace_bytes(C.c_int(n), C.c_int(int(dtype == torch.float64)))),
+                                 dtype=torch.uint8, device=dev)
         self.graph = self.graph_io = None
+        self._desc, self._filled = capi.Evaluation(), None
+        self._desc_cell = np.frombuffer(self._desc, np.float64, 9, capi.Evaluation.cell.offset)
+        self._call = (capi.lib().ai2b_evaluate, C.byref(self._desc), self.device.index)
         self._describe()
 
+    def _new_lists(self):
+        """Neighbour tensors for rows of umax slots: numneigh, firstneigh, rcs, status."""
+        self.lists = capi.NeighborBuilder.new_outputs(self.n, int(self.umax), self.dtype, self.device)
+        self.status = self.lists[3]
+
+    def _workspace(self):
+        """Scratch of the evaluation, large enough for the model as it is now."""
+        m = self.model
+        if self.kind == "mtp":
+            need = capi.lib().ai2b_mtp_workspace_bytes(self.prog.handle, C.c_int(1), C.c_int(self.n), C.c_int(int(self.nb_static["ntypes"])))
+        else:
+            need = capi.lib().ai2b_nep_workspace_bytes(C.c_int(1), C.c_int(int(self.nb_static["ntypes"])), C.c_int(int(m["n_radial"])),
+                                                       C.c_int(int(m["n_angular"])), C.c_int(int(m["chebyshev_size"])),
+                                                       C.c_int(int(self.dtype == torch.float64)))
+        if self.ws is None or self.ws.numel() < need:
+            self.ws = torch.empty(max(need, 256), dtype=torch.uint8, device=self.device)
+        return self.ws
+
+    SCALARS = {"mtp": ("chebyshev_size", "scaling", "rmax", "rmin"),
+               "nep": ("chebyshev_size", "n_radial", "n_angular", "l_max", "num_neurons", "rmax_radial", "rmax_angular")}
+    TENSORS = {"mtp": ("coeffs", "type_bias", "q_scaler", "linear_coeffs"), "nep": ("coeffs", "type_bias", "q_scaler", "w0", "b0", "w1")}
+
     def _describe(self):
-        """Everything a call needs but the positions, once (ai2b_evaluation)."""
-        m, is64 = self.model, self.dtype == torch.float64
-        self.nb_ws = torch.empty(max(256, capi.lib().ai2b_nblist_workspace_bytes(C.c_int(self.n), C.c_int(int(is64)))), dtype=torch.uint8, device=self.device)
-        if self.kind == "mtp":
-            need = capi.lib().ai2b_mtp_workspace_bytes(self.prog.handle, C.c_int(1), C.c_int(self.n), C.c_int(int(m["ntypes"])))
-        else:
-            need = capi.lib().ai2b_nep_workspace_bytes(C.c_int(1), C.c_int(int(m["ntypes"])), C.c_int(int(m["n_radial"])), C.c_int(int(m["n_angular"])),
-                                                       C.c_int(int(m["chebyshev_size"])), C.c_int(int(is64)))
-        self.ws = torch.empty(max(need, 256), dtype=torch.uint8, device=self.device)
-        d = capi.Evaluation()
-        d.is_f64, d.natoms, d.umax, d.ntypes, d.rcut = int(is64), self.n, self.umax, int(m["ntypes"]), self.rcut
-        cell = np.asarray(self.cell, np.float64 if is64 else np.float32).reshape(9)
-        for k in range(9):
-            d.cell[k] = float(cell[k])
+        """The call's arguments but the positions (ai2b_evaluation), from what the attributes hold now: cell, cutoff, row width
+        and model may be assigned or edited between calls. Only the pieces that differ from the last call's are written."""
+        m, nb = self.model, self.nb_static
+        if self.lists[1].shape[1] != self.umax:
+            self._new_lists()
+        tensors = [m[k] for k in self.TENSORS[self.kind]]
+        tensors += (nb["binum"], nb["bilist"], nb["btypes"], *self.lists, *self.out)
+        values = [self.kind, self.rcut, self.umax, nb["ntypes"], None if self.prog is None else self.prog.handle.value]
+        values += [m[k] for k in self.SCALARS[self.kind]]
+        for t in tensors:
+            if not t.is_cuda or not t.is_contiguous():
+                capi._ptr(t)       # raises
+            values.append(t.data_ptr())
+        if values != self._filled:
+            self._filled = None
+            self._fill(values[-len(tensors):])
+            self._filled = values
+        self._desc_cell[:] = np.asarray(self.cell).reshape(9)
+
+    def _fill(self, ptrs):
+        m, d = self.model, self._desc
+        d.is_f64, d.natoms, d.umax, d.ntypes, d.rcut = int(self.dtype == torch.float64), self.n, int(self.umax), int(self.nb_static["ntypes"]), float(self.rcut)
         d.chebyshev_size = int(m["chebyshev_size"])
-        ptr = lambda t: t.data_ptr()
         if self.kind == "mtp":
-            d.mtp, d.scaling, d.rmax, d.rmin, d.d_linear_coeffs = self.prog.handle.value, float(m["scaling"]), float(m["rmax"]), float(m["rmin"]), ptr(m["linear_coeffs"])
+            d.mtp, d.scaling, d.rmax, d.rmin = self.prog.handle.value, float(m["scaling"]), float(m["rmax"]), float(m["rmin"])
+            model_ptrs = ("d_coeffs", "d_type_bias", "d_q_scaler", "d_linear_coeffs")
         else:
+            d.mtp = None
             d.n_radial, d.n_angular, d.l_max, d.num_neurons = (int(m[k]) for k in ("n_radial", "n_angular", "l_max", "num_neurons"))
             d.rmax, d.rmax_angular = float(m["rmax_radial"]), float(m["rmax_angular"])
-            d.d_w0, d.d_b0, d.d_w1 = ptr(m["w0"]), ptr(m["b0"]), ptr(m["w1"])
-        d.d_coeffs, d.d_type_bias, d.d_q_scaler = ptr(m["coeffs"]), ptr(m["type_bias"]), ptr(m["q_scaler"])
-        d.d_binum, d.d_ilist, d.d_types = (ptr(self.nb_static[k]) for k in ("binum", "bilist", "btypes"))
-        d.d_numneigh, d.d_firstneigh, d.d_rcs, d.d_status = (ptr(t) for t in self.lists)
-        d.d_etot, d.d_force, d.d_virial = (ptr(t) for t in self.out)
-        d.d_nblist_workspace, d.nblist_workspace_bytes = ptr(self.nb_ws), self.nb_ws.numel()
-        d.d_workspace, d.workspace_bytes = ptr(self.ws), self.ws.numel()
-        self._desc, self._call = d, (capi.lib().ai2b_evaluate, C.byref(d), self.device.index)
+            model_ptrs = ("d_coeffs", "d_type_bias", "d_q_scaler", "d_w0", "d_b0", "d_w1")
+        names = model_ptrs + ("d_binum", "d_ilist", "d_types", "d_numneigh", "d_firstneigh", "d_rcs", "d_status", "d_etot", "d_force", "d_virial")
+        for name, p in zip(names, ptrs, strict=True):
+            setattr(d, name, p)
+        ws = self._workspace()
+        d.d_nblist_workspace, d.nblist_workspace_bytes = self.nb_ws.data_ptr(), self.nb_ws.numel()
+        d.d_workspace, d.workspace_bytes = ws.data_ptr(), ws.numel()
+
+    def _check_coords(self, coords):
+        """Buffers and types of a call are those of the structure: other positions would run over them."""
+        if not coords.is_cuda:
+            raise capi.Ai2bError("coords must be a CUDA tensor")
+        if coords.dtype is not self.dtype or coords.shape[0] != self.n or coords.numel() != 3 * self.n:
+            raise capi.Ai2bError(f"coords must be {self.n} positions of type {self.dtype}")
 
     def build_list(self, coords):
-        nn, fn, rcs, status = self.builder.build(self.cell, coords, self.rcut, self.umax, out=self.lists)
+        self._check_coords(coords)
+        if self.lists[1].shape[1] != self.umax:
+            self._new_lists()
+        nn, fn, rcs, status = self.builder.build(self.cell, coords, self.rcut, int(self.umax), out=self.lists)
         return dict(self.nb_static, bnumneigh=nn[None], bfirstneigh=fn[None], brcs=rcs[None])
 
     def evaluate(self, nb):
         if self.kind == "mtp":
             return capi.mtp_efv(self.prog, self.model, nb, out=self.out)
-        return capi.nep_efv(self.model, nb, out=self.out, ws=self.ws)
+        return capi.nep_efv(self.model, nb, out=self.out, ws=self._workspace())
 
     def compute(self, coords):
-        if coords.dtype is not self.dtype or coords.shape[0] != self.n or not coords.is_cuda or not coords.is_contiguous():
+        self._check_coords(coords)
+        if not coords.is_contiguous() or self.nb_static["nghost"]:
             return self.evaluate(self.build_list(coords))
+        self._describe()
         fn, desc, dev = self._call
         rc = fn(desc, coords.data_ptr(), capi.raw_stream(dev))
         if rc:
             capi._check(rc)
         return self.out
+
+    def _buffers(self):
+        """What a recorded call works on besides its positions: kept alive with the recording."""
+        return self.lists, self.ws, self.nb_ws, self.out, self.prog, list(self.model.values()), list(self.nb_static.values())
 
     def capture(self, coords):
         """Records one compute(coords) (neighbour build + E/F/V, every launch stream-ordered on buffers this
@@ -101,7 +152,7 @@ class Evaluator:
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g):
                 self.graph_out = self.compute(coords)
-            self.graph = g
+            self.graph, self.graph_buffers = g, (coords, self._buffers())
         except Exception:
             self.graph = None
             torch.cuda.synchronize()
@@ -116,6 +167,7 @@ class Evaluator:
         results -> pinned host buffer `host_out` (laid out like `outbuf`: E, virial 1..9, forces from element 16).
         replay_io() then costs one graph launch. Returns False if the capture is refused."""
         self.graph_io = None
+        self._describe()                                  # sizes every buffer before the capture
         try:
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
@@ -123,7 +175,7 @@ class Evaluator:
                 capi.copy_around_call(coords, host_coords)
                 self.compute(coords)
                 capi.copy_around_call(host_out, self.outbuf)
-            self.graph_io = g
+            self.graph_io, self.graph_io_buffers = g, (coords, host_coords, host_out, self.outbuf, self._buffers())
         except Exception:
             self.graph_io = None
             torch.cuda.synchronize()

@@ -85,3 +85,50 @@ def test_ordinary_launches_give_the_same(kind, monkeypatch):
     again = _host(ev.compute(coords))
     _close(plain, chained, tol)
     _close(again, chained, tol)
+
+
+@pytest.mark.parametrize("kind", ["mtp", "nep"])
+def test_changed_attributes_take_effect(kind):
+    """Cell, cutoff, row width and model may be edited or assigned between calls (a variable-cell relaxation does): the next
+    call is that of an Evaluator made with them. A recorded call goes on as it was recorded."""
+    w, dt, tol = _workload(kind, 8)
+    make = lambda model, cell, rcut: engine.Evaluator(model, cell, w["types"], rcut, 96, dt)
+    cell, model = np.array(w["cell"]), w["model"]
+    ev = engine.Evaluator(model, cell, w["types"], w["rcut"], w["umax"], dt)
+    coords = torch.from_numpy(np.ascontiguousarray(w["coords"])).to(dt).cuda()
+    before = _host(ev.compute(coords))
+    assert ev.capture(coords)
+
+    def same(want):
+        _close(_host(ev.compute(coords)), want, tol)
+        _close(_host(ev.evaluate(ev.build_list(coords))), want, tol)      # the two steps of a call one by one
+
+    strained = cell * cell.dtype.type(1.03)
+    want = _host(make(model, strained, w["rcut"]).compute(coords))
+    assert util.relerr(want[0], before[0]) > 10 * tol
+    ev.cell[:] = strained                     # edited in place
+    same(want)
+    sheared = strained.copy()
+    sheared[1, 0] += 0.5
+    ev.cell = sheared                         # another array
+    same(_host(make(model, sheared, w["rcut"]).compute(coords)))
+    ev.rcut, ev.umax = 0.75 * w["rcut"], 96   # rows of another width
+    same(_host(make(model, sheared, 0.75 * w["rcut"]).compute(coords)))
+    assert ev.lists[1].shape[1] == 96 and int(ev.status.cpu()[0]) <= 96
+    other = dict(model, coeffs=model["coeffs"] * model["coeffs"].dtype.type(0.9))
+    ev.model["coeffs"] = 0.9 * ev.model["coeffs"]
+    same(_host(make(other, sheared, 0.75 * w["rcut"]).compute(coords)))
+    _close(_host(ev.replay()), before, tol)
+
+
+def test_positions_that_do_not_fit_are_refused():
+    """The buffers of an Evaluator are those of its structure and type."""
+    w, dt, _ = _workload("nep", 6)
+    ev = engine.Evaluator(w["model"], w["cell"], w["types"], w["rcut"], w["umax"], dt)
+    coords = torch.from_numpy(np.ascontiguousarray(w["coords"])).to(dt).cuda()
+    for bad in (coords.double(), coords[:-1], torch.cat([coords, coords[:1]]), coords.cpu()):
+        for call in (ev.compute, ev.build_list):
+            with pytest.raises(engine.capi.Ai2bError):
+                call(bad)
+    strided = torch.empty(ev.n, 4, dtype=dt, device="cuda")[:, :3].copy_(coords)
+    _close(_host(ev.compute(strided)), _host(ev.compute(coords)), 1e-5)
