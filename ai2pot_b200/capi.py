@@ -4,9 +4,9 @@ PyTorch is used only as the owner of device memory and streams: every function h
 CUDA tensors, passes their raw pointers to libai2pot_b200.so and returns torch tensors. There is
 no CPU implementation behind these calls: a missing library or a non-CUDA tensor raises.
 """
+import collections
 import ctypes as C
 import os
-import sys
 
 import numpy as np
 import torch
@@ -498,6 +498,31 @@ def peer_wait(flag, value, status, max_polls=5_000_000):
     _check(lib().ai2b_peer_wait(_ptr(flag), C.c_int(int(value)), C.c_longlong(int(max_polls)), _ptr(status), _stream()))
 
 
+class _Lease:
+    """Owner of an array's memory while any array, view or buffer over it is alive; then the memory goes back to the pool."""
+    __slots__ = ("block", "pool", "__array_interface__", "__weakref__")
+
+    def __init__(self, block, interface, pool):
+        self.block, self.__array_interface__, self.pool = block, interface, pool
+
+    def __del__(self):
+        self.pool.append((self.block, self.__array_interface__))
+
+
+def _lease_array(pool, shape):
+    """A float64 array over a block of `pool` (a deque with a length limit) or, if none of its shape is free, over new
+    memory. Fresh pages cost more than the values that a step writes into them; the lease itself takes 1 us."""
+    while pool:
+        try:
+            block, interface = pool.pop()
+        except IndexError:          # another thread took the last one
+            break
+        if block.shape == shape:
+            return np.asarray(_Lease(block, interface, pool))
+    block = np.empty(shape, np.float64)
+    return np.asarray(_Lease(block, block.__array_interface__, pool))
+
+
 class MdSession:
     """ctypes wrapper of ai2b_md_session_*: the device-resident input path of an MD host
     (positions + model types in, forces on local and ghost atoms + energy + six virial components out).
@@ -505,7 +530,7 @@ class MdSession:
 
     def __init__(self, model, umax, prog=None):
         self.h = C.c_void_p()
-        self._spare = []
+        self._spare = collections.deque(maxlen=2)      # force arrays that the caller has let go of
         self._out = np.zeros(7, np.float64)      # energy, six virial components of a step
         self._out_p = (C.c_void_p(self._out.ctypes.data), C.c_void_p(self._out.ctypes.data + 8))
         f32 = lambda a: np.ascontiguousarray(np.asarray(a).ravel(), np.float32)
@@ -525,20 +550,10 @@ class MdSession:
                 C.c_int(int(model["ntypes"])), C.c_int(int(prog.nmus)), C.c_int(int(prog.ns)), *[hp(x) for x in a],
                 C.c_float(model["rmax"]), C.c_float(model["rmin"]), C.c_int(int(umax))))
 
-    def _force_array(self, n):
-        """An array for the forces of n atoms. Memory whose last array the caller has dropped is used again (two blocks at most,
-        returned with the session): fresh pages cost more than the forces themselves."""
-        for base in self._spare:
-            if base.shape[0] == n and sys.getrefcount(base) == 3:      # the list, the loop variable, the argument
-                return base.view()
-        base = np.empty((n, 3), np.float64)
-        self._spare = [base] + self._spare[:1]
-        return base.view()
-
     def compute(self, nlocal, nghost, x, model_type, want_virial=True):
         x = np.ascontiguousarray(x, np.float64)
         t = np.ascontiguousarray(model_type, np.int32)
-        f = self._force_array(nlocal + nghost)
+        f = _lease_array(self._spare, (nlocal + nghost, 3))
         out = self._out
         out[:] = 0.0
         mx = C.c_int(0)
@@ -552,6 +567,7 @@ class MdSession:
         if self.h:
             lib().ai2b_md_session_destroy(self.h)
             self.h = C.c_void_p()
+        self._spare.clear()
 
     def __del__(self):
         try:
