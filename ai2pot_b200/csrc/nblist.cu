@@ -762,7 +762,7 @@ nb_rows_kernel(NbParams<T> P, const NbGrid *__restrict__ gp, const int *__restri
                 if (lane == 0) s_n2[warp] = n2max;
                 __syncthreads();
 #pragma unroll
-                for (int k = 0; k < WPC; k++) n2max = fmaxf(n2max, s_n2[k]);
+                for (int k = 0; k < WPC; k++) n2max = fmaxf(n2max, s_n2[team * WPC + k]);
             } else {
                 __syncwarp();
             }

@@ -275,6 +275,24 @@ def test_build_at_the_edges_of_its_forms(checkers, dt, n, density, umax, pbc):
 
 
 @pytest.mark.parametrize("dt", [np.float64, np.float32])
+def test_two_warps_per_bin_with_uneven_bins(checkers, dt):
+    """Two teams share a block in the two-warp form. Drops in an otherwise empty cell make them run different numbers of bins
+    (most are empty) and tables of different length (crowded bins take several pieces), so each needs barriers of its own."""
+    chk = _chk(checkers)
+    rng = np.random.default_rng(33)
+    n, L, rcut, nb = 9000, 70.0, 5.0, 13           # 2,197 bins, 4.1 atoms per bin on average
+    drops = rng.random((60, 3)) * L
+    sizes = rng.choice([20, 60, 150, 370], size=60)
+    pos = np.concatenate([d + rng.normal(0, 2.6, (k, 3)) for d, k in zip(drops, sizes)] + [rng.random((n, 3)) * L])[:n].astype(dt)
+    cell, types = (np.eye(3) * L).astype(dt), np.zeros(n, np.int32)
+    ref = chk.nblist(cell, types, pos, rcut, 400)
+    bins = np.bincount(np.ravel_multi_index((np.floor(np.mod(pos, L) / L * nb).astype(int) % nb).T, (nb, nb, nb)), minlength=nb ** 3)
+    assert 2.5 < n / nb ** 3 < 5.5 and (bins == 0).sum() > 500 and bins.max() > 100
+    for _ in range(3):
+        util.assert_nblist_equal(_gpu(cell, types, pos, rcut, 400), ref[:3])
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.float32])
 @pytest.mark.parametrize("sizes,umax", [((600, 512, 1), 64), ((17, 16, 15), 66)])
 def test_batched_build_tiles_and_chunks(checkers, dt, sizes, umax):
     """Structures longer than one tile of the batched build, exactly one tile, and sizes around its chunk of centres."""
