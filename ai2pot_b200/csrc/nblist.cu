@@ -635,7 +635,17 @@ nb_rows_kernel(NbParams<T> P, const NbGrid *__restrict__ gp, const int *__restri
     TO *rowp = reinterpret_cast<TO *>(p_list) + (size_t)warp * 3 * P.umax;   // (staged only)
     int *rowi = reinterpret_cast<int *>(reinterpret_cast<TO *>(p_list) + (size_t)NBC_WARPS * 3 * P.umax) + warp * P.umax;
     unsigned short *list = reinterpret_cast<unsigned short *>(p_list + (staged ? (size_t)NBC_WARPS * P.umax * (sizeof(int) + 3 * sizeof(TO)) : 0)) + warp * CAP;
-    auto sync_team = [&]() { if constexpr (WPC == 1) __syncwarp(); else __syncthreads(); };
+    // The teams of a block walk over different numbers of bins (empty ones are skipped) and tables of different length, so a
+    // barrier is the team's own (numbers as constants: a number in a register would claim all sixteen).
+    static_assert(WPC == 1 || TEAMS <= 2, "a barrier per team");
+    auto sync_team = [&]() {
+        __syncwarp();
+        if constexpr (WPC > 1) {
+            if constexpr (TEAMS == 1) __syncthreads();
+            else if (team == 0) asm volatile("bar.sync 1, %0;" ::"n"(TT) : "memory");
+            else asm volatile("bar.sync 2, %0;" ::"n"(TT) : "memory");
+        }
+    };
     // no chain_release(): blocks of the next kernel that become resident now only take slots and issue cycles from this one
     // (13,824 atoms: a NEP evaluation 85.7 -> 74.5 us, an MTP evaluation 143.9 -> 127.7 us)
     chain_wait();
@@ -760,7 +770,7 @@ nb_rows_kernel(NbParams<T> P, const NbGrid *__restrict__ gp, const int *__restri
             for (int o = 16; o >= 1; o >>= 1) n2max = fmaxf(n2max, __shfl_xor_sync(FULL_MASK, n2max, o));
             if constexpr (WPC > 1) {
                 if (lane == 0) s_n2[warp] = n2max;
-                __syncthreads();
+                sync_team();
 #pragma unroll
                 for (int k = 0; k < WPC; k++) n2max = fmaxf(n2max, s_n2[team * WPC + k]);
             } else {
