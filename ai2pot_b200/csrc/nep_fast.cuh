@@ -281,11 +281,11 @@ __device__ __forceinline__ void add3(float *f, float x, float y, float z)
 __device__ __forceinline__ void add3(double *f, double x, double y, double z) { atomicAdd(f, x); atomicAdd(f + 1, y); atomicAdd(f + 2, z); }
 
 // shared-memory elements (of T) per warp behind the model table; the neighbour lists follow (two bytes per neighbour)
-template <int NMAX, int G>
-__host__ __device__ inline int nep_fast_warp_elems(int nneu, int umax, bool net)
+template <int NMAX>
+__host__ __device__ inline int nep_fast_warp_elems(int lanes, int nneu, int umax, bool net)
 {
     using D = NepFastDims<NMAX>;
-    constexpr int AW = 32 / G;
+    const int AW = 32 / lanes;
     const int stage = 32 * D::RS, es = AW * D::ESR;                 // staging rows, later the adjoints of the sums
     return (stage > es ? stage : es) + AW * 2 * D::NDP +            // descriptors, their adjoints
            (net ? AW * (nep_r32(nneu) + 4) + 96 + AW * umax * NMAX : 0);   // neurons, angular forces, cached derivatives
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_fast_kernel(const Ne
     if (early_release) chain_release();
     const NepTab<NMAX> L(A.ntypes, A.nneu, NET);
     T *tab_s = reinterpret_cast<T *>(nep_smem);
-    const int per_warp = nep_fast_warp_elems<NMAX, G>(A.nneu, A.umax, NET), NP = nep_r32(A.nneu), NPP = NP + 4;
+    const int per_warp = nep_fast_warp_elems<NMAX>(G, A.nneu, A.umax, NET), NP = nep_r32(A.nneu), NPP = NP + 4;
     T *stage = tab_s + L.total + (size_t)warp * per_warp;
     T *es = stage;                                       // [AW][ESR]
     T *q = stage + (32 * RS > AW * ESR ? 32 * RS : AW * ESR) + grp * NDP;

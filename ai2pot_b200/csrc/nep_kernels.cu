@@ -540,15 +540,42 @@ static size_t nep_ws_bytes(int B, int ntypes, int n_r, int n_a, int csp, size_t 
     return std::max(nep_ws_min(B, ntypes, n_r, n_a, csp, elem), nep_prefix_bytes(B) + NEP_TAB_BYTES);
 }
 
-template <typename T, int MODE, int NMAX, int G>
-static int launch_nep_fast_g(const NepArgs<T> &A, const T *tab, size_t tab_elems, cudaStream_t st, bool *done)
+// dynamic shared memory of a block of the specialised kernel; it shrinks as the lanes per atom grow
+template <typename T, int NMAX>
+static size_t nep_fast_smem(int lanes, const NepTab<NMAX> &L, int nneu, int umax, bool net)
 {
-    constexpr bool NET = MODE != NEP_DESC;
+    return (L.total + (size_t)NEP_WARPS * nep_fast_warp_elems<NMAX>(lanes, nneu, umax, net)) * sizeof(T) +
+           (size_t)NEP_WARPS * (32 / lanes) * umax * sizeof(unsigned short) + 16;
+}
+
+// Lanes per atom of the specialised kernel for models of at most NMAX radial and angular functions; 0: the model or the
+// neighbour width does not fit it, and the general kernel runs.
+// Few atoms: more lanes, the chip is filled by atoms x lanes. Whole call in us, fp32, 29 / 6.5 neighbours (in brackets eight
+// lanes per atom and a trip count per group):
+//   216 atoms: 32 lanes 9.8, 16 lanes 10.6 [20.2];   1,157: 12.6, 12.2 [20.3];   4,000: 16 lanes 14.7, 8 lanes 18.1 [24.5];
+//   13,824: 16 lanes 30.5, 8 lanes 30.0 [48.7];   60,000: 8 lanes 80, 4 lanes 110 [176]
+// Four lanes pay when the rows are short enough for four blocks per SM and angular neighbours are few (17 / 2.2
+// neighbours, 1,048,576 atoms: 945, eight lanes 1083 [1435]); narrow rows stand for that.
+// Where the shared memory of the wanted form exceeds a block's share, the next one with more lanes is taken (kernels alone;
+// 12 species, umax 32, 60,000 atoms: 8 lanes 103, general kernel 505; fp64, umax 128, 13,824 atoms: 16 lanes 55, 32 lanes 80).
+template <typename T, int NMAX>
+static int nep_fast_lanes(long atoms, int ntypes, int nneu, int umax, bool net)
+{
+    const NepTab<NMAX> L(ntypes, nneu, net);
+    if (ntypes > 16 || umax > 1024 || atoms >= (1L << 31) || (size_t)L.total * sizeof(T) > NEP_TAB_BYTES) return 0;
+    int lanes = 8;
+    if (net && NMAX == 4 && sizeof(T) == 4 && atoms >= 50000 && umax <= 32) lanes = 4;
+    else if (atoms <= (net ? 1000 : 4000)) lanes = 32;
+    else if (net && atoms <= 6000) lanes = 16;
+    while (lanes < 32 && nep_fast_smem<T, NMAX>(lanes, L, nneu, umax, net) > NEP_FAST_SMEM) lanes *= net || lanes == 16 ? 2 : 4;
+    return nep_fast_smem<T, NMAX>(lanes, L, nneu, umax, net) <= NEP_FAST_SMEM ? lanes : 0;
+}
+
+template <typename T, int MODE, int NMAX, int G>
+static int launch_nep_fast_g(const NepArgs<T> &A, const T *tab, const NepTab<NMAX> &L, cudaStream_t st)
+{
     constexpr int MINB = sizeof(T) == 4 ? 4 : 2;
-    *done = false;
-    const size_t smem = (tab_elems + (size_t)NEP_WARPS * nep_fast_warp_elems<NMAX, G>(A.nneu, A.umax, NET)) * sizeof(T) +
-                        (size_t)NEP_WARPS * (32 / G) * A.umax * sizeof(unsigned short) + 16;
-    if (smem > NEP_FAST_SMEM) return AI2B_OK;
+    const size_t smem = nep_fast_smem<T, NMAX>(G, L, A.nneu, A.umax, MODE != NEP_DESC);
     auto kern = nep_fast_kernel<T, G, MODE, NMAX, MINB>;
     static KernelSetup setup;
     int per_sm = 1;
@@ -559,7 +586,6 @@ static int launch_nep_fast_g(const NepArgs<T> &A, const T *tab, size_t tab_elems
     const int early = blocks * 2 <= room;
     if (blocks > room) blocks = room;
     AI2B_CUDA(launch_chained(kern, (unsigned)blocks, NEP_WARPS * 32, smem, st, A, tab, early));
-    *done = true;
     return AI2B_OK;
 }
 
@@ -570,16 +596,10 @@ static int launch_nep_fast(NepArgs<T> A, const T *coeffs, void *ws, size_t ws_by
 {
     constexpr bool NET = MODE != NEP_DESC;
     *done = false;
-    if (A.ntypes > 16 || A.umax > 1024 || (long)A.B * A.npad >= (1L << 31)) return AI2B_OK;
+    const int lanes = nep_fast_lanes<T, NMAX>((long)A.B * A.npad, A.ntypes, A.nneu, A.umax, NET);
     const NepTab<NMAX> L(A.ntypes, A.nneu, NET);
-    const size_t tab_bytes = (size_t)L.total * sizeof(T);
-    if (tab_bytes > NEP_TAB_BYTES || nep_prefix_bytes(A.B) + tab_bytes > ws_bytes) return AI2B_OK;
+    if (lanes == 0 || nep_prefix_bytes(A.B) + (size_t)L.total * sizeof(T) > ws_bytes) return AI2B_OK;
     T *tab = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(ws) + nep_prefix_bytes(A.B));
-    auto fits = [&](int lanes) {
-        const int warp = lanes == 32 ? nep_fast_warp_elems<NMAX, 32>(A.nneu, A.umax, NET) : nep_fast_warp_elems<NMAX, 8>(A.nneu, A.umax, NET);
-        return tab_bytes + (size_t)NEP_WARPS * warp * sizeof(T) + (size_t)NEP_WARPS * (32 / lanes) * A.umax * 2 + 16 <= NEP_FAST_SMEM;
-    };
-    if (!fits(32)) return AI2B_OK;
     {   // table, offsets, zeroed outputs
         T *z[3] = {NET ? A.etot : A.desc, A.force, A.virial};
         const size_t nz[3] = {NET ? (size_t)A.B : (size_t)A.B * A.npad * A.nd, NET ? 3 * (size_t)A.B * (A.npad + A.nghost) : 0, A.virial ? 9 * (size_t)A.B : 0};
@@ -590,19 +610,13 @@ static int launch_nep_fast(NepArgs<T> A, const T *coeffs, void *ws, size_t ws_by
         AI2B_CUDA(launch_chained(nep_prep_kernel<T, NMAX>, (unsigned)(tb + zb), 256, 0, st, A, coeffs, tab, const_cast<int *>(A.prefix), NET ? 1 : 0, tb,
                                  z[0], A.zero ? nz[0] : 0, z[1], A.zero ? nz[1] : 0, z[2], A.zero ? nz[2] : 0));
     }
-    const long atoms = (long)A.B * A.npad;
-    // Lanes per atom. Few atoms: more lanes, the chip is filled by atoms x lanes. Whole call in us, fp32, 29 / 6.5 neighbours
-    // (in brackets eight lanes per atom and a trip count per group):
-    //   216 atoms: 32 lanes 9.8, 16 lanes 10.6 [20.2];   1,157: 12.6, 12.2 [20.3];   4,000: 16 lanes 14.7, 8 lanes 18.1 [24.5];
-    //   13,824: 16 lanes 30.5, 8 lanes 30.0 [48.7];   60,000: 8 lanes 80, 4 lanes 110 [176]
-    // Four lanes pay when the rows are short enough for four blocks per SM and angular neighbours are few (17 / 2.2
-    // neighbours, 1,048,576 atoms: 945, eight lanes 1083 [1435]); narrow rows stand for that.
+    *done = true;
     if constexpr (NET && NMAX == 4 && sizeof(T) == 4)
-        if (atoms >= 50000 && A.umax <= 32) return launch_nep_fast_g<T, MODE, NMAX, 4>(A, tab, L.total, st, done);
-    if (atoms <= (NET ? 1000 : 4000) || !fits(8)) return launch_nep_fast_g<T, MODE, NMAX, 32>(A, tab, L.total, st, done);
+        if (lanes == 4) return launch_nep_fast_g<T, MODE, NMAX, 4>(A, tab, L, st);
     if constexpr (NET)
-        if (atoms <= 6000) return launch_nep_fast_g<T, MODE, NMAX, 16>(A, tab, L.total, st, done);
-    return launch_nep_fast_g<T, MODE, NMAX, 8>(A, tab, L.total, st, done);
+        if (lanes == 16) return launch_nep_fast_g<T, MODE, NMAX, 16>(A, tab, L, st);
+    if (lanes == 8) return launch_nep_fast_g<T, MODE, NMAX, 8>(A, tab, L, st);
+    return launch_nep_fast_g<T, MODE, NMAX, 32>(A, tab, L, st);
 }
 
 template <typename T, int CSP, int MODE>
@@ -667,6 +681,15 @@ using namespace ai2b;
 extern "C" size_t ai2b_nep_workspace_bytes(int batch_size, int ntypes, int n_radial, int n_angular, int chebyshev_size, int is_f64)
 {
     return nep_ws_bytes(batch_size, ntypes, n_radial, n_angular, chebyshev_size <= 8 ? 8 : 16, is_f64 ? 8 : 4);
+}
+
+extern "C" int ai2b_nep_lanes_per_atom(int natoms, int ntypes, int n_radial, int n_angular, int chebyshev_size, int num_neurons, int umax,
+                                       int is_f64, int descriptors_only)
+{
+    if (natoms < 0 || ntypes < 1 || num_neurons < 1 || umax < 0 || chebyshev_size > 8 || n_radial > 8 || n_angular > 8) return 0;
+    const bool net = !descriptors_only, four = n_radial <= 4 && n_angular <= 4;
+    if (is_f64) return four ? nep_fast_lanes<double, 4>(natoms, ntypes, num_neurons, umax, net) : nep_fast_lanes<double, 8>(natoms, ntypes, num_neurons, umax, net);
+    return four ? nep_fast_lanes<float, 4>(natoms, ntypes, num_neurons, umax, net) : nep_fast_lanes<float, 8>(natoms, ntypes, num_neurons, umax, net);
 }
 
 #define AI2B_DEF_NEP(SUF, T)                                                                                    \

@@ -450,6 +450,11 @@ int ai2b_nblist_build_ghost_f64_rows32(int natoms, int ncentres, const double *h
 
 size_t ai2b_nep_workspace_bytes(int batch_size, int ntypes, int n_radial, int n_angular,
                                 int chebyshev_size, int is_f64);
+/* How a call evaluates an atom: the lanes that it gets in the specialised kernel (4, 8, 16 or 32),
+ * or 0 where the general kernel runs (more than 8 functions of a kind, or tables and rows that do
+ * not fit a block's shared memory). natoms: batch size x padded atom count. */
+int ai2b_nep_lanes_per_atom(int natoms, int ntypes, int n_radial, int n_angular, int chebyshev_size,
+                            int num_neurons, int umax, int is_f64, int descriptors_only);
 
 /* Energy + force + virial. Replaces nep::find_efv_torch_launcher<T>
  * (source/descriptor/nep/gpu/include/nep_torch_launcher.cuh:34-103) and the CPU launcher

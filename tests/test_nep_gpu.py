@@ -247,3 +247,35 @@ def test_ragged_batch_warps_across_structures(checkers, dt, B, nmin, nmax):
     want = chk.nep_efv(_f64(model), dict(nb, brcs=nb["brcs"].astype(np.float64)))
     for a, b, name in zip(got, want, ("energy", "force", "virial")):
         assert util.relerr(a, b) < (1e-10 if dt == np.float64 else 1e-5), name
+
+
+@pytest.mark.parametrize("dt,ntypes,neurons,slots,umax,lanes", [
+    (np.float32, 12, 30, 50000, 32, 8),        # four lanes would be wanted, their shared memory does not fit
+    (np.float32, 10, 30, 50000, 32, 4),
+    (np.float32, 12, 30, 7000, 100, 16),       # eight do not fit, sixteen do
+    (np.float64, 3, 30, 7000, 128, 16),
+    (np.float64, 3, 30, 7000, 200, 32),
+    (np.float64, 8, 30, 7000, 64, 0),          # general kernel
+])
+def test_lanes_when_shared_memory_is_short(checkers, dt, ntypes, neurons, slots, umax, lanes):
+    """Padded slots stand for many atoms: the form of the kernel follows from them, few are filled."""
+    B, npad = 2, slots // 2
+    got_lanes = capi.lib().ai2b_nep_lanes_per_atom(B * npad, ntypes, 4, 4, 8, neurons, umax, int(dt == np.float64), 0)
+    assert got_lanes == lanes
+    chk = _chk(checkers)
+    rng = np.random.default_rng(ntypes)
+    model = synth.nep_model(ntypes, rng, dt, num_neurons=neurons)
+    lists = []
+    for n in (5, 6):
+        cell, pos = synth.cubic_lattice(n, 3.0, 0.1, rng, dt)
+        lists.append(chk.nblist(cell, rng.integers(0, ntypes, len(pos)).astype(np.int32), pos, 5.0, umax)[:4])
+    nb = synth.pad_batch(lists, ntypes, umax)
+    for k in ("bilist", "bnumneigh", "bfirstneigh", "brcs", "btypes"):
+        a = nb[k]
+        fill = np.full((B, npad) + a.shape[2:], -1 if k == "bfirstneigh" else 0, a.dtype)
+        fill[:, :a.shape[1]] = a
+        nb[k] = fill
+    got, *_ = _run(model, nb)
+    want = chk.nep_efv(_f64(model), dict(nb, brcs=nb["brcs"].astype(np.float64)))
+    for a, b, name in zip(got, want, ("energy", "force", "virial")):
+        assert util.relerr(a, b) < (1e-10 if dt == np.float64 else 1e-5), name
