@@ -275,6 +275,33 @@ def test_build_at_the_edges_of_its_forms(checkers, dt, n, density, umax, pbc):
 
 
 @pytest.mark.parametrize("dt", [np.float64, np.float32])
+def test_host_list_keeps_no_large_buffers(checkers, dt, monkeypatch):
+    """A host list above the staging limit comes back in pieces, and nothing of it stays behind."""
+    from ai2pot_b200.fromcc import nblist
+    chk = _chk(checkers)
+    w = util.small_mtp_case(10, 6, dt)
+    args = (w["cell"], w["types"], w["coords"], 5.0, 48, True, [True, True, True])
+    ref = chk.nblist(w["cell"], w["types"], w["coords"], 5.0, 48)
+    staged = nblist.find_info4mlff(*args, True)
+    held = nblist._lists
+    assert held is not None and held.host.is_pinned() and held.host.numel() <= nblist.STAGING_BYTES
+    monkeypatch.setattr(nblist, "STAGING_BYTES", held.host.numel() - 1)
+    monkeypatch.setattr(nblist, "_lists", None)
+    for piece in (8 << 20, 4096, 1000 * dt(0).itemsize):
+        monkeypatch.setattr(nblist, "PIECE_BYTES", piece)
+        plain = nblist.find_info4mlff(*args, True)
+        assert nblist._lists is None
+        for a, b in zip(plain, staged):
+            assert np.array_equal(a, b) and (np.isscalar(a) or a.dtype == b.dtype and a.shape == b.shape and a.flags.writeable)
+    util.assert_nblist_equal(nblist.find_info4mlff(*args, False)[2:5], ref[:3])
+    monkeypatch.setattr(nblist, "STAGING_BYTES", 1000)
+    with pytest.raises(ValueError, match="umax=8"):
+        nblist.find_info4mlff(*args[:4], 8, *args[5:], False)
+    empty = nblist.find_info4mlff(w["cell"], w["types"][:0], w["coords"][:0], 5.0, 48, True, [True] * 3, True)
+    assert empty[0] == 0 and empty[3].shape == (0, 48) and empty[4].shape == (0, 48, 3)
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.float32])
 def test_two_warps_per_bin_with_uneven_bins(checkers, dt):
     """Two teams share a block in the two-warp form. Drops in an otherwise empty cell make them run different numbers of bins
     (most are empty) and tables of different length (crowded bins take several pieces), so each needs barriers of its own."""
