@@ -63,8 +63,7 @@ class _Lists:
         else:
             self.coords.copy_(torch.from_numpy(np.ascontiguousarray(coords).reshape(-1)))
         hpbc = (C.c_int * 3)(*[1 if p else 0 for p in pbc])
-        hcell = np.ascontiguousarray(cell)
-        capi._check(self.build_fn(C.c_int(self.n), C.c_void_p(hcell.ctypes.data), C.c_void_p(self.coords.data_ptr()), C.c_int(1 if is_cart else 0),
+        capi._check(self.build_fn(C.c_int(self.n), C.c_void_p(cell.ctypes.data), C.c_void_p(self.coords.data_ptr()), C.c_int(1 if is_cart else 0),
                                   C.c_double(rcut), hpbc, *self.tail, stream))
         if sort:
             capi._check(self.sort_fn(*self.sort_args, stream))
@@ -123,6 +122,7 @@ def find_info4mlff(cell, types, coords, rcut, umax, is_cart, pbc, sort):
         raise TypeError("cell and coords must both be float32 or both float64")
     if types.dtype not in (np.int32, np.int64):
         raise TypeError("types must be int32 or int64")
+    cell = np.ascontiguousarray(cell).reshape(9)      # (a cell of another size raises)
     n, umax = int(coords.shape[0]), int(umax)
     key = (n, umax, torch.float64 if coords.dtype == np.float64 else torch.float32, torch.device("cuda", torch.cuda.current_device()))
     with _lock:

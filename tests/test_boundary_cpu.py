@@ -138,3 +138,11 @@ def test_predict_efv_modules_script_and_save(tmp_path):
         torch.jit.save(torch.jit.script(module), path)
         back = torch.jit.load(path)
         assert hasattr(back, "predict_efv")
+
+
+@pytest.mark.parametrize("shape", [(8,), (2, 3), (3, 4), (0,)])
+def test_host_list_refuses_cells_of_another_size(shape):
+    """The nine numbers of the cell are read from host memory: fewer would be read past their end."""
+    from ai2pot_b200.fromcc import nblist
+    with pytest.raises(ValueError):
+        nblist.find_info4mlff(np.zeros(shape), np.zeros(4, np.int32), np.zeros((4, 3)), 5.0, 8, True, [True] * 3, False)
