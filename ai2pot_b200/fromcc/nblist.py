@@ -132,7 +132,11 @@ def find_info4mlff(cell, types, coords, rcut, umax, is_cart, pbc, sort):
             _lists = lists if lists.staged else None
         else:
             lists = _lists
-        st, nn, fn, rcs = lists.run(cell, coords, float(rcut), bool(is_cart), pbc, bool(sort))
+        try:
+            st, nn, fn, rcs = lists.run(cell, coords, float(rcut), bool(is_cart), pbc, bool(sort))
+        except Exception:
+            torch.cuda.current_stream().synchronize()      # work may be under way on buffers that another stream is given next
+            raise
     if st[1]:
         raise ValueError(f"umax={umax} is smaller than the largest neighbour count {st[0]}")
     return (n, np.arange(n, dtype=np.int32), nn, fn, rcs, np.ascontiguousarray(types, dtype=np.int32), 0)

@@ -301,6 +301,22 @@ def test_host_list_keeps_no_large_buffers(checkers, dt, monkeypatch):
     assert empty[0] == 0 and empty[3].shape == (0, 48) and empty[4].shape == (0, 48, 3)
 
 
+def test_host_list_that_fails_leaves_no_work_behind(checkers):
+    """The buffers of a call that raises half-way (rows too wide to be sorted) may be given to another stream at once."""
+    from ai2pot_b200.fromcc import nblist
+    w = util.small_mtp_case(10, 6, np.float64)
+    args = (w["cell"], w["types"], w["coords"], 5.0, 1500, True, [True, True, True])
+    nblist.find_info4mlff(*args, False)         # buffers of this size are there (an allocation would wait for the device)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(100_000_000)          # tens of milliseconds in front of the call's work
+        with pytest.raises(capi.Ai2bError):
+            nblist.find_info4mlff(*args, True)
+        assert side.query()
+    ref = _chk(checkers).nblist(w["cell"], w["types"], w["coords"], 5.0, 1500)
+    util.assert_nblist_equal(nblist.find_info4mlff(*args, False)[2:5], ref[:3])
+
+
 @pytest.mark.parametrize("dt", [np.float64, np.float32])
 def test_two_warps_per_bin_with_uneven_bins(checkers, dt):
     """Two teams share a block in the two-warp form. Drops in an otherwise empty cell make them run different numbers of bins
