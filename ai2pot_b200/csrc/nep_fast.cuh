@@ -8,7 +8,7 @@
 //   * set-up: nep_prep_kernel lays the model out once per call (padded rows, signs and constants folded in) and zeroes the
 //     outputs; a block takes the table with a handful of 16-byte copies;
 //   * radial pass, lanes = neighbours of the group's atom: Chebyshev sums of all functions and their derivatives in packed
-//     pairs, cutoff from two short polynomials; g'_n(r_j) / r_j are kept per neighbour in shared memory;
+//     pairs, g'_n(r_j) / r_j are kept per neighbour in shared memory;
 //   * angular pass, lanes = angular neighbours of all atoms of the warp, back to back: only a fifth of the neighbours are
 //     inside the angular cutoff (6.5 of 29, or 2.2 of 17), so lanes that belong to one atom would mostly idle. The harmonics
 //     of a neighbour go through shared memory to the lanes that own its atom's sums S[mu][lm];
@@ -190,16 +190,6 @@ __global__ void nep_prep_kernel(const NepArgs<T> A, const T *__restrict__ coeffs
     for (size_t i = i0; i < n2; i += step) z2[i] = T(0);
 }
 
-// sin and cos of pi t / 2, 0 <= t <= 1, s = t - 1: polynomials in t^2 fitted to the functions (sin(pi t / 2) / t, and
-// cos(pi t / 2) / (1 - t^2), so that the cosine keeps its relative precision towards t = 1); relative error 1.2e-7 and 6e-8
-__device__ __forceinline__ void quarter_wave(float t, float s, float &sn, float &cs)
-{
-    const float x = t * t;
-    sn = t * fmaf(fmaf(fmaf(fmaf(1.5167852689e-04f, x, -4.6741575934e-03f), x, 7.9689927399e-02f), x, -6.4596378803e-01f), x, 1.5707963705f);
-    cs = -s * (t + 1.f) * fmaf(fmaf(fmaf(fmaf(2.3601285648e-05f, x, -8.9353672229e-04f), x, 1.9968606532e-02f), x, -2.3370051384e-01f), x, 1.f);
-}
-__device__ __forceinline__ void quarter_wave(double t, double, double &sn, double &cs) { sincospi(0.5 * t, &sn, &cs); }
-
 // 1 / sqrt(v) with a Newton step behind the hardware's estimate in single precision
 __device__ __forceinline__ float inv_sqrt(float v) { const float y = rsqrtf(v); return y * fmaf(-0.5f * v * y, y, 1.5f); }
 __device__ __forceinline__ double inv_sqrt(double v) { return rsqrt(v); }
@@ -234,7 +224,7 @@ __device__ __forceinline__ void nep_functions(const T *tc, T t, T inv_rc, Pk<T> 
         u0 = u1; u1 = u2;
     }
     T sn, cs;
-    quarter_wave(t, s, sn, cs);
+    gsincospi(T(0.5) * t, &sn, &cs);      // (polynomials of t^2 in its place saved 0.6 % of a call at 13,824 atoms, with errors up to 1.8e-7)
     const T fh = T(0.5) * cs * cs;      // half the cutoff function cos^2(pi t / 2)
     const Pk<T> f2 = pk(fh, fh);
 #pragma unroll
