@@ -4,7 +4,6 @@
 #include <algorithm>
 #include <cstring>
 #include <fstream>
-#include <queue>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -132,6 +131,96 @@ struct Blob {
         return off;
     }
 };
+
+// Deals the moments of a phase (by decreasing row count) to MTP_PAIR_WARPS warps of `groups` groups of lanes each: the first
+// nwide of them to whole warps, the others to groups, each to the least loaded place, the lowest of equals, completing a
+// moment taken as a row. choose() takes the nwide of the least cost; candidates are looked at by a lower bound of their cost,
+// so that most are never dealt.
+class RowDeal {
+public:
+    explicit RowDeal(int groups) : groups(groups), wide_rows(MTP_PAIR_WARPS), group_rows(MTP_PAIR_WARPS * groups), load(MTP_PAIR_WARPS * groups) {}
+    int nwide = 0;
+    std::vector<int> place;      // warp (of a wide moment) or group
+
+    void choose(const int4 *q, int nq)
+    {
+        n.resize(nq);
+        place.resize(nq);
+        for (int i = 0; i < nq; i++) n[i] = q[i].z - q[i].y;
+        cand.clear();
+        long rest = 0, wide = 0;
+        for (int v : n) rest += v;
+        for (int i = 0; i < nq; i++) {
+            if (i == 0 || n[i] != n[i - 1]) {      // all moments of one row count are dealt alike
+                const long sum = wide + (rest + groups - 1) / groups;
+                const long longest = std::max<long>({(sum + MTP_PAIR_WARPS - 1) / MTP_PAIR_WARPS, n[i], i ? (n[0] + groups - 1) / groups : 0});
+                cand.push_back({cost(longest, sum), i});
+            }
+            wide += (n[i] + groups - 1) / groups;
+            rest -= n[i];
+        }
+        std::stable_sort(cand.begin(), cand.end(), [](const Candidate &x, const Candidate &y) { return x.bound < y.bound; });
+        long best = -1;
+        int dealt = nwide = 0;
+        for (const Candidate &c : cand) {
+            if (best >= 0 && (c.bound > best || (c.bound == best && c.wide > nwide))) continue;
+            const long v = deal(dealt = c.wide);
+            if (best < 0 || v < best || (v == best && c.wide < nwide)) { best = v; nwide = c.wide; }
+        }
+        if (nq == 0 || dealt != nwide) deal(nwide);
+    }
+    int length(int w) const { return wide_rows[w] + *std::max_element(group_rows.begin() + w * groups, group_rows.begin() + (w + 1) * groups); }
+
+private:
+    struct Candidate { long bound; int wide; };
+    const int groups;
+    std::vector<Candidate> cand;
+    std::vector<int> n, wide_rows, group_rows, load;
+    std::vector<unsigned> at_load;      // [load][words]: which places have it
+
+    static long cost(long longest, long sum) { return 60 * longest + 5 * sum; }
+
+    // moments i0 .. i1 to `places` places with the loads load[]; a moment adds size(i) rows and one
+    template <typename Size>
+    void spread(int i0, int i1, int places, std::vector<int> &rows, Size size)
+    {
+        if (i0 == i1) return;
+        const int words = (places + 31) / 32;
+        int most = 0, low = load[0], highest = 0;
+        long total = 0;
+        for (int p = 0; p < places; p++) { low = std::min(low, load[p]); highest = std::max(highest, load[p]); total += load[p]; }
+        for (int i = i0; i < i1; i++) { most = std::max(most, size(i) + 1); total += size(i) + 1; }
+        // the least loaded place is never above the mean
+        at_load.assign((size_t)words * (std::max<long>(highest, total / places) + most + 1), 0u);
+        for (int p = 0; p < places; p++) at_load[(size_t)words * load[p] + p / 32] |= 1u << (p % 32);
+        for (int i = i0; i < i1; i++) {
+            int w = 0;
+            while (at_load[(size_t)words * low + w] == 0)
+                if (++w == words) { w = 0; low++; }
+            unsigned &set = at_load[(size_t)words * low + w];
+            const int p = 32 * w + __builtin_ctz(set);
+            set &= set - 1;
+            const int to = low + size(i) + 1;
+            at_load[(size_t)words * to + p / 32] |= 1u << (p % 32);
+            load[p] = to;
+            rows[p] += size(i);
+            place[i] = p;
+        }
+    }
+
+    long deal(int nw)
+    {
+        std::fill(wide_rows.begin(), wide_rows.end(), 0);
+        std::fill(group_rows.begin(), group_rows.end(), 0);
+        std::fill(load.begin(), load.end(), 0);
+        spread(0, nw, MTP_PAIR_WARPS, wide_rows, [&](int i) { return (n[i] + groups - 1) / groups; });
+        for (int p = MTP_PAIR_WARPS * groups - 1; p >= 0; p--) load[p] = load[p / groups];
+        spread(nw, (int)n.size(), MTP_PAIR_WARPS * groups, group_rows, [&](int i) { return n[i]; });
+        long longest = 0, sum = 0;
+        for (int w = 0; w < MTP_PAIR_WARPS; w++) { longest = std::max<long>(longest, length(w)); sum += length(w); }
+        return cost(longest, sum);
+    }
+};
 }  // namespace
 
 extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt, const int *times, int ns,
@@ -214,85 +303,74 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
     for (int m = 0; m < nm; m++) P.nlev = std::max(P.nlev, depth[m]);
     AI2B_REQUIRE(P.nlev <= MTP_MAX_LEV, AI2B_ERR_UNSUPPORTED, "product depth %d > %d", P.nlev, MTP_MAX_LEV);
 
-    // forward: destinations by depth, rows contiguous per destination, heavy destinations first
-    std::vector<std::vector<int>> rows_of(nm), occ_of(nm);
-    for (int t = 0; t < nt; t++) {
-        rows_of[times[4 * t + 3]].push_back(t);
-        occ_of[times[4 * t]].push_back(2 * t);        // entry: this moment is `a`, other = b
-        occ_of[times[4 * t + 1]].push_back(2 * t + 1);  // this moment is `b`, other = a
-    }
+    // The rows of each destination, and the places where each moment is an operand (2 t: as `a` of row t, 2 t + 1: as `b`),
+    // one moment behind another. (Everything from here on is made once per set of tables, but a user pays for it with every
+    // new model: flat arrays, no allocation per moment. Level 16: 0.25 ms with the upload, 1.06 with lists per moment, heaps
+    // and a trial of every split point.)
+    auto by_moment = [&](int entries, auto moment_of) {
+        std::pair<std::vector<int>, std::vector<int>> r{std::vector<int>(nm + 1, 0), std::vector<int>(entries)};
+        for (int i = 0; i < entries; i++) r.first[moment_of(i) + 1]++;
+        for (int m = 0; m < nm; m++) r.first[m + 1] += r.first[m];
+        std::vector<int> at(r.first.begin(), r.first.end() - 1);
+        for (int i = 0; i < entries; i++) r.second[at[moment_of(i)]++] = i;
+        return r;
+    };
+    const auto [row_at, rows_of] = by_moment(nt, [&](int t) { return times[4 * t + 3]; });
+    const auto [occ_at, occ_of] = by_moment(2 * nt, [&](int o) { return times[4 * (o >> 1) + (o & 1)]; });
+    // moments of one depth, heavy ones first
+    std::vector<int> members;
+    auto moments_of_depth = [&](int lev, const std::vector<int> &at) -> const std::vector<int> & {
+        members.clear();
+        for (int m = 0; m < nm; m++)
+            if (depth[m] == lev && at[m + 1] > at[m]) members.push_back(m);
+        std::stable_sort(members.begin(), members.end(), [&](int x, int y) { return at[x + 1] - at[x] > at[y + 1] - at[y]; });
+        return members;
+    };
+    auto bits_f = [](int mult) { const float f = (float)mult; int b; memcpy(&b, &f, 4); return b; };
+    auto bits_d = [](int mult) { const double d = mult; long long b; memcpy(&b, &d, 8); return (int)(b >> 32); };
+    // forward: destinations by depth, rows contiguous per destination. The flat streams hold the same rows with the
+    // multiplier, the moment and a flag on its last row in one word.
     std::vector<int4> fwd_dst, rev_mom;
-    std::vector<int> fwd_ab, rev_od;
-    std::vector<float> fwd_mf, rev_mf;
-    std::vector<double> fwd_md, rev_md;
-    P.fwd_lev_off[0] = 0;
-    for (int lev = 1; lev <= P.nlev; lev++) {
-        std::vector<int> ds;
-        for (int m = 0; m < nm; m++)
-            if (depth[m] == lev && !rows_of[m].empty()) ds.push_back(m);
-        std::stable_sort(ds.begin(), ds.end(), [&](int a, int b) { return rows_of[a].size() > rows_of[b].size(); });
-        for (int m : ds) {
-            int rb = (int)fwd_ab.size();
-            for (int t : rows_of[m]) {
-                fwd_ab.push_back(times[4 * t] | (times[4 * t + 1] << 16));
-                fwd_mf.push_back((float)times[4 * t + 2]);
-                fwd_md.push_back((double)times[4 * t + 2]);
+    std::vector<int2> fwd_rows, rev_ents, fwd_flat, rev_flat;
+    fwd_dst.reserve(nm); rev_mom.reserve(nm);
+    fwd_rows.reserve(nt); fwd_flat.reserve(nt); rev_ents.reserve(2 * nt); rev_flat.reserve(2 * nt);
+    auto add_row = [&](std::vector<int2> &rows, std::vector<int2> &flat, int xy, int mult, int m, bool last) {
+        rows.push_back(make_int2(xy, bits_f(mult)));
+        flat.push_back(make_int2(xy, (mult & 0xff) | (last ? 0x100 : 0) | (m << 16)));
+    };
+    P.fwd_lev_off[0] = P.fwd_lev_row[0] = 0;
+    for (int lev = 1; lev <= MTP_MAX_LEV; lev++) {
+        if (lev <= P.nlev)
+            for (int m : moments_of_depth(lev, row_at)) {
+                const int rb = (int)fwd_rows.size(), re = rb + row_at[m + 1] - row_at[m];
+                for (int i = row_at[m]; i < row_at[m + 1]; i++) {
+                    const int *r = times + 4 * rows_of[i];
+                    add_row(fwd_rows, fwd_flat, r[0] | (r[1] << 16), r[2], m, i + 1 == row_at[m + 1]);
+                }
+                fwd_dst.push_back(make_int4(m, rb, re, 0));
             }
-            fwd_dst.push_back(make_int4(m, rb, (int)fwd_ab.size(), 0));
-        }
         P.fwd_lev_off[lev] = (int)fwd_dst.size();
+        P.fwd_lev_row[lev] = (int)fwd_rows.size();
     }
-    for (int lev = P.nlev + 1; lev <= MTP_MAX_LEV; lev++) P.fwd_lev_off[lev] = P.fwd_lev_off[P.nlev];
     // reverse: sources by depth, deepest first; adjoint[m] += sum adjoint[dst] * mult * M[other]
-    P.rev_lev_off[0] = 0;
-    for (int k = 0; k < P.nlev; k++) {
-        int lev = P.nlev - 1 - k;
-        std::vector<int> ms;
-        for (int m = 0; m < nm; m++)
-            if (depth[m] == lev && !occ_of[m].empty()) ms.push_back(m);
-        std::stable_sort(ms.begin(), ms.end(), [&](int a, int b) { return occ_of[a].size() > occ_of[b].size(); });
-        for (int m : ms) {
-            int eb = (int)rev_od.size();
-            for (int o : occ_of[m]) {
-                int t = o >> 1;
-                int other = (o & 1) ? times[4 * t] : times[4 * t + 1];
-                rev_od.push_back(other | (times[4 * t + 3] << 16));
-                rev_mf.push_back((float)times[4 * t + 2]);
-                rev_md.push_back((double)times[4 * t + 2]);
+    P.rev_lev_off[0] = P.rev_lev_row[0] = 0;
+    for (int k = 0; k < MTP_MAX_LEV; k++) {
+        if (k < P.nlev)
+            for (int m : moments_of_depth(P.nlev - 1 - k, occ_at)) {
+                const int rb = (int)rev_ents.size(), re = rb + occ_at[m + 1] - occ_at[m];
+                for (int i = occ_at[m]; i < occ_at[m + 1]; i++) {
+                    const int o = occ_of[i], *r = times + 4 * (o >> 1);
+                    add_row(rev_ents, rev_flat, r[1 - (o & 1)] | (r[3] << 16), r[2], m, i + 1 == occ_at[m + 1]);
+                }
+                rev_mom.push_back(make_int4(m, rb, re, 0));
             }
-            rev_mom.push_back(make_int4(m, eb, (int)rev_od.size(), 0));
-        }
         P.rev_lev_off[k + 1] = (int)rev_mom.size();
+        P.rev_lev_row[k + 1] = (int)rev_ents.size();
     }
-    for (int k = P.nlev + 1; k <= MTP_MAX_LEV; k++) P.rev_lev_off[k] = P.rev_lev_off[P.nlev];
-
-    std::vector<int2> fwd_rows(fwd_ab.size()), rev_ents(rev_od.size());
-    for (size_t i = 0; i < fwd_ab.size(); i++) { int bits; memcpy(&bits, &fwd_mf[i], 4); fwd_rows[i] = make_int2(fwd_ab[i], bits); }
-    for (size_t i = 0; i < rev_od.size(); i++) { int bits; memcpy(&bits, &rev_mf[i], 4); rev_ents[i] = make_int2(rev_od[i], bits); }
-    // flat streams (same row order as fwd_ab / rev_od)
-    std::vector<int2> fwd_flat(fwd_ab.size()), rev_flat(rev_od.size());
-    int maxmult = 0;
-    for (int lev = 0; lev <= MTP_MAX_LEV; lev++) {
-        const int di = P.fwd_lev_off[lev];
-        P.fwd_lev_row[lev] = di < (int)fwd_dst.size() ? fwd_dst[di].y : (int)fwd_ab.size();
-        const int mi = P.rev_lev_off[lev];
-        P.rev_lev_row[lev] = mi < (int)rev_mom.size() ? rev_mom[mi].y : (int)rev_od.size();
-    }
-    for (const int4 &d : fwd_dst)
-        for (int r = d.y; r < d.z; r++) {
-            const int mult = (int)fwd_md[r];
-            maxmult = std::max(maxmult, mult);
-            fwd_flat[r] = make_int2(fwd_ab[r], (mult & 0xff) | ((r == d.z - 1) ? 0x100 : 0) | (d.x << 16));
-        }
-    for (const int4 &m : rev_mom)
-        for (int r = m.y; r < m.z; r++) {
-            const int mult = (int)rev_md[r];
-            maxmult = std::max(maxmult, mult);
-            rev_flat[r] = make_int2(rev_od[r], (mult & 0xff) | ((r == m.z - 1) ? 0x100 : 0) | (m.x << 16));
-        }
-    AI2B_REQUIRE(maxmult <= 255, AI2B_ERR_UNSUPPORTED, "product multiplier %d > 255", maxmult);
-    for (int t = 0; t < nt; t++)
+    for (int t = 0; t < nt; t++) {
+        AI2B_REQUIRE(times[4 * t + 2] <= 255, AI2B_ERR_UNSUPPORTED, "product multiplier %d > 255", times[4 * t + 2]);
         AI2B_REQUIRE(times[4 * t + 2] >= 0, AI2B_ERR_UNSUPPORTED, "negative product multiplier in row %d", t);
+    }
     std::vector<int> map(mapping, mapping + ns);
     for (int s = 0; s < ns; s++)
         AI2B_REQUIRE(map[s] >= 0 && map[s] < nm, AI2B_ERR_INVALID, "alpha_moment_mapping[%d] out of range", s);
@@ -308,143 +386,66 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
         // moments nothing uses (seed 0); every other adjoint that is read is written by a gather phase
         for (int m = 0; m < nm; m++)
             if (!is_source[m] && (is_mapped[m] || m < nb)) adj_const.push_back(m);
-        struct Row { int x, y, mult; };
-        struct Moment { int m; std::vector<Row> rows; };
-        std::vector<std::vector<Moment>> phases;
-        for (int lev = 1; lev <= P.nlev; lev++) {
-            phases.emplace_back();
-            for (int m = 0; m < nm; m++)
-                if (depth[m] == lev && !rows_of[m].empty()) {
-                    Moment q{m, {}};
-                    for (int t : rows_of[m]) q.rows.push_back(Row{times[4 * t], times[4 * t + 1], times[4 * t + 2]});
-                    phases.back().push_back(q);
-                }
-        }
-        for (int lev = P.nlev - 1; lev >= 0; lev--) {
-            phases.emplace_back();
-            for (int m = 0; m < nm; m++)
-                if (depth[m] == lev && !occ_of[m].empty()) {
-                    Moment q{m, {}};
-                    for (int o : occ_of[m]) {
-                        const int t = o >> 1;
-                        q.rows.push_back(Row{times[4 * t + 3], (o & 1) ? times[4 * t] : times[4 * t + 1], times[4 * t + 2]});
-                    }
-                    phases.back().push_back(q);
-                }
-        }
-        for (int k = 0; k < 2; k++) {
-            const size_t groups = k == 0 ? 2 : 4;
-            P.stream[k].nrows = 0;
-            if (nm > 2046 || nt == 0) continue;      // the completed moment has 11 bits
-            for (const auto &ph : phases) {
-                // A phase lasts as long as its longest warp, and a few moments have many times the rows of the others (69
-                // against 13 on average in the last phase of level 16). Moments with more rows than `wide` are therefore split
-                // over all groups of a warp; the others go to single groups. Both by decreasing row count to the least loaded
-                // place, completing a moment taken as a row. `wide` is chosen per phase by a cost: a row of the longest warp
-                // waits for about 60 cycles, a row of any warp takes about 5 of its scheduler's issue slots.
-                std::vector<size_t> order(ph.size());
-                for (size_t i = 0; i < order.size(); i++) order[i] = i;
-                std::stable_sort(order.begin(), order.end(), [&](size_t i, size_t j) { return ph[i].rows.size() > ph[j].rows.size(); });
-                using Deal = std::vector<std::vector<size_t>>;
-                Deal of_warp, of_group;
-                auto deal = [&](size_t wide, bool keep) -> size_t {
-                    using Place = std::pair<size_t, size_t>;      // load, index: the least loaded place on top, the first of equals
-                    using Heap = std::priority_queue<Place, std::vector<Place>, std::greater<Place>>;
-                    std::vector<Place> start(MTP_PAIR_WARPS, Place(0, 0));
-                    for (size_t w = 0; w < MTP_PAIR_WARPS; w++) start[w].second = w;
-                    std::vector<size_t> wrows(MTP_PAIR_WARPS, 0), wload(MTP_PAIR_WARPS, 0), grows(MTP_PAIR_WARPS * groups, 0);
-                    if (keep) { of_warp.assign(MTP_PAIR_WARPS, {}); of_group.assign(MTP_PAIR_WARPS * groups, {}); }
-                    size_t i = 0;
-                    Heap warps(std::greater<Place>(), start);
-                    for (; i < order.size() && ph[order[i]].rows.size() > wide; i++) {
-                        const Place p = warps.top();
-                        const size_t n = (ph[order[i]].rows.size() + groups - 1) / groups;
-                        warps.pop();
-                        warps.push(Place(p.first + n + 1, p.second));
-                        wload[p.second] += n + 1;
-                        wrows[p.second] += n;
-                        if (keep) of_warp[p.second].push_back(order[i]);
-                    }
-                    start.resize(MTP_PAIR_WARPS * groups);
-                    for (size_t g = 0; g < start.size(); g++) start[g] = Place(wload[g / groups], g);
-                    Heap places(std::greater<Place>(), start);
-                    for (; i < order.size(); i++) {
-                        const Place p = places.top();
-                        const size_t n = ph[order[i]].rows.size();
-                        places.pop();
-                        places.push(Place(p.first + n + 1, p.second));
-                        grows[p.second] += n;
-                        if (keep) of_group[p.second].push_back(order[i]);
-                    }
-                    size_t longest = 0, sum = 0;
-                    for (size_t w = 0; w < MTP_PAIR_WARPS; w++) {
-                        const size_t len = wrows[w] + *std::max_element(grows.begin() + w * groups, grows.begin() + (w + 1) * groups);
-                        longest = std::max(longest, len);
-                        sum += len;
-                    }
-                    return 60 * longest + 5 * sum;
-                };
-                size_t best = ~size_t(0), best_wide = 0, last = ~size_t(0);
-                for (size_t i : order) {
-                    const size_t wide = ph[i].rows.size();
-                    if (wide == last) continue;      // (sorted: every row count is tried once)
-                    last = wide;
-                    const size_t cost = deal(wide, false);
-                    if (cost < best) { best = cost; best_wide = wide; }
-                }
-                deal(best_wide, true);
-                for (size_t w = 0; w < MTP_PAIR_WARPS; w++) {
-                    std::vector<std::vector<int2>> rd(groups), rf(groups);
-                    auto put = [&](size_t g, int xy, int mult, int done) {
-                        const double md = mult;
-                        const float mf = (float)mult;
-                        long long bd;
-                        int bf;
-                        memcpy(&bd, &md, 8);
-                        memcpy(&bf, &mf, 4);
-                        rd[g].push_back(make_int2(xy, (int)(bd >> 32) | done));
-                        rf[g].push_back(make_int2(xy, bf | done));
-                    };
-                    for (size_t i : of_warp[w]) {
-                        const Moment &q = ph[i];
-                        const size_t n = (q.rows.size() + groups - 1) / groups;
-                        for (size_t r = 0; r < n; r++)
-                            for (size_t g = 0; g < groups; g++) {
-                                const size_t at = r * groups + g;
-                                const int done = r + 1 == n ? (q.m + 1) | MTP_PAIR_WIDE : 0;
-                                if (at < q.rows.size()) put(g, q.rows[at].x | (q.rows[at].y << 16), q.rows[at].mult, done);
-                                else put(g, q.rows[0].x | (q.rows[0].y << 16), 0, done);      // (operands that are written by then)
-                            }
-                    }
-                    size_t len = 0;
-                    for (size_t g = 0; g < groups; g++) {
-                        for (size_t i : of_group[w * groups + g]) {
-                            const Moment &q = ph[i];
-                            for (size_t r = 0; r < q.rows.size(); r++)
-                                put(g, q.rows[r].x | (q.rows[r].y << 16), q.rows[r].mult, r + 1 == q.rows.size() ? q.m + 1 : 0);
+    }
+    for (int k = 0; k < 2; k++) {
+        const int groups = k == 0 ? 2 : 4;
+        P.stream[k].nrows = 0;
+        if (nm > 2046 || nt == 0) continue;      // the completed moment has 11 bits
+        RowDeal deal(groups);
+        std::vector<int> row0(MTP_PAIR_WARPS), next(MTP_PAIR_WARPS * groups);      // rows that the next records of a warp, a group go to
+        stream_warp[k].reserve(2 * P.nlev * MTP_PAIR_WARPS);
+        stream_d[k].reserve(4 * nt + 64 * P.nlev);
+        stream_f[k].reserve(4 * nt + 64 * P.nlev);
+        for (int phase = 0; phase < 2 * P.nlev; phase++) {
+            // A phase lasts as long as its longest warp, and a few moments have many times the rows of the others (69
+            // against 13 on average in the last phase of level 16). The moments with the most rows are therefore split
+            // over all groups of a warp; the others go to single groups. How many are split is chosen per phase by a cost: a row
+            // of the longest warp waits for about 60 cycles, a row of any warp takes about 5 of its scheduler's issue slots.
+            const bool fwd = phase < P.nlev;
+            const int4 *q = fwd ? fwd_dst.data() + P.fwd_lev_off[phase] : rev_mom.data() + P.rev_lev_off[phase - P.nlev];
+            const int nq = fwd ? P.fwd_lev_off[phase + 1] - P.fwd_lev_off[phase] : P.rev_lev_off[phase - P.nlev + 1] - P.rev_lev_off[phase - P.nlev];
+            const std::vector<int2> &flat = fwd ? fwd_flat : rev_flat;
+            deal.choose(q, nq);
+            size_t first = stream_d[k].size();
+            for (int w = 0; w < MTP_PAIR_WARPS; w++) {
+                row0[w] = (int)(first / groups);
+                stream_warp[k].push_back(make_int2(row0[w], deal.length(w)));
+                first += (size_t)deal.length(w) * groups;
+            }
+            stream_d[k].resize(first, make_int2(0, 0));
+            stream_f[k].resize(first, make_int2(0, 0));
+            auto put = [&](int row, int g, int at, bool empty, int done) {      // record `at` of the flat stream
+                const int mult = empty ? 0 : flat[at].y & 0xff, x = flat[at].x & 0xffff, y = (flat[at].x >> 16) & 0xffff;
+                const int xy = fwd ? x | (y << 16) : y | (x << 16);             // (flat adjoint rows hold {other, dst})
+                stream_d[k][(size_t)row * groups + g] = make_int2(xy, bits_d(mult) | done);
+                stream_f[k][(size_t)row * groups + g] = make_int2(xy, bits_f(mult) | done);
+            };
+            for (int g = 0; g < MTP_PAIR_WARPS * groups; g++) next[g] = row0[g / groups];
+            for (int i = 0; i < nq; i++) {
+                const int n = q[i].z - q[i].y, place = deal.place[i];
+                if (i < deal.nwide) {
+                    const int rows = (n + groups - 1) / groups;
+                    for (int r = 0; r < rows; r++)
+                        for (int g = 0; g < groups; g++) {
+                            const int at = r * groups + g;      // (empty records: operands that are written by then)
+                            put(next[place * groups + g]++, g, at < n ? q[i].y + at : q[i].y, at >= n, r + 1 == rows ? (q[i].x + 1) | MTP_PAIR_WIDE : 0);
                         }
-                        len = std::max(len, rd[g].size());
-                    }
-                    stream_warp[k].push_back(make_int2((int)(stream_d[k].size() / groups), (int)len));
-                    for (size_t r = 0; r < len; r++)
-                        for (size_t g = 0; g < groups; g++) {
-                            stream_d[k].push_back(r < rd[g].size() ? rd[g][r] : make_int2(0, 0));
-                            stream_f[k].push_back(r < rf[g].size() ? rf[g][r] : make_int2(0, 0));
-                        }
+                } else {
+                    for (int r = 0; r < n; r++) put(next[place]++, place % groups, q[i].y + r, false, r + 1 == n ? q[i].x + 1 : 0);
                 }
             }
-            for (size_t g = 0; g < 2 * groups; g++) { stream_d[k].push_back(make_int2(0, 0)); stream_f[k].push_back(make_int2(0, 0)); }   // read ahead
-            P.stream[k].nrows = (int)(stream_d[k].size() / groups);
         }
+        for (int g = 0; g < 2 * groups; g++) { stream_d[k].push_back(make_int2(0, 0)); stream_f[k].push_back(make_int2(0, 0)); }   // read ahead
+        P.stream[k].nrows = (int)(stream_d[k].size() / groups);
     }
     P.n_adj_const = (int)adj_const.size();
 
     Blob blob;
+    blob.bytes.reserve(64 * 1024 + 128 * (size_t)(nm + nt) + 16 * (stream_d[0].size() + stream_d[1].size()));
     size_t o_ac = blob.add(adj_const), o_sd[2], o_sf[2], o_sw[2];
     for (int k = 0; k < 2; k++) { o_sd[k] = blob.add(stream_d[k]); o_sf[k] = blob.add(stream_f[k]); o_sw[k] = blob.add(stream_warp[k]); }
     size_t o_bd = blob.add(basic_dense), o_db = blob.add(dense_basic), o_e4d = blob.add(e4d), o_g = blob.add(e4g), o_m = blob.add(e4m), o_fd = blob.add(fwd_dst),
-           o_fr = blob.add(fwd_ab), o_fmf = blob.add(fwd_mf), o_fmd = blob.add(fwd_md), o_rm = blob.add(rev_mom),
-           o_re = blob.add(rev_od), o_rmf = blob.add(rev_mf), o_rmd = blob.add(rev_md), o_map = blob.add(map);
+           o_rm = blob.add(rev_mom), o_map = blob.add(map);
     size_t o_frow = blob.add(fwd_rows), o_rent = blob.add(rev_ents), o_ff = blob.add(fwd_flat), o_rf = blob.add(rev_flat);
     ai2b_mtp_program *prog = new ai2b_mtp_program;
     prog->blob_bytes = blob.bytes.size();
@@ -465,13 +466,7 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
     P.e4g = (const int4 *)(b + o_g);
     P.e4m = (const int *)(b + o_m);
     P.fwd_dst = (const int4 *)(b + o_fd);
-    P.fwd_ab = (const int *)(b + o_fr);
-    P.fwd_mult_f = (const float *)(b + o_fmf);
-    P.fwd_mult_d = (const double *)(b + o_fmd);
     P.rev_mom = (const int4 *)(b + o_rm);
-    P.rev_od = (const int *)(b + o_re);
-    P.rev_mult_f = (const float *)(b + o_rmf);
-    P.rev_mult_d = (const double *)(b + o_rmd);
     P.map = (const int *)(b + o_map);
     P.fwd_rows = (const int2 *)(b + o_frow);
     P.rev_ents = (const int2 *)(b + o_rent);

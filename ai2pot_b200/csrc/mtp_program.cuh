@@ -29,9 +29,6 @@ struct MtpProgramDev {
     const int4 *e4g;                // [ndense] basic row holding {value, d/dx, d/dy, d/dz} source (-1: none)
     const int *e4m;                 // [ndense] packed multipliers (ax+1) | (ay+1)<<8 | (az+1)<<16
     const int4 *fwd_dst;            // {dst, row_begin, row_end, -}
-    const int *fwd_ab;              // [nt] a | b<<16, rows grouped by destination
-    const float *fwd_mult_f;        // [nt] multiplier, float / double copies (no int->fp conversion on the device)
-    const double *fwd_mult_d;
     const int2 *fwd_rows;           // [nt] {a | b<<16, multiplier as float bits}: one 8-byte load per row
     const int2 *rev_ents;           // [2 nt] {other | dst<<16, multiplier as float bits}
     // flat row streams for the lanes-as-atoms kernel: rows of one depth are contiguous, a flag marks the
@@ -41,9 +38,6 @@ struct MtpProgramDev {
     int fwd_lev_row[MTP_MAX_LEV + 1];
     int rev_lev_row[MTP_MAX_LEV + 1];
     const int4 *rev_mom;            // {m, entry_begin, entry_end, -}
-    const int *rev_od;              // [2 nt] other | dst<<16
-    const float *rev_mult_f;
-    const double *rev_mult_d;
     const int *map;                 // [ns] alpha_moment_mapping
     // Row streams of the lanes-as-atoms contractions (tiles of 16 or 32 atoms, 16 bytes of atoms per lane, GL lanes per row, so
     // a warp works on 32 / GL rows at a time). Phase p < nlev is product depth p + 1 (rows {a, b}: M[dst] = sum mult * M[a] *
@@ -64,13 +58,6 @@ struct MtpProgramDev {
 constexpr int MTP_PAIR_WARPS = 32;
 constexpr int MTP_PAIR_WIDE = 0x800;
 constexpr int MTP_TILE = 32;        // atoms per tile of the workspace
-
-template <typename T> __device__ __forceinline__ const T *fwd_mult(const MtpProgramDev &P);
-template <> __device__ __forceinline__ const float *fwd_mult<float>(const MtpProgramDev &P) { return P.fwd_mult_f; }
-template <> __device__ __forceinline__ const double *fwd_mult<double>(const MtpProgramDev &P) { return P.fwd_mult_d; }
-template <typename T> __device__ __forceinline__ const T *rev_mult(const MtpProgramDev &P);
-template <> __device__ __forceinline__ const float *rev_mult<float>(const MtpProgramDev &P) { return P.rev_mult_f; }
-template <> __device__ __forceinline__ const double *rev_mult<double>(const MtpProgramDev &P) { return P.rev_mult_d; }
 
 }  // namespace ai2b
 
