@@ -78,3 +78,54 @@ def test_md_session_mtp(checkers):
     e2, f2, _, _ = ses.compute(nlocal, nghost, np.concatenate([x, gx]), np.concatenate([w["types"], gt]), want_virial=False)
     assert util.relerr(_fold(f2, nlocal, owner), f_ref[0]) < 1e-5
     ses.close()
+
+
+@pytest.mark.parametrize("n", [1, 6143, 6144, 6145, 15797, 15798, 18431, 18432, 18433, 30001])
+def test_md_session_pieces(n):
+    """Positions go to the device in pieces of 6,144 atoms through a ring of three: sizes around a piece, around what the ring
+    holds with the types, and beyond the ring; a smaller and a larger system in between."""
+    rng = np.random.default_rng(n)
+    m = synth.nep_model(3, rng, rmax_radial=4.0, rmax_angular=3.0)
+    edge = int(np.ceil(n ** (1.0 / 3.0)))
+    g = np.stack(np.meshgrid(*[np.arange(edge) * 2.5] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    x = np.ascontiguousarray(g + rng.normal(0, 0.1, (n, 3)) - 7.0)
+    t = rng.integers(0, 3, n).astype(np.int32)
+    nlocal = max(1, n - n // 3)
+    ses = capi.MdSession(m, 64)
+    want = None
+    for k in range(3):
+        e, f, v, mx = ses.compute(nlocal, n - nlocal, x, t)
+        if k == 0:
+            import torch
+            rows = capi.NeighborBuilder().build(np.eye(3), torch.from_numpy(x).cuda(), 4.0, 64, pbc=(False,) * 3, ncentres=nlocal)
+            md = capi.to_device(m)
+            nb = dict(binum=torch.tensor([nlocal], dtype=torch.int32, device="cuda"), bilist=torch.arange(nlocal, dtype=torch.int32, device="cuda")[None],
+                      bnumneigh=rows[0][None], bfirstneigh=rows[1][None], brcs=rows[2].float()[None].contiguous(),
+                      btypes=torch.from_numpy(t).cuda()[None], ntypes=3, nghost=n - nlocal)
+            want = [o.cpu().numpy() for o in capi.nep_efv(md, nb)]
+            assert mx == int(rows[3][0])
+        assert abs(e - want[0][0]) <= 1e-5 * max(1.0, abs(want[0][0])) and (n == 1 or util.relerr(f, want[1][0]) < 1e-5)
+        assert n == 1 or util.relerr(v, want[2][0][[0, 4, 8, 1, 2, 5]]) < 1e-5
+        small = max(1, n // 2) if k == 0 else n + n // 2       # the buffers serve the smaller one and grow for the larger one
+        y = np.resize(x, (small, 3)) + np.arange(small)[:, None] // n * 1000.0
+        ses.compute(small, 0, y, np.resize(t, small))
+    ses.close()
+
+
+@pytest.mark.parametrize("kind", ["nep", "mtp"])
+def test_first_step_of_a_session(kind):
+    """The first step of a session allocates what later steps use; it takes less than 1.5 ms (0.6 to 0.8; with nine
+    allocations and pinned memory for a whole step 2.1 to 5). The best of several: pinning may be slow on a busy host."""
+    import time
+    w = synth.g2(n=24) if kind == "nep" else util.small_mtp_case(16, 14, np.float32, rcut=6.0)
+    m = w["model"]
+    prog = capi.MtpProgram(m["tables"]) if kind == "mtp" else None
+    x = np.ascontiguousarray(np.mod(w["coords"].astype(np.float64), np.diag(w["cell"]).astype(np.float64)))
+    best = 1e9
+    for _ in range(8):
+        ses = capi.MdSession(m, 64, prog)
+        t0 = time.perf_counter()
+        ses.compute(len(x), 0, x, w["types"])
+        best = min(best, time.perf_counter() - t0)
+        ses.close()
+    assert best < 1.5e-3
