@@ -152,33 +152,22 @@ __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_chained_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster,
-                                          Args &&...args)
+inline cudaError_t launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[2];
+    cudaLaunchAttribute at[1];
     cfg.attrs = at;
     const char *env = std::getenv("AI2B_CHAIN");          // AI2B_CHAIN=0: ordinary launches (a switch for debugging), read per launch
     if (!(env && env[0] == '0')) {
-        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    if (cluster > 1) {
-        at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
-        at[cfg.numAttrs].val.clusterDim.x = (unsigned)cluster;
-        at[cfg.numAttrs].val.clusterDim.y = 1;
-        at[cfg.numAttrs++].val.clusterDim.z = 1;
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs = 1;
     }
     return cudaLaunchKernelEx(&cfg, kern, KArgs(static_cast<Args &&>(args))...);
-}
-template <typename... KArgs, typename... Args>
-inline cudaError_t launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args)
-{
-    return launch_chained_cluster(kern, grid, block, smem, st, 1, static_cast<Args &&>(args)...);
 }
 
 // number of monomials x^a y^b z^c with a+b+c <= k, and of exact degree d

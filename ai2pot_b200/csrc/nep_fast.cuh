@@ -279,6 +279,8 @@ __host__ __device__ inline int nep_fast_warp_elems(int lanes, int nneu, int umax
     const int stage = 32 * D::RS, es = AW * D::ESR;                 // staging rows, later the adjoints of the sums
     return (stage > es ? stage : es) + AW * 2 * D::NDP +            // descriptors, their adjoints
            (net ? AW * (nep_r32(nneu) + 4) + 96 + AW * umax * NMAX : 0);   // neurons, angular forces, cached derivatives
+    // (NMAX = 4 does not write the neurons' part. Without it 13,824 atoms take 56.0 instead of 56.6 us, 1,048,576 atoms 1,600
+    // instead of 1,592, and models of 12 species a slower form: it stays.)
 }
 
 template <typename T, int G, int MODE, int NMAX, int MINB>
