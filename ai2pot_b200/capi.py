@@ -247,6 +247,32 @@ class NeighborBuilder:
         return nn, fn, rcs, status
 
 
+def cell_heights(cell):
+    """Distances between opposite faces of a cell."""
+    c = np.asarray(cell, np.float64).reshape(3, 3)
+    return abs(np.linalg.det(c)) / np.array([np.linalg.norm(np.cross(c[(k + 1) % 3], c[(k + 2) % 3])) for k in range(3)])
+
+
+def nblist_build_launches(natoms, cell, rcut, open_extent=None):
+    """Kernels that a build of natoms atoms launches (see NeighborBuilder.build for open_extent)."""
+    heights = cell_heights(cell)
+    if open_extent is not None:
+        heights[0] *= open_extent[1] - open_extent[0]
+    bins = 1
+    for h in heights:
+        bins *= max(1, int(h / (rcut * 1.0001 + 1e-6)))
+    return lib().ai2b_nblist_build_launches(C.c_int(int(natoms)), C.c_longlong(bins))
+
+
+def nep_efv_launches(model, natoms, umax, dtype):
+    """Kernels that an energy / force / virial call launches: set-up and evaluation, or the general kernel with its three."""
+    m = model
+    lanes = lib().ai2b_nep_lanes_per_atom(C.c_int(int(natoms)), C.c_int(int(m["ntypes"])), C.c_int(int(m["n_radial"])), C.c_int(int(m["n_angular"])),
+                                          C.c_int(int(m["chebyshev_size"])), C.c_int(int(m["num_neurons"])), C.c_int(int(umax)),
+                                          C.c_int(int(dtype == torch.float64)), C.c_int(0))
+    return 2 if lanes else 4
+
+
 def nblist_build_batch(cells, binum, coords, rcut, umax, is_cart=True, pbc=(True, True, True)):
     """Neighbour tensors of a padded batch in one launch (ai2b_nblist_build_batch_*).
     cells: host array [B,3,3]; binum: CUDA int32 [B]; coords: CUDA [B,Np,3] (float32/float64).

@@ -1453,6 +1453,12 @@ extern "C" size_t ai2b_nblist_workspace_bytes(int natoms, int is_f64)
     return is_f64 ? nb_layout<double>(natoms, nb_maxbins(natoms)).total : nb_layout<float>(natoms, nb_maxbins(natoms)).total;
 }
 
+extern "C" int ai2b_nblist_build_launches(int natoms, long long bins)
+{
+    if (natoms <= 0) return 0;
+    return natoms <= BINB_MAX_ATOMS ? 2 : bins <= FILL_SCAN_BINS ? 4 : 5;
+}
+
 extern "C" int ai2b_nblist_build_f64(int natoms, const double *h_cell, const double *d_coords, int is_cart, double rcut,
                                      const int *h_pbc, int umax, int *d_numneigh, int *d_firstneigh, double *d_rcs,
                                      int *d_status, void *d_workspace, size_t workspace_bytes, void *stream)

@@ -184,20 +184,15 @@ class Evaluator:
     def replay_io(self):
         self.graph_io.replay()
 
-    # kernels of this library launched by one compute() on a fully periodic cell (memsets not counted): neighbour build =
-    # binning (one launch up to 2,048 atoms, else set-up, count, fill, with a scan between them for many bins) and rows;
-    # MTP = forward, contraction, force (plus a set-up launch when the radial coefficient rows have to be padded to eight
-    # entries); NEP = zeroing of the outputs + one kernel
     def launches_per_step(self):
-        bins = 1
-        for d in self.cell_heights():
-            bins *= max(1, int(d / (self.rcut * 1.0001 + 1e-6)))
-        build = 2 if self.n <= 2048 else 4 if bins <= 8192 else 5
+        """Kernels of this library that one compute() on a fully periodic cell launches (memsets not counted): neighbour build,
+        then forward, contraction and force of MTP (and a set-up launch when the radial coefficient rows have to be padded to
+        eight entries), or those of NEP."""
+        build = capi.nblist_build_launches(self.n, self.cell, self.rcut)
         if self.kind == "mtp":
             return build + 3 + (0 if int(self.model["chebyshev_size"]) == 8 else 1)
-        return build + 2
+        return build + capi.nep_efv_launches(self.model, self.n, self.umax, self.dtype)
 
     def cell_heights(self):
         """Distances between opposite faces of the cell."""
-        c = self.cell.astype(np.float64)
-        return abs(np.linalg.det(c)) / np.array([np.linalg.norm(np.cross(c[(k + 1) % 3], c[(k + 2) % 3])) for k in range(3)])
+        return capi.cell_heights(self.cell)

@@ -601,11 +601,13 @@ class SlabStep:
         return int(d.back.numel() * d.back.element_size()) if (d.P > 1 and self.schedule != "owner") else 0
 
     def launches_per_step(self):
-        """Kernels of this library per step: a pass = neighbour build (set-up, count, scan, fill, rows; rows only when
-        the bins are reused) + one NEP kernel."""
-        if self.dom.P == 1 or self.schedule == "serial":
-            return 6
-        return 6 + 6 + 2
+        """Kernels of this library per step: a pass = neighbour build (rows only when the bins are reused) + NEP."""
+        d, p = self.dom, self.passes
+        efv = p.capi.nep_efv_launches(p.model, d.nlocal, p.umax, d.dtype)
+        build = p.capi.nblist_build_launches(d.ntotal, p.cell, p.rcut, p.open_extent)
+        if d.P == 1 or self.schedule == "serial":
+            return build + efv
+        return 2 * (build + efv) + 1 + efv
 
     def parts_ms(self, k, flush, timed):
         """Device times of the parts of a step run one at a time (not overlapped), for the record."""

@@ -167,6 +167,9 @@ AI2B_DECL_MTP_LOSS(f32, float)
  *               buffers there, neighborList.h:550); the caller reads d_status to detect it.
  * Workspace: ai2b_nblist_workspace_bytes(natoms, is_f64). */
 size_t ai2b_nblist_workspace_bytes(int natoms, int is_f64);
+/* Kernels that a build launches when the host knows the grid of `bins` bins (all axes periodic, or
+ * the extent of the open ones given): binning and rows. */
+int ai2b_nblist_build_launches(int natoms, long long bins);
 int ai2b_nblist_build_f64(int natoms, const double *h_cell, const double *d_coords, int is_cart,
                           double rcut, const int *h_pbc, int umax, int *d_numneigh,
                           int *d_firstneigh, double *d_rcs, int *d_status, void *d_workspace,

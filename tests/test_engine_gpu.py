@@ -132,3 +132,27 @@ def test_positions_that_do_not_fit_are_refused():
                 call(bad)
     strided = torch.empty(ev.n, 4, dtype=dt, device="cuda")[:, :3].copy_(coords)
     _close(_host(ev.compute(strided)), _host(ev.compute(coords)), 1e-5)
+
+
+@pytest.mark.parametrize("kind,natoms,ntypes", [("mtp", 216, 3), ("nep", 216, 3), ("nep", 2197, 3), ("mtp", 2197, 3), ("nep", 2197, 17), ("nep", 300000, 3)])
+def test_launch_counts(kind, natoms, ntypes):
+    """launches_per_step() against the nodes of a recorded call: few atoms, several binning launches, the general NEP kernel,
+    and (sparse cell, more than 8,192 bins) a scan of its own."""
+    import ctypes as C
+    rng = np.random.default_rng(natoms)
+    spacing = 3.0 if natoms < 10000 else 6.0
+    edge = int(np.ceil(natoms ** (1.0 / 3.0) - 1e-9))
+    dt = torch.float64 if kind == "mtp" else torch.float32
+    npdt = np.float64 if kind == "mtp" else np.float32
+    cell, pos = synth.cubic_lattice(edge, spacing, 0.1, rng, npdt, nocc=natoms)
+    model = synth.mtp_model(util.tables(10), ntypes, rng, npdt, 5.0, 0.5) if kind == "mtp" else synth.nep_model(ntypes, rng, npdt)
+    ev = engine.Evaluator(model, cell, rng.integers(0, ntypes, natoms).astype(np.int32), 5.0 if kind == "mtp" else 6.0, 64, dt)
+    coords = torch.from_numpy(pos).cuda()
+    ev.compute(coords)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        ev.compute(coords)
+    nodes = C.c_size_t(0)
+    assert C.CDLL("libcudart.so.12").cudaGraphGetNodes(C.c_void_p(graph.raw_cuda_graph()), None, C.byref(nodes)) == 0
+    assert ev.launches_per_step() == nodes.value
