@@ -21,6 +21,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -216,7 +217,11 @@ __device__ __forceinline__ int bin_of(const NbParams<T> &P, const NbGrid &g, con
     }
     return (b[0] * g.nb[1] + b[1]) * g.nb[2] + b[2];
 }
-__device__ __forceinline__ int wrap_reach(const int *w) { return max(abs(w[0]), max(abs(w[1]), abs(w[2]))); }
+// (an atom out of the range of an int, or at infinity, counts as 2^31 - 1 periods away)
+__device__ __forceinline__ int wrap_reach(const int *w)
+{
+    return max(abs(max(w[0], -INT_MAX)), max(abs(max(w[1], -INT_MAX)), abs(max(w[2], -INT_MAX))));
+}
 
 // What the row kernel reads of an atom, in bin order: spos = position (type T) and index, sposw = position brought
 // into the cell in single precision and packed wrap; full wraps only when some wrap does not fit the packed form.
@@ -651,7 +656,7 @@ nb_rows_kernel(NbParams<T> P, const NbGrid *__restrict__ gp, const int *__restri
     chain_wait();
     const NbGrid g = *gp;
     const bool packed = g.maxwrap <= NB_WRAP_MAX;   // every wrap fits the packed form
-    const float pre_hi = (float)((P.rc2 + (double)g.pre_err * (1 + g.maxwrap)) * (1.0 + 1e-6));
+    const float pre_hi = (float)((P.rc2 + (double)g.pre_err * (1.0 + g.maxwrap)) * (1.0 + 1e-6));
     const int nx = 2 * g.R[0] + 1, ny = 2 * g.R[1] + 1, nz = 2 * g.R[2] + 1;
     const bool zmerge = g.zmerge != 0;
     const int nnb_full = zmerge ? nx * ny : nx * ny * nz;   // table entries of a bin away from the third axis' faces
@@ -674,7 +679,8 @@ nb_rows_kernel(NbParams<T> P, const NbGrid *__restrict__ gp, const int *__restri
         // range: the part of its 2R+1 bins that lies across the face (entries nnb_full .. 2 nnb_full - 1).
         const bool zsplit = zmerge && P.per[2] && (bz - g.R[2] < 0 || bz + g.R[2] >= g.nb[2]);
         const int nnb = zsplit ? 2 * nnb_full : nnb_full;
-        const float4 org = sposw[a_begin];
+        float4 org = sposw[a_begin];
+        if (!(fabsf(org.x) + fabsf(org.y) + fabsf(org.z) < 1e15f)) org = make_float4(0.f, 0.f, 0.f, 0.f);   // an atom that has flown off
 
         // up to 32 table entries (columns of bins, or bins) from entry `base` on, by the team's first warp; returns their candidates
         auto make_entries = [&](int base) -> int {
@@ -784,7 +790,8 @@ nb_rows_kernel(NbParams<T> P, const NbGrid *__restrict__ gp, const int *__restri
             const float4 pw = sposw[a];
             const typename Vec4<T>::type pi = spos[a];
             const float qx = pw.x - org.x, qy = pw.y - org.y, qz = pw.z - org.z;
-            const float limit = pre_hi + slack - (qx * qx + qy * qy + qz * qz);
+            // below the padding's 3e38 whatever the atoms are (infinite or undefined: the exact predicate decides about all others)
+            const float limit = fminf(pre_hi + slack - (qx * qx + qy * qy + qz * qz), 1e38f);
             const unsigned long long mx = pack2(-2.f * qx, -2.f * qx), my = pack2(-2.f * qy, -2.f * qy), mz = pack2(-2.f * qz, -2.f * qz);
             unsigned mine = 0;      // bit k: candidate 32 k + lane survives
             const ulonglong2 *cl = cq + lane;

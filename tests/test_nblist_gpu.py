@@ -301,6 +301,31 @@ def test_host_list_keeps_no_large_buffers(checkers, dt, monkeypatch):
     assert empty[0] == 0 and empty[3].shape == (0, 48) and empty[4].shape == (0, 48, 3)
 
 
+@pytest.mark.parametrize("dt", [np.float64, np.float32])
+@pytest.mark.parametrize("n,spacing,form", [(300, 3.0, ""), (3000, 3.0, ""), (9000, 3.0, ""), (9000, 4.2, ""), (9000, 5.5, ""), (3000, 3.0, "0")])
+@pytest.mark.parametrize("pbc", [(1, 1, 1), (0, 1, 0)])
+def test_atoms_that_have_flown_off(dt, n, spacing, form, pbc, monkeypatch):
+    """Infinite, undefined and enormous coordinates: such an atom has no neighbours, and the rows of all others are those of
+    the system without it (every form of the row kernel; the bad atoms lie in bins with others)."""
+    if form:
+        monkeypatch.setenv("AI2B_NBL_MIN_ATOMS", form)
+    rng = np.random.default_rng(n)
+    edge = int(np.ceil(n ** (1 / 3) - 1e-9))
+    cell, pos = synth.cubic_lattice(edge, spacing, 0.1, rng, dt, nocc=n)
+    types = np.zeros(n, np.int32)
+    want = _gpu(cell, types, pos, 5.0, 64, pbc=pbc)
+    far = 1e25 if dt == np.float32 else 1e30
+    values = [np.inf, -np.inf, np.nan, far, -far] + ([1e13, -1e13] if dt == np.float64 else [])
+    for v in values:
+        bad = pos[[0, 1, n // 2]].copy()
+        bad[0, 0], bad[1, 1], bad[2] = v, v, v
+        nn, fn, rc = _gpu(cell, np.zeros(n + 3, np.int32), np.concatenate([bad, pos]), 5.0, 64, pbc=pbc)
+        assert not nn[:3].any() and (fn[:3] == -1).all()
+        fn = np.where(fn >= 0, fn - 3, fn)
+        assert fn.min() >= -1
+        util.assert_nblist_equal((nn[3:], fn[3:], rc[3:]), want)
+
+
 def test_host_list_that_fails_leaves_no_work_behind(checkers):
     """The buffers of a call that raises half-way (rows too wide to be sorted) may be given to another stream at once."""
     from ai2pot_b200.fromcc import nblist
