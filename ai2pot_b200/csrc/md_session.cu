@@ -32,7 +32,8 @@ int nblist_build_rows32(int n, int ncentres, const double *h_cell, const double 
 
 // Positions travel in pieces of this many atoms, MD_SLOTS of which have a place in pinned memory. Pinning costs 0.9 to 2.9 ms per
 // 2 MB, of which blocks of less than 1 MB are cut: the ring has a fixed size and is made with the session, and what a
-// step brings back comes from the same 2 MB for up to 40,000 atoms.
+// step brings back comes from the same 2 MB for up to 80,000 atoms. A step of 25,239 atoms takes 188 us with three slots, 187
+// with pinned memory for all of it (medians, in turn).
 constexpr size_t MD_PIECE = 6144;
 constexpr int MD_SLOTS = 3;
 constexpr size_t MD_RING_BYTES = sizeof(double) * 3 * MD_PIECE * MD_SLOTS;
@@ -260,11 +261,11 @@ static int session_step(ai2b_md_session *s, int nlocal, int nghost, const double
     double *d_pos = reinterpret_cast<double *>(s->d_in);
     // types and the atom count travel with the last positions if the ring holds the whole step (a transfer costs 2 us)
     const bool together = in_bytes(nall) <= MD_RING_BYTES;
-    int *h_types = together ? reinterpret_cast<int *>(s->h_ring + 3 * (size_t)nall) : reinterpret_cast<int *>(s->h_types);
-    memcpy(h_types, h_model_type, sizeof(int) * nall);
-    h_types[nall] = nlocal;
     const size_t type_bytes = sizeof(int) * ((size_t)nall + 1);
-    if (!together) AI2B_CUDA(cudaMemcpyAsync(d_pos + 3 * (size_t)nall, h_types, type_bytes, cudaMemcpyHostToDevice, st));
+    auto stage_types = [&](void *dst) {
+        memcpy(dst, h_model_type, sizeof(int) * nall);
+        static_cast<int *>(dst)[nall] = nlocal;
+    };
     // positions in pieces: the copy engine takes a piece while the next one is copied and bounded
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
     const size_t pieces = ((size_t)nall + MD_PIECE - 1) / MD_PIECE;
@@ -273,9 +274,14 @@ static int session_step(ai2b_md_session *s, int nlocal, int nghost, const double
         double *h_pos = s->h_ring + 3 * MD_PIECE * slot;
         if (k >= MD_SLOTS) AI2B_CUDA(cudaEventSynchronize(s->sent[slot]));
         copy_and_bound(h_pos, h_x + 3 * i0, n, lo, hi);
-        AI2B_CUDA(cudaMemcpyAsync(d_pos + 3 * i0, h_pos, sizeof(double) * 3 * n + (together && k + 1 == pieces ? type_bytes : 0),
-                                  cudaMemcpyHostToDevice, st));
+        const bool last = k + 1 == pieces;
+        if (together && last) stage_types(h_pos + 3 * n);
+        AI2B_CUDA(cudaMemcpyAsync(d_pos + 3 * i0, h_pos, sizeof(double) * 3 * n + (together && last ? type_bytes : 0), cudaMemcpyHostToDevice, st));
         if (k + MD_SLOTS < pieces) AI2B_CUDA(cudaEventRecord(s->sent[slot], st));
+        if (!together && k == 0) {      // (copied while the first positions travel)
+            stage_types(s->h_types);
+            AI2B_CUDA(cudaMemcpyAsync(d_pos + 3 * (size_t)nall, s->h_types, type_bytes, cudaMemcpyHostToDevice, st));
+        }
     }
     const int *d_types = reinterpret_cast<const int *>(d_pos + 3 * (size_t)nall), *d_binum = d_types + nall;
     float *d_force = reinterpret_cast<float *>(s->d_out), *d_ev = d_force + 3 * (size_t)nall;

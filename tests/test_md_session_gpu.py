@@ -129,3 +129,19 @@ def test_first_step_of_a_session(kind):
         best = min(best, time.perf_counter() - t0)
         ses.close()
     assert best < 1.5e-3
+
+
+def test_atom_that_has_flown_off():
+    """A local atom at infinity or with an undefined position: nobody's neighbour, all other forces are those without it."""
+    rng = np.random.default_rng(2)
+    m = synth.nep_model(3, rng)
+    x = np.stack(np.meshgrid(*[np.arange(9) * 2.8] * 3, indexing="ij"), -1).reshape(-1, 3) + rng.normal(0, 0.1, (729, 3))
+    t = rng.integers(0, 3, 729).astype(np.int32)
+    ses = capi.MdSession(m, 96)
+    e, f, v, mx = ses.compute(729, 0, x, t)
+    lone = ses.compute(1, 0, x[:1], t[:1])[0]
+    for bad in ([np.inf, 0, 0], [0, -np.inf, 5.0], [np.nan] * 3, [1e30, 1e30, -1e30]):
+        e2, f2, v2, mx2 = ses.compute(730, 0, np.concatenate([[bad], x]), np.concatenate([t[:1], t]))
+        assert mx2 == mx and not f2[0].any() and util.relerr(f2[1:], f) < 1e-5
+        assert abs(e2 - lone - e) < 1e-5 * abs(e) and util.relerr(v2, v) < 1e-5
+    ses.close()
