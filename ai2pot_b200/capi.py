@@ -72,7 +72,9 @@ class Evaluation(C.Structure):
                 [("nblist_workspace_bytes", C.c_size_t), ("d_workspace", C.c_void_p), ("workspace_bytes", C.c_size_t)])
 
 
-CHAINED_COPY_BYTES = 1 << 20    # up to here a kernel of the chain beats the copy engine's hand-over
+# Up to here a kernel of the chain beats the copy engine's hand-over. Recorded NEP calls, both copies by the chain / the engine:
+# 2.6 KB 26.7 / 36.1 us, 166 KB 69.7 / 74.4, 0.77 MB 195 / 199, 1.04 MB 253 / 262, 1.5 MB 370 / 377, 2.4 MB 548 / 547.
+CHAINED_COPY_BYTES = 1 << 20
 
 
 def copy_around_call(dst, src):

@@ -14,7 +14,7 @@
 // A step's host work: one pass over the positions that copies them into pinned memory and finds their extent (so the
 // bin grid is known on the host and the build needs no look at the atoms first), sent off in pieces that travel while the
 // next piece is copied; one transfer back of [forces | energy, virial | status]; one pass that adds the forces. 13,824 local
-// and 11,415 ghost atoms, NEP: 183 us per step (48 copying, 68 waiting for the device, 24 taking the forces), where pageable
+// and 11,415 ghost atoms, NEP: 188 us per step (about 50 copying, 68 waiting for the device, 24 taking the forces), where pageable
 // transfers array by array, a device pass over the extents and a scalar loop over the forces took 355 us.
 #include "common.cuh"
 

@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(MTP_CWARPS * 32, 1) mtp_loss_contract_kernel(c
 // double, 32 in single precision. Two sweeps: products with their derivatives, then adjoints and second-order adjoints
 // together (a source's second-order adjoint needs the two of its products, which belong to deeper levels). A row of the second
 // sweep reads four operands where three sweeps of their own read six. Walks over the tiles with the tables staged once.
-// Level 16, fp64, 9,323 atoms: 86 us; 171 us with one row per warp, a block per tile and the table staged for each.
+// Level 16, fp64, 9,323 atoms: 83 us; 171 us with one row per warp, a block per tile and the table staged for each.
 template <typename T>
 struct LossPairSmem {
     T *M, *E, *seed;

@@ -589,9 +589,9 @@ __device__ __forceinline__ bool nb_exact(const NbParams<T> &P, const typename Ve
 }
 
 // ---- rows --------------------------------------------------------------------------------------------
-// A team of WPC warps per bin, CAP candidates of it in shared memory at a time. What bounds it is instruction issue: about
-// 600 warp instructions per atom (280 candidates, 30 survivors), half of them exact predicate and row. One warp per atom with
-// bins of half a cutoff and a table per atom took 1,750.
+// A team of WPC warps per bin, CAP candidates of it in shared memory at a time. What bounds it is instruction issue: 700 warp
+// instructions per atom at 13,824 atoms (280 candidates, 30 survivors), 540 at 1,048,576 of a sparser crystal, half of them exact
+// predicate and row. One warp per atom with bins of half a cutoff and a table per atom took 1,750.
 // TO = element type of the rcs rows (T, or float rows from double positions: what an MD host that keeps
 // double coordinates and a single-precision model does on the CPU).
 template <int WPC> __host__ __device__ constexpr int nbc_warps() { return WPC > 4 ? WPC : 4; }    // warps per block
@@ -1156,7 +1156,7 @@ static int nblist_build(int n, int ncentre, const T *h_cell, const T *d_coords, 
 //      are queued in order
 //   3. lanes = queued triples: the exact predicate, in full warps
 // Testing every triple exactly (27 x 5 warp steps per centre in double precision) took 275 us for 64 structures of 64 to 256
-// atoms; this takes about 25 us.
+// atoms; this takes 40 us.
 constexpr int NBB_WARPS = 8;
 constexpr int NBB_TILE = 512;       // atoms staged per tile
 constexpr int NBB_CPW = 2;          // centres per warp

@@ -550,12 +550,14 @@ static size_t nep_fast_smem(int lanes, const NepTab<NMAX> &L, int nneu, int umax
 
 // Lanes per atom of the specialised kernel for models of at most NMAX radial and angular functions; 0: the model or the
 // neighbour width does not fit it, and the general kernel runs.
-// Few atoms: more lanes, the chip is filled by atoms x lanes. Whole call in us, fp32, 29 / 6.5 neighbours (in brackets eight
-// lanes per atom and a trip count per group):
-//   216 atoms: 32 lanes 9.8, 16 lanes 10.6 [20.2];   1,157: 12.6, 12.2 [20.3];   4,000: 16 lanes 14.7, 8 lanes 18.1 [24.5];
-//   13,824: 16 lanes 30.5, 8 lanes 30.0 [48.7];   60,000: 8 lanes 80, 4 lanes 110 [176]
-// Four lanes pay when the rows are short enough for four blocks per SM and angular neighbours are few (17 / 2.2
-// neighbours, 1,048,576 atoms: 945, eight lanes 1083 [1435]); narrow rows stand for that.
+// Few atoms: more lanes, the chip is filled by atoms x lanes. Whole call in us, fp32, 29 / 6.5 neighbours, 32 / 16 / 8 / 4 lanes
+// (in brackets eight lanes per atom and a trip count per group):
+//   216 atoms: 9.8 / 10.7 / 12.3 / 19.1 [20.2];   1,157: 12.9 / 11.7 / 13.1 / 19.9 [20.3];   2,500: 16.2 / 12.7 / 15.4 / 20.5;
+//   4,000: 20.2 / 16.8 / 17.6 / 23.2 [24.5];   6,000: 25.2 / 21.2 / 18.2 / 24.7;   13,824: 42.8 / 30.8 / 28.3 / 29.0 [48.7];
+//   60,000: 157 / 105 / 82 / 100 [176]
+// (the line between 16 and 8 lanes stands at 6,000 atoms, the times cross at about 4,500). Four lanes pay when the rows are
+// short enough for four blocks per SM and angular neighbours are few (17 / 2.2 neighbours, 1,048,576 atoms: 833, eight lanes
+// 1,095 [1,435]); narrow rows stand for that.
 // Where the shared memory of the wanted form exceeds a block's share, the next one with more lanes is taken (kernels alone;
 // 12 species, umax 32, 60,000 atoms: 8 lanes 103, general kernel 505; fp64, umax 128, 13,824 atoms: 16 lanes 55, 32 lanes 80).
 template <typename T, int NMAX>
