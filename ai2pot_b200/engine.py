@@ -25,6 +25,7 @@ class Evaluator:
         self.prog = capi.MtpProgram(model["tables"]) if self.kind == "mtp" else None
         self.device = dev
         self.builder = capi.NeighborBuilder()
+        self.lists = ()
         self._new_lists()
         self.nb_static = dict(binum=torch.tensor([n], dtype=torch.int32, device=dev),
                               bilist=torch.arange(n, dtype=torch.int32, device=dev)[None].contiguous(),
@@ -42,8 +43,17 @@ class Evaluator:
         self._call = (capi.lib().ai2b_evaluate, C.byref(self._desc), self.device.index)
         self._describe()
 
+    @staticmethod
+    def _let_go(tensors):
+        """Buffers that are about to be replaced may still be in use on the stream of the last call, which need not be the one
+        that they were made on."""
+        for t in tensors:
+            if t is not None:
+                t.record_stream(torch.cuda.current_stream())
+
     def _new_lists(self):
         """Neighbour tensors for rows of umax slots: numneigh, firstneigh, rcs, status."""
+        self._let_go(self.lists)
         self.lists = capi.NeighborBuilder.new_outputs(self.n, int(self.umax), self.dtype, self.device)
         self.status = self.lists[3]
 
@@ -57,6 +67,7 @@ class Evaluator:
                                                        C.c_int(int(m["n_angular"])), C.c_int(int(m["chebyshev_size"])),
                                                        C.c_int(int(self.dtype == torch.float64)))
         if self.ws is None or self.ws.numel() < need:
+            self._let_go((self.ws,))
             self.ws = torch.empty(max(need, 256), dtype=torch.uint8, device=self.device)
         return self.ws
 
