@@ -114,21 +114,31 @@ def test_md_session_pieces(n):
 
 @pytest.mark.parametrize("kind", ["nep", "mtp"])
 def test_first_step_of_a_session(kind):
-    """The first step of a session allocates what later steps use; it takes less than 1.5 ms (0.6 to 0.8; with nine
-    allocations and pinned memory for a whole step 2.1 to 5). The best of several: pinning may be slow on a busy host."""
+    """The first step of a session allocates what later steps use: 0.6 to 0.8 ms on a quiet machine (2.1 to 5 with eight device
+    allocations and pinned memory for a whole step). The best of several against 1 ms and what one device allocation of that
+    size takes at the time, as other users of the machine make allocations slow."""
+    import ctypes as C
     import time
+    rt = C.CDLL("libcudart.so.12")
+
+    def allocation():
+        p = C.c_void_p()
+        t0 = time.perf_counter()
+        assert rt.cudaMalloc(C.byref(p), C.c_size_t(24 << 20)) == 0 and rt.cudaFree(p) == 0
+        return time.perf_counter() - t0
     w = synth.g2(n=24) if kind == "nep" else util.small_mtp_case(16, 14, np.float32, rcut=6.0)
     m = w["model"]
     prog = capi.MtpProgram(m["tables"]) if kind == "mtp" else None
     x = np.ascontiguousarray(np.mod(w["coords"].astype(np.float64), np.diag(w["cell"]).astype(np.float64)))
-    best = 1e9
-    for _ in range(8):
+    first, plain = [], []
+    for _ in range(10):
         ses = capi.MdSession(m, 64, prog)
         t0 = time.perf_counter()
         ses.compute(len(x), 0, x, w["types"])
-        best = min(best, time.perf_counter() - t0)
+        first.append(time.perf_counter() - t0)
         ses.close()
-    assert best < 1.5e-3
+        plain.append(allocation())
+    assert min(first) < 1e-3 + min(plain)
 
 
 def test_atom_that_has_flown_off():
