@@ -78,11 +78,11 @@ CHAINED_COPY_BYTES = 1 << 20
 
 
 def copy_around_call(dst, src):
-    """dst.copy_(src) on the current stream; between device and pinned host memory, small contiguous copies go through
-    ai2b_chained_copy."""
+    """dst.copy_(src) on the current stream; between the current device's and pinned host memory, small contiguous copies go
+    through ai2b_chained_copy."""
     n = dst.numel() * dst.element_size()
     if (n <= CHAINED_COPY_BYTES and dst.dtype == src.dtype and dst.shape == src.shape and dst.is_contiguous() and src.is_contiguous()
-            and all(t.is_cuda or t.is_pinned() for t in (dst, src))):
+            and all(t.get_device() == torch.cuda.current_device() if t.is_cuda else t.is_pinned() for t in (dst, src))):
         _check(lib().ai2b_chained_copy(C.c_void_p(dst.data_ptr()), C.c_void_p(src.data_ptr()), C.c_size_t(n), _stream()))
     else:
         dst.copy_(src, non_blocking=True)
