@@ -600,8 +600,10 @@ static int launch_nep_fast(NepArgs<T> A, const T *coeffs, void *ws, size_t ws_by
     *done = false;
     const int lanes = nep_fast_lanes<T, NMAX>((long)A.B * A.npad, A.ntypes, A.nneu, A.umax, NET);
     const NepTab<NMAX> L(A.ntypes, A.nneu, NET);
-    if (lanes == 0 || nep_prefix_bytes(A.B) + (size_t)L.total * sizeof(T) > ws_bytes) return AI2B_OK;
-    T *tab = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(ws) + nep_prefix_bytes(A.B));
+    // (the table is copied 16 bytes at a time; a workspace that does not start on such a boundary has room for the difference)
+    const size_t at = nep_prefix_bytes(A.B), shift = (16 - (reinterpret_cast<size_t>(ws) + at) % 16) % 16;
+    if (lanes == 0 || at + shift + (size_t)L.total * sizeof(T) > ws_bytes) return AI2B_OK;
+    T *tab = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(ws) + at + shift);
     {   // table, offsets, zeroed outputs
         T *z[3] = {NET ? A.etot : A.desc, A.force, A.virial};
         const size_t nz[3] = {NET ? (size_t)A.B : (size_t)A.B * A.npad * A.nd, NET ? 3 * (size_t)A.B * (A.npad + A.nghost) : 0, A.virial ? 9 * (size_t)A.B : 0};

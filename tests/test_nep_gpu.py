@@ -279,3 +279,26 @@ def test_lanes_when_shared_memory_is_short(checkers, dt, ntypes, neurons, slots,
     want = chk.nep_efv(_f64(model), dict(nb, brcs=nb["brcs"].astype(np.float64)))
     for a, b, name in zip(got, want, ("energy", "force", "virial")):
         assert util.relerr(a, b) < (1e-10 if dt == np.float64 else 1e-5), name
+
+
+@pytest.mark.parametrize("dt,shift", [(np.float32, 4), (np.float32, 8), (np.float32, 12), (np.float64, 8)])
+def test_workspace_off_a_16_byte_boundary(dt, shift):
+    """The model table of the specialised kernel is copied 16 bytes at a time, wherever the caller's workspace starts; a
+    workspace without room for the difference takes the general kernel."""
+    rng = np.random.default_rng(3)
+    cell, pos = synth.cubic_lattice(6, 3.0, 0.1, rng, dt)
+    model = synth.nep_model(3, rng, dt)
+    rows = capi.NeighborBuilder().build(cell, torch.from_numpy(pos).cuda(), 6.0, 64)
+    n = len(pos)
+    nb = dict(binum=torch.tensor([n], dtype=torch.int32, device="cuda"), bilist=torch.arange(n, dtype=torch.int32, device="cuda")[None],
+              bnumneigh=rows[0][None], bfirstneigh=rows[1][None], brcs=rows[2][None], ntypes=3, nghost=0,
+              btypes=torch.from_numpy(rng.integers(0, 3, n).astype(np.int32)).cuda()[None])
+    md = capi.to_device(model, float_dtype=torch.float64 if dt == np.float64 else torch.float32)
+    want = [o.cpu().numpy() for o in capi.nep_efv(md, nb)]
+    need = capi.lib().ai2b_nep_workspace_bytes(1, 3, 4, 4, 8, int(dt == np.float64))
+    for size in (need, 256 + 3 * 3 * 8 * 8 * dt().itemsize + 256):
+        ws = torch.empty(size + 64, dtype=torch.uint8, device="cuda")[shift:shift + size]
+        assert ws.data_ptr() % 16 == shift
+        got = [o.cpu().numpy() for o in capi.nep_efv(md, nb, ws=ws)]
+        for a, b in zip(got, want):
+            assert util.relerr(a, b) < TOL[dt]
