@@ -692,7 +692,9 @@ static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArg
     const bool pair = P.stream[1].nrows > 0 && pair_bytes <= 226 * 1024;
     // the coefficient gradient by tiles pays once they occupy half of the SMs; below that a warp per atom is over sooner
     // (level 10, fp32, 240 atoms: 11 against 14 us; level 16, fp64, 9,323 atoms: 99 against 87)
-    L.dense = pair && atoms_path && atoms_upper >= MTP_TILE * (long)sm_count() / 2 && mtp_coeff_atoms_supported(P, A.ntypes, sizeof(T));
+    // (it copies 16 bytes at a time)
+    L.dense = pair && atoms_path && atoms_upper >= MTP_TILE * (long)sm_count() / 2 && reinterpret_cast<size_t>(L.Xb) % 16 == 0 &&
+              mtp_coeff_atoms_supported(P, A.ntypes, sizeof(T));
     {
         const size_t cap = 222 * 1024;
         int rc = AI2B_ERR_UNSUPPORTED;

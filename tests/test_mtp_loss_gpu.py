@@ -199,3 +199,22 @@ def test_loss_op_keeps_the_moments(checkers, B, cs, dt):
     for _ in range(2):
         for p, a, r in zip(params, torch.autograd.grad(total, params, retain_graph=True), ref):
             assert a.shape == p.shape and util.relerr(a.cpu().numpy(), (w.double() @ r.reshape(B, -1).double()).cpu().numpy()) < tol
+
+
+def test_workspace_off_a_16_byte_boundary(checkers, monkeypatch):
+    """The coefficient gradient by tiles (enough atom slots for half of the SMs) copies 16 bytes at a time; a workspace that
+    starts elsewhere takes the other kernel."""
+    g, nb = util.training_batch(_chk(checkers), level=16, B=16, seed=5, nmin=20, nmax=160)
+    assert nb["bilist"].size >= 2368
+    prog, md, nbd, (E, F, V) = _dev(g, nb)
+    e, f, v = capi.mtp_efv(prog, md, nbd)
+    want = capi.mtp_loss_backward(prog, md, nbd, g["weights"], e, E, f, F, v, V)
+    empty = torch.empty
+
+    def shifted(*size, **kw):
+        return empty(size[0] + 8, **kw)[8:] if kw.get("dtype") is torch.uint8 else empty(*size, **kw)
+    monkeypatch.setattr(torch, "empty", shifted)
+    got = capi.mtp_loss_backward(prog, md, nbd, g["weights"], e, E, f, F, v, V)
+    monkeypatch.undo()
+    for a, b in zip(got, want):
+        assert util.relerr(a.cpu().numpy(), b.cpu().numpy()) < 1e-10
