@@ -119,6 +119,19 @@ def test_changed_attributes_take_effect(kind):
     ev.model["coeffs"] = 0.9 * ev.model["coeffs"]
     same(_host(make(other, sheared, 0.75 * w["rcut"]).compute(coords)))
     _close(_host(ev.replay()), before, tol)
+    # a tensor that the kernels cannot read is refused, also where its address is that of the last call's
+    for name, bad in (("coeffs", ev.model["coeffs"].cpu()), ("q_scaler", ev.model["q_scaler"].expand(2, -1).t()[:, 0][::2])):
+        good, ev.model[name] = ev.model[name], bad
+        with pytest.raises(engine.capi.Ai2bError):
+            ev.compute(coords)
+        ev.model[name] = good
+    for wrong in (np.eye(3)[:2], np.ones(3)):
+        good, ev.cell = ev.cell, wrong
+        with pytest.raises(ValueError):
+            ev.compute(coords)
+        ev.cell = good
+    ev.cell = list(map(list, sheared))
+    same(_host(make(other, sheared, 0.75 * w["rcut"]).compute(coords)))
 
 
 def test_positions_that_do_not_fit_are_refused():
