@@ -357,12 +357,15 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
     for (int k = 0; k < MTP_MAX_LEV; k++) {
         if (k < P.nlev)
             for (int m : moments_of_depth(P.nlev - 1 - k, occ_at)) {
-                const int rb = (int)rev_ents.size(), re = rb + occ_at[m + 1] - occ_at[m];
+                const int rb = (int)rev_ents.size();
                 for (int i = occ_at[m]; i < occ_at[m + 1]; i++) {
                     const int o = occ_of[i], *r = times + 4 * (o >> 1);
-                    add_row(rev_ents, rev_flat, r[1 - (o & 1)] | (r[3] << 16), r[2], m, i + 1 == occ_at[m + 1]);
+                    // the square of a moment: both of its places (they follow one another) in one row
+                    const bool both = !(o & 1) && r[0] == r[1] && 2 * r[2] <= 255;
+                    if (both) i++;
+                    add_row(rev_ents, rev_flat, r[1 - (o & 1)] | (r[3] << 16), both ? 2 * r[2] : r[2], m, i + 1 == occ_at[m + 1]);
                 }
-                rev_mom.push_back(make_int4(m, rb, re, 0));
+                rev_mom.push_back(make_int4(m, rb, (int)rev_ents.size(), 0));
             }
         P.rev_lev_off[k + 1] = (int)rev_mom.size();
         P.rev_lev_row[k + 1] = (int)rev_ents.size();
