@@ -13,6 +13,8 @@
 //    shared memory as [dense moment][atom], so a coefficient is one conflict-free load at a compile-time
 //    offset; the polynomial of a radial function and its gradient are evaluated by nested sums over the
 //    z, y and x exponents (two FMAs per coefficient instead of four).
+// A tile has 32 atoms, or 16, 8 or 4: with few atoms the lanes of a warp share the neighbour slots of an atom (2, 4 or 8 lanes per
+// atom, sums added up by shuffles), so that the chip is filled and the serial loop over the slots gets shorter (atom_parts).
 // The basic moments and their adjoints travel between the kernels as [tile][basic row][32 atoms], which
 // all three kernels read and write in full 256-byte rows.
 // The kernels are compiled per "signature" = the highest monomial degree of every radial function
@@ -108,12 +110,12 @@ struct PairEval {
     }
     __device__ __forceinline__ void lookup(const int *types_b) { tj = act ? types_b[nj] : 0; }
     // slot j of this lane's atom: from the staged rows, or from global memory beyond them
-    __device__ __forceinline__ void fetch(const MtpArgs<T> &A, const TileRows<T> &tr, const int *types_b, size_t row, int lane, int j, int nn)
+    __device__ __forceinline__ void fetch(const MtpArgs<T> &A, const TileRows<T> &tr, const int *types_b, size_t row, int a, int j, int nn)
     {
         if (j < TR_SLOTS) {
             act = j < nn;
-            const T *p = tr.pos + lane * TR_RS + 3 * j;
-            const int w = tr.idx[lane * TR_IS + j];
+            const T *p = tr.pos + a * TR_RS + 3 * j;
+            const int w = tr.idx[a * TR_IS + j];
             x = act ? p[0] : T(0); y = act ? p[1] : T(0); z = act ? p[2] : T(0);
             nj = w & TR_INDEX_MASK;
             tj = w >> TR_TYPE_SHIFT;
@@ -196,13 +198,30 @@ __device__ __forceinline__ int warp_max_int(int v)
     return v;
 }
 
+// How many lanes share the slots of an atom. A tile takes about (1 / parts + 1 / 6) of the time of one with a lane per atom
+// (staging and look-ups do not get shorter), and the blocks of the chip work through the tiles in rounds. Level 16, double
+// precision, whole recorded call with its copies, us with 1, 2, 4, 8 lanes per atom: 1,000 atoms 66, 59, 49, 49; 3,001 atoms 88, 70,
+// 64, 72; 5,000 atoms 100, 82, 89, 95; 9,323 atoms 122, 127, 127, 149; 13,824 atoms 147, 153, 166, 197; 20,000 atoms 222, 211, 231, 277.
+// Decided by the host for one structure, on the device for a batch, of which the host knows only the padded size. `resident`
+// blocks of the kernel run at a time.
+__host__ __device__ __forceinline__ int atom_parts(int atoms, int resident)
+{
+    int best = 1, least = 0;
+#pragma unroll
+    for (int parts = 1; parts <= 8; parts *= 2) {
+        const int tiles = (atoms + MTP_TILE / parts - 1) / (MTP_TILE / parts), time = (tiles + resident - 1) / resident * (24 / parts + 4);
+        if (parts == 1 || time < least) { least = time; best = parts; }
+    }
+    return best;
+}
+
 // ---- forward --------------------------------------------------------------------------------------
 // DERIV = false: basic moments M -> A.Mb. DERIV = true (loss gradient, linearMtpLoss.h:331-389): their directional
 // derivatives D = sum_j p_ij . dM/dr_j along the pair weights p of the loss -> L.Db; per neighbour and monomial m
 // that is a_mu m + f_mu (q . grad m) with a_mu = f'_mu (p . u), q = (p - (p . u) u) / r.
 // shared memory: radial coefficients [ntypes^2][NMUS][CSP] (rows shifted), staging [AT_CH][NV][32], tile rows
 template <typename T, typename SIG, int CSP, bool DERIV>
-__global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_kernel(const MtpProgramDev P, const MtpArgs<T> A, const LossArgs<T> L)
+__global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_kernel(const MtpProgramDev P, const MtpArgs<T> A, const LossArgs<T> L, int parts, int resident)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int NV = 3 + SIG::NMUS + (DERIV ? SIG::NMUS + 3 : 0);   // u, f [, a, q]
@@ -223,30 +242,32 @@ __global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_ke
         if (A.virial && i0 < 9 * (size_t)A.B) A.virial[i0] = T(0);
     }
     const int ntot = total_atoms(A);
-    const int ntiles = (ntot + MTP_TILE - 1) / MTP_TILE;
+    if (parts == 0) parts = atom_parts(ntot, resident);
+    const int ta = 32 / parts, a = lane & (ta - 1), part = lane / ta;      // atoms of the tile; this lane's atom and share of its slots
+    const int ntiles = (ntot + ta - 1) / ta;
 
     const bool single = A.B == 1;      // one structure: a tile's rows are known from its index alone
     const T inv_range = T(1) / (A.rmax - A.rmin);
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         if (single) {
             if (tile != (int)blockIdx.x) __syncthreads();     // the previous tile's rows are no longer read
-            tr.template request<AT_WARPS * 32>(A.rcs, A.firstneigh, A.umax, (size_t)tile * MTP_TILE, (size_t)A.npad);
+            tr.template request<AT_WARPS * 32>(A.rcs, A.firstneigh, A.umax, (size_t)tile * ta, (size_t)A.npad, ta);
         }
         TileAtom<T> at;
-        at.set(A, tile * MTP_TILE + lane, ntot);
+        at.set(A, tile * ta + a, ntot);
         const int nmax = warp_max_int(at.nn);      // the same in every warp of the block
         const size_t row = at.slot * A.umax;
         const int nstruct = at.valid ? A.binum[at.b] : 1;
-        T *out = (DERIV ? L.Db : A.Mb) + (size_t)tile * A.nbp * MTP_TILE + lane;
+        T *out = (DERIV ? L.Db : A.Mb) + (size_t)(tile * ta / MTP_TILE) * A.nbp * MTP_TILE + (tile * ta + a) % MTP_TILE;
         if (single) {
             __pipeline_wait_prior(0);
             __syncthreads();     // every thread's copies have arrived
-            tr.template complete<AT_WARPS * 32>(A.types, A.npad + A.nghost);
+            tr.template complete<AT_WARPS * 32>(A.types, A.npad + A.nghost, ta);
         } else {
             __syncthreads();     // the previous tile's rows are no longer read
-            if (warp == 0) tr.describe(lane, row, (size_t)(at.types_b - A.types), at.nn);
+            if (warp == 0 && part == 0) tr.describe(a, row, (size_t)(at.types_b - A.types), at.nn);
             __syncthreads();
-            tr.template stage<AT_WARPS * 32>(A.rcs, A.firstneigh, A.types, A.umax);
+            tr.template stage<AT_WARPS * 32>(A.rcs, A.firstneigh, A.types, A.umax, ta);
         }
 
         auto body = [&](auto gg) {
@@ -255,12 +276,12 @@ __global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_ke
             T acc[NACC > 0 ? NACC : 1];
 #pragma unroll
             for (int i = 0; i < (NACC > 0 ? NACC : 1); i++) acc[i] = T(0);
-            for (int j0 = 0; j0 < nmax; j0 += AT_CH) {
-                const int cnt = min(AT_CH, nmax - j0);
+            for (int j0 = 0; j0 < nmax; j0 += AT_CH * parts) {
+                const int cnt = min(AT_CH, (nmax - j0 + parts - 1) / parts);
                 __syncthreads();     // rows and coefficients staged / the previous round's slots consumed
                 for (int jj = warp; jj < cnt; jj += AT_WARPS) {   // this warp's slots of the round
                     PairEval<T, SIG, CSP> pe;
-                    pe.fetch(A, tr, at.types_b, row, lane, j0 + jj, at.nn);
+                    pe.fetch(A, tr, at.types_b, row, a, j0 + jj * parts + part, at.nn);
                     pe.template compute<DERIV>(A, cf, at.ti, inv_range);
                     T *s = st + (size_t)jj * NV * 32 + lane;
                     s[0] = pe.ux; s[32] = pe.uy; s[64] = pe.uz;
@@ -285,10 +306,10 @@ __global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_ke
                         const T *s = st + (size_t)jj * NV * 32 + lane;
                         Powers<T, KD> pw;
                         pw.set(s[0], s[32], s[64]);
-                        T f[SIG::NMUS], a[SIG::NMUS], dx[KD + 1], dy[KD + 1], dz[KD + 1];
+                        T f[SIG::NMUS], am[SIG::NMUS], dx[KD + 1], dy[KD + 1], dz[KD + 1];
                         static_for<0, SIG::NMUS>([&](auto mm) { f[decltype(mm)::value] = s[(3 + decltype(mm)::value) * 32]; });
                         if constexpr (DERIV) {
-                            static_for<0, SIG::NMUS>([&](auto mm) { a[decltype(mm)::value] = s[(3 + SIG::NMUS + decltype(mm)::value) * 32]; });
+                            static_for<0, SIG::NMUS>([&](auto mm) { am[decltype(mm)::value] = s[(3 + SIG::NMUS + decltype(mm)::value) * 32]; });
                             const T qx = s[(3 + 2 * SIG::NMUS) * 32], qy = s[(4 + 2 * SIG::NMUS) * 32], qz = s[(5 + 2 * SIG::NMUS) * 32];
 #pragma unroll
                             for (int k = 1; k <= KD; k++) {      // q_x d/dx of the powers, and so on
@@ -317,7 +338,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_ke
                                     static_for<0, SIG::cnt(D)>([&](auto mm) {
                                         constexpr int mu = decltype(mm)::value;
                                         constexpr int I = SIG::acc_off(D) + Q * SIG::cnt(D) + mu;
-                                        if constexpr (DERIV) acc[I] = fma(a[mu], m, fma(f[mu], dm, acc[I]));
+                                        if constexpr (DERIV) acc[I] = fma(am[mu], m, fma(f[mu], dm, acc[I]));
                                         else acc[I] = fma(f[mu], m, acc[I]);
                                     });
                                 });
@@ -326,7 +347,10 @@ __global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_ke
                     }
                 }
             }
-            // this warp's moments of the tile: one 256-byte row per moment
+            for (int o = ta; o < 32; o <<= 1)      // the lanes of an atom add up their shares
+#pragma unroll
+                for (int i = 0; i < NACC; i++) acc[i] += __shfl_xor_sync(FULL_MASK, acc[i], o);
+            // this warp's moments of the tile: one row per moment
             static_for<0, KD + 1>([&](auto dd) {
                 constexpr int D = decltype(dd)::value;
                 if constexpr (SIG::group(D) == G) {
@@ -335,7 +359,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_ke
                         static_for<0, SIG::cnt(D)>([&](auto mm) {
                             constexpr int mu = decltype(mm)::value;
                             const int r = P.dense_basic[SIG::doff(mu) + ncan(D - 1) + Q];
-                            if (r >= 0) out[(size_t)r * MTP_TILE] = acc[SIG::acc_off(D) + Q * SIG::cnt(D) + mu];
+                            if (r >= 0 && part == 0) out[(size_t)r * MTP_TILE] = acc[SIG::acc_off(D) + Q * SIG::cnt(D) + mu];
                         });
                     });
                 }
@@ -353,7 +377,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_ke
 // ---- force and virial -----------------------------------------------------------------------------
 // shared memory: radial coefficients, adjoints [NDENSE][32]
 template <typename T, int MODE, typename SIG, int CSP>
-__global__ void __launch_bounds__(AT_WARPS * 32, 3) mtp_force_atoms_kernel(const MtpProgramDev P, const MtpArgs<T> A)
+__global__ void __launch_bounds__(AT_WARPS * 32, 3) mtp_force_atoms_kernel(const MtpProgramDev P, const MtpArgs<T> A, int parts, int resident)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int KD = SIG::KD;
@@ -366,7 +390,9 @@ __global__ void __launch_bounds__(AT_WARPS * 32, 3) mtp_force_atoms_kernel(const
     stage_coefficients<T, SIG, CSP>(A, cf);   // model constants: staged while the contraction drains
     chain_wait();
     const int ntot = total_atoms(A);
-    const int ntiles = (ntot + MTP_TILE - 1) / MTP_TILE;
+    if (parts == 0) parts = atom_parts(ntot, resident);
+    const int ta = 32 / parts, a = lane & (ta - 1), part = lane / ta;      // as in the forward kernel
+    const int ntiles = (ntot + ta - 1) / ta;
     const bool single = A.B == 1;      // one structure: a tile's rows are known from its index alone
     const T inv_range = T(1) / (A.rmax - A.rmin);
 
@@ -374,26 +400,30 @@ __global__ void __launch_bounds__(AT_WARPS * 32, 3) mtp_force_atoms_kernel(const
         if (tile != (int)blockIdx.x) __syncthreads();     // the previous tile's adjoints and rows are no longer read
         {   // The contraction leaves the adjoints of a tile in dense monomial order, [dense][32 atoms] in one piece: they are
             // requested here with asynchronous 16-byte copies and awaited only before the neighbour loop.
-            const T *ein = A.Eb + (size_t)tile * A.ndp * MTP_TILE;
+            const T *ein = A.Eb + (size_t)(tile * ta / MTP_TILE) * A.ndp * MTP_TILE + (tile * ta) % MTP_TILE;
             constexpr int CH = 16 / (int)sizeof(T);
-            for (int c = threadIdx.x; c < SIG::NDENSE * 32 / CH; c += AT_WARPS * 32) __pipeline_memcpy_async(Es + c * CH, ein + c * CH, 16);
+            const int cpr = ta / CH;      // chunks of a row
+            for (int c = threadIdx.x; c < SIG::NDENSE * cpr; c += AT_WARPS * 32) {
+                const int e = c / cpr * 32 + c % cpr * CH;
+                __pipeline_memcpy_async(Es + e, ein + e, 16);
+            }
             __pipeline_commit();
         }
-        if (single) tr.template request<AT_WARPS * 32>(A.rcs, A.firstneigh, A.umax, (size_t)tile * MTP_TILE, (size_t)A.npad);
+        if (single) tr.template request<AT_WARPS * 32>(A.rcs, A.firstneigh, A.umax, (size_t)tile * ta, (size_t)A.npad, ta);
         TileAtom<T> at;
-        at.set(A, tile * MTP_TILE + lane, ntot);
+        at.set(A, tile * ta + a, ntot);
         const int nmax = warp_max_int(at.nn);
         const size_t row = at.slot * A.umax;
         T *frc = A.force + (size_t)at.b * (A.npad + A.nghost) * 3;
         if (single) {
             __pipeline_wait_prior(0);     // the adjoints and the rows requested at the top of the tile
             __syncthreads();
-            tr.template complete<AT_WARPS * 32>(A.types, A.npad + A.nghost);
+            tr.template complete<AT_WARPS * 32>(A.types, A.npad + A.nghost, ta);
         } else {
             __syncthreads();     // the previous tile's rows are no longer read
-            if (warp == 0) tr.describe(lane, row, (size_t)(at.types_b - A.types), at.nn);
+            if (warp == 0 && part == 0) tr.describe(a, row, (size_t)(at.types_b - A.types), at.nn);
             __syncthreads();
-            tr.template stage<AT_WARPS * 32>(A.rcs, A.firstneigh, A.types, A.umax);
+            tr.template stage<AT_WARPS * 32>(A.rcs, A.firstneigh, A.types, A.umax, ta);
             __pipeline_wait_prior(0);     // the adjoints requested at the top of the tile
         }
         __syncthreads();
@@ -402,10 +432,10 @@ __global__ void __launch_bounds__(AT_WARPS * 32, 3) mtp_force_atoms_kernel(const
         T vir[9];
 #pragma unroll
         for (int k = 0; k < 9; k++) vir[k] = T(0);
-        const T *el = Es + lane;
-        for (int j = warp; j < nmax; j += AT_WARPS) {
+        const T *el = Es + a;
+        for (int j0 = warp * parts; j0 < nmax; j0 += AT_WARPS * parts) {
             PairEval<T, SIG, CSP> pe;
-            pe.fetch(A, tr, at.types_b, row, lane, j, at.nn);
+            pe.fetch(A, tr, at.types_b, row, a, j0 + part, at.nn);
             pe.template compute<true>(A, cf, at.ti, inv_range);
             // powers of the unit vector and their derivatives k u^(k-1)
             T X[KD + 1], Y[KD + 1], Z[KD + 1], dX[KD + 1], dY[KD + 1], dZ[KD + 1];
@@ -426,26 +456,26 @@ __global__ void __launch_bounds__(AT_WARPS * 32, 3) mtp_force_atoms_kernel(const
                 // polynomial of this radial function in (ux, uy, uz) and its gradient, by nested sums
                 T Pv = T(0), Gx = T(0), Gy = T(0), Gz = T(0);
                 static_for<0, K + 1>([&](auto aa) {
-                    constexpr int a = decltype(aa)::value;
+                    constexpr int x = decltype(aa)::value;
                     T S = T(0), Sy = T(0), Sz = T(0);
-                    static_for<0, K - a + 1>([&](auto bb) {
+                    static_for<0, K - x + 1>([&](auto bb) {
                         constexpr int b = decltype(bb)::value;
                         T R = T(0), Rz = T(0);
-                        static_for<0, K - a - b + 1>([&](auto cc) {
+                        static_for<0, K - x - b + 1>([&](auto cc) {
                             constexpr int c = decltype(cc)::value;
-                            const T e = el[(base + canon_index(a, b, c)) * 32];
+                            const T e = el[(base + canon_index(x, b, c)) * 32];
                             if constexpr (c == 0) R = e; else R = fma(e, Z[c], R);
                             if constexpr (c == 1) Rz = e; else if constexpr (c > 1) Rz = fma(e, dZ[c], Rz);
                         });
                         if constexpr (b == 0) S = R; else S = fma(Y[b], R, S);
                         if constexpr (b == 1) Sy = R; else if constexpr (b > 1) Sy = fma(dY[b], R, Sy);
-                        if constexpr (K - a - b >= 1) { if constexpr (b == 0) Sz = Rz; else Sz = fma(Y[b], Rz, Sz); }
+                        if constexpr (K - x - b >= 1) { if constexpr (b == 0) Sz = Rz; else Sz = fma(Y[b], Rz, Sz); }
                     });
-                    if constexpr (a == 0) Pv = S; else Pv = fma(X[a], S, Pv);
-                    if constexpr (a == 1) Gx = S; else if constexpr (a > 1) Gx = fma(dX[a], S, Gx);
-                    if constexpr (K - a >= 1) {
-                        if constexpr (a == 0) { Gy = Sy; Gz = Sz; }
-                        else { Gy = fma(X[a], Sy, Gy); Gz = fma(X[a], Sz, Gz); }
+                    if constexpr (x == 0) Pv = S; else Pv = fma(X[x], S, Pv);
+                    if constexpr (x == 1) Gx = S; else if constexpr (x > 1) Gx = fma(dX[x], S, Gx);
+                    if constexpr (K - x >= 1) {
+                        if constexpr (x == 0) { Gy = Sy; Gz = Sz; }
+                        else { Gy = fma(X[x], Sy, Gy); Gz = fma(X[x], Sz, Gz); }
                     }
                 });
                 const T ug = pe.ux * Gx + pe.uy * Gy + pe.uz * Gz;
@@ -467,7 +497,10 @@ __global__ void __launch_bounds__(AT_WARPS * 32, 3) mtp_force_atoms_kernel(const
                 }
             }
         }
-        if (at.valid && warp < at.nn) {      // this warp saw at least one slot of the atom
+        for (int o = ta; o < 32; o <<= 1) {      // the lanes of an atom add up their shares
+            fcx += __shfl_xor_sync(FULL_MASK, fcx, o); fcy += __shfl_xor_sync(FULL_MASK, fcy, o); fcz += __shfl_xor_sync(FULL_MASK, fcz, o);
+        }
+        if (at.valid && part == 0 && warp * parts < at.nn) {      // this warp saw at least one slot of the atom
             atomicAdd(frc + 3 * at.ci + 0, fcx);
             atomicAdd(frc + 3 * at.ci + 1, fcy);
             atomicAdd(frc + 3 * at.ci + 2, fcz);
@@ -491,7 +524,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32, 3) mtp_force_atoms_kernel(const
                     for (int w = 0; w < AT_WARPS; w++) s += vred[w][threadIdx.x];
                     atomicAdd(A.virial + 9 * b0 + threadIdx.x, s);
                 }
-            } else if (at.valid && warp < at.nn) {
+            } else if (at.valid && warp * parts + part < at.nn) {
 #pragma unroll
                 for (int k = 0; k < 9; k++) atomicAdd(A.virial + 9 * at.b + k, vir[k]);
             }
@@ -733,10 +766,10 @@ static int launch_fwd_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, const L
     static KernelSetup setup;
     int per_sm = 1;
     if (int rc = kernel_setup(setup, kern, smem, AT_WARPS * 32, &per_sm)) return rc;
-    long tiles = ((long)A.B * A.npad + MTP_TILE - 1) / MTP_TILE;
-    long blocks = (long)sm_count() * per_sm;
-    if (blocks > tiles) blocks = tiles;
-    AI2B_CUDA(launch_chained(kern, (unsigned)blocks, AT_WARPS * 32, smem, st, P, A, L));
+    const int resident = sm_count() * per_sm;
+    const int parts = A.B == 1 ? atom_parts(A.npad, resident) : 0;
+    const long tiles = ((long)A.B * A.npad * (parts ? parts : 8) + 31) / 32;
+    AI2B_CUDA(launch_chained(kern, (unsigned)(tiles < resident ? tiles : resident), AT_WARPS * 32, smem, st, P, A, L, parts, resident));
     return AI2B_OK;
 }
 
@@ -749,10 +782,10 @@ static int launch_force_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, cudaS
     static KernelSetup setup;
     int per_sm = 1;
     if (int rc = kernel_setup(setup, kern, smem, AT_WARPS * 32, &per_sm)) return rc;
-    long tiles = ((long)A.B * A.npad + MTP_TILE - 1) / MTP_TILE;
-    long blocks = (long)sm_count() * per_sm;
-    if (blocks > tiles) blocks = tiles;
-    AI2B_CUDA(launch_chained(kern, (unsigned)blocks, AT_WARPS * 32, smem, st, P, A));
+    const int resident = sm_count() * per_sm;
+    const int parts = A.B == 1 ? atom_parts(A.npad, resident) : 0;
+    const long tiles = ((long)A.B * A.npad * (parts ? parts : 8) + 31) / 32;
+    AI2B_CUDA(launch_chained(kern, (unsigned)(tiles < resident ? tiles : resident), AT_WARPS * 32, smem, st, P, A, parts, resident));
     return AI2B_OK;
 }
 

@@ -7,7 +7,8 @@
 // elements), all of them in flight together, and the lanes then read their row from shared memory:
 //   pos[atom][TR_RS]   r_j - r_i of slots 0 .. TR_SLOTS-1 (row stride odd: the 32 rows start in different banks)
 //   idx[atom][TR_IS]   neighbour index | neighbour type << 26 (0 for empty slots)
-// Slots beyond TR_SLOTS (rows longer than 32 neighbours) are read from global memory by the caller.
+// Slots beyond TR_SLOTS (rows longer than 32 neighbours) are read from global memory by the caller. A tile may have fewer atoms
+// (`atoms`, a power of two): only their rows are copied then.
 #pragma once
 #include <cuda_pipeline.h>
 #include "common.cuh"
@@ -55,7 +56,7 @@ struct TileRows {
     // all NT threads of the block, after a barrier behind describe(); a barrier must follow
     template <int NT>
     __device__ __forceinline__ void stage(const T *__restrict__ rcs, const int *__restrict__ firstneigh, const int *__restrict__ types,
-                                          int umax)
+                                          int umax, int atoms = 32)
     {
         const int lim = 3 * (umax < TR_SLOTS ? umax : TR_SLOTS);
         constexpr int TP = 32 * 3 * TR_SLOTS, TI = 32 * TR_SLOTS;           // elements of the two copies
@@ -65,12 +66,12 @@ struct TileRows {
 #pragma unroll
         for (int k = 0; k < NI; k++) {
             const int e = threadIdx.x + k * NT, a = (e >> 5) & 31, j = e & 31;
-            nj[k] = (e < TI && j < nn[a]) ? firstneigh[row[a] + j] : -1;
+            nj[k] = (e < atoms * TR_SLOTS && j < nn[a]) ? firstneigh[row[a] + j] : -1;
         }
 #pragma unroll
         for (int k = 0; k < NP; k++) {
             const int e = threadIdx.x + k * NT, a = (e / (3 * TR_SLOTS)) & 31, o = e % (3 * TR_SLOTS);
-            v[k] = (e < TP && o < lim) ? rcs[row[a] * 3 + o] : T(0);
+            v[k] = (e < atoms * 3 * TR_SLOTS && o < lim) ? rcs[row[a] * 3 + o] : T(0);
         }
 #pragma unroll
         for (int k = 0; k < NI; k++) {
@@ -80,12 +81,12 @@ struct TileRows {
 #pragma unroll
         for (int k = 0; k < NP; k++) {
             const int e = threadIdx.x + k * NT, a = e / (3 * TR_SLOTS), o = e % (3 * TR_SLOTS);
-            if (e < TP) pos[a * TR_RS + o] = v[k];
+            if (e < atoms * 3 * TR_SLOTS) pos[a * TR_RS + o] = v[k];
         }
 #pragma unroll
         for (int k = 0; k < NI; k++) {
             const int e = threadIdx.x + k * NT, a = e >> 5, j = e & 31;
-            if (e < TI) idx[a * TR_IS + j] = w[k];
+            if (e < atoms * TR_SLOTS) idx[a * TR_IS + j] = w[k];
         }
     }
 
@@ -96,14 +97,14 @@ struct TileRows {
     // by all NT threads; a barrier must follow complete().
     template <int NT>
     __device__ __forceinline__ void request(const T *__restrict__ rcs, const int *__restrict__ firstneigh, int umax, size_t first_slot,
-                                            size_t nslots)
+                                            size_t nslots, int atoms)
     {
         const int lim = umax < TR_SLOTS ? umax : TR_SLOTS;
-        for (int e = threadIdx.x; e < 32 * 3 * TR_SLOTS; e += NT) {
+        for (int e = threadIdx.x; e < atoms * 3 * TR_SLOTS; e += NT) {
             const int a = e / (3 * TR_SLOTS), o = e % (3 * TR_SLOTS);
             if (o < 3 * lim && first_slot + a < nslots) __pipeline_memcpy_async(pos + a * TR_RS + o, rcs + (first_slot + a) * umax * 3 + o, sizeof(T));
         }
-        for (int e = threadIdx.x; e < 32 * TR_SLOTS; e += NT) {
+        for (int e = threadIdx.x; e < atoms * TR_SLOTS; e += NT) {
             const int a = e >> 5, j = e & 31;
             if (j < lim && first_slot + a < nslots) __pipeline_memcpy_async(raw + a * TR_IS + j, firstneigh + (first_slot + a) * umax + j, sizeof(int));
             else raw[a * TR_IS + j] = -1;
@@ -111,21 +112,21 @@ struct TileRows {
         __pipeline_commit();
     }
     template <int NT>
-    __device__ __forceinline__ void complete(const int *__restrict__ types, int ids)
+    __device__ __forceinline__ void complete(const int *__restrict__ types, int ids, int atoms)
     {
         constexpr int NI = (32 * TR_SLOTS + NT - 1) / NT;
         int nj[NI], w[NI];
 #pragma unroll
         for (int k = 0; k < NI; k++) {
             const int e = threadIdx.x + k * NT;
-            nj[k] = e < 32 * TR_SLOTS ? raw[(e >> 5) * TR_IS + (e & 31)] : -1;
+            nj[k] = e < atoms * TR_SLOTS ? raw[(e >> 5) * TR_IS + (e & 31)] : -1;
         }
 #pragma unroll
         for (int k = 0; k < NI; k++) w[k] = (nj[k] >= 0 && nj[k] < ids) ? (nj[k] | (types[nj[k]] << TR_TYPE_SHIFT)) : 0;
 #pragma unroll
         for (int k = 0; k < NI; k++) {
             const int e = threadIdx.x + k * NT;
-            if (e < 32 * TR_SLOTS) idx[(e >> 5) * TR_IS + (e & 31)] = w[k];
+            if (e < atoms * TR_SLOTS) idx[(e >> 5) * TR_IS + (e & 31)] = w[k];
         }
     }
 };

@@ -75,6 +75,27 @@ def test_g1_full_size_vs_checker(checkers):
     assert max(errs.values()) < 1e-10, errs
 
 
+@pytest.mark.parametrize("natoms,level,dt", [(3, 16, np.float64), (133, 16, np.float32), (1777, 16, np.float64), (2370, 10, np.float64), (3001, 10, np.float32),
+                                             (5003, 10, np.float64), (15001, 6, np.float64)])
+def test_lanes_share_the_slots_of_an_atom(checkers, natoms, level, dt):
+    """Structures of a size for 8, 4, 2 and 1 lanes per atom and for contraction tiles of 16 and 32 atoms, the last tile ragged, some
+    atoms at an open side with few neighbours; fp32 against the model in double precision (every input is a single)."""
+    rng = np.random.default_rng(natoms)
+    edge = int(np.ceil(natoms ** (1 / 3) - 1e-9))
+    cell, pos = synth.cubic_lattice(max(edge, 4), 3.0, 0.1, rng, np.float64, nocc=natoms)
+    w = util.small_mtp_case(level, 2, dt)
+    w.update(cell=cell, coords=pos.astype(dt).astype(np.float64), types=rng.integers(0, 3, natoms).astype(np.int32))
+    chk = _chk(checkers)
+    nb = util.nblist_batch(chk, w)
+    if dt == np.float32:
+        nb["brcs"] = nb["brcs"].astype(dt)
+    (e, f, v), *_ = _run(w, nb)
+    model = util.to64(w["model"])
+    er, fr, vr = chk.mtp_efv(model, dict(nb, brcs=nb["brcs"].astype(np.float64)))
+    for a, r, name in ((e, er, "energy"), (f, fr, "force"), (v, vr, "virial")):
+        assert util.relerr(a, r) < TOL[dt], name
+
+
 def test_many_neighbours_and_ragged_batch(checkers):
     """> 32 neighbours per atom (two lane chunks), padded batch with an empty structure and ghosts."""
     chk = _chk(checkers)
