@@ -4,26 +4,32 @@
 // (ai2pot/models/potential_utils.py:217-268). Here everything but the positions is described once; a call then is
 // the neighbour build and the evaluation back to back, with no argument handling in between: at a few hundred atoms
 // the host's share of a call through two separate entry points (50 us) exceeded the device's (31 us).
-#include "common.cuh"
+#include "nep_setup.cuh"
 
 using namespace ai2b;
+
+namespace ai2b {
+template <typename T>
+int nblist_build_periodic(int n, const T *h_cell, const T *d_coords, double rcut, int umax, int *d_numneigh, int *d_firstneigh, T *d_rcs, int *d_status,
+                          void *ws, size_t ws_bytes, cudaStream_t st, const NepSetup &side);
+}
 
 template <typename T>
 static int evaluate_t(const ai2b_evaluation *e, const T *coords, void *stream)
 {
-    const int pbc[3] = {1, 1, 1};
     T cell[9];
     for (int k = 0; k < 9; k++) cell[k] = (T)e->cell[k];
-    int rc;
-    if constexpr (sizeof(T) == 8)
-        rc = ai2b_nblist_build_f64(e->natoms, cell, coords, 1, e->rcut, pbc, e->umax, e->d_numneigh, e->d_firstneigh, (T *)e->d_rcs, e->d_status,
-                                   e->d_nblist_workspace, e->nblist_workspace_bytes, stream);
-    else
-        rc = ai2b_nblist_build_f32(e->natoms, cell, coords, 1, e->rcut, pbc, e->umax, e->d_numneigh, e->d_firstneigh, (T *)e->d_rcs, e->d_status,
-                                   e->d_nblist_workspace, e->nblist_workspace_bytes, stream);
-    if (rc != AI2B_OK) return rc;
+    cudaStream_t st = (cudaStream_t)stream;
     T *etot = (T *)e->d_etot, *force = (T *)e->d_force, *virial = (T *)e->d_virial;
     const T *co = (const T *)e->d_coeffs, *bias = (const T *)e->d_type_bias, *qs = (const T *)e->d_q_scaler, *rcs = (const T *)e->d_rcs;
+    const T *w0 = (const T *)e->d_w0, *b0 = (const T *)e->d_b0, *w1 = (const T *)e->d_w1;
+    // what the evaluation has to set up goes out with a launch of the build
+    NepSetup side;
+    const bool carried = !e->mtp && nep_plan_setup<T>(etot, force, virial, e->chebyshev_size, e->n_radial, e->n_angular, e->l_max, e->num_neurons, co,
+                                                      w0, b0, w1, e->natoms, e->d_binum, e->ntypes, e->umax, 0, qs, e->d_workspace, e->workspace_bytes, &side);
+    if (int rc = nblist_build_periodic<T>(e->natoms, cell, coords, e->rcut, e->umax, e->d_numneigh, e->d_firstneigh, (T *)e->d_rcs, e->d_status,
+                                          e->d_nblist_workspace, e->nblist_workspace_bytes, st, side))
+        return rc;
     if (e->mtp) {
         const T *lin = (const T *)e->d_linear_coeffs;
         if constexpr (sizeof(T) == 8)
@@ -35,7 +41,10 @@ static int evaluate_t(const ai2b_evaluation *e, const T *coords, void *stream)
                                     e->d_numneigh, e->d_firstneigh, rcs, e->d_types, e->ntypes, e->umax, 0, (T)e->rmax, (T)e->rmin, qs,
                                     e->d_workspace, e->workspace_bytes, stream);
     }
-    const T *w0 = (const T *)e->d_w0, *b0 = (const T *)e->d_b0, *w1 = (const T *)e->d_w1;
+    if (carried)
+        return nep_efv_prepared<T>(etot, force, virial, e->chebyshev_size, e->n_radial, e->n_angular, e->l_max, e->num_neurons, co, w0, b0, w1, bias,
+                                   e->natoms, e->d_binum, e->d_ilist, e->d_numneigh, e->d_firstneigh, rcs, e->d_types, e->ntypes, e->umax, 0, (T)e->rmax,
+                                   (T)e->rmax_angular, qs, e->d_workspace, e->workspace_bytes, st);
     if constexpr (sizeof(T) == 8)
         return ai2b_nep_efv_f64(etot, force, virial, e->chebyshev_size, e->n_radial, e->n_angular, e->l_max, e->num_neurons, co, w0, b0, w1, bias, 1,
                                 e->natoms, e->d_binum, e->d_ilist, e->d_numneigh, e->d_firstneigh, rcs, e->d_types, e->ntypes, e->umax, 0, e->rmax,

@@ -14,9 +14,9 @@
 // A step's host work: one pass over the positions that copies them into pinned memory and finds their extent (so the
 // bin grid is known on the host and the build needs no look at the atoms first), sent off in pieces that travel while the
 // next piece is copied; one transfer back of [forces | energy, virial | status]; one pass that adds the forces. 13,824 local
-// and 11,415 ghost atoms, NEP: 188 us per step (about 50 copying, 68 waiting for the device, 24 taking the forces), where pageable
-// transfers array by array, a device pass over the extents and a scalar loop over the forces took 355 us.
-#include "common.cuh"
+// and 11,415 ghost atoms, NEP: 164 us per step, where pageable transfers array by array, a device pass over the extents and a scalar
+// loop over the forces took 355 us.
+#include "nep_setup.cuh"
 
 #include <cstring>
 #if defined(__SSE2__)
@@ -27,7 +27,7 @@ using namespace ai2b;
 
 namespace ai2b {
 int nblist_build_rows32(int n, int ncentres, const double *h_cell, const double *d_coords, double rcut, const int *h_pbc, const double *open_ext, int umax,
-                        int *d_numneigh, int *d_firstneigh, float *d_rcs, int *d_status, void *ws, size_t ws_bytes, cudaStream_t st);
+                        int *d_numneigh, int *d_firstneigh, float *d_rcs, int *d_status, void *ws, size_t ws_bytes, cudaStream_t st, const NepSetup &side);
 }
 
 // Positions travel in pieces of this many atoms, MD_SLOTS of which have a place in pinned memory. Pinning costs 0.9 to 2.9 ms per
@@ -133,7 +133,7 @@ int common_init(ai2b_md_session *s)
     return AI2B_OK;
 }
 
-// dst = src for n positions; the lowest and highest coordinates are folded into lo and hi
+// dst = src for n positions; the lowest and highest coordinates are folded into lo and hi.
 void copy_and_bound(double *dst, const double *src, size_t n, double *lo, double *hi)
 {
     size_t i = 0;
@@ -289,11 +289,19 @@ static int session_step(ai2b_md_session *s, int nlocal, int nghost, const double
     const double cell[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};   // no periodic axis: only the extents of the atoms matter
     const int pbc[3] = {0, 0, 0};
     const double ext[6] = {lo[0], lo[1], lo[2], hi[0], hi[1], hi[2]};
-    int rc = nblist_build_rows32(nall, nlocal, cell, d_pos, s->rcut, pbc, ext, s->umax, s->d_numneigh, s->d_firstneigh, s->d_rcs, d_status, s->d_nbws,
-                                 s->nbws, st);
-    if (rc) return rc;
     float *d_vir = want_virial ? d_ev + 1 : nullptr;
-    if (s->kind == 0)
+    // what the evaluation has to set up goes out with a launch of the build
+    NepSetup side;
+    const bool carried = s->kind == 0 && nep_plan_setup<float>(d_ev, d_force, d_vir, s->cs, s->n_r, s->n_a, s->l_max, s->nneu, s->d_coeffs, s->d_w0, s->d_b0,
+                                                               s->d_w1, nlocal, d_binum, s->ntypes, s->umax, nghost, s->d_qs, s->d_ws, s->ws, &side);
+    int rc = nblist_build_rows32(nall, nlocal, cell, d_pos, s->rcut, pbc, ext, s->umax, s->d_numneigh, s->d_firstneigh, s->d_rcs, d_status, s->d_nbws,
+                                 s->nbws, st, side);
+    if (rc) return rc;
+    if (carried)
+        rc = nep_efv_prepared<float>(d_ev, d_force, d_vir, s->cs, s->n_r, s->n_a, s->l_max, s->nneu, s->d_coeffs, s->d_w0, s->d_b0, s->d_w1, s->d_bias,
+                                     nlocal, d_binum, s->d_ilist, s->d_numneigh, s->d_firstneigh, s->d_rcs, d_types, s->ntypes, s->umax, nghost, s->rc_r,
+                                     s->rc_a, s->d_qs, s->d_ws, s->ws, st);
+    else if (s->kind == 0)
         rc = ai2b_nep_efv_f32(d_ev, d_force, d_vir, s->cs, s->n_r, s->n_a, s->l_max, s->nneu, s->d_coeffs, s->d_w0, s->d_b0, s->d_w1,
                               s->d_bias, 1, nlocal, d_binum, s->d_ilist, s->d_numneigh, s->d_firstneigh, s->d_rcs, d_types, s->ntypes,
                               s->umax, nghost, s->rc_r, s->rc_a, s->d_qs, s->d_ws, s->ws, st);

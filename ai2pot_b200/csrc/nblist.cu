@@ -17,7 +17,7 @@
 // range of atoms: the table of a bin holds 9 ranges (plus the wrapped remainders next to a periodic face).
 // Binning is one launch of one block for systems of up to 2,048 atoms, else a chain of set-up, count, scan and fill
 // (launch_chained() in common.cuh).
-#include "common.cuh"
+#include "nep_setup.cuh"
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -297,8 +297,14 @@ template <typename T>
 __global__ void __launch_bounds__(BINB_THREADS, 1)
 nb_bin_block_kernel(NbParams<T> P, NbGrid host_grid, int have_grid, const T *__restrict__ coords, NbGrid *__restrict__ gp,
                     int *__restrict__ bin_start, typename Vec4<T>::type *__restrict__ spos, float4 *__restrict__ sposw,
-                    int4 *__restrict__ sinfo, int *__restrict__ status)
+                    int4 *__restrict__ sinfo, int *__restrict__ status, const NepSetup side)
 {
+    if (blockIdx.x > 0) {      // blocks of another kernel's set-up
+        chain_release();
+        chain_wait();
+        nep_setup_any(side, blockIdx.x - 1);
+        return;
+    }
     __shared__ int cnt[BINB_MAX_BINS];           // counters, then the starts of the bins
     __shared__ int ws[32];
     __shared__ double wext[32][6], bext[6];
@@ -514,8 +520,14 @@ template <typename T, bool SCAN>
 __global__ void __launch_bounds__(FILL_THREADS)
 nb_fill_kernel(NbParams<T> P, const T *__restrict__ coords, const int2 *__restrict__ ainfo, const int *__restrict__ bin_count,
                int *__restrict__ bin_start, typename Vec4<T>::type *__restrict__ spos, float4 *__restrict__ sposw, int4 *__restrict__ sinfo,
-               const NbGrid *__restrict__ gp)
+               const NbGrid *__restrict__ gp, int own, const NepSetup side)
 {
+    if ((int)blockIdx.x >= own) {      // blocks of another kernel's set-up
+        chain_release();
+        chain_wait();
+        nep_setup_any(side, blockIdx.x - own);
+        return;
+    }
     __shared__ int s_start[SCAN ? FILL_SCAN_BINS : 1];
     __shared__ int ws[32];
     chain_release();
@@ -1012,7 +1024,7 @@ static int launch_rows(const NbParams<T> &P, const NbGrid *grid, const int *star
 template <typename T, typename TO = T>
 static int nblist_build(int n, int ncentre, const T *h_cell, const T *d_coords, int is_cart, double rcut_in, const int *pbc, int umax,
                         int *d_numneigh, int *d_firstneigh, TO *d_rcs, int *d_status, void *ws, size_t ws_bytes, cudaStream_t st,
-                        int cbegin = 0, bool reuse_bins = false, const double *open_ext = nullptr)
+                        int cbegin = 0, bool reuse_bins = false, const double *open_ext = nullptr, const NepSetup &side = NepSetup())
 {
     AI2B_REQUIRE(h_cell && pbc && d_status, AI2B_ERR_INVALID, "ai2b_nblist_build: NULL argument");
     AI2B_REQUIRE(n >= 0 && umax >= 0 && rcut_in > 0 && ncentre >= 0 && ncentre <= n && cbegin >= 0 && cbegin <= ncentre,
@@ -1098,8 +1110,8 @@ static int nblist_build(int n, int ncentre, const T *h_cell, const T *d_coords, 
     if (reuse_bins) {
         // bins and bin-ordered positions are in the workspace already
     } else if (n <= BINB_MAX_ATOMS) {
-        AI2B_CUDA(launch_chained(nb_bin_block_kernel<T>, 1, BINB_THREADS, 0, st, P, hg, host_grid ? 1 : 0, d_coords, grid, start, spos, sposw,
-                                 sinfo, d_status));
+        AI2B_CUDA(launch_chained(nb_bin_block_kernel<T>, 1 + side.blocks, BINB_THREADS, 0, st, P, hg, host_grid ? 1 : 0, d_coords, grid, start, spos, sposw,
+                                 sinfo, d_status, side));
     } else {
         const int nblk = (n + FILL_THREADS - 1) / FILL_THREADS;
         if (host_grid) {
@@ -1114,10 +1126,12 @@ static int nblist_build(int n, int ncentre, const T *h_cell, const T *d_coords, 
         }
         AI2B_CUDA(launch_chained(nb_count_kernel<T>, nblk, FILL_THREADS, 0, st, P, grid, d_coords, ainfo, count));
         if ((host_grid ? prod : (long)maxbins) <= FILL_SCAN_BINS) {
-            AI2B_CUDA(launch_chained(nb_fill_kernel<T, true>, nblk, FILL_THREADS, 0, st, P, d_coords, ainfo, count, start, spos, sposw, sinfo, grid));
+            AI2B_CUDA(launch_chained(nb_fill_kernel<T, true>, nblk + side.blocks, FILL_THREADS, 0, st, P, d_coords, ainfo, count, start, spos, sposw, sinfo, grid,
+                                     nblk, side));
         } else {
             AI2B_CUDA(launch_chained(nb_scan_kernel, SCAN_CLUSTER, SCAN_BLOCK, 0, st, grid, count, start));
-            AI2B_CUDA(launch_chained(nb_fill_kernel<T, false>, nblk, FILL_THREADS, 0, st, P, d_coords, ainfo, count, start, spos, sposw, sinfo, grid));
+            AI2B_CUDA(launch_chained(nb_fill_kernel<T, false>, nblk + side.blocks, FILL_THREADS, 0, st, P, d_coords, ainfo, count, start, spos, sposw, sinfo, grid,
+                                     nblk, side));
         }
     }
     // rows leave as 16-byte stores when they start on 16-byte boundaries and one warp's row fits its share of shared memory
@@ -1426,13 +1440,25 @@ static int nblist_build_batch(int B, int npad, const int *d_binum, const T *d_ce
     return AI2B_OK;
 }
 
-// rows in single precision from double positions; open_ext (optional): lowest and highest fractional coordinates
+// Builds that carry the set-up of the kernel that reads the rows (nep_setup.cuh), as blocks of the last binning launch.
+// Rows in single precision from double positions; open_ext: lowest and highest fractional coordinates.
 int nblist_build_rows32(int n, int ncentres, const double *h_cell, const double *d_coords, double rcut, const int *h_pbc, const double *open_ext, int umax,
-                        int *d_numneigh, int *d_firstneigh, float *d_rcs, int *d_status, void *ws, size_t ws_bytes, cudaStream_t st)
+                        int *d_numneigh, int *d_firstneigh, float *d_rcs, int *d_status, void *ws, size_t ws_bytes, cudaStream_t st, const NepSetup &side)
 {
     return nblist_build<double, float>(n, ncentres, h_cell, d_coords, 1, rcut, h_pbc, umax, d_numneigh, d_firstneigh, d_rcs, d_status, ws, ws_bytes, st, 0,
-                                       false, open_ext);
+                                       false, open_ext, side);
 }
+template <typename T>
+int nblist_build_periodic(int n, const T *h_cell, const T *d_coords, double rcut, int umax, int *d_numneigh, int *d_firstneigh, T *d_rcs, int *d_status,
+                          void *ws, size_t ws_bytes, cudaStream_t st, const NepSetup &side)
+{
+    const int pbc[3] = {1, 1, 1};
+    return nblist_build<T>(n, n, h_cell, d_coords, 1, rcut, pbc, umax, d_numneigh, d_firstneigh, d_rcs, d_status, ws, ws_bytes, st, 0, false, nullptr, side);
+}
+template int nblist_build_periodic<double>(int, const double *, const double *, double, int, int *, int *, double *, int *, void *, size_t, cudaStream_t,
+                                           const NepSetup &);
+template int nblist_build_periodic<float>(int, const float *, const float *, double, int, int *, int *, float *, int *, void *, size_t, cudaStream_t,
+                                          const NepSetup &);
 
 }  // namespace ai2b
 

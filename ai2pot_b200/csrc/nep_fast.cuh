@@ -5,8 +5,9 @@
 // Same math as the general kernel (nep.h:320-529). A warp evaluates 32 / G atoms, G lanes each, and all of its lanes run the
 // same trip counts: with loops per group (8 lanes, own neighbour count) the four groups of a warp drift apart and every phase
 // is issued up to four times. What bounds it is instruction issue, so every phase is written for few instructions:
-//   * set-up: nep_prep_kernel lays the model out once per call (padded rows, signs and constants folded in) and zeroes the
-//     outputs; a block takes the table with a handful of 16-byte copies;
+//   * set-up (nep_setup.cuh): lays the model out once per call (padded rows, signs and constants folded in) and zeroes the
+//     outputs, in a launch of its own or as blocks of a launch of the neighbour build; a block takes the table with a handful
+//     of 16-byte copies;
 //   * radial pass, lanes = neighbours of the group's atom: Chebyshev sums of all functions and their derivatives in packed
 //     pairs, g'_n(r_j) / r_j are kept per neighbour in shared memory;
 //   * angular pass, lanes = angular neighbours of all atoms of the warp, back to back: only a fifth of the neighbours are
@@ -99,95 +100,6 @@ __device__ __forceinline__ void load_pk(const double *p, Pk<double> (&v)[N])
         const double2 t = reinterpret_cast<const double2 *>(p)[i];
         v[i].a = t.x; v[i].b = t.y;
     }
-}
-
-// padded descriptor count: rows of the network's first layer are 16-byte aligned and an odd
-// number of 16-byte chunks long (conflict-free when eight lanes read eight rows)
-template <int NMAX>
-struct NepFastDims {
-    static constexpr int ND = 5 * NMAX;                                   // >= n_r + n_a * l_max
-    static constexpr int NDP = ((ND / 4) & 1) ? ND : ND + 4;
-    static constexpr int CS = 8;                                          // Chebyshev rows
-    static constexpr int TROW = 2 * NMAX * CS + 4;                        // one type pair; rows of different pairs start in different banks
-    static constexpr int RS = NMAX + NEP_NLM + (NMAX == 8 ? 4 : 0);       // staging row: g[NMAX] | B_lm[24], conflict-free 16-byte stores
-    static constexpr int ESR = NMAX * NEP_NLM + 4;                        // adjoints of an atom's sums, [mu][24]
-};
-__host__ __device__ inline int nep_r4(int n) { return (n + 3) & ~3; }
-__host__ __device__ inline int nep_r32(int n) { return (n + 31) & ~31; }   // neurons per type, padded
-
-// The model as the kernel reads it (elements of T): Chebyshev rows [ti][tj][k][radial | angular], then (unless descriptors
-// only) first-layer rows [type][neuron][NDP], biases, second-layer weights, 1 / q_scaler
-template <int NMAX>
-struct NepTab {
-    int w0, b0, w1, iqs, total;
-    __host__ __device__ NepTab(int ntypes, int nneu, bool net)
-    {
-        using D = NepFastDims<NMAX>;
-        const int nrow = ntypes * nep_r32(nneu);
-        w0 = nep_r4(ntypes * ntypes * D::TROW);
-        b0 = w0 + (net ? nrow * D::NDP : 0);
-        w1 = b0 + (net ? nrow : 0);
-        iqs = w1 + (net ? nrow : 0);
-        total = iqs + (net ? nep_r4(D::NDP) : 0);
-    }
-};
-
-// One launch in front of the kernel: the table, the structures' atom offsets, zeroed outputs.
-// Row 0 of a function holds 2 c_0 + sum_k c_k (the constant part of sum c_k (T_k + 1)); row k holds s_k c_k with the signs
-// s = + + - - + + - -, which turn the recurrences T_k+1 = 2 x T_k - T_k-1 and T'_k+1 = 2 T_k + 2 x T'_k - T'_k-1 into sums.
-template <typename T, int NMAX>
-__global__ void nep_prep_kernel(const NepArgs<T> A, const T *__restrict__ coeffs, T *__restrict__ tab, int *__restrict__ prefix, int net, int tab_blocks,
-                                T *__restrict__ z0, size_t n0, T *__restrict__ z1, size_t n1, T *__restrict__ z2, size_t n2)
-{
-    using D = NepFastDims<NMAX>;
-    chain_release();
-    chain_wait();
-    if ((int)blockIdx.x < tab_blocks) {
-        const NepTab<NMAX> L(A.ntypes, A.nneu, net != 0);
-        const int NP = nep_r32(A.nneu), nfun = A.n_r + A.n_a;
-        if (blockIdx.x == 0 && A.B > 1 && threadIdx.x < 32) {      // exclusive sum of the structures' sizes
-            int carry = 0;
-            for (int b0 = 0; b0 < A.B; b0 += 32) {
-                const int b = b0 + threadIdx.x;
-                int inc = b < A.B ? A.binum[b] : 0;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(FULL_MASK, inc, o); if ((int)threadIdx.x >= o) inc += v; }
-                if (b < A.B) prefix[b + 1] = carry + inc;
-                carry += __shfl_sync(FULL_MASK, inc, 31);
-            }
-            if (threadIdx.x == 0) prefix[0] = 0;
-        }
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < L.total; i += tab_blocks * blockDim.x) {
-            T v = T(0);
-            if (i < L.w0) {
-                const int pair = i / D::TROW, o = i % D::TROW, k = o / (2 * NMAX), f = o % (2 * NMAX);
-                const int row = f < NMAX ? (f < A.n_r ? f : -1) : (f - NMAX < A.n_a ? A.n_r + f - NMAX : -1);
-                if (pair < A.ntypes * A.ntypes && k < A.cs && row >= 0) {
-                    const T *c = coeffs + ((size_t)pair * nfun + row) * A.cs;
-                    if (k == 0) {
-                        v = T(2) * c[0];
-                        for (int q = 1; q < A.cs; q++) v += c[q];
-                    } else {
-                        v = (k & 2) ? -c[k] : c[k];
-                    }
-                }
-            } else if (i < L.b0) {
-                const int row = (i - L.w0) / D::NDP, k = (i - L.w0) % D::NDP, t = row / NP, p = row % NP;
-                if (k < A.nd && p < A.nneu) v = A.w0[((size_t)t * A.nneu + p) * A.nd + k];
-            } else if (i < L.iqs) {
-                const int row = (i - L.b0) % (A.ntypes * NP), t = row / NP, p = row % NP;
-                if (p < A.nneu) v = (i < L.w1 ? A.b0 : A.w1)[t * A.nneu + p];
-            } else if (i - L.iqs < A.nd) {
-                v = T(1) / A.qs[i - L.iqs];
-            }
-            tab[i] = v;
-        }
-        return;
-    }
-    const size_t i0 = (size_t)(blockIdx.x - tab_blocks) * blockDim.x + threadIdx.x, step = (size_t)(gridDim.x - tab_blocks) * blockDim.x;
-    for (size_t i = i0; i < n0; i += step) z0[i] = T(0);
-    for (size_t i = i0; i < n1; i += step) z1[i] = T(0);
-    for (size_t i = i0; i < n2; i += step) z2[i] = T(0);
 }
 
 // 1 / sqrt(v) with a Newton step behind the hardware's estimate in single precision

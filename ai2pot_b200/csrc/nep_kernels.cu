@@ -14,7 +14,7 @@
 //   4. force passes: radial  g = (sum_n dE/dq_n g'_n) u;
 //      angular g = sum_mu [ g'_mu P u + g_mu/r (G - (u.G) u) ],  P = sum_lm e_lm B_lm(u),
 //      G = sum_lm e_lm grad B_lm(u);  F_i += g, F_j -= g, V -= g (x) r
-#include "common.cuh"
+#include "nep_setup.cuh"
 #include <cuda_pipeline.h>
 
 #include <cstring>
@@ -26,7 +26,6 @@ constexpr int NEP_GROUP = 8;                  // lanes per atom
 constexpr int NEP_APW = 32 / NEP_GROUP;       // atoms per warp
 constexpr int NEP_WARPS = 4;
 constexpr int NEP_APB = NEP_APW * NEP_WARPS;  // atoms per block
-constexpr int NEP_NLM = 24;
 
 enum NepMode { NEP_EFV = 0, NEP_EF = 1, NEP_DESC = 2 };
 
@@ -41,6 +40,7 @@ struct NepArgs {
     int B, npad, ntypes, umax, nghost, cs, n_r, n_a, l_max, nneu, nd, nS;
     T rc_r, rc_a;
     int zero = 0;          // the outputs are zeroed before anything is added to them
+    int prepared = 0;      // the set-up has been done by an earlier launch of the chain (one structure, specialised kernel)
 };
 
 // 3-body coefficients as the reference stores them: double literals, some written with an `f`
@@ -591,29 +591,52 @@ static int launch_nep_fast_g(const NepArgs<T> &A, const T *tab, const NepTab<NMA
     return AI2B_OK;
 }
 
-// Specialised kernel for n_radial, n_angular <= NMAX. *done = false if the model's tables, the neighbour width or the
-// workspace do not fit its plan (the general kernel then runs).
+// The set-up launch of the specialised kernel, alone
+__global__ void __launch_bounds__(NEP_SETUP_THREADS) nep_prep_kernel(const NepSetup S)
+{
+    chain_release();
+    chain_wait();
+    nep_setup_any(S, blockIdx.x);
+}
+
+// Set-up of a call of the specialised kernel and its lanes per atom. 0: the model's tables, the neighbour width or the workspace
+// do not fit its plan (the general kernel then runs).
+template <typename T, int NMAX>
+static int nep_fast_plan(const NepArgs<T> &A, bool net, const T *coeffs, void *ws, size_t ws_bytes, NepSetup *S)
+{
+    const int lanes = nep_fast_lanes<T, NMAX>((long)A.B * A.npad, A.ntypes, A.nneu, A.umax, net);
+    const NepTab<NMAX> L(A.ntypes, A.nneu, net);
+    // (the table is copied 16 bytes at a time; a workspace that does not start on such a boundary has room for the difference)
+    const size_t at = nep_prefix_bytes(A.B), shift = (16 - (reinterpret_cast<size_t>(ws) + at) % 16) % 16;
+    if (lanes == 0 || at + shift + (size_t)L.total * sizeof(T) > ws_bytes) return 0;
+    S->tab_blocks = (L.total + 4 * NEP_SETUP_THREADS - 1) / (4 * NEP_SETUP_THREADS);
+    S->wide = NMAX == 8; S->is_f64 = sizeof(T) == 8; S->net = net;
+    S->ntypes = A.ntypes; S->n_r = A.n_r; S->n_a = A.n_a; S->cs = A.cs; S->nneu = A.nneu; S->nd = A.nd; S->B = A.B;
+    S->binum = A.binum; S->prefix = reinterpret_cast<int *>(ws);
+    S->coeffs = coeffs; S->w0 = A.w0; S->b0 = A.b0; S->w1 = A.w1; S->qs = A.qs;
+    S->tab = reinterpret_cast<unsigned char *>(ws) + at + shift;
+    T *z[3] = {net ? A.etot : A.desc, A.force, A.virial};
+    const size_t nz[3] = {net ? (size_t)A.B : (size_t)A.B * A.npad * A.nd, net ? 3 * (size_t)A.B * (A.npad + A.nghost) : 0, A.virial ? 9 * (size_t)A.B : 0};
+    size_t total = 0;
+    for (int k = 0; k < 3; k++) { S->z[k] = z[k]; S->nz[k] = A.zero ? nz[k] : 0; total += S->nz[k]; }
+    size_t zb = (total + 4 * NEP_SETUP_THREADS - 1) / (4 * NEP_SETUP_THREADS);
+    if (zb > 4096) zb = 4096;
+    S->blocks = S->tab_blocks + (int)zb;
+    return lanes;
+}
+
+// *done = false if the specialised kernel for n_radial, n_angular <= NMAX does not take the call
 template <typename T, int MODE, int NMAX>
 static int launch_nep_fast(NepArgs<T> A, const T *coeffs, void *ws, size_t ws_bytes, cudaStream_t st, bool *done)
 {
     constexpr bool NET = MODE != NEP_DESC;
     *done = false;
-    const int lanes = nep_fast_lanes<T, NMAX>((long)A.B * A.npad, A.ntypes, A.nneu, A.umax, NET);
+    NepSetup S;
+    const int lanes = nep_fast_plan<T, NMAX>(A, NET, coeffs, ws, ws_bytes, &S);
+    if (lanes == 0) return AI2B_OK;
     const NepTab<NMAX> L(A.ntypes, A.nneu, NET);
-    // (the table is copied 16 bytes at a time; a workspace that does not start on such a boundary has room for the difference)
-    const size_t at = nep_prefix_bytes(A.B), shift = (16 - (reinterpret_cast<size_t>(ws) + at) % 16) % 16;
-    if (lanes == 0 || at + shift + (size_t)L.total * sizeof(T) > ws_bytes) return AI2B_OK;
-    T *tab = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(ws) + at + shift);
-    {   // table, offsets, zeroed outputs
-        T *z[3] = {NET ? A.etot : A.desc, A.force, A.virial};
-        const size_t nz[3] = {NET ? (size_t)A.B : (size_t)A.B * A.npad * A.nd, NET ? 3 * (size_t)A.B * (A.npad + A.nghost) : 0, A.virial ? 9 * (size_t)A.B : 0};
-        const size_t nzero = A.zero ? nz[0] + nz[1] + nz[2] : 0;
-        size_t zb = (nzero + 4 * 256 - 1) / (4 * 256);
-        if (zb > 4096) zb = 4096;
-        const int tb = (L.total + 4 * 256 - 1) / (4 * 256);
-        AI2B_CUDA(launch_chained(nep_prep_kernel<T, NMAX>, (unsigned)(tb + zb), 256, 0, st, A, coeffs, tab, const_cast<int *>(A.prefix), NET ? 1 : 0, tb,
-                                 z[0], A.zero ? nz[0] : 0, z[1], A.zero ? nz[1] : 0, z[2], A.zero ? nz[2] : 0));
-    }
+    const T *tab = static_cast<const T *>(S.tab);
+    if (!A.prepared) AI2B_CUDA(launch_chained(nep_prep_kernel, (unsigned)S.blocks, NEP_SETUP_THREADS, 0, st, S));
     *done = true;
     if constexpr (NET && NMAX == 4 && sizeof(T) == 4)
         if (lanes == 4) return launch_nep_fast_g<T, MODE, NMAX, 4>(A, tab, L, st);
@@ -677,6 +700,41 @@ static int launch_nep(NepArgs<T> A, const T *coeffs, void *ws, size_t ws_bytes, 
     if (A.cs <= 8) return launch_nep_csp<T, 8, MODE>(A, coeffs, ws, ws_bytes, st);
     return launch_nep_csp<T, 16, MODE>(A, coeffs, ws, ws_bytes, st);
 }
+
+template <typename T>
+bool nep_plan_setup(T *etot, T *force, T *virial, int cs, int n_r, int n_a, int l_max, int nneu, const T *coeffs, const T *w0, const T *b0,
+                    const T *w1, int npad, const int *binum, int ntypes, int umax, int nghost, const T *qs, void *ws, size_t ws_bytes, NepSetup *out)
+{
+    // what ai2b_nep_efv_* refuses is left to it
+    if (!etot || !force || !coeffs || !w0 || !b0 || !w1 || !qs || !binum || !ws) return false;
+    if (cs < 1 || cs > 8 || l_max < 0 || l_max > 4 || n_r < 0 || n_a < 0 || n_r + n_a < 1 || n_r > 8 || n_a > 8 || nneu < 1 || ntypes < 1 ||
+        npad < 1 || umax < 0 || umax >= 65536 || nghost < 0 || ws_bytes < nep_ws_min(1, ntypes, n_r, n_a, 8, sizeof(T)))
+        return false;
+    NepArgs<T> A{etot, force, virial, nullptr, nullptr, w0, b0, w1, nullptr, qs, binum};
+    A.B = 1; A.npad = npad; A.ntypes = ntypes; A.umax = umax; A.nghost = nghost; A.cs = cs; A.n_r = n_r; A.n_a = n_a; A.nneu = nneu;
+    A.nd = l_max == 0 ? n_r : n_r + n_a * l_max;
+    A.zero = 1;
+    return (n_r <= 4 && n_a <= 4 ? nep_fast_plan<T, 4>(A, true, coeffs, ws, ws_bytes, out) : nep_fast_plan<T, 8>(A, true, coeffs, ws, ws_bytes, out)) != 0;
+}
+template <typename T>
+int nep_efv_prepared(T *etot, T *force, T *virial, int cs, int n_r, int n_a, int l_max, int nneu, const T *coeffs, const T *w0, const T *b0,
+                     const T *w1, const T *bias, int npad, const int *binum, const int *bilist, const int *numneigh, const int *firstneigh,
+                     const T *rcs, const int *types, int ntypes, int umax, int nghost, T rc_r, T rc_a, const T *qs, void *ws, size_t ws_bytes,
+                     cudaStream_t st)
+{
+    AI2B_REQUIRE(bias && bilist && numneigh && firstneigh && rcs && types, AI2B_ERR_INVALID, "ai2b_nep_efv: NULL argument");
+    NepArgs<T> A{etot, force, virial, nullptr, nullptr, w0, b0, w1, bias, qs, binum, bilist, numneigh, firstneigh, types, rcs, nullptr,
+                 1, npad, ntypes, umax, nghost, cs, n_r, n_a, l_max, nneu, 0, 0, rc_r, rc_a, 1, 1};
+    return virial ? launch_nep<T, NEP_EFV>(A, coeffs, ws, ws_bytes, st) : launch_nep<T, NEP_EF>(A, coeffs, ws, ws_bytes, st);
+}
+#define AI2B_NEP_PREPARED(T)                                                                                                                    \
+    template bool nep_plan_setup<T>(T *, T *, T *, int, int, int, int, int, const T *, const T *, const T *, const T *, int, const int *, int,     \
+                                    int, int, const T *, void *, size_t, NepSetup *);                                                           \
+    template int nep_efv_prepared<T>(T *, T *, T *, int, int, int, int, int, const T *, const T *, const T *, const T *, const T *, int,          \
+                                     const int *, const int *, const int *, const int *, const T *, const int *, int, int, int, T, T, const T *, \
+                                     void *, size_t, cudaStream_t);
+AI2B_NEP_PREPARED(double)
+AI2B_NEP_PREPARED(float)
 
 }  // namespace ai2b
 

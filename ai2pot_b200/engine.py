@@ -209,11 +209,12 @@ class Evaluator:
     def launches_per_step(self):
         """Kernels of this library that one compute() on a fully periodic cell launches (memsets not counted): neighbour build,
         then forward, contraction and force of MTP (and a set-up launch when the radial coefficient rows have to be padded to
-        eight entries), or those of NEP."""
+        eight entries), or those of NEP (whose set-up goes out with a launch of the build)."""
         build = capi.nblist_build_launches(self.n, self.cell, self.rcut)
         if self.kind == "mtp":
             return build + 3 + (0 if int(self.model["chebyshev_size"]) == 8 else 1)
-        return build + capi.nep_efv_launches(self.model, self.n, self.umax, self.dtype)
+        efv = capi.nep_efv_launches(self.model, self.n, self.umax, self.dtype)
+        return build + (1 if efv == 2 else efv)
 
     def cell_heights(self):
         """Distances between opposite faces of the cell."""
