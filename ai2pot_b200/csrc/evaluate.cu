@@ -80,8 +80,11 @@ extern "C" int ai2b_chained_copy(void *dst, const void *src, size_t bytes, void 
 {
     if (bytes == 0) return AI2B_OK;
     AI2B_REQUIRE(dst && src, AI2B_ERR_INVALID, "ai2b_chained_copy: NULL argument");
-    size_t blocks = (bytes + 16 * 256 - 1) / (16 * 256);
+    // Few blocks: every SM that takes part has to reach the host's memory first (14 KB in one block of 1,024 threads or in four of
+    // 256: a recorded call of 1,157 atoms 27.1 against 28.7 us, and its time depends less on where the blocks land)
+    constexpr int THREADS = 1024;
+    size_t blocks = (bytes + 16 * THREADS - 1) / (16 * THREADS);
     if (blocks > 148) blocks = 148;
-    AI2B_CUDA(launch_chained(chained_copy_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, (unsigned char *)dst, (const unsigned char *)src, bytes));
+    AI2B_CUDA(launch_chained(chained_copy_kernel, (unsigned)blocks, THREADS, 0, (cudaStream_t)stream, (unsigned char *)dst, (const unsigned char *)src, bytes));
     return AI2B_OK;
 }
