@@ -14,6 +14,12 @@ int nblist_build_periodic(int n, const T *h_cell, const T *d_coords, double rcut
                           void *ws, size_t ws_bytes, cudaStream_t st, const NepSetup &side);
 }
 
+static bool apart(const void *a, size_t na, const void *b, size_t nb)
+{
+    const size_t x = reinterpret_cast<size_t>(a), y = reinterpret_cast<size_t>(b);
+    return x + na <= y || y + nb <= x;
+}
+
 template <typename T>
 static int evaluate_t(const ai2b_evaluation *e, const T *coords, void *stream)
 {
@@ -23,10 +29,13 @@ static int evaluate_t(const ai2b_evaluation *e, const T *coords, void *stream)
     T *etot = (T *)e->d_etot, *force = (T *)e->d_force, *virial = (T *)e->d_virial;
     const T *co = (const T *)e->d_coeffs, *bias = (const T *)e->d_type_bias, *qs = (const T *)e->d_q_scaler, *rcs = (const T *)e->d_rcs;
     const T *w0 = (const T *)e->d_w0, *b0 = (const T *)e->d_b0, *w1 = (const T *)e->d_w1;
-    // what the evaluation has to set up goes out with a launch of the build
+    // What the evaluation has to set up goes out with a launch of the build, unless one buffer serves build and evaluation in turn
+    // (scratch of both, or positions that the forces replace).
     NepSetup side;
-    const bool carried = !e->mtp && nep_plan_setup<T>(etot, force, virial, e->chebyshev_size, e->n_radial, e->n_angular, e->l_max, e->num_neurons, co,
-                                                      w0, b0, w1, e->natoms, e->d_binum, e->ntypes, e->umax, 0, qs, e->d_workspace, e->workspace_bytes, &side);
+    bool carried = !e->mtp && apart(e->d_workspace, e->workspace_bytes, e->d_nblist_workspace, e->nblist_workspace_bytes) &&
+                   apart(force, 3 * sizeof(T) * (size_t)e->natoms, coords, 3 * sizeof(T) * (size_t)e->natoms);
+    carried = carried && nep_plan_setup<T>(etot, force, virial, e->chebyshev_size, e->n_radial, e->n_angular, e->l_max, e->num_neurons, co, w0, b0, w1,
+                                           e->natoms, e->d_binum, e->ntypes, e->umax, 0, qs, e->d_workspace, e->workspace_bytes, &side);
     if (int rc = nblist_build_periodic<T>(e->natoms, cell, coords, e->rcut, e->umax, e->d_numneigh, e->d_firstneigh, (T *)e->d_rcs, e->d_status,
                                           e->d_nblist_workspace, e->nblist_workspace_bytes, st, side))
         return rc;

@@ -87,6 +87,19 @@ def test_ordinary_launches_give_the_same(kind, monkeypatch):
     _close(again, chained, tol)
 
 
+@pytest.mark.parametrize("n", [8, 14])
+def test_build_and_evaluation_share_scratch(n):
+    """One buffer as the scratch of the neighbour build and of the evaluation, below and above the size from which atoms are binned
+    by several launches: the evaluation's set-up does not run ahead of the build then."""
+    w, dt, tol = _workload("nep", n)
+    ev = engine.Evaluator(w["model"], w["cell"], w["types"], w["rcut"], w["umax"], dt)
+    coords = torch.from_numpy(np.ascontiguousarray(w["coords"])).to(dt).cuda()
+    apart = _host(ev.compute(coords))
+    ev.ws = ev.nb_ws = torch.empty(max(ev.ws.numel(), ev.nb_ws.numel()), dtype=torch.uint8, device="cuda")
+    ev._filled = None
+    _close(_host(ev.compute(coords)), apart, tol)
+
+
 @pytest.mark.parametrize("kind", ["mtp", "nep"])
 def test_changed_attributes_take_effect(kind):
     """Cell, cutoff, row width and model may be edited or assigned between calls (a variable-cell relaxation does): the next
