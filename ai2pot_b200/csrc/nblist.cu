@@ -1166,15 +1166,17 @@ static int nblist_build(int n, int ncentre, const T *h_cell, const T *d_coords, 
 // structure's positions are staged through shared memory in tiles; one warp per centre:
 //   1. lanes = images: an image whose atoms (bounding box of the tile) cannot reach the centre is dropped. Of the 27
 //      images of a cell of 15 A about six are left at a cutoff of 6 A.
-//   2. lanes = atoms of the tile, single precision: triples that are certainly outside the cutoff are dropped, the others
-//      are queued in order
+//   2. lanes = atoms of the tile, single precision, |q_j|^2 - 2 q_i q_j < limit for two atoms at a time as in the rows kernel:
+//      triples that are certainly outside the cutoff are dropped, the others are queued in order
 //   3. lanes = queued triples: the exact predicate, in full warps
-// Testing every triple exactly (27 x 5 warp steps per centre in double precision) took 275 us for 64 structures of 64 to 256
-// atoms; this takes 40 us.
+// 64 structures of 64 to 256 atoms, 32 warps per SM: 32 us; with differences of coordinates, one atom per lane and step,
+// image numbers taken apart by divisions and 94 registers (two blocks per SM) 40 us and 2,000 warp instructions per centre; testing
+// every triple exactly 275 us.
 constexpr int NBB_WARPS = 8;
 constexpr int NBB_TILE = 512;       // atoms staged per tile
 constexpr int NBB_CPW = 2;          // centres per warp
 constexpr int NBB_CPB = NBB_WARPS * NBB_CPW;
+constexpr int NBB_MINB = 4;         // blocks per SM
 constexpr int NBB_QUEUE = 64;       // queued triples per warp: less than a warp's worth left over + one warp step
 
 template <typename T>
@@ -1186,17 +1188,17 @@ struct NbBatchParams {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(NBB_WARPS * 32)
+__global__ void __launch_bounds__(NBB_WARPS * 32, NBB_MINB)
 nb_batch_kernel(NbBatchParams<T> P, const int *__restrict__ binum, const T *__restrict__ cells, const T *__restrict__ coords,
                 int *__restrict__ bilist, int *__restrict__ bnumneigh, int *__restrict__ bfirstneigh, T *__restrict__ brcs,
                 int *__restrict__ status)
 {
     extern __shared__ __align__(16) unsigned char nbb_smem[];     // rows under construction (staged)
     __shared__ T s_pos[NBB_TILE * 3];
-    __shared__ float s_posf[NBB_TILE * 3];
+    __shared__ ulonglong2 s_cq[NBB_TILE];      // atoms e and e + 32 of every 64, relative to the first: 32 x {x, x', y, y'}, 32 x {z, z', q^2, q'^2}
     __shared__ T s_cell[9];
     __shared__ int s_e[3];
-    __shared__ float s_box[NBB_WARPS][6];
+    __shared__ float s_box[NBB_WARPS][7];
     __shared__ int s_queue[NBB_WARPS][NBB_QUEUE], s_img[NBB_WARPS][NBB_QUEUE];
     const int b = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1253,19 +1255,46 @@ nb_batch_kernel(NbBatchParams<T> P, const int *__restrict__ binum, const T *__re
         float c[9];
 #pragma unroll
         for (int k = 0; k < 9; k++) c[k] = (float)s_cell[k];
+        // image of lane l among the images g0 .. g0 + 31: packed numbers, shift in single precision
+        int im_packed = 0;
+        float im_x = 0.f, im_y = 0.f, im_z = 0.f;
+        auto set_image = [&](int g0) {
+            const int im = g0 + lane, i0 = im / (m1 * m2), i1 = (im / m2) % m1, i2 = im % m2;
+            const float f0 = (float)(i0 - e0), f1 = (float)(i1 - e1), f2 = (float)(i2 - e2);
+            im_packed = i0 | (i1 << 10) | (i2 << 20);      // (at most 2 * 499 + 1 images per axis)
+            im_x = f0 * c[0] + f1 * c[3] + f2 * c[6]; im_y = f0 * c[1] + f1 * c[4] + f2 * c[7]; im_z = f0 * c[2] + f1 * c[5] + f2 * c[8];
+        };
+        set_image(0);
         for (int t0 = 0; t0 < n; t0 += NBB_TILE) {
             const int tn = min(NBB_TILE, n - t0);
             __syncthreads();
-            float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
-            for (int j = threadIdx.x; j < tn; j += blockDim.x) {
-                T p[3];
-                cart(t0 + j, p[0], p[1], p[2]);
+            T org[3];
+            cart(t0, org[0], org[1], org[2]);
 #pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    const float f = (float)p[k];
-                    s_pos[3 * j + k] = p[k]; s_posf[3 * j + k] = f;
-                    lo[k] = fminf(lo[k], f); hi[k] = fmaxf(hi[k], f);
+            for (int k = 0; k < 3; k++) if (!(fabs((double)org[k]) < 1e15)) org[k] = T(0);      // an atom that has flown off
+            float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f}, n2max = 0.f;
+            for (int s = threadIdx.x; s < ((tn + 63) & ~63) / 2; s += blockDim.x) {
+                float q[2][4];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int j = (s & ~31) * 2 + (s & 31) + 32 * h;
+                    q[h][0] = q[h][1] = q[h][2] = 0.f; q[h][3] = 3e38f;      // (padding never passes)
+                    if (j < tn) {
+                        T p[3];
+                        cart(t0 + j, p[0], p[1], p[2]);
+#pragma unroll
+                        for (int k = 0; k < 3; k++) {
+                            const float f = (float)(p[k] - org[k]);
+                            s_pos[3 * j + k] = p[k]; q[h][k] = f;
+                            lo[k] = fminf(lo[k], f); hi[k] = fmaxf(hi[k], f);
+                        }
+                        q[h][3] = q[h][0] * q[h][0] + q[h][1] * q[h][1] + q[h][2] * q[h][2];
+                        n2max = fmaxf(n2max, q[h][3]);      // (an atom without a position is nobody's neighbour)
+                    }
                 }
+                ulonglong2 *dst = s_cq + 2 * (s & ~31) + (s & 31);
+                dst[0] = make_ulonglong2(pack2(q[0][0], q[1][0]), pack2(q[0][1], q[1][1]));
+                dst[32] = make_ulonglong2(pack2(q[0][2], q[1][2]), pack2(q[0][3], q[1][3]));
             }
 #pragma unroll
             for (int k = 0; k < 3; k++) {
@@ -1276,22 +1305,26 @@ nb_batch_kernel(NbBatchParams<T> P, const int *__restrict__ binum, const T *__re
                 }
                 if (lane == 0) { s_box[warp][k] = lo[k]; s_box[warp][3 + k] = hi[k]; }
             }
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1) n2max = fmaxf(n2max, __shfl_xor_sync(FULL_MASK, n2max, o));
+            if (lane == 0) s_box[warp][6] = n2max;
             __syncthreads();
             float reach = 0.f;
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 for (int w = 0; w < NBB_WARPS; w++) { lo[k] = fminf(lo[k], s_box[w][k]); hi[k] = fmaxf(hi[k], s_box[w][3 + k]); }
-                reach += fmaxf(fabsf(lo[k]), fabsf(hi[k])) + e0 * fabsf(c[k]) + e1 * fabsf(c[3 + k]) + e2 * fabsf(c[6 + k]);
+                reach += fmaxf(fabsf(lo[k]), fabsf(hi[k])) + fabsf((float)org[k]) + e0 * fabsf(c[k]) + e1 * fabsf(c[3 + k]) + e2 * fabsf(c[6 + k]);
             }
+            for (int w = 0; w < NBB_WARPS; w++) n2max = fmaxf(n2max, s_box[w][6]);
 #pragma unroll 1
             for (int q = 0; q < NBB_CPW; q++) {
                 const int i = c_begin + warp * NBB_CPW + q;
                 if (i >= n) continue;
                 T cx, cy, cz;
                 cart(i, cx, cy, cz);
-                const float fx = (float)cx, fy = (float)cy, fz = (float)cz;
+                const float fx = (float)(cx - org[0]), fy = (float)(cy - org[1]), fz = (float)(cz - org[2]);
                 // d^2 near the cutoff from single-precision coordinates no larger than `reach`: off by less than 64 eps reach rc
-                const float rmax = reach + fabsf(fx) + fabsf(fy) + fabsf(fz);
+                const float rmax = reach + fabsf((float)cx) + fabsf((float)cy) + fabsf((float)cz);
                 const float limit = ((float)P.rc2 + 64.f * 6e-8f * rmax * (float)P.rcut) * 1.000002f;
                 int *frow = staged ? rowi : bfirstneigh + ((size_t)b * P.npad + i) * P.umax;
                 T *rrow = staged ? rowp : brcs + ((size_t)b * P.npad + i) * P.umax * 3;
@@ -1304,7 +1337,7 @@ nb_batch_kernel(NbBatchParams<T> P, const int *__restrict__ binum, const T *__re
                     if (lane < m) {
                         j = s_queue[warp][lane];
                         const int img = s_img[warp][lane];
-                        const T f0 = T(img / (m1 * m2) - e0), f1 = T((img / m2) % m1 - e1), f2 = T(img % m2 - e2);
+                        const T f0 = T((img & 1023) - e0), f1 = T(((img >> 10) & 1023) - e1), f2 = T((img >> 20) - e2);
                         // this image's shift, applied in the reference's order ((r + a0 n0) + a1 n1) + a2 n2
                         const T ix = add_rn(add_rn(add_rn(s_pos[3 * j], mul_rn(s_cell[0], f0)), mul_rn(s_cell[3], f1)), mul_rn(s_cell[6], f2));
                         const T iy = add_rn(add_rn(add_rn(s_pos[3 * j + 1], mul_rn(s_cell[1], f0)), mul_rn(s_cell[4], f1)), mul_rn(s_cell[7], f2));
@@ -1335,30 +1368,42 @@ nb_batch_kernel(NbBatchParams<T> P, const int *__restrict__ binum, const T *__re
                 };
                 for (int g0 = 0; g0 < nimg; g0 += 32) {
                     // lanes = images: centre relative to the image, distance to the tile's bounding box
-                    const int im = g0 + lane;
-                    const float f0 = (float)(im / (m1 * m2) - e0), f1 = (float)((im / m2) % m1 - e1), f2 = (float)(im % m2 - e2);
-                    const float qx = fx - (f0 * c[0] + f1 * c[3] + f2 * c[6]), qy = fy - (f0 * c[1] + f1 * c[4] + f2 * c[7]),
-                                qz = fz - (f0 * c[2] + f1 * c[5] + f2 * c[8]);
+                    if (nimg > 32) set_image(g0);
+                    const float qx = fx - im_x, qy = fy - im_y, qz = fz - im_z;
                     const float gx = fmaxf(fmaxf(lo[0] - qx, qx - hi[0]), 0.f), gy = fmaxf(fmaxf(lo[1] - qy, qy - hi[1]), 0.f),
                                 gz = fmaxf(fmaxf(lo[2] - qz, qz - hi[2]), 0.f);
-                    unsigned near = __ballot_sync(FULL_MASK, im < nimg && gx * gx + gy * gy + gz * gz < limit);
+                    unsigned near = __ballot_sync(FULL_MASK, g0 + lane < nimg && gx * gx + gy * gy + gz * gz < limit);
                     while (near) {
                         const int l = __ffs(near) - 1;
                         near &= near - 1;
                         const float px = __shfl_sync(FULL_MASK, qx, l), py = __shfl_sync(FULL_MASK, qy, l), pz = __shfl_sync(FULL_MASK, qz, l);
-                        for (int j0 = 0; j0 < tn; j0 += 32) {
-                            const int j = j0 + lane;
-                            bool pass = false;
-                            if (j < tn) {
-                                const float dx = s_posf[3 * j] - px, dy = s_posf[3 * j + 1] - py, dz = s_posf[3 * j + 2] - pz;
-                                pass = dx * dx + dy * dy + dz * dz < limit;
+                        const int packed = __shfl_sync(FULL_MASK, im_packed, l);
+                        const float p2 = px * px + py * py + pz * pz, size = n2max + p2;
+                        unsigned mine = 0;      // bit k: atom 32 k + lane of the tile survives
+                        if (size < 1e30f) {
+                            // rounding of |q_j|^2 - 2 q_i q_j + |q_i|^2: less than 1e-6 of the squares
+                            const float lim = fminf(limit + 2e-6f * size - p2, 1e38f);      // (below the padding)
+                            const unsigned long long mx = pack2(-2.f * px, -2.f * px), my = pack2(-2.f * py, -2.f * py), mz = pack2(-2.f * pz, -2.f * pz);
+                            const ulonglong2 *cl = s_cq + lane;
+#pragma unroll 2
+                            for (int k = 0; 32 * k < tn; k += 2, cl += 64) {
+                                const ulonglong2 a2 = cl[0], b2 = cl[32];
+                                float v0, v1;
+                                unpack2(fma2(mx, a2.x, fma2(my, a2.y, fma2(mz, b2.x, b2.y))), v0, v1);
+                                if (v0 < lim) mine |= 1u << k;
+                                if (v1 < lim) mine |= 2u << k;
                             }
+                        } else {                // coordinates whose squares leave the single-precision range, or none: no pre-test
+                            for (int k = 0; 32 * k + lane < tn; k++) mine |= 1u << k;
+                        }
+                        for (unsigned any = __reduce_or_sync(FULL_MASK, mine); any; any &= any - 1) {
+                            const int k = __ffs(any) - 1;
+                            const bool pass = (mine >> k) & 1u;
                             const unsigned bal = __ballot_sync(FULL_MASK, pass);
-                            if (!bal) continue;
                             if (pass) {
                                 const int p = queued + __popc(bal & lt_mask);
-                                s_queue[warp][p] = j;
-                                s_img[warp][p] = g0 + l;
+                                s_queue[warp][p] = 32 * k + lane;
+                                s_img[warp][p] = packed;
                             }
                             queued += __popc(bal);
                             __syncwarp();

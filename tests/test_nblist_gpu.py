@@ -376,3 +376,38 @@ def test_batched_build_tiles_and_chunks(checkers, dt, sizes, umax):
         nn, fn, rc, ty, mx = chk.nblist(cells[b], np.zeros(n, np.int32), coords[b, :n], 4.0, umax)
         util.assert_nblist_equal((out["bnumneigh"][b, :n].cpu().numpy(), out["bfirstneigh"][b, :n].cpu().numpy(),
                                   out["brcs"][b, :n].cpu().numpy()), (nn, fn, rc))
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.float32])
+def test_batched_build_pre_test(checkers, dt):
+    """The single-precision test of the batched build drops no neighbour: a structure far from the origin (first atom of the tile or
+    not), more than 32 images, an odd count, and atoms with infinite, undefined or enormous coordinates beside whole ones."""
+    chk = _chk(checkers)
+    rng = np.random.default_rng(12)
+    cells, plain = [], []
+    for n, L, shift in ((65, 12.0, 0.0), (65, 12.0, 2500.0), (3, 2.1, 0.0), (130, 15.0, -40.0)):
+        cells.append(np.eye(3) * L)
+        plain.append(rng.random((n, 3)) * L + shift)
+    plain[3][1:] += 37 * cells[3][0]                   # the first atom alone in another period
+    cells, plain = np.stack(cells).astype(dt), [p.astype(dt) for p in plain]
+
+    def build(frames):
+        npad = max(map(len, frames))
+        coords = np.zeros((len(frames), npad, 3), dt)
+        for b, p in enumerate(frames):
+            coords[b, :len(p)] = p
+        out = capi.nblist_build_batch(cells, torch.tensor([len(p) for p in frames], dtype=torch.int32).cuda(), torch.from_numpy(coords).cuda(), 4.0, 128)
+        return [tuple(out[k][b, :len(p)].cpu().numpy() for k in ("bnumneigh", "bfirstneigh", "brcs")) for b, p in enumerate(frames)]
+
+    want = build(plain)
+    for b, p in enumerate(plain):
+        nn, fn, rc, ty, mx = chk.nblist(cells[b], np.zeros(len(p), np.int32), p, 4.0, 128)
+        util.assert_nblist_equal(want[b], (nn, fn, rc))
+    for v in (np.inf, -np.inf, np.nan, 1e25, -1e25) + ((1e13,) if dt == np.float64 else ()):
+        bad = np.array([[v, 1.0, 1.0], [1.0, v, 1.0]], dt)
+        for got, w in zip(build([np.concatenate([bad, p]) for p in plain]), want):
+            nn, fn, rc = got
+            assert not nn[:2].any() and (fn[:2] == -1).all()
+            fn = np.where(fn >= 0, fn - 2, fn)
+            assert fn.min() >= -1
+            util.assert_nblist_equal((nn[2:], fn[2:], rc[2:]), w)
