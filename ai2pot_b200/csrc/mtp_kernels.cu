@@ -438,11 +438,12 @@ __global__ void __launch_bounds__(MTP_CWARPS * 32, 1) mtp_contract_kernel(const 
 
 
 // ---- kernel B: products and adjoints out of shared memory (row loop: mtp_pairs.cuh) -----------------------
-// Tiles of TA = 32 or 16 atoms, one block per SM walking over them; the next tile's rows travel in registers while the current tile
-// is processed. A moment is finished with a plain store by the group of lanes that owns it, so the result is the same bit for
+// Tiles of TA = 32 or 16 atoms, blocks of W warps (32, one block per SM; 8 for small tables) walking over them; the next tile's rows
+// travel in registers while the current tile is processed. A moment is finished with a plain store by the group of lanes that owns it, so the result is the same bit for
 // bit from run to run. Shared memory: M[nm][TA], E[nm][TA] (not for descriptors), row records, adjoint seeds, small tables.
 constexpr int MTP_PAIR_EWARPS = 8;   // warps that sum the site energies of a tile
 template <typename T> constexpr int pair_gl(int ta) { return ta * (int)sizeof(T) / 16; }      // lanes per row
+template <typename T> constexpr int pair_stream(int ta, int warps) { return (pair_gl<T>(ta) == 16 ? 0 : 1) + (warps == MTP_PAIR_FEW ? 2 : 0); }
 template <typename T>
 struct PairSmem {
     T *M, *E, *seed, *wsc;     // wsc[s] = lin[s] / q[s]; seed[m] = sum of wsc over the scalars mapped to moment m
@@ -450,16 +451,16 @@ struct PairSmem {
     int2 *row, *warp;
     int *map, *db;             // moment of scalar s; basic moment of dense index d (-1: none)
 };
-template <typename T, int MODE, int TA>
+template <typename T, int MODE, int TA, int W>
 __host__ __device__ inline size_t pair_smem_layout(const MtpProgramDev &P, unsigned char *base, PairSmem<T> *out)
 {
-    constexpr int K = pair_gl<T>(TA) == 16 ? 0 : 1, G = 32 / pair_gl<T>(TA);
+    constexpr int K = pair_stream<T>(TA, W), G = 32 / pair_gl<T>(TA);
     size_t o = 0;
     auto take = [&](size_t bytes) { size_t r = o; o += (bytes + 15) & ~size_t(15); return r; };
     const size_t oM = take(sizeof(T) * (size_t)P.nm * TA);
     const size_t oE = MODE == MODE_DESC ? oM : take(sizeof(T) * (size_t)P.nm * TA);
     const size_t orow = take(sizeof(int2) * (size_t)P.stream[K].nrows * G);
-    const size_t ow = take(sizeof(int2) * (size_t)(2 * P.nlev) * MTP_PAIR_WARPS);
+    const size_t ow = take(sizeof(int2) * (size_t)(2 * P.nlev) * W);
     const size_t os = take(sizeof(T) * (size_t)P.nm);
     const size_t osc = take(sizeof(T) * (size_t)P.ns);
     const size_t oep = take(MODE == MODE_DESC ? 0 : sizeof(T) * MTP_PAIR_EWARPS * 32);
@@ -474,23 +475,23 @@ __host__ __device__ inline size_t pair_smem_layout(const MtpProgramDev &P, unsig
     }
     return o;
 }
-template <typename T, int MODE, int TA>
+template <typename T, int MODE, int TA, int W = MTP_PAIR_WARPS>
 static bool pair_fits(const MtpProgramDev &P)
 {
-    return P.stream[pair_gl<T>(TA) == 16 ? 0 : 1].nrows > 0 && pair_smem_layout<T, MODE, TA>(P, nullptr, nullptr) <= 226 * 1024;
+    return P.stream[pair_stream<T>(TA, W)].nrows > 0 && pair_smem_layout<T, MODE, TA, W>(P, nullptr, nullptr) <= 226 * 1024;
 }
 
-template <typename T, int MODE, int TA>
-__global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_contract_pair_kernel(const MtpProgramDev P, const MtpArgs<T> A)
+template <typename T, int MODE, int TA, int W>
+__global__ void __launch_bounds__(W * 32, W == MTP_PAIR_FEW ? 4 : 1) mtp_contract_pair_kernel(const MtpProgramDev P, const MtpArgs<T> A)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int NT = MTP_PAIR_WARPS * 32, GL = pair_gl<T>(TA), G = 32 / GL, K = GL == 16 ? 0 : 1;
-    constexpr int RW = 32 / TA, NR = MTP_PAIR_WARPS * RW;      // rows of a warp, of the block when lanes are atoms
+    constexpr int NT = W * 32, GL = pair_gl<T>(TA), G = 32 / GL, K = pair_stream<T>(TA, W);
+    constexpr int RW = 32 / TA, NR = W * RW;      // rows of a warp, of the block when lanes are atoms
     constexpr int PREF = MTP_PREF / RW;                        // rows fetched ahead per thread
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int at = lane % TA, rw = warp * RW + lane / TA;
     PairSmem<T> S;
-    pair_smem_layout<T, MODE, TA>(P, smem_raw, &S);
+    pair_smem_layout<T, MODE, TA, W>(P, smem_raw, &S);
     chain_release();
     const int ntot = total_atoms(A);
     const int ntiles = (ntot + TA - 1) / TA;
@@ -500,7 +501,7 @@ __global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_contract_pair_kern
     }
     // tables, staged once per block
     for (int i = threadIdx.x; i < P.stream[K].nrows * G; i += NT) S.row[i] = stream_rows<T>(P.stream[K])[i];
-    for (int i = threadIdx.x; i < 2 * P.nlev * MTP_PAIR_WARPS; i += NT) S.warp[i] = P.stream[K].warp[i];
+    for (int i = threadIdx.x; i < 2 * P.nlev * W; i += NT) S.warp[i] = P.stream[K].warp[i];
     for (int s = threadIdx.x; s < P.ns; s += NT) S.map[s] = P.map[s];
     if (MODE != MODE_DESC) {
         for (int i = threadIdx.x; i < P.nm; i += NT) S.seed[i] = T(0);
@@ -535,7 +536,7 @@ __global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_contract_pair_kern
     const unsigned ml = (unsigned)__cvta_generic_to_shared(S.M) + 16u * (lane % GL), el = (unsigned)__cvta_generic_to_shared(S.E) + 16u * (lane % GL);
     const unsigned a_row = (unsigned)__cvta_generic_to_shared(S.row) + 8u * (lane / GL), a_seed = (unsigned)__cvta_generic_to_shared(S.seed);
     auto run_phase = [&](int p, auto seeded, unsigned xl, unsigned yl, unsigned dl) {
-        const int2 w = S.warp[p * MTP_PAIR_WARPS + warp];
+        const int2 w = S.warp[p * W + warp];
         pair_phase<T, GL, decltype(seeded)::value>(a_row + 8u * G * (unsigned)w.x, w.y, xl, yl, dl, a_seed);
     };
 
@@ -836,15 +837,16 @@ static int launch_contract(const MtpProgramDev &P, const MtpArgs<T> &A, long ato
     return AI2B_OK;
 }
 
-template <typename T, int MODE, int TA>
+template <typename T, int MODE, int TA, int W>
 static int launch_pair(const MtpProgramDev &P, const MtpArgs<T> &A, long tiles, cudaStream_t st)
 {
-    const size_t smem = pair_smem_layout<T, MODE, TA>(P, nullptr, nullptr);
-    auto kern = mtp_contract_pair_kernel<T, MODE, TA>;
+    const size_t smem = pair_smem_layout<T, MODE, TA, W>(P, nullptr, nullptr);
+    auto kern = mtp_contract_pair_kernel<T, MODE, TA, W>;
     static KernelSetup setup;
-    if (int rc = kernel_setup(setup, kern, smem)) return rc;
-    if (tiles > sm_count()) tiles = sm_count();      // persistent: one block per SM walks over the tiles
-    AI2B_CUDA(launch_chained(kern, (unsigned)tiles, MTP_PAIR_WARPS * 32, smem, st, P, A));
+    int per_sm = 1;
+    if (int rc = kernel_setup(setup, kern, smem, W * 32, &per_sm)) return rc;
+    const long room = (long)sm_count() * per_sm;      // persistent: the blocks walk over the tiles
+    AI2B_CUDA(launch_chained(kern, (unsigned)(tiles < room ? tiles : room), W * 32, smem, st, P, A));
     return AI2B_OK;
 }
 
@@ -860,9 +862,10 @@ static int dispatch_contract(const MtpProgramDev &P, const MtpArgs<T> &A, long a
     // each on a tile of 16). Single precision stays at 32 atoms: its rows are as short as the double ones of 16.
     if (pair_fits<T, MODE, 32>(P)) {
         constexpr int SMALL = sizeof(T) == 8 ? 16 : 32;
-        const long small_tiles = (atoms_upper + SMALL - 1) / SMALL;
-        if (small_tiles <= sm_count()) return launch_pair<T, MODE, SMALL>(P, A, small_tiles, st);
-        return launch_pair<T, MODE, 32>(P, A, (atoms_upper + 31) / 32, st);
+        const long small_tiles = (atoms_upper + SMALL - 1) / SMALL, tiles = (atoms_upper + 31) / 32;
+        if (small_tiles <= sm_count()) return launch_pair<T, MODE, SMALL, MTP_PAIR_WARPS>(P, A, small_tiles, st);
+        if (tiles > sm_count() && pair_fits<T, MODE, 32, MTP_PAIR_FEW>(P)) return launch_pair<T, MODE, 32, MTP_PAIR_FEW>(P, A, tiles, st);
+        return launch_pair<T, MODE, 32, MTP_PAIR_WARPS>(P, A, tiles, st);
     }
 #define AI2B_TRY(TA_)                                                                                       \
     if ((long)P.nm * (TA_ + 1) <= 65535) {                                                                  \

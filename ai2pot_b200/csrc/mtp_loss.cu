@@ -397,13 +397,13 @@ struct LossPairSmem {
     int *map, *db;
 };
 template <typename T> constexpr int loss_ta() { return 8 * 16 / (int)sizeof(T); }
-template <typename T>
+template <typename T, int W>
 __host__ __device__ inline size_t loss_pair_smem(const MtpProgramDev &P, unsigned char *base, LossPairSmem<T> *out)
 {
     size_t o = 0;
     auto take = [&](size_t bytes) { size_t r = o; o += (bytes + 15) & ~size_t(15); return r; };
     const size_t oM = take(sizeof(T) * 2 * (size_t)P.nm * loss_ta<T>()), oE = take(sizeof(T) * 2 * (size_t)P.nm * loss_ta<T>());
-    const size_t orow = take(sizeof(int2) * (size_t)P.stream[1].nrows * 4), ow = take(sizeof(int2) * (size_t)(2 * P.nlev) * MTP_PAIR_WARPS);
+    const size_t orow = take(sizeof(int2) * (size_t)P.stream[W == MTP_PAIR_FEW ? 3 : 1].nrows * 4), ow = take(sizeof(int2) * (size_t)(2 * P.nlev) * W);
     const size_t os = take(sizeof(T) * (size_t)P.nm), om = take(sizeof(int) * (size_t)P.ns), od = take(sizeof(int) * (size_t)P.ndense);
     if (out) {
         out->db = reinterpret_cast<int *>(base + od);
@@ -413,20 +413,20 @@ __host__ __device__ inline size_t loss_pair_smem(const MtpProgramDev &P, unsigne
     return o;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_loss_pair_kernel(const MtpProgramDev P, const MtpArgs<T> A, const LossArgs<T> L)
+template <typename T, int W>
+__global__ void __launch_bounds__(W * 32, W == MTP_PAIR_FEW ? 4 : 1) mtp_loss_pair_kernel(const MtpProgramDev P, const MtpArgs<T> A, const LossArgs<T> L)
 {
     extern __shared__ __align__(32) unsigned char smem_raw[];
-    constexpr int NT = MTP_PAIR_WARPS * 32, TA = loss_ta<T>(), RW = 32 / TA, G = 4;    // RW: moment rows per warp when lanes are atoms
+    constexpr int NT = W * 32, TA = loss_ta<T>(), RW = 32 / TA, G = 4, K = W == MTP_PAIR_FEW ? 3 : 1;    // RW: moment rows per warp when lanes are atoms
     LossPairSmem<T> S;
-    loss_pair_smem<T>(P, smem_raw, &S);
+    loss_pair_smem<T, W>(P, smem_raw, &S);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int at = lane % TA, rw = warp * RW + lane / TA;
     T *D = S.M + (size_t)P.nm * TA, *Gm = S.E + (size_t)P.nm * TA;
     const unsigned off = (unsigned)(sizeof(T) * (size_t)P.nm * TA);
     chain_release();
-    for (int i = threadIdx.x; i < P.stream[1].nrows * G; i += NT) S.row[i] = stream_rows<T>(P.stream[1])[i];
-    for (int i = threadIdx.x; i < 2 * P.nlev * MTP_PAIR_WARPS; i += NT) S.warp[i] = P.stream[1].warp[i];
+    for (int i = threadIdx.x; i < P.stream[K].nrows * G; i += NT) S.row[i] = stream_rows<T>(P.stream[K])[i];
+    for (int i = threadIdx.x; i < 2 * P.nlev * W; i += NT) S.warp[i] = P.stream[K].warp[i];
     for (int s = threadIdx.x; s < P.ns; s += NT) S.map[s] = P.map[s];
     for (int d = threadIdx.x; d < P.ndense; d += NT) S.db[d] = P.dense_basic[d];
     for (int i = threadIdx.x; i < P.nm; i += NT) S.seed[i] = T(0);
@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_loss_pair_kernel(c
     for (int s = threadIdx.x; s < P.ns; s += NT) atomicAdd(S.seed + P.map[s], A.lin[s] / A.qs[s]);
     __syncthreads();
     // moments no product reads: adjoint = seed, no second-order adjoint
-    for (int i = rw; i < P.n_adj_const; i += MTP_PAIR_WARPS * RW) {
+    for (int i = rw; i < P.n_adj_const; i += W * RW) {
         const int m = P.adj_const[i];
         S.E[m * TA + at] = S.seed[m];
         Gm[m * TA + at] = T(0);
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_loss_pair_kernel(c
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int t = tile * TA + at;
         const bool valid = t < ntot;
-        for (int i = rw; i < P.nb; i += MTP_PAIR_WARPS * RW) {
+        for (int i = rw; i < P.nb; i += W * RW) {
             // rows per atom, or [tile of 32 atoms][row][32]
             const size_t src = A.tiled ? ((size_t)(t >> 5) * A.nbp + i) * 32 + (t & 31) : (size_t)t * A.nbp + i;
             S.M[i * TA + at] = valid ? A.Mb[src] : T(0);
@@ -463,18 +463,18 @@ __global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_loss_pair_kernel(c
         }
         __syncthreads();
         for (int p = 0; p < P.nlev; p++) {
-            const int2 w = S.warp[p * MTP_PAIR_WARPS + warp];
+            const int2 w = S.warp[p * W + warp];
             pair_phase_deriv<T, 8>(a_row + 8u * G * (unsigned)w.x, w.y, ml, off);
             __syncthreads();
         }
         for (int p = P.nlev; p < 2 * P.nlev; p++) {
-            const int2 w = S.warp[p * MTP_PAIR_WARPS + warp];
+            const int2 w = S.warp[p * W + warp];
             pair_phase_second<T, 8>(a_row + 8u * G * (unsigned)w.x, w.y, el, ml, off, a_seed);
             __syncthreads();
         }
         // for the coefficient kernel: E and X = ce E + G of the basic moments
         if (L.dense) {
-            for (int d = rw; d < P.ndense; d += MTP_PAIR_WARPS * RW) {
+            for (int d = rw; d < P.ndense; d += W * RW) {
                 const int i = S.db[d];
                 const T e = i >= 0 ? S.E[i * TA + at] : T(0), g = i >= 0 ? Gm[i * TA + at] : T(0);
                 const size_t o = ((size_t)(t >> 5) * A.ndp + d) * 32 + (t & 31);
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_loss_pair_kernel(c
                 reinterpret_cast<typename Vec2<T>::type *>(L.Xb)[o] = ex;
             }
         } else if (valid)
-            for (int i = rw; i < P.nb; i += MTP_PAIR_WARPS * RW) {
+            for (int i = rw; i < P.nb; i += W * RW) {
                 const T e = S.E[i * TA + at];
                 A.Eb[(size_t)t * A.nbp + i] = e;
                 L.Xb[(size_t)t * A.nbp + i] = fma(ce, e, Gm[i * TA + at]);
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(MTP_PAIR_WARPS * 32, 1) mtp_loss_pair_kernel(c
         // gradients w.r.t. the linear coefficients and the type bias: one atomic per entry when the tile lies in one structure
         const int b0 = __shfl_sync(FULL_MASK, b, 0);
         const bool uniform = __all_sync(FULL_MASK, !valid || b == b0);      // (the same in every warp: they share the tile's atoms)
-        for (int s0 = 0; s0 < P.ns; s0 += MTP_PAIR_WARPS * RW) {
+        for (int s0 = 0; s0 < P.ns; s0 += W * RW) {
             const int s = s0 + rw;
             T val = T(0);
             if (s < P.ns && valid) {
@@ -688,8 +688,9 @@ static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArg
         kern<<<(unsigned)blocks, MTP_WARPS * 32, smem, st>>>(P, A, L);
         AI2B_CUDA(cudaGetLastError());
     }
-    const size_t pair_bytes = loss_pair_smem<T>(P, nullptr, nullptr);
+    const size_t pair_bytes = loss_pair_smem<T, MTP_PAIR_WARPS>(P, nullptr, nullptr);
     const bool pair = P.stream[1].nrows > 0 && pair_bytes <= 226 * 1024;
+    const long pair_tiles = (atoms_upper + loss_ta<T>() - 1) / loss_ta<T>();
     // the coefficient gradient by tiles pays once they occupy half of the SMs; below that a warp per atom is over sooner
     // (level 10, fp32, 240 atoms: 11 against 14 us; level 16, fp64, 9,323 atoms: 99 against 87)
     // (it copies 16 bytes at a time)
@@ -700,12 +701,20 @@ static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArg
         int rc = AI2B_ERR_UNSUPPORTED;
         bool done = false;
         if (pair) {
-            auto kern = mtp_loss_pair_kernel<T>;
-            static KernelSetup setup;
-            if ((rc = kernel_setup(setup, kern, pair_bytes))) return rc;
-            long tiles = (atoms_upper + loss_ta<T>() - 1) / loss_ta<T>();
-            if (tiles > sm_count()) tiles = sm_count();
-            AI2B_CUDA(launch_chained(kern, (unsigned)tiles, MTP_PAIR_WARPS * 32, pair_bytes, st, P, A, L));
+            auto run = [&](auto w) -> int {
+                constexpr int W = decltype(w)::value;
+                const size_t bytes = loss_pair_smem<T, W>(P, nullptr, nullptr);
+                auto kern = mtp_loss_pair_kernel<T, W>;
+                static KernelSetup setup;
+                int per_sm = 1;
+                if (int e = kernel_setup(setup, kern, bytes, W * 32, &per_sm)) return e;
+                const long room = (long)sm_count() * per_sm;
+                AI2B_CUDA(launch_chained(kern, (unsigned)(pair_tiles < room ? pair_tiles : room), W * 32, bytes, st, P, A, L));
+                return AI2B_OK;
+            };
+            // (few warps per block as in the contraction of the forces)
+            const bool few = pair_tiles > sm_count() && P.stream[3].nrows > 0 && loss_pair_smem<T, MTP_PAIR_FEW>(P, nullptr, nullptr) <= 226 * 1024;
+            rc = few ? run(std::integral_constant<int, MTP_PAIR_FEW>{}) : run(std::integral_constant<int, MTP_PAIR_WARPS>{});
             done = true;
         }
 #define AI2B_TRY(TA_)                                                                                                   \

@@ -132,13 +132,13 @@ struct Blob {
     }
 };
 
-// Deals the moments of a phase (by decreasing row count) to MTP_PAIR_WARPS warps of `groups` groups of lanes each: the first
+// Deals the moments of a phase (by decreasing row count) to `warps` warps of `groups` groups of lanes each: the first
 // nwide of them to whole warps, the others to groups, each to the least loaded place, the lowest of equals, completing a
 // moment taken as a row. choose() takes the nwide of the least cost; candidates are looked at by a lower bound of their cost,
 // so that most are never dealt.
 class RowDeal {
 public:
-    explicit RowDeal(int groups) : groups(groups), wide_rows(MTP_PAIR_WARPS), group_rows(MTP_PAIR_WARPS * groups), load(MTP_PAIR_WARPS * groups) {}
+    RowDeal(int warps, int groups) : warps(warps), groups(groups), wide_rows(warps), group_rows(warps * groups), load(warps * groups) {}
     int nwide = 0;
     std::vector<int> place;      // warp (of a wide moment) or group
 
@@ -153,7 +153,7 @@ public:
         for (int i = 0; i < nq; i++) {
             if (i == 0 || n[i] != n[i - 1]) {      // all moments of one row count are dealt alike
                 const long sum = wide + (rest + groups - 1) / groups;
-                const long longest = std::max<long>({(sum + MTP_PAIR_WARPS - 1) / MTP_PAIR_WARPS, n[i], i ? (n[0] + groups - 1) / groups : 0});
+                const long longest = std::max<long>({(sum + warps - 1) / warps, n[i], i ? (n[0] + groups - 1) / groups : 0});
                 cand.push_back({cost(longest, sum), i});
             }
             wide += (n[i] + groups - 1) / groups;
@@ -173,7 +173,7 @@ public:
 
 private:
     struct Candidate { long bound; int wide; };
-    const int groups;
+    const int warps, groups;
     std::vector<Candidate> cand;
     std::vector<int> n, wide_rows, group_rows, load;
     std::vector<unsigned> at_load;      // [load][words]: which places have it
@@ -213,11 +213,11 @@ private:
         std::fill(wide_rows.begin(), wide_rows.end(), 0);
         std::fill(group_rows.begin(), group_rows.end(), 0);
         std::fill(load.begin(), load.end(), 0);
-        spread(0, nw, MTP_PAIR_WARPS, wide_rows, [&](int i) { return (n[i] + groups - 1) / groups; });
-        for (int p = MTP_PAIR_WARPS * groups - 1; p >= 0; p--) load[p] = load[p / groups];
-        spread(nw, (int)n.size(), MTP_PAIR_WARPS * groups, group_rows, [&](int i) { return n[i]; });
+        spread(0, nw, warps, wide_rows, [&](int i) { return (n[i] + groups - 1) / groups; });
+        for (int p = warps * groups - 1; p >= 0; p--) load[p] = load[p / groups];
+        spread(nw, (int)n.size(), warps * groups, group_rows, [&](int i) { return n[i]; });
         long longest = 0, sum = 0;
-        for (int w = 0; w < MTP_PAIR_WARPS; w++) { longest = std::max<long>(longest, length(w)); sum += length(w); }
+        for (int w = 0; w < warps; w++) { longest = std::max<long>(longest, length(w)); sum += length(w); }
         return cost(longest, sum);
     }
 };
@@ -379,7 +379,7 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
         AI2B_REQUIRE(map[s] >= 0 && map[s] < nm, AI2B_ERR_INVALID, "alpha_moment_mapping[%d] out of range", s);
 
     // row streams (see mtp_program.cuh)
-    std::vector<int2> stream_d[2], stream_f[2], stream_warp[2];
+    std::vector<int2> stream_d[4], stream_f[4], stream_warp[4];
     std::vector<int> adj_const;
     {
         std::vector<char> is_source(nm, 0), is_mapped(nm, 0);
@@ -390,13 +390,13 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
         for (int m = 0; m < nm; m++)
             if (!is_source[m] && (is_mapped[m] || m < nb)) adj_const.push_back(m);
     }
-    for (int k = 0; k < 2; k++) {
-        const int groups = k == 0 ? 2 : 4;
+    for (int k = 0; k < 4; k++) {
+        const int groups = k % 2 == 0 ? 2 : 4, warps = k < 2 ? MTP_PAIR_WARPS : MTP_PAIR_FEW;
         P.stream[k].nrows = 0;
-        if (nm > 2046 || nt == 0) continue;      // the completed moment has 11 bits
-        RowDeal deal(groups);
-        std::vector<int> row0(MTP_PAIR_WARPS), next(MTP_PAIR_WARPS * groups);      // rows that the next records of a warp, a group go to
-        stream_warp[k].reserve(2 * P.nlev * MTP_PAIR_WARPS);
+        if (nm > 2046 || nt == 0 || (k >= 2 && nt > MTP_PAIR_FEW_ROWS)) continue;      // the completed moment has 11 bits
+        RowDeal deal(warps, groups);
+        std::vector<int> row0(warps), next(warps * groups);      // rows that the next records of a warp, a group go to
+        stream_warp[k].reserve(2 * P.nlev * warps);
         stream_d[k].reserve(4 * nt + 64 * P.nlev);
         stream_f[k].reserve(4 * nt + 64 * P.nlev);
         for (int phase = 0; phase < 2 * P.nlev; phase++) {
@@ -410,7 +410,7 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
             const std::vector<int2> &flat = fwd ? fwd_flat : rev_flat;
             deal.choose(q, nq);
             size_t first = stream_d[k].size();
-            for (int w = 0; w < MTP_PAIR_WARPS; w++) {
+            for (int w = 0; w < warps; w++) {
                 row0[w] = (int)(first / groups);
                 stream_warp[k].push_back(make_int2(row0[w], deal.length(w)));
                 first += (size_t)deal.length(w) * groups;
@@ -423,7 +423,7 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
                 stream_d[k][(size_t)row * groups + g] = make_int2(xy, bits_d(mult) | done);
                 stream_f[k][(size_t)row * groups + g] = make_int2(xy, bits_f(mult) | done);
             };
-            for (int g = 0; g < MTP_PAIR_WARPS * groups; g++) next[g] = row0[g / groups];
+            for (int g = 0; g < warps * groups; g++) next[g] = row0[g / groups];
             for (int i = 0; i < nq; i++) {
                 const int n = q[i].z - q[i].y, place = deal.place[i];
                 if (i < deal.nwide) {
@@ -445,8 +445,8 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
 
     Blob blob;
     blob.bytes.reserve(64 * 1024 + 128 * (size_t)(nm + nt) + 16 * (stream_d[0].size() + stream_d[1].size()));
-    size_t o_ac = blob.add(adj_const), o_sd[2], o_sf[2], o_sw[2];
-    for (int k = 0; k < 2; k++) { o_sd[k] = blob.add(stream_d[k]); o_sf[k] = blob.add(stream_f[k]); o_sw[k] = blob.add(stream_warp[k]); }
+    size_t o_ac = blob.add(adj_const), o_sd[4], o_sf[4], o_sw[4];
+    for (int k = 0; k < 4; k++) { o_sd[k] = blob.add(stream_d[k]); o_sf[k] = blob.add(stream_f[k]); o_sw[k] = blob.add(stream_warp[k]); }
     size_t o_bd = blob.add(basic_dense), o_db = blob.add(dense_basic), o_e4d = blob.add(e4d), o_g = blob.add(e4g), o_m = blob.add(e4m), o_fd = blob.add(fwd_dst),
            o_rm = blob.add(rev_mom), o_map = blob.add(map);
     size_t o_frow = blob.add(fwd_rows), o_rent = blob.add(rev_ents), o_ff = blob.add(fwd_flat), o_rf = blob.add(rev_flat);
@@ -476,7 +476,7 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
     P.fwd_flat = (const int2 *)(b + o_ff);
     P.rev_flat = (const int2 *)(b + o_rf);
     P.adj_const = (const int *)(b + o_ac);
-    for (int k = 0; k < 2; k++) {
+    for (int k = 0; k < 4; k++) {
         P.stream[k].row_d = (const int2 *)(b + o_sd[k]);
         P.stream[k].row_f = (const int2 *)(b + o_sf[k]);
         P.stream[k].warp = (const int2 *)(b + o_sw[k]);

@@ -49,13 +49,17 @@ struct MtpProgramDev {
     // zero for integers up to 255. The groups of a warp have equally many rows in a phase (empty ones where needed).
     struct Stream {
         const int2 *row_d, *row_f;      // [nrows][groups of a warp]
-        const int2 *warp;               // [2 nlev][MTP_PAIR_WARPS] {first row, rows}
-        int nrows;                      // 0: the tables do not fit the encoding
-    } stream[2];                        // GL = 16, GL = 8
+        const int2 *warp;               // [2 nlev][warps] {first row, rows}
+        int nrows;                      // 0: the tables do not fit the encoding, or have too many rows for few warps
+    } stream[4];                        // GL = 16, GL = 8 for MTP_PAIR_WARPS warps; the same for MTP_PAIR_FEW
     const int *adj_const;           // [n_adj_const] moments whose adjoint is only their seed (no product reads them)
     int n_adj_const;
 };
-constexpr int MTP_PAIR_WARPS = 32;
+// Warps of a block of the contractions. A phase of a small table is over before 32 warps have met: where there are more tiles than
+// SMs such tables (levels up to 10, of 42 products; level 16 has 969 and fills 32 warps) take blocks of eight warps, four of which share
+// an SM. Level 10, whole call, us, 32 / 8 warps: fp64 6,000 atoms 51.6 / 48.5, 13,824 atoms 73.2 / 67.2, 100,000 atoms 361 / 303; with a
+// tile per SM 32 warps are sooner over it (2,500 atoms 34.8 / 37.2).
+constexpr int MTP_PAIR_WARPS = 32, MTP_PAIR_FEW = 8, MTP_PAIR_FEW_ROWS = 128;
 constexpr int MTP_PAIR_WIDE = 0x800;
 constexpr int MTP_TILE = 32;        // atoms per tile of the workspace
 

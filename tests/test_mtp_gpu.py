@@ -76,9 +76,9 @@ def test_g1_full_size_vs_checker(checkers):
 
 
 @pytest.mark.parametrize("natoms,level,dt", [(3, 16, np.float64), (133, 16, np.float32), (1777, 16, np.float64), (2370, 10, np.float64), (3001, 10, np.float32),
-                                             (5003, 10, np.float64), (15001, 6, np.float64)])
+                                             (5003, 10, np.float64), (9001, 10, np.float32), (15001, 6, np.float64)])
 def test_lanes_share_the_slots_of_an_atom(checkers, natoms, level, dt):
-    """Structures of a size for 8, 4, 2 and 1 lanes per atom and for contraction tiles of 16 and 32 atoms, the last tile ragged, some
+    """Structures of a size for 8, 4, 2 and 1 lanes per atom, contraction tiles of 16 and 32 atoms, blocks of 32 and 8 warps, the last tile ragged, some
     atoms at an open side with few neighbours; fp32 against the model in double precision (every input is a single)."""
     rng = np.random.default_rng(natoms)
     edge = int(np.ceil(natoms ** (1 / 3) - 1e-9))

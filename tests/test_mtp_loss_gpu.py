@@ -147,7 +147,7 @@ def test_loss_op_autograd(checkers):
 
 @pytest.mark.parametrize("dt", [torch.float64, torch.float32])
 @pytest.mark.parametrize("level,B,nmin,nmax", [(6, 1, 1, 2), (6, 3, 8, 40), (10, 5, 1, 17), (16, 1, 16, 17), (16, 9, 1, 34),
-                                                 (6, 120, 1, 34), (16, 96, 1, 40)])
+                                                 (6, 120, 1, 34), (10, 150, 1, 34), (16, 96, 1, 40)])
 def test_contraction_tile_edges(checkers, level, B, nmin, nmax, dt):
     """Structures of 1 to 33 atoms: tiles of 16 and 32 atoms that are nearly empty, full, ragged and shared by several
     structures, at every template level, forward and gradients."""
