@@ -2,7 +2,7 @@
 //
 // Tables of the reference's template levels 6 to 16 (monomial degree <= 6, four radial functions at most):
 //   mtp_fwd_atoms_kernel    (mtp_atoms.cu) lanes = atoms, basic moments in registers -> Mb[tile][basic row][32 atoms]
-//   mtp_contract_pair_kernel lanes = atoms, one tile of 32 atoms per block at a time: the product rows and the adjoint
+//   mtp_contract_pair_kernel lanes = atoms, a tile of 32 or 16 atoms per block at a time: the product rows and the adjoint
 //                           sweep run out of shared memory, every moment owned by a group of lanes; site energies; adjoints
 //                           of the basic moments -> Eb[tile][dense monomial][32 atoms] (or the descriptors)
 //   mtp_force_atoms_kernel  (mtp_atoms.cu) lanes = atoms: polynomial of every radial function and its gradient per
