@@ -100,6 +100,24 @@ def test_build_and_evaluation_share_scratch(n):
     _close(_host(ev.compute(coords)), apart, tol)
 
 
+@pytest.mark.parametrize("n", [8, 14])
+@pytest.mark.parametrize("where", ["nb_ws", "coords"])
+def test_results_in_memory_that_the_build_reads(n, where):
+    """Energy, forces and virial in the build's scratch or over the positions: both are free once the rows stand, so the call
+    is answered, and its set-up, which zeroes them, waits for the build."""
+    w, dt, tol = _workload("nep", n)
+    ev = engine.Evaluator(w["model"], w["cell"], w["types"], w["rcut"], w["umax"], dt)
+    coords = torch.from_numpy(np.ascontiguousarray(w["coords"])).to(dt).cuda()
+    apart = _host(ev.compute(coords))
+    memory = ev.nb_ws.view(-1) if where == "nb_ws" else coords.view(-1).view(torch.uint8)
+    kept = ev.out
+    for k in range(3):      # one at a time, at the beginning of the memory
+        moved = memory[:kept[k].numel() * kept[k].element_size()].view(dt).view(kept[k].shape)
+        ev.out = kept[:k] + (moved,) + kept[k + 1:]
+        _close(_host(ev.compute(coords)), apart, tol)
+        coords.copy_(torch.from_numpy(np.ascontiguousarray(w["coords"])).to(dt))
+
+
 @pytest.mark.parametrize("kind", ["mtp", "nep"])
 def test_changed_attributes_take_effect(kind):
     """Cell, cutoff, row width and model may be edited or assigned between calls (a variable-cell relaxation does): the next
