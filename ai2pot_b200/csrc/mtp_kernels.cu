@@ -287,17 +287,9 @@ __global__ void __launch_bounds__(MTP_CWARPS * 32, 1) mtp_contract_kernel(const 
     const int nthreads = MTP_CWARPS * 32;
     if ((int)blockIdx.x >= ntiles) return;
 
-    // row tables, staged once, with the moment indices already scaled to element offsets (index * LD fits 16 bits)
-    auto scale = [](int2 r) {
-        return make_int2(((r.x & 0xffff) * LD) | (((r.x >> 16) & 0xffff) * LD) << 16, (r.y & 0xffff) | (((r.y >> 16) & 0xffff) * LD) << 16);
-    };
-    if (SMEMTAB) {
-#pragma unroll 4
-        for (int i = threadIdx.x; i < P.nt; i += nthreads) s_fwd[i] = scale(P.fwd_flat[i]);
-        if (MODE != MODE_DESC)
-#pragma unroll 4
-            for (int i = threadIdx.x; i < 2 * P.nt; i += nthreads) s_rev[i] = scale(P.rev_flat[i]);
-    }
+    // row tables, staged once
+    const ScaledRow<LD, true> scale;
+    if (SMEMTAB) stage_product_rows(P, P.fwd_flat, P.rev_flat, MODE != MODE_DESC, s_fwd, threadIdx.x, nthreads, scale);
     // large tables (template levels above 16) stay in global memory
     auto frow = [&](int r) { return SMEMTAB ? s_fwd[r] : scale(P.fwd_flat[r]); };
     auto rrow = [&](int r) { return SMEMTAB ? s_rev[r] : scale(P.rev_flat[r]); };

@@ -220,13 +220,8 @@ __global__ void __launch_bounds__(MTP_CWARPS * 32, 1) mtp_loss_contract_kernel(c
     const int nthreads = MTP_CWARPS * 32;
 
     for (int i = threadIdx.x; i < 4 * (int)narr; i += nthreads) M[i] = T(0);
-    auto scale = [](int2 r) { return make_int2(((r.x & 0xffff) * LD) | (((r.x >> 16) & 0xffff) * LD) << 16, r.y); };
-    if (SMEMTAB) {
-#pragma unroll 4
-        for (int i = threadIdx.x; i < P.nt; i += nthreads) s_fwd[i] = scale(P.fwd_rows[i]);
-#pragma unroll 4
-        for (int i = threadIdx.x; i < 2 * P.nt; i += nthreads) s_rev[i] = scale(P.rev_ents[i]);
-    }
+    const ScaledRow<LD, false> scale;
+    if (SMEMTAB) stage_product_rows(P, P.fwd_rows, P.rev_ents, true, s_fwd, threadIdx.x, nthreads, scale);
     auto frow = [&](int r) { return SMEMTAB ? s_fwd[r] : scale(P.fwd_rows[r]); };
     auto rrow = [&](int r) { return SMEMTAB ? s_rev[r] : scale(P.rev_ents[r]); };
     __syncthreads();

@@ -30,11 +30,11 @@ struct MtpProgramDev {
     const int *e4m;                 // [ndense] packed multipliers (ax+1) | (ay+1)<<8 | (az+1)<<16
     const int4 *fwd_dst;            // {dst, row_begin, row_end, -}
     const int2 *fwd_rows;           // [nt] {a | b<<16, multiplier as float bits}: one 8-byte load per row
-    const int2 *rev_ents;           // [2 nt] {other | dst<<16, multiplier as float bits}
+    const int2 *rev_ents;           // [adjoint_rows()] {other | dst<<16, multiplier as float bits}
     // flat row streams for the lanes-as-atoms kernel: rows of one depth are contiguous, a flag marks the
     // last row of each destination, so any contiguous share of a depth's rows can be given to a worker
     const int2 *fwd_flat;           // [nt]   {a | b<<16, mult | last<<8 | dst<<16}
-    const int2 *rev_flat;           // [2 nt] {other | dst<<16, mult | last<<8 | source<<16}
+    const int2 *rev_flat;           // [adjoint_rows()] {other | dst<<16, mult | last<<8 | source<<16}
     int fwd_lev_row[MTP_MAX_LEV + 1];
     int rev_lev_row[MTP_MAX_LEV + 1];
     const int4 *rev_mom;            // {m, entry_begin, entry_end, -}
@@ -54,7 +54,30 @@ struct MtpProgramDev {
     } stream[4];                        // GL = 16, GL = 8 for MTP_PAIR_WARPS warps; the same for MTP_PAIR_FEW
     const int *adj_const;           // [n_adj_const] moments whose adjoint is only their seed (no product reads them)
     int n_adj_const;
+    // two per product, one for the square of a moment (unless twice its multiplier exceeds 255)
+    __host__ __device__ int adjoint_rows() const { return rev_lev_row[nlev]; }
 };
+
+// A row with its moment indices scaled to element offsets in [moment][LD] (index * LD fits 16 bits); FLAT: the moment in the high half
+// of the second word too.
+template <int LD, bool FLAT>
+struct ScaledRow {
+    __host__ __device__ int2 operator()(int2 r) const
+    {
+        return make_int2(((r.x & 0xffff) * LD) | (((r.x >> 16) & 0xffff) * LD) << 16,
+                         FLAT ? (r.y & 0xffff) | (((r.y >> 16) & 0xffff) * LD) << 16 : r.y);
+    }
+};
+// Product rows, then (if `adjoints`) adjoint rows to to[0 .. nt + adjoint_rows()), by thread t of n.
+template <typename Rows, typename Scale>
+__host__ __device__ inline void stage_product_rows(const MtpProgramDev &P, Rows fwd, Rows rev, bool adjoints, int2 *to, int t, int n, Scale scale)
+{
+#pragma unroll 4
+    for (int i = t; i < P.nt; i += n) to[i] = scale(fwd[i]);
+    if (adjoints)
+#pragma unroll 4
+        for (int i = t; i < P.adjoint_rows(); i += n) to[P.nt + i] = scale(rev[i]);
+}
 // Warps of a block of the contractions. A phase of a small table is over before 32 warps have met: where there are more tiles than
 // SMs such tables (levels up to 10, of 42 products; level 16 has 969 and fills 32 warps) take blocks of eight warps, four of which share
 // an SM. Level 10, whole call, us, 32 / 8 warps: fp64 6,000 atoms 51.6 / 48.5, 13,824 atoms 73.2 / 67.2, 100,000 atoms 361 / 303; with a

@@ -1,0 +1,48 @@
+// Compiles MTP tables into host memory (malloc and memcpy take the place of the device's) and reports, as one line of
+// numbers, what the kernels would read of them. Input: int32 nm nb nt ns nmus, basic, times, mapping.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include "mtp_program.cuh"
+
+template <typename P> static cudaError_t host_malloc(P **p, size_t n) { *p = (P *)malloc(n); return cudaSuccess; }
+static cudaError_t host_free(void *p) { free(p); return cudaSuccess; }
+static cudaError_t host_device(int *d) { *d = 0; return cudaSuccess; }
+static cudaError_t host_copy(void *d, const void *s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
+#define cudaMalloc host_malloc
+#define cudaFree host_free
+#define cudaGetDevice host_device
+#define cudaMemcpy host_copy
+#include "mtp_program.cu"
+
+struct Watched {      // an array of the tables: remembers how far it was read, and reads nothing
+    int *read;
+    int2 operator[](int i) const { *read = std::max(*read, i + 1); return make_int2(0, 0); }
+};
+
+int main(int, char **argv)
+{
+    std::vector<int> in;
+    FILE *f = fopen(argv[1], "rb");
+    for (int v; fread(&v, 4, 1, f) == 1;) in.push_back(v);
+    fclose(f);
+    const int nm = in[0], nb = in[1], nt = in[2], ns = in[3], nmus = in[4];
+    ai2b_mtp_program *prog = nullptr;
+    if (ai2b_mtp_program_create(nm, nb, &in[5], nt, &in[5 + 4 * nb], ns, &in[5 + 4 * nb + 4 * nt], nmus, &prog)) {
+        fprintf(stderr, "%s\n", ai2b_last_error_string());
+        return 1;
+    }
+    const MtpProgramDev &P = prog->dev;
+    const unsigned char *end = (const unsigned char *)prog->d_blob + prog->blob_bytes;
+    std::vector<int2> to(3 * (size_t)nt);      // what the kernels keep for the rows
+    const int threads = 1024;
+    for (int adjoints = 0; adjoints < 2; adjoints++) {
+        int fwd = 0, rev = 0;
+        for (int t = 0; t < threads; t++)
+            stage_product_rows(P, Watched{&fwd}, Watched{&rev}, adjoints, to.data(), t, threads, ScaledRow<17, true>());
+        printf("%d %d ", fwd, rev);
+    }
+    // adjoint rows that the kernels' loops walk through, and the room that rev_flat has
+    printf("%d %ld\n", P.rev_lev_row[P.nlev], (long)((end - (const unsigned char *)P.rev_flat) / sizeof(int2)));
+    ai2b_mtp_program_destroy(prog);
+}

@@ -172,6 +172,46 @@ def test_contraction_tile_edges(checkers, level, B, nmin, nmax, dt):
         assert util.relerr(capi.mtp_descriptors(prog, md, nbd).cpu().numpy(), chk.mtp_descriptors(g["model"], nb)) < tol
 
 
+@pytest.mark.parametrize("nm,nt,dt", [(600, 2000, torch.float64), (600, 6000, torch.float64), (1000, 2000, torch.float64), (900, 2000, torch.float32)])
+def test_tables_too_large_for_a_tile_of_32(checkers, nm, nt, dt):
+    """Tables whose moments and adjoints of 32 atoms do not fit shared memory (levels above 16 are such): contraction in tiles of 16 or 8
+    atoms, product rows in shared memory or not, squares and doubled multipliers beyond eight bits among them; energy, forces, virial,
+    descriptors and the loss gradient. Single precision: four times the distance of the CPU code's own single-precision
+    result from the double one (the sums run in another order)."""
+    chk = _chk(checkers)
+    np_dt = np.float64 if dt == torch.float64 else np.float32
+    g, nb = util.training_batch(chk, level=util.synthetic_tables(nm, nt), B=5, seed=5, nmin=1, nmax=40)
+    m, rng = g["model"], np.random.default_rng(nm)
+    m["coeffs"] = rng.normal(0, 0.1, m["coeffs"].shape)
+    m["linear_coeffs"] = rng.normal(0, 1, m["linear_coeffs"].shape)
+    desc = chk.mtp_descriptors(m, nb)
+    m["q_scaler"] = np.abs(desc[np.arange(desc.shape[1])[None] < nb["binum"][:, None]]).max(0)      # every scalar counts
+    g["model"] = {k: (v.astype(np_dt) if isinstance(v, np.ndarray) and v.dtype == np.float64 else v) for k, v in m.items()}
+    nb = dict(nb, brcs=nb["brcs"].astype(np_dt))
+    t = {k: v.astype(np_dt) for k, v in g["targets"].items()}
+    g["targets"] = t
+    npad = nb["bilist"].shape[1]
+
+    def reference(model, nb, ft):
+        e, f, v = (a.astype(ft) for a in chk.mtp_efv(model, nb))
+        grads = chk.mtp_loss_backward(model, nb, g["weights"], e, t["E"].astype(ft), f, t["F"][:, :npad].astype(ft), v, t["V"].astype(ft))
+        return (e, f, v, chk.mtp_descriptors(model, nb)) + tuple(grads)
+
+    ref = reference(util.to64(g["model"]), dict(nb, brcs=nb["brcs"].astype(np.float64)), np.float64)
+    tol = [1e-10] * 7 if dt == torch.float64 else [max(1e-5, 4 * util.relerr(a, r)) for a, r in zip(reference(g["model"], nb, np.float32), ref)]
+    prog, md, nbd, (E, F, V) = _dev(g, nb, dt)
+    got = list(capi.mtp_efv(prog, md, nbd)) + [capi.mtp_descriptors(prog, md, nbd)]
+    if nm == 600 or dt == torch.float32:      # (four arrays of eight atoms)
+        e, f, v = (torch.from_numpy(x).to(dt).cuda() for x in ref[:3])
+        got += list(capi.mtp_loss_backward(prog, md, nbd, g["weights"], e, E, f, F, v, V))
+    else:
+        e, f, v = got[:3]
+        with pytest.raises(capi.Ai2bError):
+            capi.mtp_loss_backward(prog, md, nbd, g["weights"], e, E, f, F, v, V)
+    for a, r, x, name in zip(got, ref, tol, ("energy", "force", "virial", "descriptors", "coeffs", "linear", "bias")):
+        assert util.relerr(a.cpu().numpy(), r) < x, name
+
+
 @pytest.mark.parametrize("B,cs,dt", [(1, 8, torch.float64), (9, 8, torch.float64), (9, 8, torch.float32), (3, 9, torch.float64)])
 def test_loss_op_keeps_the_moments(checkers, B, cs, dt):
     """Backward of the op on the moments of its forward (and, with nine Chebyshev functions, without) against the backward

@@ -1,12 +1,14 @@
 """Compilation of the MTP tables (host code; a user pays for it with every new model)."""
 import ctypes as C
+import os
+import subprocess
 import time
 
 import numpy as np
 import pytest
 
 import util
-from ai2pot_b200 import capi
+from ai2pot_b200 import _build, capi
 
 
 def _create(t):
@@ -37,3 +39,33 @@ def test_bad_rows_are_refused(row, value, why):
     t["alpha_index_times"][5, row] = value
     rc, _ = _create(t)
     assert rc in (-1, -2) and why in capi.lib().ai2b_last_error_string().decode()
+
+
+@pytest.fixture(scope="module")
+def host_tables(tmp_path_factory):
+    """The table compiler as a program of its own, its device memory on the host: tables -> the numbers it reports."""
+    d = tmp_path_factory.mktemp("tables")
+    here = os.path.dirname(os.path.abspath(__file__))
+    subprocess.check_call([_build._nvcc(), "-O1", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", _build.CSRC, "-o", str(d / "host"),
+                           os.path.join(here, "mtp_tables_host.cu")])
+
+    def run(t):
+        arrays = [np.ascontiguousarray(t[k], np.int32).ravel() for k in ("alpha_index_basic", "alpha_index_times", "alpha_moment_mapping")]
+        head = [int(t["alpha_moments_count"]), len(t["alpha_index_basic"]), len(t["alpha_index_times"]), len(t["alpha_moment_mapping"]), int(t["nmus"])]
+        np.concatenate([np.array(head, np.int32)] + arrays).tofile(d / "in")
+        return [int(v) for v in subprocess.run([str(d / "host"), str(d / "in")], check=True, capture_output=True, text=True).stdout.split()]
+
+    return run
+
+
+@pytest.mark.parametrize("tables", [util.tables(6), util.tables(10), util.tables(16), util.synthetic_tables(600, 2000), util.synthetic_tables(64, 96, squares=0.0)],
+                         ids=["6", "10", "16", "600x2000", "few_squares"])
+def test_rows_are_read_to_their_ends(host_tables, tables):
+    """A kernel that keeps the rows of the tables in shared memory reads the products' rows and the adjoints' rows, all of them and
+    nothing behind them: the square of a moment has one adjoint row where twice its multiplier fits eight bits, other products two."""
+    r = tables["alpha_index_times"]
+    adjoints = 2 * len(r) - int(((r[:, 0] == r[:, 1]) & (2 * r[:, 2] <= 255)).sum())
+    fwd0, rev0, fwd1, rev1, walked, room = host_tables(tables)
+    assert (fwd0, rev0, fwd1) == (len(r), 0, len(r))
+    assert walked == adjoints
+    assert rev1 == adjoints <= room

@@ -13,6 +13,29 @@ def tables(level):
     return _tables.load(level)
 
 
+def synthetic_tables(nmoments, nproducts, nscalars=40, squares=0.15, kmu=(4, 2, 0), levels=3, seed=17):
+    """Alpha tables of any size, with the properties of the template files: dense basic moments up to degree kmu[mu], products in
+    `levels` depths whose operands are complete before they are read, several products per moment, squares among them (some with a
+    multiplier that does not fit eight bits twice), scalars that are basic moments or products."""
+    rng = np.random.default_rng(seed)
+    basic = [(mu, a, b, k - a - b) for mu, top in enumerate(kmu) for k in range(top + 1) for a in range(k, -1, -1) for b in range(k - a, -1, -1)]
+    nb = len(basic)
+    level_of = np.concatenate([np.zeros(nb, int), np.sort(rng.integers(1, levels + 1, nmoments - nb))])
+    level_of[nb:nb + levels] = level_of[nmoments - levels:] = np.arange(1, levels + 1)
+    level_of[nb:] = np.sort(level_of[nb:])
+    dst = np.concatenate([np.arange(nb, nmoments), rng.integers(nb, nmoments, nproducts - (nmoments - nb))])
+    dst = dst[np.argsort(level_of[dst], kind="stable")]
+    times = np.zeros((nproducts, 4), np.int32)
+    for t, m in enumerate(dst):
+        below = int(np.searchsorted(level_of, level_of[m]))                   # moments of the depths before this one
+        a = int(rng.integers(np.searchsorted(level_of, level_of[m] - 1), below))      # one operand of the depth just before
+        b = a if rng.random() < squares else int(rng.integers(0, below))
+        times[t] = (a, b, int(rng.choice([1, 2, 3, 6, 90, 130])), m)
+    mapping = np.sort(rng.permutation(nmoments)[:nscalars])
+    return dict(alpha_moments_count=nmoments, nmus=len(kmu), alpha_index_basic=np.array(basic, np.int32), alpha_index_times=times,
+                alpha_moment_mapping=mapping.astype(np.int32))
+
+
 def canonical_nblist(numneigh, firstneigh, rcs):
     """Order-independent form: per atom, rows sorted by (neighbour index, rcs bits)."""
     n, umax = firstneigh.shape
@@ -97,8 +120,8 @@ def nblist_batch(chk, w):
 
 
 def training_batch(chk, level=10, B=3, seed=21, nmin=20, nmax=40):
-    """A small padded batch with random targets, shaped like the training configuration."""
-    g = synth.g3(tables(level), seed=seed, batch=B, nmin=nmin, nmax=nmax)
+    """A small padded batch with random targets, shaped like the training configuration. level: of the template, or tables."""
+    g = synth.g3(level if isinstance(level, dict) else tables(level), seed=seed, batch=B, nmin=nmin, nmax=nmax)
     lists = []
     for s in g["structs"]:
         nn, fn, rc, ty, mx = chk.nblist(s["cell"], s["types"], s["coords"], 5.0, g["umax"] * 2)
