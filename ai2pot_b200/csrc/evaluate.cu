@@ -30,14 +30,16 @@ static int evaluate_t(const ai2b_evaluation *e, const T *coords, void *stream)
     const T *co = (const T *)e->d_coeffs, *bias = (const T *)e->d_type_bias, *qs = (const T *)e->d_q_scaler, *rcs = (const T *)e->d_rcs;
     const T *w0 = (const T *)e->d_w0, *b0 = (const T *)e->d_b0, *w1 = (const T *)e->d_w1;
     // What the evaluation has to set up goes out with a launch of the build, unless it writes to memory that the build still works
-    // with (one buffer as the scratch of both, results in the build's scratch, or forces that replace the positions).
+    // with (one buffer as the scratch of both, results in the build's scratch, forces that replace the positions, or its status words in
+    // the scratch).
     NepSetup side;
     const void *set_up[4] = {e->d_workspace, etot, force, virial};
     const size_t n3 = 3 * sizeof(T) * (size_t)e->natoms, set_up_bytes[4] = {e->workspace_bytes, sizeof(T), n3, 9 * sizeof(T)};
     bool carried = !e->mtp;
     for (int k = 0; k < 4; k++)
         carried = carried && (!set_up[k] || (apart(set_up[k], set_up_bytes[k], e->d_nblist_workspace, e->nblist_workspace_bytes) &&
-                                             apart(set_up[k], set_up_bytes[k], coords, n3)));
+                                             apart(set_up[k], set_up_bytes[k], coords, n3) &&
+                                             apart(set_up[k], set_up_bytes[k], e->d_status, 2 * sizeof(int))));
     carried = carried && nep_plan_setup<T>(etot, force, virial, e->chebyshev_size, e->n_radial, e->n_angular, e->l_max, e->num_neurons, co, w0, b0, w1,
                                            e->natoms, e->d_binum, e->ntypes, e->umax, 0, qs, e->d_workspace, e->workspace_bytes, &side);
     if (int rc = nblist_build_periodic<T>(e->natoms, cell, coords, e->rcut, e->umax, e->d_numneigh, e->d_firstneigh, (T *)e->d_rcs, e->d_status,

@@ -118,6 +118,20 @@ def test_results_in_memory_that_the_build_reads(n, where):
         coords.copy_(torch.from_numpy(np.ascontiguousarray(w["coords"])).to(dt))
 
 
+@pytest.mark.parametrize("n", [8, 14])
+def test_status_words_in_the_scratch_of_the_evaluation(n):
+    """The build's status words where the evaluation lays its model table: they are the build's until the rows stand, and the memory is
+    the evaluation's after that. (Negative values: the build would raise them to its counts.)"""
+    w, dt, tol = _workload("nep", n)
+    w["model"]["coeffs"] = -np.abs(w["model"]["coeffs"])
+    ev = engine.Evaluator(w["model"], w["cell"], w["types"], w["rcut"], w["umax"], dt)
+    coords = torch.from_numpy(np.ascontiguousarray(w["coords"])).to(dt).cuda()
+    apart = _host(ev.compute(coords))
+    ev.lists = ev.lists[:3] + (ev.ws[256:264].view(torch.int32),)      # (the table follows the offsets of one structure)
+    ev._filled = None
+    _close(_host(ev.compute(coords)), apart, tol)
+
+
 @pytest.mark.parametrize("kind", ["mtp", "nep"])
 def test_changed_attributes_take_effect(kind):
     """Cell, cutoff, row width and model may be edited or assigned between calls (a variable-cell relaxation does): the next
