@@ -855,7 +855,8 @@ static int dispatch_contract(const MtpProgramDev &P, const MtpArgs<T> &A, long a
     if (pair_fits<T, MODE, 32>(P)) {
         constexpr int SMALL = sizeof(T) == 8 ? 16 : 32;
         const long small_tiles = (atoms_upper + SMALL - 1) / SMALL, tiles = (atoms_upper + 31) / 32;
-        if (small_tiles <= sm_count()) return launch_pair<T, MODE, SMALL, MTP_PAIR_WARPS>(P, A, small_tiles, st);
+        // (its rows may be longer in all, where a phase has fewer moments than groups of lanes: more than half a tile saves)
+        if (small_tiles <= sm_count() && pair_fits<T, MODE, SMALL>(P)) return launch_pair<T, MODE, SMALL, MTP_PAIR_WARPS>(P, A, small_tiles, st);
         if (tiles > sm_count() && pair_fits<T, MODE, 32, MTP_PAIR_FEW>(P)) return launch_pair<T, MODE, 32, MTP_PAIR_FEW>(P, A, tiles, st);
         return launch_pair<T, MODE, 32, MTP_PAIR_WARPS>(P, A, tiles, st);
     }

@@ -96,6 +96,30 @@ def test_lanes_share_the_slots_of_an_atom(checkers, natoms, level, dt):
         assert util.relerr(a, r) < TOL[dt], name
 
 
+@pytest.mark.parametrize("natoms", [27, 2400])
+def test_tables_that_fit_tiles_of_32_atoms_only(checkers, natoms):
+    """Sixteen moments in a chain, each the sum of 300 products: the rows of a tile of 16 atoms (four groups of lanes per warp, of
+    which one moment fills one) take twice the shared memory of those of 32, more than the tile itself saves."""
+    levels, rows = 16, 300
+    rng = np.random.default_rng(natoms)
+    tables = dict(alpha_moments_count=4 + levels, nmus=1, alpha_moment_mapping=np.arange(4 + levels, dtype=np.int32),
+                  alpha_index_basic=np.array([[0, 0, 0, 0], [0, 1, 0, 0], [0, 0, 1, 0], [0, 0, 0, 1]], np.int32),
+                  alpha_index_times=np.array([(3 + k if k else 0, r % 4, 1, 4 + k) for k in range(levels) for r in range(rows)], np.int32))
+    cell, pos = synth.cubic_lattice(int(np.ceil(natoms ** (1 / 3) - 1e-9)), 3.0, 0.1, rng, np.float64, nocc=natoms)
+    w = dict(cell=cell, coords=pos, types=rng.integers(0, 3, natoms).astype(np.int32), rcut=5.0, umax=48,
+             model=synth.mtp_model(tables, 3, rng, np.float64, 5.0, 0.5, sigma=0.1))
+    chk = _chk(checkers)
+    nb = util.nblist_batch(chk, w)
+    desc = chk.mtp_descriptors(w["model"], nb)
+    w["model"].update(q_scaler=np.abs(desc[0]).max(0), linear_coeffs=rng.normal(0, 1, desc.shape[2]))      # every scalar counts
+    (e, f, v), prog, md, nbd = _run(w, nb)
+    e2, f2 = capi.mtp_efv(prog, md, nbd, virial=False)
+    er, fr, vr = chk.mtp_efv(w["model"], nb)
+    for a, r, name in ((e, er, "energy"), (f, fr, "force"), (v, vr, "virial"), (e2.cpu().numpy(), er, "energy"), (f2.cpu().numpy(), fr, "force"),
+                       (capi.mtp_descriptors(prog, md, nbd).cpu().numpy(), desc, "descriptors")):
+        assert util.relerr(a, r) < 1e-10, name
+
+
 def test_many_neighbours_and_ragged_batch(checkers):
     """> 32 neighbours per atom (two lane chunks), padded batch with an empty structure and ghosts."""
     chk = _chk(checkers)
