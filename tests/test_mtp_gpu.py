@@ -120,6 +120,23 @@ def test_tables_that_fit_tiles_of_32_atoms_only(checkers, natoms):
         assert util.relerr(a, r) < 1e-10, name
 
 
+@pytest.mark.parametrize("level,dt,natoms", [(6, np.float64, 5003), (10, np.float64, 4737), (10, np.float32, 9001)])
+def test_blocks_of_eight_warps_without_virial(checkers, level, dt, natoms):
+    """Small tables with more tiles than SMs: energy and forces without the virial, and descriptors."""
+    rng = np.random.default_rng(natoms)
+    cell, pos = synth.cubic_lattice(int(np.ceil(natoms ** (1 / 3) - 1e-9)), 3.0, 0.1, rng, np.float64, nocc=natoms)
+    w = util.small_mtp_case(level, 2, dt)
+    w.update(cell=cell, coords=pos.astype(dt).astype(np.float64), types=rng.integers(0, 3, natoms).astype(np.int32))
+    chk = _chk(checkers)
+    nb = util.nblist_batch(chk, w)
+    nb["brcs"] = nb["brcs"].astype(dt)
+    model, nb64 = util.to64(w["model"]), dict(nb, brcs=nb["brcs"].astype(np.float64))
+    (e, f), prog, md, nbd = _run(w, nb, virial=False)
+    er, fr, _ = chk.mtp_efv(model, nb64)
+    for a, r, name in ((e, er, "energy"), (f, fr, "force"), (capi.mtp_descriptors(prog, md, nbd).cpu().numpy(), chk.mtp_descriptors(model, nb64), "descriptors")):
+        assert util.relerr(a, r) < TOL[dt], name
+
+
 def test_many_neighbours_and_ragged_batch(checkers):
     """> 32 neighbours per atom (two lane chunks), padded batch with an empty structure and ghosts."""
     chk = _chk(checkers)
