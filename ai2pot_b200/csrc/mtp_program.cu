@@ -317,13 +317,18 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
     };
     const auto [row_at, rows_of] = by_moment(nt, [&](int t) { return times[4 * t + 3]; });
     const auto [occ_at, occ_of] = by_moment(2 * nt, [&](int o) { return times[4 * (o >> 1) + (o & 1)]; });
-    // moments of one depth, heavy ones first
+    // The square of a moment: both of its places as an operand (they follow one another) are one adjoint row.
+    auto both_places = [&](const int *r) { return r[0] == r[1] && r[2] <= 127; };
+    std::vector<int> fwd_count(nm), rev_count(nm);      // rows of each moment
+    for (int m = 0; m < nm; m++) { fwd_count[m] = row_at[m + 1] - row_at[m]; rev_count[m] = occ_at[m + 1] - occ_at[m]; }
+    for (int t = 0; t < nt; t++) rev_count[times[4 * t]] -= both_places(times + 4 * t);
+    // moments of one depth, those with the most rows first
     std::vector<int> members;
-    auto moments_of_depth = [&](int lev, const std::vector<int> &at) -> const std::vector<int> & {
+    auto moments_of_depth = [&](int lev, const std::vector<int> &count) -> const std::vector<int> & {
         members.clear();
         for (int m = 0; m < nm; m++)
-            if (depth[m] == lev && at[m + 1] > at[m]) members.push_back(m);
-        std::stable_sort(members.begin(), members.end(), [&](int x, int y) { return at[x + 1] - at[x] > at[y + 1] - at[y]; });
+            if (depth[m] == lev && count[m] > 0) members.push_back(m);
+        std::stable_sort(members.begin(), members.end(), [&](int x, int y) { return count[x] > count[y]; });
         return members;
     };
     auto bits_f = [](int mult) { const float f = (float)mult; int b; memcpy(&b, &f, 4); return b; };
@@ -341,8 +346,8 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
     P.fwd_lev_off[0] = P.fwd_lev_row[0] = 0;
     for (int lev = 1; lev <= MTP_MAX_LEV; lev++) {
         if (lev <= P.nlev)
-            for (int m : moments_of_depth(lev, row_at)) {
-                const int rb = (int)fwd_rows.size(), re = rb + row_at[m + 1] - row_at[m];
+            for (int m : moments_of_depth(lev, fwd_count)) {
+                const int rb = (int)fwd_rows.size(), re = rb + fwd_count[m];
                 for (int i = row_at[m]; i < row_at[m + 1]; i++) {
                     const int *r = times + 4 * rows_of[i];
                     add_row(fwd_rows, fwd_flat, r[0] | (r[1] << 16), r[2], m, i + 1 == row_at[m + 1]);
@@ -356,12 +361,11 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
     P.rev_lev_off[0] = P.rev_lev_row[0] = 0;
     for (int k = 0; k < MTP_MAX_LEV; k++) {
         if (k < P.nlev)
-            for (int m : moments_of_depth(P.nlev - 1 - k, occ_at)) {
+            for (int m : moments_of_depth(P.nlev - 1 - k, rev_count)) {
                 const int rb = (int)rev_ents.size();
                 for (int i = occ_at[m]; i < occ_at[m + 1]; i++) {
                     const int o = occ_of[i], *r = times + 4 * (o >> 1);
-                    // the square of a moment: both of its places (they follow one another) in one row
-                    const bool both = !(o & 1) && r[0] == r[1] && 2 * r[2] <= 255;
+                    const bool both = !(o & 1) && both_places(r);
                     if (both) i++;
                     add_row(rev_ents, rev_flat, r[1 - (o & 1)] | (r[3] << 16), both ? 2 * r[2] : r[2], m, i + 1 == occ_at[m + 1]);
                 }

@@ -42,7 +42,18 @@ int main(int, char **argv)
             stage_product_rows(P, Watched{&fwd}, Watched{&rev}, adjoints, to.data(), t, threads, ScaledRow<17, true>());
         printf("%d %d ", fwd, rev);
     }
-    // adjoint rows that the kernels' loops walk through, and the room that rev_flat has
-    printf("%d %ld\n", P.rev_lev_row[P.nlev], (long)((end - (const unsigned char *)P.rev_flat) / sizeof(int2)));
+    // adjoint rows that the kernels' loops walk through, the room that rev_flat has, and the phases whose moments do not come with the
+    // most rows first
+    int unordered = 0;
+    auto look = [&](const int4 *q, const int *off) {
+        for (int lev = 0; lev < P.nlev; lev++) {
+            bool ordered = true;
+            for (int i = off[lev] + 1; i < off[lev + 1]; i++) ordered = ordered && q[i].z - q[i].y <= q[i - 1].z - q[i - 1].y;
+            unordered += !ordered;
+        }
+    };
+    look(P.fwd_dst, P.fwd_lev_off);
+    look(P.rev_mom, P.rev_lev_off);
+    printf("%d %ld %d\n", P.rev_lev_row[P.nlev], (long)((end - (const unsigned char *)P.rev_flat) / sizeof(int2)), unordered);
     ai2b_mtp_program_destroy(prog);
 }

@@ -58,14 +58,23 @@ def host_tables(tmp_path_factory):
     return run
 
 
-@pytest.mark.parametrize("tables", [util.tables(6), util.tables(10), util.tables(16), util.synthetic_tables(600, 2000), util.synthetic_tables(64, 96, squares=0.0)],
-                         ids=["6", "10", "16", "600x2000", "few_squares"])
+ANY_TABLES = pytest.mark.parametrize("tables", [util.tables(6), util.tables(10), util.tables(16), util.synthetic_tables(600, 2000),
+                                                util.synthetic_tables(64, 96, squares=0.0)], ids=["6", "10", "16", "600x2000", "few_squares"])
+
+
+@ANY_TABLES
 def test_rows_are_read_to_their_ends(host_tables, tables):
     """A kernel that keeps the rows of the tables in shared memory reads the products' rows and the adjoints' rows, all of them and
     nothing behind them: the square of a moment has one adjoint row where twice its multiplier fits eight bits, other products two."""
     r = tables["alpha_index_times"]
     adjoints = 2 * len(r) - int(((r[:, 0] == r[:, 1]) & (2 * r[:, 2] <= 255)).sum())
-    fwd0, rev0, fwd1, rev1, walked, room = host_tables(tables)
+    fwd0, rev0, fwd1, rev1, walked, room, _ = host_tables(tables)
     assert (fwd0, rev0, fwd1) == (len(r), 0, len(r))
     assert walked == adjoints
     assert rev1 == adjoints <= room
+
+
+@ANY_TABLES
+def test_moments_are_dealt_in_order_of_their_rows(host_tables, tables):
+    """The deal of a phase's rows to warps takes the moments with the most rows first, equal ones side by side."""
+    assert host_tables(tables)[-1] == 0
