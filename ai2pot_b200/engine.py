@@ -209,7 +209,8 @@ class Evaluator:
     def launches_per_step(self):
         """Kernels of this library that one compute() on a fully periodic cell launches (memsets not counted): neighbour build,
         then forward, contraction and force of MTP (and a set-up launch when the radial coefficient rows have to be padded to
-        eight entries), or those of NEP (whose set-up goes out with a launch of the build)."""
+        eight entries), or those of NEP (whose set-up goes out with a launch of the build: one more where buffers were replaced by ones
+        that it shares with the build)."""
         build = capi.nblist_build_launches(self.n, self.cell, self.rcut)
         if self.kind == "mtp":
             return build + 3 + (0 if int(self.model["chebyshev_size"]) == 8 else 1)

@@ -209,7 +209,8 @@ def run_md_benchmark(w, steps, warmup, dist, sampler):
                 "note": "host-timed synchronous call; the kernels are those of the nep workload", "max_neighbours": int(mx),
                 "local_atoms": nlocal, "ghost_atoms": nghost}
     nall = nlocal + nghost
-    return dict(t_dev=t, t_e2e=t, clocks=clocks, launches=(4 + 1) * steps, h2d=nall * 28, d2h=nall * 12 + 48, units=nlocal,
+    # kernels of a step: three of binning (the last with the set-up of the evaluation), rows, evaluation, copy of the results
+    return dict(t_dev=t, t_e2e=t, clocks=clocks, launches=(3 + 1 + 1 + 1) * steps, h2d=nall * 28, d2h=nall * 12 + 48, units=nlocal,
                 e2e_path="host double positions + types of local and ghost atoms -> ai2b_md_session_compute -> host forces (+=), energy, virial[6]",
                 roofline=roofline, parts_ms=None, host_ms_per_call=1e3 * t / steps)
 
