@@ -386,13 +386,12 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
     std::vector<int2> stream_d[4], stream_f[4], stream_warp[4];
     std::vector<int> adj_const;
     {
-        std::vector<char> is_source(nm, 0), is_mapped(nm, 0);
+        std::vector<char> is_source(nm, 0);
         for (int t = 0; t < nt; t++) { is_source[times[4 * t]] = 1; is_source[times[4 * t + 1]] = 1; }
-        for (int s = 0; s < ns; s++) is_mapped[mapping[s]] = 1;
-        // moments whose adjoint is just their seed: scalars that are no operand of any product, and basic
-        // moments nothing uses (seed 0); every other adjoint that is read is written by a gather phase
+        // moments whose adjoint is just their seed (0 where no scalar is mapped to them, as for products that nothing uses);
+        // every other adjoint is written by a gather phase
         for (int m = 0; m < nm; m++)
-            if (!is_source[m] && (is_mapped[m] || m < nb)) adj_const.push_back(m);
+            if (!is_source[m]) adj_const.push_back(m);
     }
     for (int k = 0; k < 4; k++) {
         const int groups = k % 2 == 0 ? 2 : 4, warps = k < 2 ? MTP_PAIR_WARPS : MTP_PAIR_FEW;

@@ -1,5 +1,6 @@
 // Compiles MTP tables into host memory (malloc and memcpy take the place of the device's) and reports, as one line of
-// numbers, what the kernels would read of them. Input: int32 nm nb nt ns nmus, basic, times, mapping.
+// numbers, what the kernels would read of them; with a second argument, what they would read before it is written.
+// Input: int32 nm nb nt ns nmus, basic, times, mapping.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -20,7 +21,7 @@ struct Watched {      // an array of the tables: remembers how far it was read, 
     int2 operator[](int i) const { *read = std::max(*read, i + 1); return make_int2(0, 0); }
 };
 
-int main(int, char **argv)
+int main(int argc, char **argv)
 {
     std::vector<int> in;
     FILE *f = fopen(argv[1], "rb");
@@ -33,6 +34,15 @@ int main(int, char **argv)
         return 1;
     }
     const MtpProgramDev &P = prog->dev;
+    if (argc > 2) {      // adjoints of products that the adjoint rows read, and that neither a row nor the list of seeds finishes
+        std::vector<char> written(nm, 0);
+        for (int i = 0; i < P.n_adj_const; i++) written[P.adj_const[i]] = 1;
+        for (int i = 0; i < P.rev_lev_off[P.nlev]; i++) written[P.rev_mom[i].x] = 1;
+        int missing = 0;
+        for (int i = 0; i < P.adjoint_rows(); i++) missing += !written[P.rev_ents[i].x >> 16 & 0xffff];
+        printf("%d\n", missing);
+        return 0;
+    }
     const unsigned char *end = (const unsigned char *)prog->d_blob + prog->blob_bytes;
     std::vector<int2> to(3 * (size_t)nt);      // what the kernels keep for the rows
     const int threads = 1024;

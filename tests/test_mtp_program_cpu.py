@@ -49,11 +49,11 @@ def host_tables(tmp_path_factory):
     subprocess.check_call([_build._nvcc(), "-O1", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", _build.CSRC, "-o", str(d / "host"),
                            os.path.join(here, "mtp_tables_host.cu")])
 
-    def run(t):
+    def run(t, *mode):
         arrays = [np.ascontiguousarray(t[k], np.int32).ravel() for k in ("alpha_index_basic", "alpha_index_times", "alpha_moment_mapping")]
         head = [int(t["alpha_moments_count"]), len(t["alpha_index_basic"]), len(t["alpha_index_times"]), len(t["alpha_moment_mapping"]), int(t["nmus"])]
         np.concatenate([np.array(head, np.int32)] + arrays).tofile(d / "in")
-        return [int(v) for v in subprocess.run([str(d / "host"), str(d / "in")], check=True, capture_output=True, text=True).stdout.split()]
+        return [int(v) for v in subprocess.run([str(d / "host"), str(d / "in"), *mode], check=True, capture_output=True, text=True).stdout.split()]
 
     return run
 
@@ -78,3 +78,9 @@ def test_rows_are_read_to_their_ends(host_tables, tables):
 def test_moments_are_dealt_in_order_of_their_rows(host_tables, tables):
     """The deal of a phase's rows to warps takes the moments with the most rows first, equal ones side by side."""
     assert host_tables(tables)[-1] == 0
+
+
+@ANY_TABLES
+def test_every_adjoint_that_is_read_is_written(host_tables, tables):
+    """A product that no other product and no scalar uses has the adjoint zero, and the rows of its operands read it."""
+    assert host_tables(tables, "uses") == [0]
