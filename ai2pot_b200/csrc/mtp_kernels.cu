@@ -533,6 +533,7 @@ __global__ void __launch_bounds__(W * 32, W == MTP_PAIR_FEW ? 4 : 1) mtp_contrac
     };
 
     __syncthreads();         // tables staged
+    for (int i = rw; i < P.n_empty; i += NR) S.M[P.empty[i] * TA + at] = T(0);
     if (MODE != MODE_DESC) {
         // moments no product reads: their adjoint is their seed for every atom of every tile, written once
         for (int i = rw; i < P.n_adj_const; i += NR) {

@@ -428,6 +428,7 @@ __global__ void __launch_bounds__(W * 32, W == MTP_PAIR_FEW ? 4 : 1) mtp_loss_pa
     __syncthreads();
     for (int s = threadIdx.x; s < P.ns; s += NT) atomicAdd(S.seed + P.map[s], A.lin[s] / A.qs[s]);
     __syncthreads();
+    for (int i = rw; i < P.n_empty; i += W * RW) S.M[P.empty[i] * TA + at] = D[P.empty[i] * TA + at] = T(0);
     // moments no product reads: adjoint = seed, no second-order adjoint
     for (int i = rw; i < P.n_adj_const; i += W * RW) {
         const int m = P.adj_const[i];

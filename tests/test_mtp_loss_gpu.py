@@ -212,6 +212,23 @@ def test_tables_too_large_for_a_tile_of_32(checkers, nm, nt, dt):
         assert util.relerr(a.cpu().numpy(), r) < x, name
 
 
+@pytest.mark.parametrize("B", [3, 200])
+def test_idle_moments(checkers, B):
+    """Tables with products that nothing uses and moments that nothing fills, in blocks of 32 and of eight warps."""
+    chk = _chk(checkers)
+    g, nb = util.training_batch(chk, level=util.tables_with_idle_moments(), B=B, seed=B, nmin=20, nmax=40)
+    rng = np.random.default_rng(B)
+    g["model"].update(coeffs=rng.normal(0, 0.1, g["model"]["coeffs"].shape), linear_coeffs=rng.normal(0, 1, g["model"]["linear_coeffs"].shape))
+    prog, md, nbd, (E, F, V) = _dev(g, nb)
+    t, npad = g["targets"], nb["bilist"].shape[1]
+    e, f, v = capi.mtp_efv(prog, md, nbd)
+    er, fr, vr = ref = chk.mtp_efv(g["model"], nb)
+    got = [e, f, v, capi.mtp_descriptors(prog, md, nbd)] + list(capi.mtp_loss_backward(prog, md, nbd, g["weights"], e, E, f, F, v, V))
+    ref = list(ref) + [chk.mtp_descriptors(g["model"], nb)] + list(chk.mtp_loss_backward(g["model"], nb, g["weights"], er, t["E"], fr, t["F"][:, :npad], vr, t["V"]))
+    for a, r, name in zip(got, ref, ("energy", "force", "virial", "descriptors", "coeffs", "linear", "bias")):
+        assert util.relerr(a.cpu().numpy(), r) < 1e-10, name
+
+
 @pytest.mark.parametrize("B,cs,dt", [(1, 8, torch.float64), (9, 8, torch.float64), (9, 8, torch.float32), (3, 9, torch.float64)])
 def test_loss_op_keeps_the_moments(checkers, B, cs, dt):
     """Backward of the op on the moments of its forward (and, with nine Chebyshev functions, without) against the backward

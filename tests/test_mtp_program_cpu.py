@@ -84,3 +84,8 @@ def test_moments_are_dealt_in_order_of_their_rows(host_tables, tables):
 def test_every_adjoint_that_is_read_is_written(host_tables, tables):
     """A product that no other product and no scalar uses has the adjoint zero, and the rows of its operands read it."""
     assert host_tables(tables, "uses") == [0]
+
+
+def test_idle_moments_are_filled(host_tables):
+    """Moments that are neither basic nor a product are zero, and nothing reads what was not written."""
+    assert host_tables(util.tables_with_idle_moments(), "uses") == [0]

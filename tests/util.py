@@ -36,6 +36,17 @@ def synthetic_tables(nmoments, nproducts, nscalars=40, squares=0.15, kmu=(4, 2, 
                 alpha_moment_mapping=mapping.astype(np.int32))
 
 
+def tables_with_idle_moments():
+    """Level 10 with moments that the templates do not have: a product that nothing uses, a moment that no product fills and a scalar is mapped
+    to, and another one that is an operand (their value is zero)."""
+    t = {k: (v.copy() if isinstance(v, np.ndarray) else v) for k, v in tables(10).items()}
+    m = int(t["alpha_moments_count"])
+    t["alpha_index_times"] = np.concatenate([t["alpha_index_times"], np.array([(0, 1, 2, m), (3, m + 2, 3, m + 3)], np.int32)])
+    t["alpha_moment_mapping"] = np.concatenate([t["alpha_moment_mapping"], np.array([m + 1, m + 3], np.int32)])
+    t["alpha_moments_count"] = m + 4
+    return t
+
+
 def canonical_nblist(numneigh, firstneigh, rcs):
     """Order-independent form: per atom, rows sorted by (neighbour index, rcs bits)."""
     n, umax = firstneigh.shape
