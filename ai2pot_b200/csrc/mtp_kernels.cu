@@ -533,13 +533,11 @@ __global__ void __launch_bounds__(W * 32, W == MTP_PAIR_FEW ? 4 : 1) mtp_contrac
     };
 
     __syncthreads();         // tables staged
-    for (int i = rw; i < P.n_empty; i += NR) S.M[P.empty[i] * TA + at] = T(0);
-    if (MODE != MODE_DESC) {
-        // moments no product reads: their adjoint is their seed for every atom of every tile, written once
-        for (int i = rw; i < P.n_adj_const; i += NR) {
-            const int m = P.adj_const[i];
-            S.E[m * TA + at] = S.seed[m];
-        }
+    // written once, for every atom of every tile: adjoints that are only their seed, moments that are always zero
+    for (int i = rw + (MODE == MODE_DESC ? P.n_adj_const : 0); i < P.n_constant; i += NR) {
+        const int m = P.constant[i];
+        if (MODE != MODE_DESC && i < P.n_adj_const) S.E[m * TA + at] = S.seed[m];
+        else S.M[m * TA + at] = T(0);
     }
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         // (no barrier here: the last adjoint phase ended with one, after which the moments are no longer read, and the

@@ -428,12 +428,11 @@ __global__ void __launch_bounds__(W * 32, W == MTP_PAIR_FEW ? 4 : 1) mtp_loss_pa
     __syncthreads();
     for (int s = threadIdx.x; s < P.ns; s += NT) atomicAdd(S.seed + P.map[s], A.lin[s] / A.qs[s]);
     __syncthreads();
-    for (int i = rw; i < P.n_empty; i += W * RW) S.M[P.empty[i] * TA + at] = D[P.empty[i] * TA + at] = T(0);
-    // moments no product reads: adjoint = seed, no second-order adjoint
-    for (int i = rw; i < P.n_adj_const; i += W * RW) {
-        const int m = P.adj_const[i];
-        S.E[m * TA + at] = S.seed[m];
-        Gm[m * TA + at] = T(0);
+    // adjoints that are only their seed (no second-order adjoint), moments that are always zero
+    for (int i = rw; i < P.n_constant; i += W * RW) {
+        const int m = P.constant[i];
+        (i < P.n_adj_const ? S.E : S.M)[m * TA + at] = i < P.n_adj_const ? S.seed[m] : T(0);
+        (i < P.n_adj_const ? Gm : D)[m * TA + at] = T(0);
     }
     chain_wait();        // everything above reads the program's tables and the model only
     const int ntot = A.prefix[A.B], ntiles = (ntot + TA - 1) / TA;

@@ -384,16 +384,18 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
 
     // row streams (see mtp_program.cuh)
     std::vector<int2> stream_d[4], stream_f[4], stream_warp[4];
-    std::vector<int> adj_const, empty;
+    std::vector<int> constant;
     {
         std::vector<char> is_source(nm, 0);
         for (int t = 0; t < nt; t++) { is_source[times[4 * t]] = 1; is_source[times[4 * t + 1]] = 1; }
         // moments whose adjoint is just their seed (0 where no scalar is mapped to them, as for products that nothing uses);
         // every other adjoint is written by a gather phase
         for (int m = 0; m < nm; m++)
-            if (!is_source[m]) adj_const.push_back(m);
+            if (!is_source[m]) constant.push_back(m);
+        P.n_adj_const = (int)constant.size();
         for (int m = nb; m < nm; m++)
-            if (fwd_count[m] == 0) empty.push_back(m);
+            if (fwd_count[m] == 0) constant.push_back(m);
+        P.n_constant = (int)constant.size();
     }
     for (int k = 0; k < 4; k++) {
         const int groups = k % 2 == 0 ? 2 : 4, warps = k < 2 ? MTP_PAIR_WARPS : MTP_PAIR_FEW;
@@ -446,12 +448,10 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
         for (int g = 0; g < 2 * groups; g++) { stream_d[k].push_back(make_int2(0, 0)); stream_f[k].push_back(make_int2(0, 0)); }   // read ahead
         P.stream[k].nrows = (int)(stream_d[k].size() / groups);
     }
-    P.n_adj_const = (int)adj_const.size();
-    P.n_empty = (int)empty.size();
 
     Blob blob;
     blob.bytes.reserve(64 * 1024 + 128 * (size_t)(nm + nt) + 16 * (stream_d[0].size() + stream_d[1].size()));
-    size_t o_ac = blob.add(adj_const), o_em = blob.add(empty), o_sd[4], o_sf[4], o_sw[4];
+    size_t o_c = blob.add(constant), o_sd[4], o_sf[4], o_sw[4];
     for (int k = 0; k < 4; k++) { o_sd[k] = blob.add(stream_d[k]); o_sf[k] = blob.add(stream_f[k]); o_sw[k] = blob.add(stream_warp[k]); }
     size_t o_bd = blob.add(basic_dense), o_db = blob.add(dense_basic), o_e4d = blob.add(e4d), o_g = blob.add(e4g), o_m = blob.add(e4m), o_fd = blob.add(fwd_dst),
            o_rm = blob.add(rev_mom), o_map = blob.add(map);
@@ -481,8 +481,7 @@ extern "C" int ai2b_mtp_program_create(int nm, int nb, const int *basic, int nt,
     P.rev_ents = (const int2 *)(b + o_rent);
     P.fwd_flat = (const int2 *)(b + o_ff);
     P.rev_flat = (const int2 *)(b + o_rf);
-    P.adj_const = (const int *)(b + o_ac);
-    P.empty = (const int *)(b + o_em);
+    P.constant = (const int *)(b + o_c);
     for (int k = 0; k < 4; k++) {
         P.stream[k].row_d = (const int2 *)(b + o_sd[k]);
         P.stream[k].row_f = (const int2 *)(b + o_sf[k]);

@@ -52,9 +52,8 @@ struct MtpProgramDev {
         const int2 *warp;               // [2 nlev][warps] {first row, rows}
         int nrows;                      // 0: the tables do not fit the encoding, or have too many rows for few warps
     } stream[4];                        // GL = 16, GL = 8 for MTP_PAIR_WARPS warps; the same for MTP_PAIR_FEW
-    const int *adj_const;           // [n_adj_const] moments whose adjoint is only their seed (no product reads them)
-    const int *empty;               // [n_empty] moments that are neither basic nor a product: zero
-    int n_adj_const, n_empty;
+    const int *constant;            // [n_adj_const] moments whose adjoint is only their seed (no product reads them), then, up to
+    int n_adj_const, n_constant;    // n_constant, moments that are neither basic nor a product: zero
     // two per product, one for the square of a moment (unless twice its multiplier exceeds 255)
     __host__ __device__ int adjoint_rows() const { return rev_lev_row[nlev]; }
 };

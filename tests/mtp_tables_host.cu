@@ -37,9 +37,9 @@ int main(int argc, char **argv)
     if (argc > 2) {      // operands of products and of scalars that nothing fills, adjoints that neither a row nor the list of seeds finishes
         std::vector<char> filled(nm, 0), finished(nm, 0);
         for (int m = 0; m < nb; m++) filled[m] = 1;
-        for (int i = 0; i < P.n_empty; i++) filled[P.empty[i]] = 1;
+        for (int i = P.n_adj_const; i < P.n_constant; i++) filled[P.constant[i]] = 1;
         for (int i = 0; i < P.fwd_lev_off[P.nlev]; i++) filled[P.fwd_dst[i].x] = 1;
-        for (int i = 0; i < P.n_adj_const; i++) finished[P.adj_const[i]] = 1;
+        for (int i = 0; i < P.n_adj_const; i++) finished[P.constant[i]] = 1;
         for (int i = 0; i < P.rev_lev_off[P.nlev]; i++) finished[P.rev_mom[i].x] = 1;
         int missing = 0;
         for (int i = 0; i < P.nt; i++) missing += !filled[P.fwd_rows[i].x & 0xffff] + !filled[P.fwd_rows[i].x >> 16 & 0xffff];
