@@ -470,7 +470,7 @@ __host__ __device__ inline size_t pair_smem_layout(const MtpProgramDev &P, unsig
 template <typename T, int MODE, int TA, int W = MTP_PAIR_WARPS>
 static bool pair_fits(const MtpProgramDev &P)
 {
-    return P.stream[pair_stream<T>(TA, W)].nrows > 0 && pair_smem_layout<T, MODE, TA, W>(P, nullptr, nullptr) <= 226 * 1024;
+    return P.stream[pair_stream<T>(TA, W)].nrows > 0 && pair_smem_layout<T, MODE, TA, W>(P, nullptr, nullptr) <= (W == MTP_PAIR_FEW ? MTP_PAIR_FEW_BYTES : MTP_PAIR_BYTES);
 }
 
 template <typename T, int MODE, int TA, int W>

@@ -684,7 +684,7 @@ static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArg
         AI2B_CUDA(cudaGetLastError());
     }
     const size_t pair_bytes = loss_pair_smem<T, MTP_PAIR_WARPS>(P, nullptr, nullptr);
-    const bool pair = P.stream[1].nrows > 0 && pair_bytes <= 226 * 1024;
+    const bool pair = P.stream[1].nrows > 0 && pair_bytes <= MTP_PAIR_BYTES;
     const long pair_tiles = (atoms_upper + loss_ta<T>() - 1) / loss_ta<T>();
     // the coefficient gradient by tiles pays once they occupy half of the SMs; below that a warp per atom is over sooner
     // (level 10, fp32, 240 atoms: 11 against 14 us; level 16, fp64, 9,323 atoms: 99 against 87)
@@ -708,7 +708,7 @@ static int launch_loss_bwd_v(const ai2b_mtp_program *prog, MtpArgs<T> A, LossArg
                 return AI2B_OK;
             };
             // (few warps per block as in the contraction of the forces)
-            const bool few = pair_tiles > sm_count() && P.stream[3].nrows > 0 && loss_pair_smem<T, MTP_PAIR_FEW>(P, nullptr, nullptr) <= 226 * 1024;
+            const bool few = pair_tiles > sm_count() && P.stream[3].nrows > 0 && loss_pair_smem<T, MTP_PAIR_FEW>(P, nullptr, nullptr) <= MTP_PAIR_FEW_BYTES;
             rc = few ? run(std::integral_constant<int, MTP_PAIR_FEW>{}) : run(std::integral_constant<int, MTP_PAIR_WARPS>{});
             done = true;
         }

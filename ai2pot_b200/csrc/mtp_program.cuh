@@ -81,8 +81,10 @@ __host__ __device__ inline void stage_product_rows(const MtpProgramDev &P, Rows 
 // Warps of a block of the contractions. A phase of a small table is over before 32 warps have met: where there are more tiles than
 // SMs such tables (levels up to 10, of 42 products; level 16 has 969 and fills 32 warps) take blocks of eight warps, four of which share
 // an SM. Level 10, whole call, us, 32 / 8 warps: fp64 6,000 atoms 51.6 / 48.5, 13,824 atoms 73.2 / 67.2, 100,000 atoms 361 / 303; with a
-// tile per SM 32 warps are sooner over it (2,500 atoms 34.8 / 37.2).
+// tile per SM 32 warps are sooner over it (2,500 atoms 34.8 / 37.2). Tables whose moments leave room for fewer than three such blocks
+// stay with 32 warps: 20,000 atoms, fp64, 100 products, 230 moments 155 us with eight warps, 142 with 32; 128 products, 90 moments 104 / 113.
 constexpr int MTP_PAIR_WARPS = 32, MTP_PAIR_FEW = 8, MTP_PAIR_FEW_ROWS = 128;
+constexpr size_t MTP_PAIR_BYTES = 226 * 1024, MTP_PAIR_FEW_BYTES = 75 * 1024;      // shared memory of a block at most
 constexpr int MTP_PAIR_WIDE = 0x800;
 constexpr int MTP_TILE = 32;        // atoms per tile of the workspace
 

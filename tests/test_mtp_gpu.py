@@ -137,6 +137,28 @@ def test_blocks_of_eight_warps_without_virial(checkers, level, dt, natoms):
         assert util.relerr(a, r) < TOL[dt], name
 
 
+@pytest.mark.parametrize("nm,nt,kmu,dt", [(110, 64, (4, 2, 0), np.float64), (230, 100, (6, 4, 2, 0), np.float64), (230, 100, (6, 4, 2, 0), np.float32)])
+def test_few_products_over_many_moments(checkers, nm, nt, kmu, dt):
+    """Few products, more tiles than SMs: blocks of 32 warps where three of eight do not fit an SM (the second case). Single precision:
+    four times the distance of the CPU code's own single-precision result."""
+    natoms = 5003
+    rng = np.random.default_rng(nm)
+    cell, pos = synth.cubic_lattice(int(np.ceil(natoms ** (1 / 3) - 1e-9)), 3.0, 0.1, rng, np.float64, nocc=natoms)
+    model = synth.mtp_model(util.synthetic_tables(nm, nt, kmu=kmu), 3, rng, np.float64, 5.0, 0.5, sigma=0.1)
+    w = dict(cell=cell, coords=pos.astype(dt).astype(np.float64), types=rng.integers(0, 3, natoms).astype(np.int32), rcut=5.0, umax=48, model=model)
+    chk = _chk(checkers)
+    nb = util.nblist_batch(chk, w)
+    desc = chk.mtp_descriptors(model, nb)
+    model.update(q_scaler=np.abs(desc[0]).max(0), linear_coeffs=rng.normal(0, 1, desc.shape[2]))      # every scalar counts
+    w["model"] = {k: (v.astype(dt) if isinstance(v, np.ndarray) and v.dtype == np.float64 else v) for k, v in model.items()}
+    nb["brcs"] = nb["brcs"].astype(dt)
+    got, *_ = _run(w, nb)
+    ref = chk.mtp_efv(util.to64(w["model"]), dict(nb, brcs=nb["brcs"].astype(np.float64)))
+    own = ref if dt == np.float64 else chk.mtp_efv(w["model"], nb)
+    for a, r, o, name in zip(got, ref, own, ("energy", "force", "virial")):
+        assert util.relerr(a, r) < max(TOL[dt], 4 * util.relerr(o, r)), name
+
+
 def test_many_neighbours_and_ragged_batch(checkers):
     """> 32 neighbours per atom (two lane chunks), padded batch with an empty structure and ghosts."""
     chk = _chk(checkers)
