@@ -198,18 +198,23 @@ __device__ __forceinline__ int warp_max_int(int v)
     return v;
 }
 
-// How many lanes share the slots of an atom. A tile takes about (1 / parts + 1 / 6) of the time of one with a lane per atom
-// (staging and look-ups do not get shorter), and the blocks of the chip work through the tiles in rounds. Level 16, double
-// precision, whole recorded call with its copies, us with 1, 2, 4, 8 lanes per atom: 1,000 atoms 66, 59, 49, 49; 3,001 atoms 88, 70,
-// 64, 72; 5,000 atoms 100, 82, 89, 95; 9,323 atoms 122, 127, 127, 149; 13,824 atoms 147, 153, 166, 197; 20,000 atoms 222, 211, 231, 277.
+// How many lanes share the slots of an atom. A tile takes 1 / parts of the time that its slots take with a lane per atom, plus an overhead
+// (staging, look-ups and, in the forward kernel, the walk that all groups share do not get shorter), and the blocks of the chip work
+// through the tiles in rounds. Whole call, us, with 1 / 2 / 4 / 8 lanes per atom:
+//   level 16 fp64   3,000 atoms 73 / 63 / 56 / 64;  7,000 100 / 82 / 90;  13,824 121 / 128 / 143;  20,000 194 / 184;  30,000 264 / 259
+//   level 10 fp64   3,000 atoms 44 / 40 / 37 / 40;  7,000  56 / 50 / 55;  13,824  67 /  71 /  81;  20,000 109 / 107;  30,000 120 / 124
+//   level 16 fp32   3,000 atoms 58 / 50 / 46 / 53;  7,000  75 / 64 / 72;  13,824  88 /  96 / 108;  20,000 135 / 133;  30,000 185 / 193
+//   level  6 fp32   3,000 atoms 37 / 34 / 32 / 34;  7,000  47 / 43 / 46;  13,824  57 /  58 /  64;  20,000  93 /  92;  30,000  98 / 102
 // Decided by the host for one structure, on the device for a batch, of which the host knows only the padded size. `resident`
 // blocks of the kernel run at a time.
+template <typename T>
 __host__ __device__ __forceinline__ int atom_parts(int atoms, int resident)
 {
+    constexpr int OVERHEAD = sizeof(T) == 8 ? 4 : 6;      // of 24
     int best = 1, least = 0;
 #pragma unroll
     for (int parts = 1; parts <= 8; parts *= 2) {
-        const int tiles = (atoms + MTP_TILE / parts - 1) / (MTP_TILE / parts), time = (tiles + resident - 1) / resident * (24 / parts + 4);
+        const int tiles = (atoms + MTP_TILE / parts - 1) / (MTP_TILE / parts), time = (tiles + resident - 1) / resident * (24 / parts + OVERHEAD);
         if (parts == 1 || time < least) { least = time; best = parts; }
     }
     return best;
@@ -242,7 +247,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_ke
         if (A.virial && i0 < 9 * (size_t)A.B) A.virial[i0] = T(0);
     }
     const int ntot = total_atoms(A);
-    if (parts == 0) parts = atom_parts(ntot, resident);
+    if (parts == 0) parts = atom_parts<T>(ntot, resident);
     const int ta = 32 / parts, a = lane & (ta - 1), part = lane / ta;      // atoms of the tile; this lane's atom and share of its slots
     const int ntiles = (ntot + ta - 1) / ta;
 
@@ -390,7 +395,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32, 3) mtp_force_atoms_kernel(const
     stage_coefficients<T, SIG, CSP>(A, cf);   // model constants: staged while the contraction drains
     chain_wait();
     const int ntot = total_atoms(A);
-    if (parts == 0) parts = atom_parts(ntot, resident);
+    if (parts == 0) parts = atom_parts<T>(ntot, resident);
     const int ta = 32 / parts, a = lane & (ta - 1), part = lane / ta;      // as in the forward kernel
     const int ntiles = (ntot + ta - 1) / ta;
     const bool single = A.B == 1;      // one structure: a tile's rows are known from its index alone
@@ -776,7 +781,7 @@ static int launch_fwd_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, const L
     int per_sm = 1;
     if (int rc = kernel_setup(setup, kern, smem, AT_WARPS * 32, &per_sm)) return rc;
     const int resident = sm_count() * per_sm;
-    const int parts = A.B == 1 ? atom_parts(A.npad, resident) : 0;
+    const int parts = A.B == 1 ? atom_parts<T>(A.npad, resident) : 0;
     const long tiles = ((long)A.B * A.npad * (parts ? parts : 8) + 31) / 32;
     AI2B_CUDA(launch_chained(kern, (unsigned)(tiles < resident ? tiles : resident), AT_WARPS * 32, smem, st, P, A, L, parts, resident));
     return AI2B_OK;
@@ -792,7 +797,7 @@ static int launch_force_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, cudaS
     int per_sm = 1;
     if (int rc = kernel_setup(setup, kern, smem, AT_WARPS * 32, &per_sm)) return rc;
     const int resident = sm_count() * per_sm;
-    const int parts = A.B == 1 ? atom_parts(A.npad, resident) : 0;
+    const int parts = A.B == 1 ? atom_parts<T>(A.npad, resident) : 0;
     const long tiles = ((long)A.B * A.npad * (parts ? parts : 8) + 31) / 32;
     AI2B_CUDA(launch_chained(kern, (unsigned)(tiles < resident ? tiles : resident), AT_WARPS * 32, smem, st, P, A, parts, resident));
     return AI2B_OK;
