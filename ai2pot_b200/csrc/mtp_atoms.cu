@@ -381,7 +381,10 @@ __global__ void __launch_bounds__(AT_WARPS * 32, DERIV ? 2 : 3) mtp_fwd_atoms_ke
 
 // ---- force and virial -----------------------------------------------------------------------------
 // shared memory: radial coefficients, adjoints [NDENSE][32]
-template <typename T, int MODE, typename SIG, int CSP>
+// FULL: a lane per atom, known when the kernel is compiled. In single precision the kernel of level 16 takes longer where the share of the slots is
+// a variable (13,824 atoms 23.6 us, with FULL 21.7; 100,000 atoms 138, 122). Shorter polynomials gain less or lose (whole call, 100,000 atoms,
+// level 10 253, 251; level 6 234, 241). In double precision both take the same (35.4, 35.1 us).
+template <typename T, int MODE, typename SIG, int CSP, bool FULL>
 __global__ void __launch_bounds__(AT_WARPS * 32, 3) mtp_force_atoms_kernel(const MtpProgramDev P, const MtpArgs<T> A, int parts, int resident)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -395,7 +398,8 @@ __global__ void __launch_bounds__(AT_WARPS * 32, 3) mtp_force_atoms_kernel(const
     stage_coefficients<T, SIG, CSP>(A, cf);   // model constants: staged while the contraction drains
     chain_wait();
     const int ntot = total_atoms(A);
-    if (parts == 0) parts = atom_parts<T>(ntot, resident);
+    if (FULL) parts = 1;
+    else if (parts == 0) parts = atom_parts<T>(ntot, resident);
     const int ta = 32 / parts, a = lane & (ta - 1), part = lane / ta;      // as in the forward kernel
     const int ntiles = (ntot + ta - 1) / ta;
     const bool single = A.B == 1;      // one structure: a tile's rows are known from its index alone
@@ -792,14 +796,23 @@ static int launch_force_atoms(const MtpProgramDev &P, const MtpArgs<T> &A, cudaS
 {
     const size_t ncf = (size_t)cf_elems<SIG, AT_CSP>(A.ntypes);
     const size_t smem = sizeof(T) * (ncf + (size_t)SIG::NDENSE * 32) + tile_rows_bytes<T>();
-    auto kern = mtp_force_atoms_kernel<T, MODE, SIG, AT_CSP>;
+    auto kern = mtp_force_atoms_kernel<T, MODE, SIG, AT_CSP, false>;
     static KernelSetup setup;
     int per_sm = 1;
     if (int rc = kernel_setup(setup, kern, smem, AT_WARPS * 32, &per_sm)) return rc;
     const int resident = sm_count() * per_sm;
     const int parts = A.B == 1 ? atom_parts<T>(A.npad, resident) : 0;
     const long tiles = ((long)A.B * A.npad * (parts ? parts : 8) + 31) / 32;
-    AI2B_CUDA(launch_chained(kern, (unsigned)(tiles < resident ? tiles : resident), AT_WARPS * 32, smem, st, P, A, parts, resident));
+    const unsigned blocks = (unsigned)(tiles < resident ? tiles : resident);
+    if constexpr (sizeof(T) == 4 && SIG::KD > 4)
+        if (parts == 1) {
+            auto full = mtp_force_atoms_kernel<T, MODE, SIG, AT_CSP, true>;
+            static KernelSetup full_setup;
+            if (int rc = kernel_setup(full_setup, full, smem)) return rc;
+            AI2B_CUDA(launch_chained(full, blocks, AT_WARPS * 32, smem, st, P, A, parts, resident));
+            return AI2B_OK;
+        }
+    AI2B_CUDA(launch_chained(kern, blocks, AT_WARPS * 32, smem, st, P, A, parts, resident));
     return AI2B_OK;
 }
 

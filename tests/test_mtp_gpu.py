@@ -96,6 +96,25 @@ def test_lanes_share_the_slots_of_an_atom(checkers, natoms, level, dt):
         assert util.relerr(a, r) < TOL[dt], name
 
 
+@pytest.mark.parametrize("natoms", [7201, 14211])
+def test_a_lane_per_atom_in_single_precision(checkers, natoms):
+    """Level 16, fp32: the force kernel of full tiles (first size), and the one of shared slots right beyond a round of full tiles; with and without
+    virial. Against the model in double precision; four times the distance of the CPU code's own single-precision result."""
+    rng = np.random.default_rng(natoms)
+    cell, pos = synth.cubic_lattice(int(np.ceil(natoms ** (1 / 3) - 1e-9)), 3.0, 0.1, rng, np.float64, nocc=natoms)
+    w = util.small_mtp_case(16, 2, np.float32)
+    w.update(cell=cell, coords=pos.astype(np.float32).astype(np.float64), types=rng.integers(0, 3, natoms).astype(np.int32))
+    chk = _chk(checkers)
+    nb = util.nblist_batch(chk, w)
+    nb["brcs"] = nb["brcs"].astype(np.float32)
+    (e, f, v), prog, md, nbd = _run(w, nb)
+    e2, f2 = capi.mtp_efv(prog, md, nbd, virial=False)
+    ref = chk.mtp_efv(util.to64(w["model"]), dict(nb, brcs=nb["brcs"].astype(np.float64)))
+    tol = [max(TOL[np.float32], 4 * util.relerr(o, r)) for o, r in zip(chk.mtp_efv(w["model"], nb), ref)]
+    for a, k, name in ((e, 0, "energy"), (f, 1, "force"), (v, 2, "virial"), (e2.cpu().numpy(), 0, "energy"), (f2.cpu().numpy(), 1, "force")):
+        assert util.relerr(a, ref[k]) < tol[k], name
+
+
 @pytest.mark.parametrize("natoms", [27, 2400])
 def test_tables_that_fit_tiles_of_32_atoms_only(checkers, natoms):
     """Sixteen moments in a chain, each the sum of 300 products: the rows of a tile of 16 atoms (four groups of lanes per warp, of
