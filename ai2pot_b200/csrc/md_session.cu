@@ -14,8 +14,8 @@
 // A step's host work: one pass over the positions that copies them into pinned memory and finds their extent (so the
 // bin grid is known on the host and the build needs no look at the atoms first), sent off in pieces that travel while the
 // next piece is copied; one transfer back of [forces | energy, virial | status]; one pass that adds the forces. 13,824 local
-// and 11,415 ghost atoms, NEP: 164 us per step, where pageable transfers array by array, a device pass over the extents and a scalar
-// loop over the forces took 355 us.
+// and 11,415 ghost atoms, NEP: 159 to 178 us per step, by the host, where pageable transfers array by array, a device pass over the extents
+// and a scalar loop over the forces took 355 us.
 #include "nep_setup.cuh"
 
 #include <cstring>
@@ -32,8 +32,8 @@ int nblist_build_rows32(int n, int ncentres, const double *h_cell, const double 
 
 // Positions travel in pieces of this many atoms, MD_SLOTS of which have a place in pinned memory. Pinning costs 0.9 to 2.9 ms per
 // 2 MB, of which blocks of less than 1 MB are cut: the ring has a fixed size and is made with the session, and what a
-// step brings back comes from the same 2 MB for up to 80,000 atoms. A step of 25,239 atoms takes 188 us with three slots, 187
-// with pinned memory for all of it (medians, in turn).
+// step brings back comes from the same 2 MB for up to 80,000 atoms. A step of 25,239 atoms takes as long with three slots as with pinned
+// memory for all of it (188 and 187 us when the stores still went through the caches; medians, in turn).
 constexpr size_t MD_PIECE = 6144;
 constexpr int MD_SLOTS = 3;
 constexpr size_t MD_RING_BYTES = sizeof(double) * 3 * MD_PIECE * MD_SLOTS;

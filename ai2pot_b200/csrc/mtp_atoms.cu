@@ -15,8 +15,8 @@
 //    z, y and x exponents (two FMAs per coefficient instead of four).
 // A tile has 32 atoms, or 16, 8 or 4: with few atoms the lanes of a warp share the neighbour slots of an atom (2, 4 or 8 lanes per
 // atom, sums added up by shuffles), so that the chip is filled and the serial loop over the slots gets shorter (atom_parts).
-// The basic moments and their adjoints travel between the kernels as [tile][basic row][32 atoms], which
-// all three kernels read and write in full 256-byte rows.
+// The basic moments and their adjoints travel between the kernels as [tile of 32 atoms][basic row][32 atoms]; a smaller tile
+// reads and writes its part of the rows (16 to 256 bytes).
 // The kernels are compiled per "signature" = the highest monomial degree of every radial function
 // (non-increasing, at most four functions); other tables take the warp-per-atom kernels.
 #include <cuda_pipeline.h>

@@ -431,8 +431,9 @@ __global__ void __launch_bounds__(MTP_CWARPS * 32, 1) mtp_contract_kernel(const 
 
 // ---- kernel B: products and adjoints out of shared memory (row loop: mtp_pairs.cuh) -----------------------
 // Tiles of TA = 32 or 16 atoms, blocks of W warps (32, one block per SM; 8 for small tables) walking over them; the next tile's rows
-// travel in registers while the current tile is processed. A moment is finished with a plain store by the group of lanes that owns it, so the result is the same bit for
-// bit from run to run. Shared memory: M[nm][TA], E[nm][TA] (not for descriptors), row records, adjoint seeds, small tables.
+// travel in registers while the current tile is processed. A moment is finished with a plain store by the group of lanes that owns it,
+// so the result is the same bit for bit from run to run. Level 16, fp64, 13,824 atoms, 44 us alone: the data stage of the load/store
+// unit is busy 57 % of the launch, warps wait for shared memory and at the barriers of the phases. Shared memory: M[nm][TA], E[nm][TA] (not for descriptors), row records, adjoint seeds, small tables.
 constexpr int MTP_PAIR_EWARPS = 8;   // warps that sum the site energies of a tile
 template <typename T> constexpr int pair_gl(int ta) { return ta * (int)sizeof(T) / 16; }      // lanes per row
 template <typename T> constexpr int pair_stream(int ta, int warps) { return (pair_gl<T>(ta) == 16 ? 0 : 1) + (warps == MTP_PAIR_FEW ? 2 : 0); }

@@ -1169,7 +1169,7 @@ static int nblist_build(int n, int ncentre, const T *h_cell, const T *d_coords, 
 //   2. lanes = atoms of the tile, single precision, |q_j|^2 - 2 q_i q_j < limit for two atoms at a time as in the rows kernel:
 //      triples that are certainly outside the cutoff are dropped, the others are queued in order
 //   3. lanes = queued triples: the exact predicate, in full warps
-// 64 structures of 64 to 256 atoms, 32 warps per SM: 32 us; with differences of coordinates, one atom per lane and step,
+// 64 structures of 64 to 256 atoms, 32 warps per SM: 32 us (64 registers, in double precision with 48 bytes of spills); with differences of coordinates, one atom per lane and step,
 // image numbers taken apart by divisions and 94 registers (two blocks per SM) 40 us and 2,000 warp instructions per centre; testing
 // every triple exactly 275 us.
 constexpr int NBB_WARPS = 8;

@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(NEP_WARPS * 32, MINB) nep_fast_kernel(const Ne
     }
     // descriptors and their adjoints are read as NDP-long vectors: the padding stays zero
     for (int i = lane; i < AW * 2 * NDP; i += 32) (q - grp * NDP)[i] = T(0);
-    chain_wait();        // the table and the offsets are the previous launch's
+    chain_wait();        // the table and the offsets come from an earlier launch of the chain (each of its kernels waits)
     for (int i = threadIdx.x; i < L.total * (int)sizeof(T) / 16; i += NEP_WARPS * 32)
         __pipeline_memcpy_async(reinterpret_cast<float4 *>(tab_s) + i, reinterpret_cast<const float4 *>(tab) + i, 16);
     __pipeline_commit();
